@@ -169,3 +169,66 @@ def test_coordinate_gradient_is_deterministic(torch):
         np.testing.assert_array_equal(gx, grads[0][0])
         np.testing.assert_array_equal(gy, grads[0][1])
     assert np.abs(grads[0][0]).max() > 0
+
+
+@pytest.mark.parametrize("shape_in,shape_out,angle,change", [
+    ((16, 16), (12, 12), 0.0, "none"),       # near-parallel edges
+    ((33, 17), (20, 31), 0.3, "none"),       # rotated, odd, cells of unequal sides
+    ((64, 64), (3, 2), 0.2, "none"),         # hundreds of entries per output cell
+    ((2, 3), (40, 33), 0.1, "none"),         # output cells inside single input cells
+    ((1, 1), (1, 1), 0.1, "none"),
+    ((24, 24), (18, 18), 0.2, "flip"),       # output grid of the other orientation
+    ((24, 24), (18, 18), 0.2, "weights"),    # signed and zero input weights
+    ((24, 24), (18, 18), 0.2, "dart"),       # an output cell that is not convex
+    ((16, 16), (12, 12), 0.0, "lines"),      # output columns on input columns
+    ((24, 24), (18, 18), 0.2, "offset"),     # coordinates far from zero
+])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_edge_gradient_matches_polygon_gradient(torch, shape_in, shape_out, angle, change, dtype):
+    """The edges' crossings against the clipped polygons (which run when the
+    recomputed weights are asked for).  A crossing parameter is off by a few
+    2^-53 of a coordinate over a cell side and the sine of the angle: with
+    sides of 1/64 and angles from 1e-4 up, under 1e-9."""
+    import regridding_gb300 as rg
+    from regridding_gb300 import _device, _lib
+
+    rng = np.random.default_rng(11)
+    a, b = (np.linspace(-1, 1, n + 1) for n in shape_in)
+    x, y = np.meshgrid(a, b, indexing="ij")
+    xi = x * np.cos(angle) - y * np.sin(angle)
+    yi = x * np.sin(angle) + y * np.cos(angle)
+    if change != "lines":
+        xi, yi = xi + 0.02 * np.sin(np.pi * yi), yi + 0.02 * np.sin(np.pi * xi)
+    xo, yo = np.meshgrid(*(np.linspace(-0.9, 0.9, n + 1) for n in shape_out), indexing="ij")
+    xo, yo = (c + rng.normal(0, 1e-4, c.shape) for c in (xo, yo))
+    w_in = None
+    if change == "flip":
+        xo, yo = xo[::-1].copy(), yo[::-1].copy()
+    elif change == "weights":
+        w_in = rng.normal(0, 1, shape_in)
+        w_in[::3] = 0
+    elif change == "dart":
+        xo[9, 9] += 0.08
+        yo[9, 9] += 0.08
+    elif change == "lines":
+        xo[:] = a[2:15, None]
+    elif change == "offset":
+        xi, yi, xo, yo = xi + 1000, yi - 3000, xo + 1000, yo - 3000
+    t = lambda v: torch.from_numpy(np.ascontiguousarray(v)).cuda()
+    gi, go = (t(xi), t(yi)), (t(xo), t(yo))
+    w = None if w_in is None else t(w_in)
+    dw = rg.build_conservative_2d(gi, go, w)
+    v = t(rng.normal(0, 1, (5, dw.n_in)).astype(dtype))
+    g = t(rng.normal(0, 1, (5, dw.n_out)).astype(dtype))
+    g[:, : dw.n_out // 7] = 0
+    got = []
+    for check in (None, torch.empty(dw.nnz, dtype=torch.float64, device="cuda")):
+        gx, gy = torch.empty_like(go[0]), torch.empty_like(go[1])
+        p = _device.ptr
+        _lib.call("rg_conservative_2d_grad_output", dw.handle, p(gi[0]), p(gi[1]), *gi[0].shape, p(go[0]), p(go[1]),
+                  *go[0].shape, p(w), p(v), p(g), _lib.RG_F32 if dtype == "float32" else _lib.RG_F64, 5, p(gx), p(gy),
+                  p(check), _device.stream())
+        got.append(torch.stack((gx, gy)).cpu().numpy())
+    assert np.abs(got[1]).max() > 0
+    tol = 1e-6 if change == "offset" else 1e-9  # 4000 times the coordinates
+    np.testing.assert_allclose(got[0], got[1], rtol=0, atol=tol * np.abs(got[1]).max())
