@@ -10,6 +10,7 @@
 // stack chunk, so the weights are read once per chunk instead of once per
 // array.
 #include "common.cuh"
+#include "patch.cuh"
 
 namespace rg {
 namespace {
@@ -38,6 +39,9 @@ __device__ __forceinline__ int64_t tile_row(const Tile& T, int64_t tile, int tid
 // MODE 1: exact double update rounded to float32 after every entry (numpy's
 //         in-place float32 output)
 // MODE 2: fast, accumulate in the output type with FMA
+// MODE 3: compensated (float32 input, float64 output): the float-float sums
+//         of the patch kernel, two slices at a time, for footprints too large
+//         for its boxes
 template <typename Tin, typename Tout, int MODE, typename Tw>
 __global__ void __launch_bounds__(APPLY_BLOCK)
     apply_kernel(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
@@ -56,6 +60,43 @@ __global__ void __launch_bounds__(APPLY_BLOCK)
         c[k] = k < nk ? col[s + k] : 0;
         w[k] = k < nk ? val[s + k] : (Tw)0;
     }
+    if constexpr (MODE == 3) {
+        float hi[CACHED], lo[CACHED];
+#pragma unroll
+        for (int k = 0; k < CACHED; k++) {
+            hi[k] = (float)w[k];
+            lo[k] = __double2float_rn(__dsub_rn(w[k], (double)hi[k]));
+        }
+        for (int64_t d = d0; d < d1; d += 2) {
+            const Tin* a = vin + d * n_in;
+            const Tin* b = d + 1 < d1 ? a + n_in : a;
+            uint64_t h2 = 0ull, l2 = 0ull;
+            auto step = [&](int32_t cell, float wh, float wl) {
+                ff_step2(h2, l2, f2_pack(wh, wh), f2_pack(-wh, -wh), f2_pack(wl, wl),
+                         f2_pack(ldg_cast(a + cell), ldg_cast(b + cell)));
+            };
+#pragma unroll
+            for (int k = 0; k < CACHED; k++)
+                if (k < nk) step(c[k], hi[k], lo[k]);
+            for (int64_t k = s + CACHED; k < e; k++) {
+                const float wh = (float)val[k];
+                step(col[k], wh, __double2float_rn(__dsub_rn(val[k], (double)wh)));
+            }
+            const float2 h = f2_unpack(h2), l = f2_unpack(l2);
+            auto store = [&](int64_t dd, const Tin* x, float hv, float lv) {
+                double r = 0.0;
+                if (finite_bits(hv) && finite_bits(lv)) {
+                    r = __dadd_rn(widen(hv), widen(lv));
+                } else {  // as the patch kernel: this output and slice in float64, stored order
+                    for (int64_t k = s; k < e; k++)
+                        r = __dadd_rn(r, __dmul_rn((double)val[k], (double)ldg_cast(x + col[k])));
+                }
+                vout[dd * n_out + o] = (Tout)r;
+            };
+            store(d, a, h.x, l.x);
+            if (d + 1 < d1) store(d + 1, b, h.y, l.y);
+        }
+    } else
     for (int64_t d = d0; d < d1; d++) {
         const Tin* a = vin + d * n_in;
         if (MODE == 0) {
@@ -132,7 +173,10 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
     RG_CHECK(acc == RG_ACC_EXACT || acc == RG_ACC_FAST || acc == RG_ACC_COMPENSATED, RG_ERR_ARG,
              "apply: bad accumulation mode");
     if (stack <= 0 || n_rows <= 0) return RG_OK;
-    if (acc != RG_ACC_FAST) {  // exact, or compensated where the staged kernel does not take the call
+    if (acc == RG_ACC_COMPENSATED && dtype_in == RG_F32 && dtype_out == RG_F64)
+        return launch<float, double, 3, double>(row_ptr, col, val, n_rows, shape0, shape1, vin, n_cols, vout, stack,
+                                                s);
+    if (acc != RG_ACC_FAST) {
         if (dtype_out == RG_F64) {
             if (dtype_in == RG_F32)
                 return launch<float, double, 0, double>(row_ptr, col, val, n_rows, shape0, shape1, vin, n_cols,
@@ -165,7 +209,9 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
 
 int tiled_lists_for(rg_weights_s* W, const float* vin, cudaStream_t s, int* g, bool* made);
 int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s);
-bool box_usable(const rg_weights_s* W, const float* vin, int64_t stack);
+bool box_usable(const rg_weights_s* W, int64_t stack);
+int box_load(const rg_weights_s* W, const float* vin, int64_t stack);
+int box_order_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_perm_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int ff_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
@@ -203,7 +249,7 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     // (the patch lists keep a float32 copy of the weights in gather order)
     const bool need32 = ((acc == RG_ACC_FAST && dtype_out == RG_F32) || exact_box || ff_box) && W->nnz > 0;
     int g = 0;
-    bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false;
+    bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false, ff_direct = false;
     {
         std::lock_guard<std::mutex> lock(W->mu);
         bool made = false;
@@ -218,33 +264,44 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
                 transposed ? W->t_val : W->val, *v32, W->nnz);
             made = true;
         }
-        if (tiled && box_usable(W, (const float*)vin, stack)) {
+        int load = -1;  // how the patch kernel fills its stages, -1: it does not take the call
+        if (((tiled && W->in_shape1 % 4 == 0) || exact_box || ff_box) && box_usable(W, stack)) {
             RG_TRY(box_lists_for(W, s, &made));
-            use_box = W->box_state == 1;
-            if (use_box && W->box_cfg[stack_class(stack)] == -1) {
+            load = box_load(W, (const float*)vin, stack);
+        }
+        // (rows that are no whole 16-byte chunks: the row residues' copies cost
+        // the fast mode more than its gathers; 1601^2 -> 1201^2, 32 slices 243 us
+        // against 189 us of the warp-staged kernel, where the compensated mode
+        // goes from 2200 us of FP64 gathers to 330 us)
+        if (tiled && load >= 0 && load != LOAD_RESIDUES) {
+            use_box = true;
+            RG_TRY(box_order_for(W, s, &made));
+            if (load == LOAD_SWIZZLED && W->box_cfg[stack_class(stack)] == -1) {
                 if (made) RG_CUDA(cudaStreamSynchronize(s));
                 made = false;
                 RG_TRY(tune_box_fast(W, (const float*)vin, (float*)vout, stack, s));
             }
-            use_box = use_box && W->box_cfg[stack_class(stack)] >= 0;
+            use_box = load != LOAD_SWIZZLED || W->box_cfg[stack_class(stack)] >= 0;
         }
-        if (exact_box && box_usable(W, (const float*)vin, stack)) {
-            RG_TRY(box_lists_for(W, s, &made));
-            use_box_exact = W->box_state == 1;
-            if (use_box_exact) RG_TRY(box_perm_for(W, s, &made));
+        if (exact_box && load >= 0) {
+            use_box_exact = true;
+            RG_TRY(box_perm_for(W, s, &made));
         }
-        if (ff_box && box_usable(W, (const float*)vin, stack)) {
-            RG_TRY(box_lists_for(W, s, &made));
-            use_box_ff = W->box_state == 1;
-            if (use_box_ff) RG_TRY(ff_lists_for(W, s, &made));
-            if (use_box_ff && W->box_cfg_ff[stack_class(stack)] == -1) {
+        // footprints too large for any box; handles without shapes and stacks
+        // off a 16-byte boundary of the swizzled box compute as exact
+        ff_direct = ff_box && W->box_state == -1;
+        if (ff_box && load >= 0) {
+            use_box_ff = true;
+            RG_TRY(ff_lists_for(W, s, &made));
+            if (load == LOAD_SWIZZLED && W->box_cfg_ff[stack_class(stack)] == -1) {
                 if (made) RG_CUDA(cudaStreamSynchronize(s));
                 made = false;
                 RG_TRY(tune_box_ff(W, (const float*)vin, (double*)vout, stack, s));
             }
-            use_box_ff = use_box_ff && W->box_cfg_ff[stack_class(stack)] >= 0;
+            use_box_ff = load != LOAD_SWIZZLED || W->box_cfg_ff[stack_class(stack)] >= 0;
         }
-        if (tiled && !use_box) RG_TRY(rows_usable(W, (const float*)vin, stack, s, &made, &use_rows));
+        if (tiled && !use_box)
+            RG_TRY(rows_usable(W, (const float*)vin, stack, s, &made, &use_rows));
         if (tiled && !use_box && !use_rows) RG_TRY(tiled_lists_for(W, (const float*)vin, s, &g, &made));
         if (made) RG_CUDA(cudaStreamSynchronize(s));
     }
@@ -270,9 +327,11 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     if (tiled) return apply_tiled(W, g, (const float*)vin, (float*)vout, stack, s);
     if (!transposed)
         return apply_csr(W->row_ptr, W->col, W->val, W->val32, W->nnz, W->n_out, W->n_in, W->out_shape0,
-                         W->out_shape1, vin, dtype_in, vout, dtype_out, stack, acc, s);
+                         W->out_shape1, vin, dtype_in, vout, dtype_out, stack,
+                         acc == RG_ACC_COMPENSATED && !ff_direct ? RG_ACC_EXACT : acc, s);
+    // (a compensated call is defined for the matrix itself; its transpose computes as exact)
     return apply_csr(W->t_row_ptr, W->t_col, W->t_val, W->t_val32, W->nnz, W->n_in, W->n_out, 0, 0, vin,
-                     dtype_in, vout, dtype_out, stack, acc, s);
+                     dtype_in, vout, dtype_out, stack, acc == RG_ACC_COMPENSATED ? RG_ACC_EXACT : acc, s);
 }
 
 }  // namespace rg

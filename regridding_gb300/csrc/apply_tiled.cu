@@ -28,6 +28,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "patch.cuh"
 
 namespace rg {
 namespace {
@@ -35,9 +36,6 @@ namespace {
 constexpr int WARPS = 8;        // warp tiles per block
 constexpr int TR = 4, TC = 8;   // warp tile: TR output rows x TC output columns
 constexpr int PREP_MAX = 1024;  // entries of one warp tile sorted in shared memory (4 KB per warp)
-constexpr int CACHED_T = 8;     // row entries kept in registers across slices
-constexpr int FF_EXTRA = 3;     // compensated mode: further row entries kept in shared memory
-constexpr int ROW_EXTRA = 2;    // fast and exact modes: further row entries kept in shared memory
 constexpr int SLICES = 4;       // stack slices staged per step
 
 struct TileShape {
@@ -167,18 +165,6 @@ __global__ void max_i64(const int64_t* a, int64_t n, unsigned long long* out) {
         atomicMax(out, (unsigned long long)a[k]);
 }
 
-// Direct gathers for one lane's row (tiles whose list does not fit).
-__device__ __forceinline__ void apply_direct(const int64_t s, const int64_t e, const int32_t* __restrict__ col,
-                                             const float* __restrict__ val, const float* __restrict__ vin,
-                                             int64_t n_in, float* out, int64_t n_out, int64_t d0, int64_t d1) {
-    for (int64_t d = d0; d < d1; d++) {
-        const float* a = vin + d * n_in;
-        float acc = 0.f;
-        for (int64_t k = s; k < e; k++) acc = fmaf(val[k], __ldg(a + col[k]), acc);
-        out[d * n_out] = acc;
-    }
-}
-
 // Vector variant: the list holds 32-byte sectors (8 cells, at most 32 per
 // tile; longer lists take the scalar kernel).  A sector is fetched as two
 // 16-byte halves, one per lane ("half h" = sector h / 2, half h % 2), so the
@@ -289,162 +275,66 @@ __global__ void __launch_bounds__(32 * WARPS)
     }
 }
 
-// ---------------------------------------------------------------------------
-// TMA variant.  A block of 8 warps owns a 16 x 16 patch of output cells
-// (4 x 2 warp tiles of 4 x 8).  The input footprint of every patch lies in a
-// box of box_rows x 32 input cells (the same box size for all patches, the
-// origin per patch, its column a multiple of 4 so that a copy starts on a
-// 16-byte boundary).  A ring of NST stages, each holding SPS slices of the
-// patch's box, is filled by one 3D tensor copy per stage (columns x rows x
-// slices) issued by thread 0 and completed by the stage's "full" mbarrier
-// transaction count; every warp arrives on the stage's "empty" mbarrier when
-// it has read the stage, and thread 0 waits for all 8 before refilling it.
-// The copies run on the TMA unit, so the load/store pipe only carries the
-// gathers of the reduction (one 32-bit shared load per entry and slice).
-// Box rows are 128 bytes and written with the 128-byte swizzle (16-byte
-// chunk c of row r lands at chunk c ^ (r & 7) of that row), which spreads
-// the gathers of vertically neighbouring cells over different banks; the
-// entries' slots carry the swizzle.  Waits are bounded: a copy that does not
-// land sets FLAG_TIMEOUT and the block leaves after a bounded drain.
-// ---------------------------------------------------------------------------
-
-constexpr int PATCH = 16;      // output cells per patch side
-constexpr int PATCH_WARPS = 8; // 4 x 2 warp tiles of 4 x 8
-constexpr int PBOX_C = 32;     // box columns: one 128-byte swizzle span
-constexpr int PBOX_MAX_R = 32; // box rows at most
-constexpr int PLANE = PBOX_MAX_R * PBOX_C;  // floats of one slice's plane in a stage (4 KB)
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-// try_wait with a suspend-time hint (ns): the thread sleeps instead of spinning
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait: gives up after 2^16 polls (each suspends at most ~20 us)
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity) {
-    for (int it = 0; it < (1 << 16); it++)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-__device__ __forceinline__ void tma_load_3d(float* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];\n" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-
-struct PatchGrid {
-    int64_t n0, n1;     // output cells
-    int64_t patches1;   // patches along axis 1
-};
-
-__device__ __forceinline__ int64_t patch_cell(const PatchGrid& P, int64_t p, int r, int c) {
-    const int64_t pi = p / P.patches1, pj = p - pi * P.patches1;
-    const int64_t i = pi * PATCH + r, j = pj * PATCH + c;
-    return (i < P.n0 && j < P.n1) ? i * P.n1 + j : -1;
-}
-
-// One block of 256 threads per patch, a thread per output cell.  PASS 0:
-// footprint (origin, extent) of every patch; PASS 1: patches that fit the
-// box get their entries' swizzled slots, the others are marked for direct
-// gathers (origin row -2).
-template <int PASS>
-__global__ void __launch_bounds__(256)
-    prepare_patch(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col, PatchGrid P, FastDiv nd,
-                  int2* __restrict__ origin, int2* __restrict__ extent, unsigned* __restrict__ stats, int BR,
-                  uint16_t* __restrict__ slot) {
-    __shared__ int red[4][8];
+// The input footprint of every patch, one block of 256 threads each, a thread
+// per output cell: its first row and column (a multiple of 4, where a tensor
+// copy can start) and its extent, (-1, -1) and 0 without entries.  stats: the
+// most rows and columns, and the patches larger than 32 x 32.
+__global__ void __launch_bounds__(32 * PATCH_WARPS)
+    patch_footprints(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col, PatchGrid P, FastDiv nd,
+                     int2* __restrict__ origin, int2* __restrict__ extent, unsigned* __restrict__ stats) {
+    __shared__ int red[4][PATCH_WARPS];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int64_t p = blockIdx.x;
-    const int64_t o = patch_cell(P, p, t / PATCH, t % PATCH);
+    const int64_t o = patch_cell(P, p, t >> P.cb, t & ((1 << P.cb) - 1));
     int64_t s = 0, e = 0;
     if (o >= 0) {
         s = row_ptr[o];
         e = row_ptr[o + 1];
     }
-    if (PASS == 0) {
-        int rmin = INT_MAX, rmax = -1, cmin = INT_MAX, cmax = -1;
-        for (int64_t k = s; k < e; k++) {
-            const int c = col[k];
-            const int r = (int)nd.div((uint32_t)c), cc = c - r * (int)nd.d;
-            rmin = min(rmin, r);
-            rmax = max(rmax, r);
-            cmin = min(cmin, cc);
-            cmax = max(cmax, cc);
-        }
-        rmin = __reduce_min_sync(0xffffffffu, rmin);
-        cmin = __reduce_min_sync(0xffffffffu, cmin);
-        rmax = __reduce_max_sync(0xffffffffu, rmax);
-        cmax = __reduce_max_sync(0xffffffffu, cmax);
-        if (lane == 0) {
-            red[0][warp] = rmin;
-            red[1][warp] = cmin;
-            red[2][warp] = rmax;
-            red[3][warp] = cmax;
-        }
-        __syncthreads();
-        if (t == 0) {
-            for (int w = 1; w < 8; w++) {
-                rmin = min(rmin, red[0][w]);
-                cmin = min(cmin, red[1][w]);
-                rmax = max(rmax, red[2][w]);
-                cmax = max(cmax, red[3][w]);
-            }
-            if (rmax < 0) {
-                origin[p] = make_int2(-1, -1);
-                extent[p] = make_int2(0, 0);
-            } else {
-                const int c0 = cmin & ~3;
-                origin[p] = make_int2(rmin, c0);
-                extent[p] = make_int2(rmax - rmin + 1, cmax - c0 + 1);
-                atomicMax(&stats[0], (unsigned)(rmax - rmin + 1));
-                atomicMax(&stats[1], (unsigned)(cmax - c0 + 1));
-            }
-        }
-        return;
-    }
-    const int2 org = origin[p];
-    const int2 ext = extent[p];
-    if (org.x < 0) return;
-    if (ext.x > BR || ext.y > PBOX_C) {
-        __syncthreads();  // every thread has read origin before it changes
-        if (t == 0) {
-            origin[p] = make_int2(-2, -2);
-            atomicAdd(&stats[2], 1u);
-        }
-        return;
-    }
+    int rmin = INT_MAX, rmax = -1, cmin = INT_MAX, cmax = -1;
     for (int64_t k = s; k < e; k++) {
         const int c = col[k];
-        const int row = (int)nd.div((uint32_t)c);
-        const int r = row - org.x, cc = c - row * (int)nd.d - org.y;
-        slot[k] = (uint16_t)(r * PBOX_C + ((((cc >> 2) ^ (r & 7)) << 2) | (cc & 3)));
+        const int r = (int)nd.div((uint32_t)c), cc = c - r * (int)nd.d;
+        rmin = min(rmin, r);
+        rmax = max(rmax, r);
+        cmin = min(cmin, cc);
+        cmax = max(cmax, cc);
     }
+    rmin = __reduce_min_sync(0xffffffffu, rmin);
+    cmin = __reduce_min_sync(0xffffffffu, cmin);
+    rmax = __reduce_max_sync(0xffffffffu, rmax);
+    cmax = __reduce_max_sync(0xffffffffu, cmax);
+    if (lane == 0) {
+        red[0][warp] = rmin;
+        red[1][warp] = cmin;
+        red[2][warp] = rmax;
+        red[3][warp] = cmax;
+    }
+    __syncthreads();
+    if (t != 0) return;
+    for (int w = 1; w < PATCH_WARPS; w++) {
+        rmin = min(rmin, red[0][w]);
+        cmin = min(cmin, red[1][w]);
+        rmax = max(rmax, red[2][w]);
+        cmax = max(cmax, red[3][w]);
+    }
+    if (rmax < 0) {
+        origin[p] = make_int2(-1, -1);
+        extent[p] = make_int2(0, 0);
+        return;
+    }
+    const int c0 = cmin & ~3, rows = rmax - rmin + 1, cols = cmax - c0 + 1;
+    origin[p] = make_int2(rmin, c0);
+    extent[p] = make_int2(rows, cols);
+    atomicMax(&stats[0], (unsigned)rows);
+    atomicMax(&stats[1], (unsigned)cols);
+    if (rows > PBOX_MAX_R || cols > PBOX_C) atomicAdd(&stats[2], 1u);
 }
 
-// Box slot of input cell c (the slot prepare_patch gives it).
-__device__ __forceinline__ int box_slot_of(int c, int2 org, FastDiv nd) {
-    const int row = (int)nd.div((uint32_t)c);
-    const int r = row - org.x, cc = c - row * (int)nd.d - org.y;
-    return r * PBOX_C + ((((cc >> 2) ^ (r & 7)) << 2) | (cc & 3));
+// Marks the patches larger than 32 x 32 for direct gathers (origin row -2).
+__global__ void mark_large_patches(int64_t n, const int2* __restrict__ extent, int2* __restrict__ origin) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
+        if (extent[p].x > PBOX_MAX_R || extent[p].y > PBOX_C) origin[p] = make_int2(-2, -2);
 }
 
 // The part of a float64 weight that its float32 rounding hi = (float)w
@@ -473,9 +363,9 @@ __device__ __forceinline__ float weight_rest(double w, float hi) {
 // 2.15 (stored order) -> 1.56 (greedy) -> 1.28 (with the augmentation) for
 // the warp tiles and 2.68 -> 2.11 -> 1.65 for the row-length layout.)  A
 // lane's turn is taken by the whole warp: lane c tests the lane's candidate
-// c, ballots give the pick, and the step's picks are written at its end.  The entries' natural slots come from
-// slot_in, or from their columns when it is null; writes the reordered
-// slots, float32 weights and (lo_out non-null) the weights' float32 rests.
+// c, ballots give the pick, and the step's picks are written at its end.
+// Writes the reordered slots, float32 weights and (lo_out non-null) the
+// weights' float32 rests.
 // The CSR itself, which fixes the exact paths' order, is unchanged.  Lanes
 // with more than ORDER_MAX entries keep the stored order.
 constexpr int ORDER_MAX = 16;
@@ -483,8 +373,8 @@ constexpr int ORDER_MAX = 16;
 __global__ void __launch_bounds__(32 * PATCH_WARPS)
     order_patch(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col, FastDiv nd,
                 const float* __restrict__ val32, const double* __restrict__ val, PatchGrid P,
-                const int2* __restrict__ origin, const uint8_t* __restrict__ perm, const uint16_t* slot_in,
-                uint16_t* slot_out, float* __restrict__ hi_out, float* __restrict__ lo_out) {
+                const int2* __restrict__ origin, BoxShape box, const uint8_t* __restrict__ perm,
+                uint16_t* __restrict__ slot_out, float* __restrict__ hi_out, float* __restrict__ lo_out) {
     __shared__ uint16_t cand[PATCH_WARPS][32][ORDER_MAX];  // every lane's natural slots
     __shared__ uint16_t owner[PATCH_WARPS][32];            // the word each bank serves at this step
     __shared__ int8_t owner_lane[PATCH_WARPS][32];          // the lane that holds the bank (first to take it)
@@ -493,11 +383,12 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS)
     __shared__ unsigned left_of[PATCH_WARPS][32];           // every lane's entries not yet placed
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int64_t p = blockIdx.x;
-    int pr = 4 * (warp >> 1) + (lane >> 3), pc = 8 * (warp & 1) + (lane & 7);
+    int pr, pc;
+    tile_cell(P, t, &pr, &pc);
     if (perm) {
-        const int raw = perm[p * (PATCH * PATCH) + t];
-        pr = raw / PATCH;
-        pc = raw % PATCH;
+        const int raw = perm[p * (32 * PATCH_WARPS) + t];
+        pr = raw >> P.cb;
+        pc = raw & ((1 << P.cb) - 1);
     }
     const int64_t o = patch_cell(P, p, pr, pc);
     int64_t s = 0, e = 0;
@@ -509,7 +400,9 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS)
     const int2 org = origin[p];
     if (org.x < 0) return;  // block-uniform
     auto natural = [&](int64_t k) -> uint16_t {
-        return slot_in ? slot_in[k] : (uint16_t)box_slot_of(col[k], org, nd);
+        return (uint16_t)(box.residues ? box_slot_of<LOAD_RESIDUES>(col[k], org, nd, box)
+                          : box.pitch  ? box_slot_of<LOAD_WIDE>(col[k], org, nd, box)
+                                       : box_slot_of<LOAD_SWIZZLED>(col[k], org, nd, box));
     };
     if (nk > ORDER_MAX) {
         for (int64_t k = s; k < e; k++) {
@@ -623,17 +516,17 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS)
 // keeps more of a warp's cells near each other, so that more lanes share
 // input words, for a little more divergence); ties by cell.  A bitonic sort
 // of 256 keys in shared memory; one block per patch.
-__global__ void __launch_bounds__(PATCH * PATCH)
+__global__ void __launch_bounds__(32 * PATCH_WARPS)
     perm_patch(const int64_t* __restrict__ row_ptr, PatchGrid P, int group, uint8_t* __restrict__ perm) {
-    __shared__ unsigned key[PATCH * PATCH];
+    __shared__ unsigned key[32 * PATCH_WARPS];
     const int t = threadIdx.x;
     const int64_t p = blockIdx.x;
-    const int64_t o = patch_cell(P, p, t / PATCH, t % PATCH);
+    const int64_t o = patch_cell(P, p, t >> P.cb, t & ((1 << P.cb) - 1));
     int64_t nk = o >= 0 ? row_ptr[o + 1] - row_ptr[o] : 0;
     if (nk > 255) nk = 255;
     key[t] = ((unsigned)((255 - nk) / group) << 8) | (unsigned)t;
     __syncthreads();
-    for (int k = 2; k <= PATCH * PATCH; k <<= 1) {
+    for (int k = 2; k <= 32 * PATCH_WARPS; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
             const int ixj = t ^ j;
             if (ixj > t) {
@@ -647,459 +540,7 @@ __global__ void __launch_bounds__(PATCH * PATCH)
             __syncthreads();
         }
     }
-    perm[p * (PATCH * PATCH) + t] = (uint8_t)(key[t] & 255u);
-}
-
-// Whether a float32 is finite, from its exponent bits.
-__device__ __forceinline__ bool finite_bits(float f) {
-    return (__float_as_uint(f) & 0x7f800000u) != 0x7f800000u;
-}
-
-// Whether a float32 is normal (neither zero, subnormal, infinite nor NaN).
-__device__ __forceinline__ bool normal_bits(unsigned u) {
-    return (u & 0x7f800000u) - 0x00800000u < 0x7f000000u;
-}
-
-// widen() of a normal float32, from its bits: the double's high word is the
-// sign, the exponent rebiased by 1023 - 127 and the top 20 fraction bits;
-// the low word the last 3 fraction bits.
-__device__ __forceinline__ double widen_normal(unsigned u) {
-    const unsigned hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20));
-    return __hiloint2double((int)hi, (int)(u << 29));
-}
-
-// Accumulation modes of the TMA apply.
-//  MODE_FAST:  float32 output, acc = fmaf(w, x, acc) with float32 weights in
-//              the bank-aware gather order.
-//  MODE_EXACT: the upstream float64 apply bit for bit (float32 input, float64
-//              weights and output): every entry in stored (CSR) order as
-//              acc = acc + w * (double)x with one rounding per operation, from 0.0.
-//  MODE_FF:    float64 output from float-float arithmetic on the FP32 pipe
-//              (the GB300 runs FP32 at 64x its FP64 rate): each weight as
-//              hi + lo floats, each product x * hi split exactly into p + e
-//              by an FMA (Dekker's product), the running sum kept as an
-//              unevaluated pair (h, l) with Knuth's two-sum, and h + l added
-//              in double once per output.  Entries in the gather order.
-constexpr int MODE_FAST = 0, MODE_EXACT = 1, MODE_FF = 2;
-
-// Packed pairs of float32 (two slices of one output): the sm_100-family
-// f32x2 instructions apply one IEEE operation, rounded to nearest, to both
-// halves, at the issue cost of one scalar instruction.
-__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-// One float-float step on a pair of slices: (h, l) += x * (wh + wl), with
-// the weight given as the pairs wh, -wh and wl.  Per half the operations
-// and their results are those of the scalar step
-//     p = x wh;  e = fma(x, wh, -p);  r = fma(x, wl, e);
-//     t = h + p;  bp = t - h;  err = (h - (t - bp)) + (p - bp);
-//     h = t;  l = l + (err + r)
-// (Dekker's product, Knuth's two-sum), written with pn = x (-wh) = -p so
-// that no operand needs negating: fma(x, wh, pn) = x wh - p, h - pn = h + p,
-// and p - bp = -(pn + bp), subtracted from h - (t - bp).  (The only
-// difference is the sign of an exact zero p - bp, which cannot reach the
-// sum: h - (t - bp) is never -0, as h starts at +0.)
-__device__ __forceinline__ void ff_step2(uint64_t& h, uint64_t& l, uint64_t wh, uint64_t whn, uint64_t wl,
-                                         uint64_t x) {
-    const uint64_t pn = f2_mul(x, whn);
-    const uint64_t e = f2_fma(x, wh, pn);
-    const uint64_t r = f2_fma(x, wl, e);
-    const uint64_t t = f2_sub(h, pn);
-    const uint64_t bp = f2_sub(t, h);
-    const uint64_t err = f2_sub(f2_sub(h, f2_sub(t, bp)), f2_add(pn, bp));
-    h = t;
-    l = f2_add(l, f2_add(err, r));
-}
-
-template <int SPS, int NST, int MINB, int MODE, int CT = CACHED_T>
-__global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
-    apply_patch_tma(const __grid_constant__ CUtensorMap tmap, const int64_t* __restrict__ row_ptr,
-                    const int32_t* __restrict__ col, const uint16_t* __restrict__ slot,
-                    const float* __restrict__ bval, const float* __restrict__ blo, const float* __restrict__ val,
-                    const double* __restrict__ dval, double* __restrict__ vout64, FastDiv nd,
-                    PatchGrid P, int64_t n_patches, const int2* __restrict__ origin, int BR, int stage_floats,
-                    unsigned box_bytes, const float* __restrict__ vin, int64_t n_in, float* __restrict__ vout,
-                    int64_t n_out, int64_t stack, int64_t chunk, unsigned* __restrict__ flags,
-                    const uint8_t* __restrict__ perm) {
-    constexpr bool EXACT = MODE == MODE_EXACT;
-    constexpr bool OUT64 = MODE != MODE_FAST;
-    // The float64-output modes give every slice of a stage its own 4 KB plane
-    // (constant gather offsets; one box copy per slice) and let the last warp
-    // done with a stage refill it.  The float32 mode, whose gathers are few
-    // instructions, keeps one box copy per stage (slices packed BR rows
-    // apart) and a producer thread that waits for the warps; measured faster
-    // for it.
-    constexpr bool PLANES = MODE != MODE_FAST;
-    __shared__ __align__(8) uint64_t full[NST], empty[NST];
-    __shared__ unsigned done[NST];  // warps done with each stage, counted over all its uses
-    // entries CT .. CT + NX - 1 of every thread's row, read once per patch
-    // (rows one or two entries longer than the registers hold are common;
-    // reading those entries from global memory at every stage held back the
-    // warp with the longest rows, and with it the stage's refill): their
-    // slots, and their float32 weights (fast), float32 weight and rest
-    // (compensated) or float64 weights (exact)
-    constexpr int NX = CT > 0 ? (MODE == MODE_FF ? FF_EXTRA : ROW_EXTRA) : 1;
-    constexpr int NXF = MODE != MODE_EXACT ? NX : 1, NXL = MODE == MODE_FF ? NX : 1;
-    constexpr int NXD = MODE == MODE_EXACT ? NX : 1;
-    __shared__ uint16_t ex_slot[NX][32 * PATCH_WARPS];
-    __shared__ float ex_hi[NXF][32 * PATCH_WARPS], ex_lo[NXL][32 * PATCH_WARPS];
-    __shared__ double ex_d[NXD][32 * PATCH_WARPS];
-    extern __shared__ __align__(1024) float ring[];
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int64_t p = blockIdx.x;
-    // the thread's output: the warp tile layout, or for the exact and
-    // compensated applies the patch's outputs by row length (a warp's lanes
-    // then run chains of similar length)
-    const int64_t d0 = (int64_t)blockIdx.y * chunk;
-    const int64_t d1 = d0 + chunk < stack ? d0 + chunk : stack;
-    const int2 org = origin[p];
-    const int64_t ngroups = (d1 - d0 + SPS - 1) / SPS;
-    // PLANES: one box copy per slice of the group (slices past the chunk are
-    // not loaded); else one copy of box_bytes for the whole stage
-    auto issue = [&](int st, int64_t grp) {
-        const int64_t z0 = d0 + grp * SPS;
-        if constexpr (PLANES) {
-            const int n = (int)(d1 - z0 < SPS ? d1 - z0 : SPS);
-            mbar_expect_tx(&full[st], (unsigned)n * box_bytes);
-            for (int q = 0; q < n; q++)
-                tma_load_3d(ring + (int64_t)st * stage_floats + q * PLANE, &tmap, org.y, org.x, (int)(z0 + q),
-                            &full[st]);
-        } else {
-            mbar_expect_tx(&full[st], box_bytes);
-            tma_load_3d(ring + (int64_t)st * stage_floats, &tmap, org.y, org.x, (int)z0, &full[st]);
-        }
-    };
-    // the first stages' copies start before the threads fetch their rows, so
-    // that the copies and the row fetches overlap (the barriers are ready for
-    // the other threads after the __syncthreads below)
-    if (org.x >= 0 && t == 0) {
-        for (int k = 0; k < NST; k++) {
-            mbar_init(&full[k], 1);
-            mbar_init(&empty[k], PATCH_WARPS);
-            done[k] = 0u;
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        for (int k = 0; k < NST && k < ngroups; k++) issue(k, k);
-    }
-    int pr = 4 * (warp >> 1) + (lane >> 3), pc = 8 * (warp & 1) + (lane & 7);
-    if (OUT64 && perm) {
-        const int raw = perm[p * (PATCH * PATCH) + t];
-        pr = raw / PATCH;
-        pc = raw % PATCH;
-    }
-    const int64_t o = patch_cell(P, p, pr, pc);
-    int64_t s = 0, e = 0;
-    if (o >= 0) {
-        s = row_ptr[o];
-        e = row_ptr[o + 1];
-    }
-    const int nk = (int)(e - s);
-    float* out = vout + (o >= 0 ? o : 0);
-    if (org.x < 0) {
-        // no entries (all zeros) or a footprint larger than the box: the whole block
-        if (o >= 0) {
-            if constexpr (OUT64) {
-                for (int64_t d = d0; d < d1; d++) {
-                    const float* a = vin + d * n_in;
-                    double acc = 0.0;
-                    for (int64_t k = s; k < e; k++) acc = __dadd_rn(acc, __dmul_rn(dval[k], (double)__ldg(a + col[k])));
-                    vout64[d * n_out + o] = acc;
-                }
-            } else {
-                apply_direct(s, e, col, val, vin, n_in, out, n_out, d0, d1);
-            }
-        }
-        return;
-    }
-    // The compensated apply runs every lane of a warp to the warp's longest
-    // row (a uniform bound, no divergent branch per entry).  A lane's entries
-    // past its own row have zero weights and slot 0: such a step leaves the
-    // pair (h, l) unchanged for a finite input word; a non-finite one makes
-    // the sum NaN, which sends that output and slice to the exact loop.
-    const int kwarp = MODE == MODE_FF ? __reduce_max_sync(0xffffffffu, nk) : nk;
-    // PLANES: every slice of a stage has its own 4 KB plane, 1024-byte
-    // aligned, so all slices see the same swizzle phase and a gather's
-    // slices differ by constant offsets.  Otherwise the rows of slice q start
-    // at row q * BR of the swizzle pattern: with BR a multiple of 4, odd
-    // slices see the pattern shifted by 4 rows, which is the chunk index
-    // xor 4 (slot xor 16).
-    const int plane = PLANES ? PLANE : BR * PBOX_C;
-    const int flip = PLANES ? 0 : ((BR & 4) ? 16 : 0);
-    // (CT = 0 keeps a single dummy slot: every entry is read from memory)
-    int li[CT > 0 ? CT : 1];
-    float w[CT > 0 ? CT : 1];
-    double wd[CT > 0 ? CT : 1];
-    // the compensated mode's weights as packed pairs (wh, wh), (-wh, -wh), (wl, wl)
-    uint64_t fh[CT > 0 ? CT : 1], fhn[CT > 0 ? CT : 1], fl[CT > 0 ? CT : 1];
-#pragma unroll
-    for (int k = 0; k < CT; k++) {
-        if constexpr (EXACT) {
-            li[k] = k < nk ? box_slot_of(col[s + k], org, nd) : 0;
-            wd[k] = k < nk ? dval[s + k] : 0.0;
-            w[k] = 0.f;
-        } else if constexpr (MODE == MODE_FF) {
-            li[k] = k < nk ? (int)slot[s + k] : 0;
-            const float a = k < nk ? bval[s + k] : 0.f, b = k < nk ? blo[s + k] : 0.f;
-            fh[k] = f2_pack(a, a);
-            fhn[k] = f2_pack(-a, -a);
-            fl[k] = f2_pack(b, b);
-        } else {
-            li[k] = k < nk ? (int)slot[s + k] : 0;
-            w[k] = k < nk ? bval[s + k] : 0.f;
-            wd[k] = 0.0;
-        }
-    }
-    if constexpr (CT > 0) {
-#pragma unroll
-        for (int j = 0; j < NX; j++) {
-            const bool has = CT + j < nk;
-            if constexpr (EXACT) {
-                ex_slot[j][t] = has ? (uint16_t)box_slot_of(col[s + CT + j], org, nd) : (uint16_t)0;
-                ex_d[j][t] = has ? dval[s + CT + j] : 0.0;
-            } else {
-                ex_slot[j][t] = has ? slot[s + CT + j] : (uint16_t)0;
-                ex_hi[j][t] = has ? bval[s + CT + j] : 0.f;
-                if constexpr (MODE == MODE_FF) ex_lo[j][t] = has ? blo[s + CT + j] : 0.f;
-            }
-        }
-    }
-    __syncthreads();
-    for (int64_t grp = 0; grp < ngroups; grp++) {
-        const int st = (int)(grp % NST);
-        const unsigned ph = (unsigned)((grp / NST) & 1);
-        const bool got = mbar_wait_bounded(&full[st], ph);
-        if (!__all_sync(0xffffffffu, got)) {
-            if (lane == 0) {
-                atomicOr(flags, FLAG_TIMEOUT);
-                // copies of this block that may still be in flight: bounded wait before leaving
-                for (int64_t q = grp + 1; q < grp + NST && q < ngroups; q++)
-                    (void)mbar_wait_bounded(&full[q % NST], (unsigned)((q / NST) & 1));
-            }
-            return;
-        }
-        const float* buf = ring + (int64_t)st * stage_floats;
-        const int64_t ds = d0 + grp * SPS;
-        if constexpr (EXACT) {
-            if (o >= 0) {
-                double acc[SPS];
-#pragma unroll
-                for (int q = 0; q < SPS; q++) acc[q] = 0.0;
-#pragma unroll
-                for (int k = 0; k < CT; k++) {
-                    if (k < nk) {
-#pragma unroll
-                        for (int q = 0; q < SPS; q++)
-                            acc[q] = __dadd_rn(
-                                acc[q], __dmul_rn(wd[k], widen(buf[q * plane + (li[k] ^ ((q & 1) ? flip : 0))])));
-                    }
-                }
-                if constexpr (CT > 0) {
-#pragma unroll
-                    for (int j = 0; j < NX; j++) {
-                        if (CT + j < nk) {
-                            const double wk = ex_d[j][t];
-                            const int sk = ex_slot[j][t];
-#pragma unroll
-                            for (int q = 0; q < SPS; q++)
-                                acc[q] = __dadd_rn(acc[q],
-                                                   __dmul_rn(wk, widen(buf[q * plane + (sk ^ ((q & 1) ? flip : 0))])));
-                        }
-                    }
-                }
-                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < e; k++) {
-                    const double wk = dval[k];
-                    const int sk = box_slot_of(col[k], org, nd);
-#pragma unroll
-                    for (int q = 0; q < SPS; q++)
-                        acc[q] = __dadd_rn(acc[q], __dmul_rn(wk, widen(buf[q * plane + (sk ^ ((q & 1) ? flip : 0))])));
-                }
-#pragma unroll
-                for (int q = 0; q < SPS; q++)
-                    if (ds + q < d1) vout64[(ds + q) * n_out + o] = acc[q];
-            }
-        } else if constexpr (MODE == MODE_FF) {
-            if (o >= 0) {
-                // slices 2j and 2j + 1 of the stage as one packed pair
-                static_assert(SPS % 2 == 0, "the compensated apply stages slices in pairs");
-                uint64_t h2[SPS / 2], l2[SPS / 2];
-#pragma unroll
-                for (int j = 0; j < SPS / 2; j++) h2[j] = l2[j] = 0ull;
-#pragma unroll
-                for (int k = 0; k < CT; k++) {
-                    if (k < kwarp) {
-                        const int a = li[k], b = li[k] ^ flip;
-#pragma unroll
-                        for (int j = 0; j < SPS / 2; j++)
-                            ff_step2(h2[j], l2[j], fh[k], fhn[k], fl[k],
-                                     f2_pack(buf[2 * j * plane + a], buf[(2 * j + 1) * plane + b]));
-                    }
-                }
-                if constexpr (CT > 0) {
-#pragma unroll
-                    for (int j = 0; j < NX; j++) {
-                        if (CT + j < kwarp) {
-                            const float wk = ex_hi[j][t], wlk = ex_lo[j][t];
-                            const uint64_t kh = f2_pack(wk, wk), khn = f2_pack(-wk, -wk), kl = f2_pack(wlk, wlk);
-                            const int a = ex_slot[j][t], b = a ^ flip;
-#pragma unroll
-                            for (int q = 0; q < SPS / 2; q++)
-                                ff_step2(h2[q], l2[q], kh, khn, kl,
-                                         f2_pack(buf[2 * q * plane + a], buf[(2 * q + 1) * plane + b]));
-                        }
-                    }
-                }
-                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < e; k++) {
-                    const float wk = bval[k], wlk = blo[k];
-                    const uint64_t kh = f2_pack(wk, wk), khn = f2_pack(-wk, -wk), kl = f2_pack(wlk, wlk);
-                    const int a = slot[k], b = a ^ flip;
-#pragma unroll
-                    for (int j = 0; j < SPS / 2; j++)
-                        ff_step2(h2[j], l2[j], kh, khn, kl,
-                                 f2_pack(buf[2 * j * plane + a], buf[(2 * j + 1) * plane + b]));
-                }
-                float h[SPS], l[SPS];
-#pragma unroll
-                for (int j = 0; j < SPS / 2; j++) {
-                    const float2 hv = f2_unpack(h2[j]), lv = f2_unpack(l2[j]);
-                    h[2 * j] = hv.x;
-                    h[2 * j + 1] = hv.y;
-                    l[2 * j] = lv.x;
-                    l[2 * j + 1] = lv.y;
-                }
-                // The usual stage (every slice in range, every h and l a
-                // normal float) is tested once, with bitwise ands and a single
-                // branch, and stored without further tests (per-slice tests
-                // and branches were a measured share of the instruction
-                // stream).  Anything else takes the per-slice path.
-                bool usual = ds + SPS <= d1;
-#pragma unroll
-                for (int q = 0; q < SPS; q++)
-                    usual = usual & normal_bits(__float_as_uint(h[q])) & normal_bits(__float_as_uint(l[q]));
-                if (usual) {
-                    double* dst = vout64 + ds * n_out + o;
-#pragma unroll
-                    for (int q = 0; q < SPS; q++)
-                        dst[q * n_out] =
-                            __dadd_rn(widen_normal(__float_as_uint(h[q])), widen_normal(__float_as_uint(l[q])));
-                } else {
-#pragma unroll
-                    for (int q = 0; q < SPS; q++) {
-                        if (ds + q >= d1) continue;
-                        double r;
-                        const unsigned uh = __float_as_uint(h[q]), ul = __float_as_uint(l[q]);
-                        if (normal_bits(uh) && normal_bits(ul)) {
-                            r = __dadd_rn(widen_normal(uh), widen_normal(ul));
-                        } else if (nk == 0) {
-                            r = 0.0;
-                        } else if (finite_bits(h[q]) && finite_bits(l[q])) {
-                            r = __dadd_rn(widen(h[q]), widen(l[q]));
-                        } else {
-                            // a float32 partial sum overflowed, or an input or
-                            // a weight is not finite (or a padded step read a
-                            // non-finite word): this output and slice in
-                            // float64, stored order (the exact apply's sum)
-                            r = 0.0;
-                            for (int64_t k = s; k < e; k++)
-                                r = __dadd_rn(r, __dmul_rn(dval[k], widen(buf[q * plane + (box_slot_of(col[k], org, nd) ^
-                                                                                         ((q & 1) ? flip : 0))])));
-                        }
-                        vout64[(ds + q) * n_out + o] = r;
-                    }
-                }
-            }
-        } else if (o >= 0) {
-            float acc[SPS];
-#pragma unroll
-            for (int q = 0; q < SPS; q++) acc[q] = 0.f;
-#pragma unroll
-            for (int k = 0; k < CT; k++) {
-                if (k < nk) {
-#pragma unroll
-                    for (int q = 0; q < SPS; q++)
-                        acc[q] = fmaf(w[k], buf[q * plane + (li[k] ^ ((q & 1) ? flip : 0))], acc[q]);
-                }
-            }
-            if constexpr (CT > 0) {
-#pragma unroll
-                for (int j = 0; j < NX; j++) {
-                    if (CT + j < nk) {
-                        const float wk = ex_hi[j][t];
-                        const int sk = ex_slot[j][t];
-#pragma unroll
-                        for (int q = 0; q < SPS; q++)
-                            acc[q] = fmaf(wk, buf[q * plane + (sk ^ ((q & 1) ? flip : 0))], acc[q]);
-                    }
-                }
-            }
-            for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < e; k++) {
-                const float wk = bval[k];
-                const int sk = slot[k];
-#pragma unroll
-                for (int q = 0; q < SPS; q++) acc[q] = fmaf(wk, buf[q * plane + (sk ^ ((q & 1) ? flip : 0))], acc[q]);
-            }
-#pragma unroll
-            for (int q = 0; q < SPS; q++)
-                if (ds + q < d1) out[(ds + q) * n_out] = acc[q];
-        }
-        // The last warp done with the stage refills it, so no warp waits for
-        // the others (the slowest warp, with the longest rows, no longer
-        // holds a producer thread back).  Its lanes' reads of the stage are
-        // ordered before the count (syncwarp, then a release fence); the last
-        // one acquires them all before the async-proxy copy overwrites it.
-        __syncwarp();
-        if constexpr (PLANES) {
-            if (lane == 0) {
-                __threadfence_block();
-                const unsigned n = atomicAdd(&done[st], 1u) + 1u;
-                if (n == (unsigned)(grp / NST + 1) * PATCH_WARPS && grp + NST < ngroups) {
-                    __threadfence_block();
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    issue(st, grp + NST);
-                }
-            }
-        } else {
-            if (lane == 0) mbar_arrive(&empty[st]);  // this warp is done with the stage
-            if (t == 0 && grp + NST < ngroups) {
-                if (!mbar_wait_bounded(&empty[st], ph)) {
-                    atomicOr(flags, FLAG_TIMEOUT);
-                    for (int64_t q = grp + 1; q < grp + NST && q < ngroups; q++)
-                        (void)mbar_wait_bounded(&full[q % NST], (unsigned)((q / NST) & 1));
-                    return;
-                }
-                // the warps' generic-proxy reads of the stage before the async-proxy writes
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                issue(st, grp + NST);
-            }
-        }
-    }
+    perm[p * (32 * PATCH_WARPS) + t] = (uint8_t)(key[t] & 255u);
 }
 
 // ---------------------------------------------------------------------------
@@ -1213,25 +654,6 @@ __global__ void max_row_len(const int64_t* __restrict__ row_ptr, int64_t n, unsi
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-    static std::once_flag once;
-    static EncodeTiledFn fn = nullptr;
-    std::call_once(once, []() {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-        cudaGetLastError();
-    });
-    return fn;
-}
-
 // Scalar variant (slices not 16-byte aligned): single cells, PER per lane.
 template <int PER>
 __global__ void __launch_bounds__(32 * WARPS)
@@ -1334,6 +756,52 @@ TileShape tile_shape(const rg_weights_s* W) {
 }
 
 }  // namespace
+
+namespace {
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled() {
+    static std::once_flag once;
+    static EncodeTiledFn fn = nullptr;
+    std::call_once(once, []() {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = (EncodeTiledFn)p;
+        cudaGetLastError();
+    });
+    return fn;
+}
+
+}  // namespace
+
+// Tensor map of the input stack: columns x rows x slices, boxes of box_rows
+// rows and `bs` slices of 32 columns with the 128-byte swizzle, or (wide)
+// box_pitch columns as they lie; or (LOAD_RESIDUES) groups of four rows x
+// their number.
+bool encode_stack(const rg_weights_s* W, const float* vin, int64_t stack, int bs, CUtensorMap* map) {
+    const bool wide = W->box_pitch > 0;
+    if (W->box_residues) {
+        const cuuint64_t dims[2] = {(cuuint64_t)W->in_shape1 * 4, (cuuint64_t)(stack * W->in_shape0 / 4)};
+        const cuuint64_t strides[1] = {(cuuint64_t)W->in_shape1 * 16};
+        const cuuint32_t box[2] = {(cuuint32_t)W->box_pitch, (cuuint32_t)((W->box_rows + 3) / 4)};
+        const cuuint32_t estr[2] = {1, 1};
+        return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)vin, dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    const cuuint64_t dims[3] = {(cuuint64_t)W->in_shape1, (cuuint64_t)W->in_shape0, (cuuint64_t)stack};
+    const cuuint64_t strides[2] = {(cuuint64_t)W->in_shape1 * 4, (cuuint64_t)W->n_in * 4};
+    const cuuint32_t box[3] = {(cuuint32_t)(wide ? W->box_pitch : PBOX_C), (cuuint32_t)W->box_rows, (cuuint32_t)bs};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)vin, dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Build the warp-tile lists of W for the given grain (8: 32-byte sectors for
 // aligned inputs, 1: single cells), stream ordered, synchronising once.
@@ -1454,45 +922,89 @@ int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int
     return RG_OK;
 }
 
-// Whether the TMA apply can take this call: output and input grid shapes
-// known, input rows of whole 16-byte chunks, 16-byte aligned slices.
-bool box_usable(const rg_weights_s* W, const float* vin, int64_t stack) {
+// Whether the patch kernel may take calls with this handle: output and input
+// grid shapes known.
+bool box_usable(const rg_weights_s* W, int64_t stack) {
     return W->box_state >= 0 && W->out_shape0 > 0 && W->out_shape1 > 0 &&
            W->out_shape0 * W->out_shape1 == W->n_out && W->in_shape0 > 0 && W->in_shape1 > 0 &&
-           W->in_shape1 % 4 == 0 && W->in_shape0 * W->in_shape1 == W->n_in && ((uintptr_t)vin & 15) == 0 &&
-           stack >= 1 && W->n_in < INT32_MAX && stack < INT32_MAX && encode_tiled() != nullptr;
+           W->in_shape0 * W->in_shape1 == W->n_in && stack >= 1 && W->n_in < INT32_MAX && stack < INT32_MAX &&
+           encode_tiled() != nullptr;
 }
+
+// How the patch kernel would fill its stages for this call, -1 when it does
+// not take it (the caller holds the handle's lock, box_lists_for has run).
+int box_load(const rg_weights_s* W, const float* vin, int64_t stack) {
+    const bool aligned = W->in_shape1 % 4 == 0 && ((uintptr_t)vin & 15) == 0;
+    if (W->box_state == 1) return aligned ? LOAD_SWIZZLED : -1;
+    if (W->box_state != 2) return -1;
+    if (((uintptr_t)vin & 15) != 0) return -1;
+    if (W->box_residues == 0) return LOAD_WIDE;
+    // the box within the tensor of row groups
+    return stack * W->in_shape0 / 4 >= (W->box_rows + 3) / 4 ? LOAD_RESIDUES : -1;
+}
+
+BoxShape box_shape(const rg_weights_s* W) { return BoxShape{W->box_pitch, W->box_residues}; }
 
 PatchGrid patch_grid(const rg_weights_s* W) {
     PatchGrid P;
     P.n0 = W->out_shape0;
     P.n1 = W->out_shape1;
-    P.patches1 = (P.n1 + PATCH - 1) / PATCH;
+    P.cb = W->box_cb;
+    P.patches1 = (P.n1 + (1 << P.cb) - 1) >> P.cb;
     return P;
 }
 
-// Build the patch lists of W (the caller holds the handle's lock; *made set
-// when anything was launched).  Leaves box_state -1 when the footprints do
-// not fit a box (more than 1 % of the patches, and more than 4, would need
-// direct gathers).
+int64_t patch_count(const PatchGrid& P) {
+    const int64_t rows = 256 >> P.cb;
+    return (P.n0 + rows - 1) / rows * P.patches1;
+}
+
 // The exact apply's per-patch thread order (made once, with the box lists).
 int box_perm_for(rg_weights_s* W, cudaStream_t s, bool* made) {
-    if (W->box_perm || W->box_state != 1) return RG_OK;
+    if (W->box_perm || W->box_state < 1) return RG_OK;
     *made = true;
-    RG_TRY(dalloc(&W->box_perm, (size_t)W->box_patches * PATCH * PATCH, s));
-    perm_patch<<<(unsigned)W->box_patches, PATCH * PATCH, 0, s>>>(W->row_ptr, patch_grid(W), 1, W->box_perm);
+    RG_TRY(dalloc(&W->box_perm, (size_t)W->box_patches * 256, s));
+    perm_patch<<<(unsigned)W->box_patches, 32 * PATCH_WARPS, 0, s>>>(W->row_ptr, patch_grid(W), 1, W->box_perm);
     RG_CUDA(cudaGetLastError());
+    return RG_OK;
+}
+
+// The fast apply's entry order: slots and float32 weights in the order its
+// threads gather them.
+int box_order_for(rg_weights_s* W, cudaStream_t s, bool* made) {
+    if (W->box_val || W->box_state < 1) return RG_OK;
+    *made = true;
+    uint16_t* slot = nullptr;
+    float* hi = nullptr;
+    int st = dalloc(&slot, (size_t)W->nnz, s);
+    if (st == RG_OK) st = dalloc(&hi, (size_t)W->nnz, s);
+    if (st == RG_OK) {
+        order_patch<<<(unsigned)W->box_patches, 32 * PATCH_WARPS, 0, s>>>(
+            W->row_ptr, W->col, FastDiv((uint32_t)W->in_shape1), W->val32, W->val, patch_grid(W), W->box_origin,
+            box_shape(W), nullptr, slot, hi, nullptr);
+        if (cudaGetLastError() != cudaSuccess) {
+            set_error("apply (entry order): launch failed");
+            st = RG_ERR_CUDA;
+        }
+    }
+    if (st != RG_OK) {
+        dfree(slot, s);
+        dfree(hi, s);
+        return st;
+    }
+    W->box_slot = slot;
+    W->box_val = hi;
     return RG_OK;
 }
 
 // The compensated apply's per-patch thread order (row lengths in classes of 3).
 constexpr int FF_LENGTH_CLASS = 3;
 int ff_perm_for(rg_weights_s* W, cudaStream_t s, bool* made) {
-    if (W->ff_perm || W->box_state != 1) return RG_OK;
+    if (W->ff_perm || W->box_state < 1) return RG_OK;
     *made = true;
-    RG_TRY(dalloc(&W->ff_perm, (size_t)W->box_patches * PATCH * PATCH, s));
-    perm_patch<<<(unsigned)W->box_patches, PATCH * PATCH, 0, s>>>(W->row_ptr, patch_grid(W), FF_LENGTH_CLASS,
-                                                                  W->ff_perm);
+    RG_TRY(dalloc(&W->ff_perm, (size_t)W->box_patches * 256, s));
+    perm_patch<<<(unsigned)W->box_patches, 32 * PATCH_WARPS, 0, s>>>(W->row_ptr, patch_grid(W), FF_LENGTH_CLASS,
+                                                                     W->ff_perm);
     RG_CUDA(cudaGetLastError());
     return RG_OK;
 }
@@ -1502,7 +1014,7 @@ int ff_perm_for(rg_weights_s* W, cudaStream_t s, bool* made) {
 // lane's entries are ordered for that layout with their float32 weights and
 // the weights' float32 rests.
 int ff_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
-    if (W->ff_slot || W->box_state != 1) return RG_OK;
+    if (W->ff_slot || W->box_state < 1) return RG_OK;
     RG_TRY(ff_perm_for(W, s, made));
     *made = true;
     int st = RG_OK;
@@ -1511,8 +1023,8 @@ int ff_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
         if ((st = dalloc(&W->ff_hi, (size_t)W->nnz, s))) break;
         if ((st = dalloc(&W->ff_lo, (size_t)W->nnz, s))) break;
         order_patch<<<(unsigned)W->box_patches, 32 * PATCH_WARPS, 0, s>>>(
-            W->row_ptr, W->col, FastDiv((uint32_t)W->in_shape1), W->val32, W->val, patch_grid(W), W->box_origin, W->ff_perm, nullptr,
-            W->ff_slot, W->ff_hi, W->ff_lo);
+            W->row_ptr, W->col, FastDiv((uint32_t)W->in_shape1), W->val32, W->val, patch_grid(W), W->box_origin,
+            box_shape(W), W->ff_perm, W->ff_slot, W->ff_hi, W->ff_lo);
         if (cudaGetLastError() != cudaSuccess) {
             set_error("apply (compensated lists): launch failed");
             st = RG_ERR_CUDA;
@@ -1529,67 +1041,120 @@ int ff_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
     return st;
 }
 
+// A wide box that holds rows x cols cells: rows a multiple of 4 floats apart
+// and no multiple of 8, so that the rows of a column fall on eight groups of
+// banks.  Where rows are no whole 16-byte chunks, up to 6 floats before the
+// cells, and the four row residues each from a 128-byte boundary on.  (A few
+// floats of stagger between the residues, to put neighbouring rows on
+// different banks, measured no faster: the boxes grow by half.)
+struct WideBox {
+    int rows, pitch, residues;
+    int cells() const { return residues ? 4 * residues : rows * pitch; }
+};
+static WideBox wide_box(const unsigned* extent, int64_t row) {
+    WideBox b{(int)extent[0], (int)((extent[1] + (row % 4 ? 6 : 0) + 3) & ~3u), 0};
+    if (b.pitch % 8 == 0) b.pitch += 4;
+    if (row % 4) b.residues = ((b.rows + 3) / 4 * b.pitch + 31) & ~31;
+    return b;
+}
+
+// Build the patch list of W (the caller holds the handle's lock; *made set
+// when anything was launched).  One box size serves all patches:
+//  state 1: 32 swizzled columns and up to 32 rows, for patches of 16 x 16
+//           cells whose input rows are whole 16-byte chunks; up to 1 % of
+//           them (or 4) may be larger and gather directly;
+//  state 2: a wide box of up to WIDE_MAX cells, for larger footprints
+//           (output grids rotated by more than about 0.3 rad at 0.75 of the
+//           input's cells a side, or coarser ones) and for rows of any
+//           length.  Patches are 16 x 16, or of the sides from 64 x 4 to
+//           4 x 64 with the smallest box where 16 x 16 needs more than 1536
+//           cells (input cells of unequal sides);
+//  state -1: larger yet.
+constexpr int WIDE_MAX = 3584;
+
 int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
     if (W->box_state != 0) return RG_OK;
     *made = true;
-    const PatchGrid P = patch_grid(W);
-    const int64_t patches = ((P.n0 + PATCH - 1) / PATCH) * P.patches1;
-    RG_CHECK(patches < 0x7fffffff, RG_ERR_UNSUPPORTED, "apply: too many output patches");
-    int2* extent = nullptr;
-    unsigned* stats = nullptr;
+    const FastDiv nd((uint32_t)W->in_shape1);
+    // the candidates' patches, log2 of their columns; 16 x 16 first
+    const int sides[5] = {4, 3, 5, 2, 6};
+    int64_t most = 0;
+    for (int c : sides) {
+        W->box_cb = c;
+        most = std::max(most, patch_count(patch_grid(W)));
+    }
+    W->box_cb = 4;
+    RG_CHECK(most < 0x7fffffff, RG_ERR_UNSUPPORTED, "apply: too many output patches");
+    unsigned* stats = nullptr;  // [candidate][rows, columns, larger than 32 x 32, -]
     int st = RG_OK;
+    int state = -1;
+    auto footprints = [&](int k) {
+        W->box_cb = sides[k];
+        const PatchGrid P = patch_grid(W);
+        patch_footprints<<<(unsigned)patch_count(P), 32 * PATCH_WARPS, 0, s>>>(W->row_ptr, W->col, P, nd, W->box_origin,
+                                                                               W->box_extent, stats + 4 * k);
+    };
+    unsigned h[5][4] = {};
+    auto read = [&]() {
+        small_to_host(h, stats, sizeof(h), s);
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) return (int)RG_OK;
+        set_error("apply (patch lists): %s", cudaGetErrorString(e));
+        return (int)RG_ERR_CUDA;
+    };
     do {
-        if ((st = dalloc(&W->box_origin, (size_t)patches, s))) break;
-        if ((st = dalloc(&extent, (size_t)patches, s))) break;
-        if ((st = dalloc(&stats, 4, s))) break;
-        if ((st = dalloc(&W->box_slot, (size_t)W->nnz, s))) break;
+        if ((st = dalloc(&W->box_origin, (size_t)most, s))) break;
+        if ((st = dalloc(&W->box_extent, (size_t)most, s))) break;
+        if ((st = dalloc(&stats, 20, s))) break;
         if (W->dflags == nullptr) {
             if ((st = dalloc(&W->dflags, 1, s))) break;
             cudaMemsetAsync(W->dflags, 0, sizeof(unsigned), s);
         }
-        cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned), s);
-        prepare_patch<0><<<(unsigned)patches, 256, 0, s>>>(W->row_ptr, W->col, P, FastDiv((uint32_t)W->in_shape1), W->box_origin,
-                                                           extent, stats, 0, nullptr);
-        unsigned h[4] = {0, 0, 0, 0};
-        small_to_host(h, stats, sizeof(h), s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_error("apply (patch lists): %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
-            break;
-        }
+        cudaMemsetAsync(stats, 0, 20 * sizeof(unsigned), s);
+        footprints(0);
+        if ((st = read())) break;
         // box rows: a multiple of 4 (keeps the swizzle phase of every slice at 0 or 4)
-        const int BR = (int)((std::min<unsigned>(std::max<unsigned>(h[0], 1u), PBOX_MAX_R) + 3) & ~3u);
-        prepare_patch<1><<<(unsigned)patches, 256, 0, s>>>(W->row_ptr, W->col, P, FastDiv((uint32_t)W->in_shape1), W->box_origin,
-                                                           extent, stats, BR, W->box_slot);
-        small_to_host(h, stats, sizeof(h), s);
-        e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_error("apply (patch lists): %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
+        const int BR = (int)((std::min<unsigned>(std::max<unsigned>(h[0][0], 1u), PBOX_MAX_R) + 3) & ~3u);
+        const int64_t patches = patch_count(patch_grid(W));
+        if (W->in_shape1 % 4 == 0 && ((int64_t)h[0][2] * 100 <= patches || h[0][2] <= 4) && BR <= W->in_shape0 &&
+            PBOX_C <= W->in_shape1) {
+            if (h[0][2])
+                mark_large_patches<<<grid_for(patches, 256), 256, 0, s>>>(patches, W->box_extent, W->box_origin);
+            state = 1;
+            W->box_rows = BR;
+            W->box_cols = PBOX_C;
+            W->box_pitch = W->box_residues = 0;
+            W->box_patches = patches;
             break;
         }
-        W->box_rows = BR;
-        W->box_cols = PBOX_C;
-        W->box_patches = patches;
-        const bool few = (int64_t)h[2] * 100 <= patches || h[2] <= 4;  // patches left to direct gathers
-        W->box_state = few && BR <= W->in_shape0 && PBOX_C <= W->in_shape1 ? 1 : -1;
-        if (W->box_state != 1) break;  // footprints too large for a box: no entry order needed
-        if ((st = dalloc(&W->box_val, (size_t)W->nnz, s))) break;
-        order_patch<<<(unsigned)patches, 32 * PATCH_WARPS, 0, s>>>(W->row_ptr, W->col, FastDiv((uint32_t)W->in_shape1),
-                                                                   W->val32, W->val, P, W->box_origin, nullptr,
-                                                                   W->box_slot, W->box_slot, W->box_val, nullptr);
+        int best = 0;
+        if (wide_box(h[0], W->in_shape1).cells() > 1536) {
+            for (int k = 1; k < 5; k++) footprints(k);
+            if ((st = read())) break;
+            for (int k = 1; k < 5; k++)
+                if (wide_box(h[k], W->in_shape1).cells() < wide_box(h[best], W->in_shape1).cells()) best = k;
+            footprints(best);
+        }
+        const WideBox b = wide_box(h[best], W->in_shape1);
+        W->box_patches = patch_count(patch_grid(W));
+        // the box has to lie in a tensor's extent
+        if (b.rows == 0 || b.rows > 256 || b.pitch > 256 || b.cells() > WIDE_MAX) break;
+        if (b.residues ? b.pitch > 4 * W->in_shape1 : b.rows > W->in_shape0 || b.pitch > W->in_shape1) break;
+        state = 2;
+        W->box_rows = b.rows;
+        W->box_cols = W->box_pitch = b.pitch;
+        W->box_residues = b.residues;
     } while (0);
-    dfree(extent, s);
     dfree(stats, s);
-    if (st != RG_OK || W->box_state != 1) {
+    if (st == RG_OK) W->box_state = state;
+    if (st != RG_OK || state != 2) {
+        dfree(W->box_extent, s);
+        W->box_extent = nullptr;
+    }
+    if (st != RG_OK || state == -1) {
         dfree(W->box_origin, s);
-        dfree(W->box_slot, s);
-        dfree(W->box_val, s);
         W->box_origin = nullptr;
-        W->box_slot = nullptr;
-        W->box_val = nullptr;
-        if (st == RG_OK) W->box_state = -1;
+        W->box_cb = 4;
     }
     return st;
 }
@@ -1646,21 +1211,9 @@ int launch_patch(const rg_weights_s* W, const CUtensorMap& map, int box_slices, 
         map, W->row_ptr, W->col, FF ? W->ff_slot : W->box_slot, FF ? W->ff_hi : W->box_val, FF ? W->ff_lo : nullptr,
         W->val32, W->val, OUT64 ? (double*)vout : nullptr, FastDiv((uint32_t)W->in_shape1), patch_grid(W), patches, W->box_origin, BR,
         stage_floats, box_bytes, vin, W->n_in, OUT64 ? nullptr : (float*)vout, W->n_out, stack, chunk, W->dflags,
-        FF ? W->ff_perm : (OUT64 ? W->box_perm : nullptr));
+        FF ? W->ff_perm : (OUT64 ? W->box_perm : nullptr), BoxShape{0, 0}, nullptr);
     RG_CUDA(cudaGetLastError());
     return RG_OK;
-}
-
-// Tensor map of the input stack: columns x rows x slices, boxes of
-// 32 columns x box_rows x bs slices, 128-byte swizzle.
-bool encode_stack(const rg_weights_s* W, const float* vin, int64_t stack, int bs, CUtensorMap* map) {
-    const cuuint64_t dims[3] = {(cuuint64_t)W->in_shape1, (cuuint64_t)W->in_shape0, (cuuint64_t)stack};
-    const cuuint64_t strides[2] = {(cuuint64_t)W->in_shape1 * 4, (cuuint64_t)W->n_in * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)PBOX_C, (cuuint32_t)W->box_rows, (cuuint32_t)bs};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)vin, dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int MODE>
@@ -1802,10 +1355,13 @@ int tune_box(rg_weights_s* W, int mode, const float* vin, void* vout, int64_t st
     return RG_OK;
 }
 
+int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s);
+
 // Launch the TMA apply; returns RG_ERR_UNSUPPORTED (nothing launched) when
 // the tuned configuration does not take this call, so the caller can take
 // another kernel.
 int apply_box(const rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
+    if (W->box_state == 2) return apply_wide(W, MODE_FAST, box_load(W, vin, stack), vin, vout, stack, s);
     const int cfg = W->box_cfg[stack_class(stack)];
     if (cfg < 0) return RG_ERR_UNSUPPORTED;
     return launch_box_config(W, MODE_FAST, cfg, vin, vout, stack, s);
@@ -1814,6 +1370,7 @@ int apply_box(const rg_weights_s* W, const float* vin, float* vout, int64_t stac
 // The compensated (float-float) TMA apply with its tuned configuration.
 int apply_box_ff(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
     const int cfg = W->box_cfg_ff[stack_class(stack)];
+    if (W->box_state == 2) return apply_wide(W, MODE_FF, box_load(W, vin, stack), vin, vout, stack, s);
     if (W->box_state != 1 || cfg < 0 || !W->ff_slot || !W->ff_perm) return RG_ERR_UNSUPPORTED;
     return launch_box_config(W, MODE_FF, cfg, vin, vout, stack, s);
 }
@@ -1829,6 +1386,7 @@ int tune_box_ff(rg_weights_s* W, const float* vin, double* vout, int64_t stack, 
 // The exact (float64) TMA apply: 4 slices per stage, 2 stages (FP64 issue,
 // not the staging, bounds it).
 int apply_box_exact(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
+    if (W->box_state == 2) return apply_wide(W, MODE_EXACT, box_load(W, vin, stack), vin, vout, stack, s);
     if (W->box_state != 1) return RG_ERR_UNSUPPORTED;
     const int bs = (int)std::min<int64_t>(4, stack);
     CUtensorMap map;

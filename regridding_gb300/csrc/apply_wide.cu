@@ -1,0 +1,97 @@
+// The patch kernel with wide boxes (box_state 2): footprints that exceed the
+// 32 x 32 swizzled box, and input rows that are no whole 16-byte chunks.
+// Without them those handles gathered from global memory, the exact and
+// compensated modes with FP64 sums whose lanes ran rows of unequal length.
+// Measured, before and after: 2048^2 -> 1536^2 rotated by 0.45 rad, 64 float32
+// slices, compensated 7.17 -> 0.60 ms (HBM 0.36 ms; the kernel is bound by its
+// instruction stream) and fast 0.50 -> 0.35 ms (a mean over three rotations);
+// 1601^2 -> 1201^2, 32 slices, compensated 2.20 -> 0.33 ms; 777 x 611 -> 583 x
+// 458, 32 slices, exact 0.44 -> 0.25 ms (FP64 issue).
+#include <algorithm>
+
+#include "common.cuh"
+#include "patch.cuh"
+
+namespace rg {
+
+bool encode_stack(const rg_weights_s* W, const float* vin, int64_t stack, int bs, CUtensorMap* map);
+PatchGrid patch_grid(const rg_weights_s* W);
+BoxShape box_shape(const rg_weights_s* W);
+
+namespace {
+
+template <int PL, int SPS, int NST, int MODE, int LOAD>
+int launch_wide(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+    constexpr int CT = MODE == MODE_FF ? 6 : CACHED_T;
+    const auto kernel = apply_patch_tma<SPS, NST, 0, MODE, CT, LOAD, PL>;
+    const size_t smem = (size_t)NST * SPS * PL * sizeof(float);
+    static std::once_flag attr;
+    std::call_once(attr, [&]() {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaGetLastError();
+    });
+    CUtensorMap map = {};
+    if (!encode_stack(W, vin, stack, 1, &map)) return RG_ERR_UNSUPPORTED;
+    const int64_t patches = W->box_patches;
+    // split the stack over gridDim.y only when the patches alone give less
+    // than ~4 waves of 4 blocks per SM on 152 SMs
+    const int64_t target_blocks = 152 * 4 * 4;
+    const int64_t chunks = std::max<int64_t>(1, (target_blocks + patches - 1) / patches);
+    int64_t chunk = (stack + chunks - 1) / chunks;
+    chunk = (chunk + SPS - 1) / SPS * SPS;
+    if ((stack + chunk - 1) / chunk > 65535) chunk = ((stack + 65534) / 65535 + SPS - 1) / SPS * SPS;
+    const dim3 grid((unsigned)patches, (unsigned)((stack + chunk - 1) / chunk));
+    // bytes of one copy: a slice's box, or the rows of one residue
+    const int rows = LOAD == LOAD_RESIDUES ? (W->box_rows + 3) / 4 : W->box_rows;
+    const unsigned box_bytes = (unsigned)(rows * W->box_pitch * 4);
+    constexpr bool OUT64 = MODE != MODE_FAST;
+    constexpr bool FF = MODE == MODE_FF;
+    kernel<<<grid, 32 * PATCH_WARPS, smem, s>>>(
+        map, W->row_ptr, W->col, FF ? W->ff_slot : W->box_slot, FF ? W->ff_hi : W->box_val, FF ? W->ff_lo : nullptr,
+        W->val32, W->val, OUT64 ? (double*)vout : nullptr, FastDiv((uint32_t)W->in_shape1), patch_grid(W), patches,
+        W->box_origin, W->box_rows, SPS * PL, box_bytes, vin, W->n_in,
+        OUT64 ? nullptr : (float*)vout, W->n_out, stack, chunk, W->dflags,
+        FF ? W->ff_perm : (OUT64 ? W->box_perm : nullptr), box_shape(W), W->box_extent);
+    RG_CUDA(cudaGetLastError());
+    return RG_OK;
+}
+
+// Slices per stage: a stage computes all its slices, also those past the end
+// of the stack, so one or two slices take stages of two; the largest boxes
+// too, to keep three blocks on an SM.
+template <int PL, int MODE, int LOAD>
+int launch_plane(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+    if constexpr (PL <= 2304)
+        if (stack > 2) return launch_wide<PL, 4, 2, MODE, LOAD>(W, vin, vout, stack, s);
+    return launch_wide<PL, 2, 2, MODE, LOAD>(W, vin, vout, stack, s);
+}
+
+// A slice's plane in a stage, the smallest of a few sizes that holds the box
+// (a constant, so that a gather's slices differ by constant offsets).
+template <int MODE, int LOAD>
+int launch_mode(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+    const int cells = W->box_residues ? 4 * W->box_residues : W->box_rows * W->box_pitch;
+    if (cells <= 1024) return launch_plane<1024, MODE, LOAD>(W, vin, vout, stack, s);
+    if (cells <= 1536) return launch_plane<1536, MODE, LOAD>(W, vin, vout, stack, s);
+    if (cells <= 2304) return launch_plane<2304, MODE, LOAD>(W, vin, vout, stack, s);
+    return launch_plane<3584, MODE, LOAD>(W, vin, vout, stack, s);
+}
+
+template <int MODE>
+int launch_load(const rg_weights_s* W, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+    if (load == LOAD_WIDE) return launch_mode<MODE, LOAD_WIDE>(W, vin, vout, stack, s);
+    if constexpr (MODE != MODE_FAST) return launch_mode<MODE, LOAD_RESIDUES>(W, vin, vout, stack, s);
+    return RG_ERR_UNSUPPORTED;
+}
+
+}  // namespace
+
+int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+    switch (mode) {
+        case MODE_FAST: return launch_load<MODE_FAST>(W, load, vin, vout, stack, s);
+        case MODE_EXACT: return launch_load<MODE_EXACT>(W, load, vin, vout, stack, s);
+        default: return launch_load<MODE_FF>(W, load, vin, vout, stack, s);
+    }
+}
+
+}  // namespace rg

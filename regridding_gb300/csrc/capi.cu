@@ -140,6 +140,19 @@ int column_order(rg_weights_s* W, int32_t** row_of, uint32_t** perm, int64_t** c
     return st;
 }
 
+// Frees what box_lists_for and the entry orders made (no work in flight).
+void drop_patch_lists(rg_weights_s* W) {
+    for (void* p : {(void*)W->box_origin, (void*)W->box_extent, (void*)W->box_slot, (void*)W->box_val,
+                    (void*)W->box_perm, (void*)W->ff_perm, (void*)W->ff_slot, (void*)W->ff_hi, (void*)W->ff_lo})
+        dfree(p, nullptr);
+    W->box_origin = W->box_extent = nullptr;
+    W->box_slot = W->ff_slot = nullptr;
+    W->box_val = W->ff_hi = W->ff_lo = nullptr;
+    W->box_perm = W->ff_perm = nullptr;
+    W->box_state = 0;
+    W->box_cb = 4;
+}
+
 void free_weights(rg_weights_s* W, cudaStream_t s) {
     dfree(W->row_ptr, s);
     dfree(W->col, s);
@@ -155,6 +168,7 @@ void free_weights(rg_weights_s* W, cudaStream_t s) {
         dfree(W->t_slot[g], s);
     }
     dfree(W->box_origin, s);
+    dfree(W->box_extent, s);
     dfree(W->box_slot, s);
     dfree(W->box_val, s);
     dfree(W->ff_slot, s);
@@ -484,8 +498,12 @@ int rg_weights_set_output_shape(rg_weights w, int64_t n0, int64_t n1) {
              (long long)n0, (long long)n1, (long long)w->n_out);
     std::lock_guard<std::mutex> lock(w->mu);
     if (w->out_shape0 == n0 && w->out_shape1 == n1) return RG_OK;
-    RG_CHECK(!w->tiled_ready[0] && !w->tiled_ready[1], RG_ERR_ARG,
+    RG_CHECK(!w->tiled_ready[0] && !w->tiled_ready[1] && !w->box_val, RG_ERR_ARG,
              "rg_weights_set_output_shape: the output tiling is fixed once a fast float32 apply has run");
+    if (w->box_state != 0) {  // patch lists of the former shape, perhaps in use on some stream
+        RG_CUDA(cudaDeviceSynchronize());
+        drop_patch_lists(w);
+    }
     w->out_shape0 = n0;
     w->out_shape1 = n1;
     return RG_OK;
@@ -516,6 +534,12 @@ int rg_weights_set_input_shape(rg_weights w, int64_t n0, int64_t n1) {
              (long long)n1, (long long)w->n_in);
     std::lock_guard<std::mutex> lock(w->mu);
     if (w->in_shape0 == n0 && w->in_shape1 == n1) return RG_OK;
+    if (w->box_state != 0 && w->in_shape1 % 4 != 0 && !w->box_val) {
+        // exact or compensated applies made patch lists for rows that are
+        // not whole 16-byte chunks; they may still be in use on some stream
+        RG_CUDA(cudaDeviceSynchronize());
+        drop_patch_lists(w);
+    }
     RG_CHECK(w->box_state == 0, RG_ERR_ARG,
              "rg_weights_set_input_shape: the input tiling is fixed once a fast float32 apply has run");
     w->in_shape0 = n0;
@@ -632,7 +656,8 @@ int rg_weights_device_bytes(rg_weights w, int64_t* bytes) {
     if (w->t_val32) b += nnz * 4;
     for (int g = 0; g < 2; g++)
         if (w->tiled_ready[g]) b += (w->t_tiles + 1) * 8 + nnz * 2;  // list pointers + slots (lists are small)
-    if (w->box_state == 1) b += w->box_patches * 8 + nnz * 6;  // origins; slot and float32 weight per entry
+    if (w->box_state >= 1) b += w->box_patches * (w->box_extent ? 16 : 8);  // origins, extents
+    if (w->box_val) b += nnz * 6;                                // slot and float32 weight per entry
     if (w->ff_slot) b += nnz * 10;                              // compensated: slot, hi and lo per entry
     if (w->box_perm) b += w->box_patches * 256;
     if (w->ff_perm) b += w->box_patches * 256;

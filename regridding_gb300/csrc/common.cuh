@@ -234,12 +234,15 @@ struct rg_weights_s {
     // origin (row, column) of a fixed box_rows x box_cols box of input cells
     // holding its footprint (row -1: no entries, -2: footprint larger than
     // the box), and per entry its (swizzled) offset in the box
-    int box_state = 0;  // 0 not built, 1 ready, -1 not applicable
-    int box_rows = 0, box_cols = 0;
+    // in a wide box (state 2, of box_pitch columns) it is not swizzled, and
+    // patches are of 256 >> box_cb rows and 1 << box_cb columns
+    int box_state = 0;  // 0 not built, 1 ready, 2 ready with wide boxes, -1 not applicable
+    int box_rows = 0, box_cols = 0, box_pitch = 0, box_residues = 0, box_cb = 4;
     int64_t box_patches = 0;
     // configuration chosen by the autotuner per stack class (-1 not tuned, -2 none fits)
     int box_cfg[rg::kStackClasses] = {-1, -1, -1, -1, -1, -1, -1};
     int2* box_origin = nullptr;
+    int2* box_extent = nullptr;    // wide boxes: rows and columns of every patch's footprint
     uint16_t* box_slot = nullptr;  // per entry, in the order the TMA kernel gathers them
     uint8_t* box_perm = nullptr;   // exact apply: per patch, thread -> output (longest rows first)
     float* box_val = nullptr;      // float32 weights in that order
