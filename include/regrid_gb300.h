@@ -122,6 +122,18 @@ int rg_build_conservative_2d_batch(int64_t n, const double* const* d_xi, const d
 int rg_weights_from_coo(const int64_t* d_in, const int64_t* d_out, const double* d_val, int64_t nnz,
                         int64_t n_in, int64_t n_out, rg_stream_t stream, rg_weights* out);
 
+/* The block diagonal matrix of nd elements in the saved layout, as
+ * rg_conservative_1d and rg_multilinear_1d leave them: those of element d
+ * start at d * stride, d_count[d] of them (d_count NULL: stride of them).
+ * Element d maps its n_in inputs, columns d * n_in on, to outputs d * n_out on,
+ * so one apply of (stack, nd * n_in) values serves all elements; entries of
+ * one output keep their order.  nd * n_in and nd * n_out below 2^31.
+ * Synchronises `stream`.  Replaces the loop over the elements of
+ * regridding/_regrid/_regrid_from_weights.py:150-162. */
+int rg_weights_block_diagonal(const int64_t* d_in, const int64_t* d_out, const double* d_val,
+                              const int64_t* d_count, int64_t nd, int64_t stride, int64_t n_in, int64_t n_out,
+                              rg_stream_t stream, rg_weights* out);
+
 /* Number of stored entries and the matrix shape. */
 int rg_weights_info(rg_weights w, int64_t* nnz, int64_t* n_in, int64_t* n_out);
 

@@ -199,6 +199,16 @@ class DeviceWeights:
                   stream(), ctypes.byref(h))
         return cls(h, shape_out, shape_in)
 
+    @classmethod
+    def block_diagonal(cls, ind_in, ind_out, val, count, n_in: int, n_out: int) -> "DeviceWeights":
+        """One matrix over the elements of (elements, stride) CUDA tensors in
+        the saved layout (``count[d]`` entries of row ``d``, all of them when
+        None): element ``d`` maps columns ``d * n_in`` on to rows ``d * n_out`` on."""
+        h = ctypes.c_void_p()
+        _lib.call("rg_weights_block_diagonal", ptr(ind_in), ptr(ind_out), ptr(val), ptr(count), ind_in.shape[0],
+                  ind_in.shape[1], int(n_in), int(n_out), stream(), ctypes.byref(h))
+        return cls(h)
+
     def export(self):
         """Entries in the saved layout, sorted by (input, output), as CUDA tensors."""
         t = torch()

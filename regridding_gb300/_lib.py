@@ -48,6 +48,7 @@ SIGNATURES = {
     "rg_fill_median": [_P, _C, _P, _I, _I, _P, _P],
     "rg_build_conservative_2d_batch": [_I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
     "rg_weights_from_coo": [_P, _P, _P, _I, _I, _I, _P, ctypes.POINTER(_P)],
+    "rg_weights_block_diagonal": [_P, _P, _P, _P, _I, _I, _I, _I, _P, ctypes.POINTER(_P)],
     "rg_weights_info": [_P, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I)],
     "rg_weights_set_output_shape": [_P, _I, _I],
     "rg_weights_export_coo": [_P, _P, _P, _P, _P],

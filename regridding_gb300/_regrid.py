@@ -13,7 +13,7 @@ from typing import Literal, Sequence
 import numpy as np
 
 from . import _device, _util
-from ._weights import _weights_device
+from ._weights import Entries, _weights_device
 
 __all__ = ["regrid_from_weights", "regrid"]
 
@@ -61,6 +61,12 @@ def regrid_from_weights(
     in float-float arithmetic on the FP32 pipe, about 5x faster than
     ``"exact"`` on GB300 (other inputs compute as ``"exact"``).
     """
+    return _apply(weights, shape_input, shape_output, values_input, values_output, axis_input, axis_output, accumulate)
+
+
+def _apply(weights, shape_input, shape_output, values_input, values_output, axis_input, axis_output, accumulate):
+    """:func:`regrid_from_weights`; ``weights`` may also be the 1D
+    :class:`Entries` of a build that never left the device."""
     if accumulate not in ("exact", "fast", "compensated"):
         raise ValueError(f"accumulate must be 'exact', 'fast' or 'compensated', got {accumulate!r}")
     unit = getattr(values_input, "unit", None)
@@ -72,7 +78,21 @@ def regrid_from_weights(
         shape_input, shape_output, values_input.shape if np.ndim(values_input) > 0 else (), axis_input,
         axis_output)
 
-    w_arr = np.broadcast_to(np.array(weights), shape_orth, subok=True)
+    entries = element = None
+    if isinstance(weights, Entries):
+        n_cells = [int(np.prod([shape[ax] for ax in axes])) for shape, axes in
+                   ((full_in, axis_input), (full_out, axis_output))]
+        if weights.ind_in.shape[0] == 1:
+            one = np.empty(weights.shape, dtype=object)
+            one[...] = _DeviceElement(_device.DeviceWeights.block_diagonal(
+                weights.ind_in, weights.ind_out, weights.val, weights.count, *n_cells))
+            weights = one
+        else:
+            entries = weights
+            element = np.arange(entries.ind_in.shape[0]).reshape(entries.shape)
+            element = np.broadcast_to(element, shape_orth).reshape(-1)
+            weights = np.empty(0, dtype=object)
+    w_arr = weights if entries is not None else np.broadcast_to(np.array(weights), shape_orth, subok=True)
     values_input = np.broadcast_to(values_input, full_in, subok=True)
 
     out_dtype = np.float64
@@ -117,12 +137,20 @@ def regrid_from_weights(
             first[key] = d
         groups[key].append(d)
 
-    # one weights element and a row-major output view: the device result is
-    # copied straight into values_output
+    if entries is None and len(axis_input) == 1:
+        entries, element = _short_elements(flat, groups, first)
+    if entries is not None:
+        groups = {}
+
+    # one matrix and a row-major output view: the device result is copied
+    # straight into values_output
     direct = None
-    if len(groups) == 1 and v_out_view.flags.c_contiguous and v_out_view.dtype == out_np_dtype:
-        direct = v_out_view.reshape(flat.size, n_out)
-    result = None if direct is not None else np.empty((flat.size, n_out), dtype=out_np_dtype)
+    if (len(groups) == 1 or entries is not None) and v_out_view.flags.c_contiguous and \
+            v_out_view.dtype == out_np_dtype:
+        direct = v_out_view.reshape(v_in.shape[0], n_out)
+    result = None if direct is not None else np.empty((v_in.shape[0], n_out), dtype=out_np_dtype)
+    if entries is not None:
+        _apply_blocks(entries, n_in, n_out, element, v_in, in_dtype, result if direct is None else direct, accumulate)
     d_all = None
     if len(groups) == 1:
         d_all = _device.upload(v_in, in_dtype)
@@ -162,6 +190,68 @@ def regrid_from_weights(
     return values_output << unit
 
 
+# Saved 1D elements of up to this many entries on average are applied as one
+# block diagonal matrix, uploaded on each call: an element of its own takes
+# about 0.2 ms (with its device copy kept) to 0.45 ms of launches and copies,
+# and the upload of 16384 entries about 0.1 ms.
+SHORT_ELEMENT = 16384
+
+
+def _short_elements(flat: np.ndarray, groups: dict, first: dict):
+    """The short saved elements of ``groups`` as device :class:`Entries` and
+    the element of every flat slice, or ``(None, None)`` where they are long
+    or few or not used by equally many slices."""
+    if len(groups) < 4 or len({len(rows) for rows in groups.values()}) > 1:
+        return None, None
+    elements = [flat[first[key]] for key in groups]
+    if any(isinstance(e, _DeviceElement) for e in elements):
+        return None, None
+    arrays = [(np.asarray(ii), np.asarray(oo), np.asarray(getattr(vv, "value", vv), dtype=np.float64))
+              for ii, oo, vv in elements]
+    count = np.array([vv.size for *_, vv in arrays], dtype=np.int64)
+    stride = int(count.max())
+    if stride * len(arrays) > 2 * int(count.sum()) or count.mean() > SHORT_ELEMENT or any(
+            a.ndim != 1 or a.size != c for e, c in zip(arrays, count) for a in e):
+        return None, None
+    element = np.empty(flat.size, dtype=np.int64)
+    for k, rows in enumerate(groups.values()):
+        element[rows] = k
+    host = [np.zeros((len(arrays), stride), dtype=dtype) for dtype in (np.int64, np.int64, np.float64)]
+    for k, e in enumerate(arrays):
+        for h, a in zip(host, e):
+            h[k, :a.size] = a
+    return Entries(*(_device.upload(h) for h in host), _device.upload(count), (len(arrays),)), element
+
+
+def _apply_blocks(entries, n_in: int, n_out: int, element: np.ndarray, v_in: np.ndarray, in_dtype, out: np.ndarray,
+                  accumulate: str) -> None:
+    """Slice ``d`` of ``v_in`` through element ``element[d]`` of the device
+    ``entries`` into ``out[d]``: block diagonal matrices over as many
+    elements as 2^31 cells hold, each with one apply.  (The elements one by
+    one, 256 spectra of 512 -> 384 cells: 118 ms.)"""
+    t = _device.torch()
+    if element.size == 0:
+        return
+    nd, stride = entries.ind_in.shape
+    most = max(1, min((2**31 - 2) // max(n_in, n_out, 1), (2**32 - 2) // max(stride, 1)))
+    # slices of an element side by side: (slices, elements)
+    order = np.argsort(element, kind="stable").reshape(nd, -1)
+    for d in range(0, nd, most):
+        rows = order[d:d + most].T
+        count = None if entries.count is None else entries.count[d:d + most]
+        dw = _device.DeviceWeights.block_diagonal(entries.ind_in[d:d + most], entries.ind_out[d:d + most],
+                                                  entries.val[d:d + most], count, n_in, n_out)
+        whole = rows.size == element.size and np.array_equal(rows.reshape(-1), np.arange(element.size))
+        src = _device.upload(v_in if whole else v_in[rows.reshape(-1)], in_dtype)
+        dst = t.empty((rows.shape[0], rows.shape[1] * n_out), dtype=_device.torch_dtype(out.dtype), device="cuda")
+        dw.apply(src.reshape(rows.shape[0], -1), out=dst, accumulate=accumulate)
+        if whole:
+            t.from_numpy(out).copy_(dst.reshape(-1, n_out))
+        else:
+            out[rows.reshape(-1)] = _device.download(dst).reshape(-1, n_out)
+        dw.free()
+
+
 class _DeviceElement:
     """Stand-in for a saved-layout element whose weights live only on the GPU."""
 
@@ -194,10 +284,11 @@ def regrid(
     the weights through host memory; the result is bit-identical to
     ``regrid_from_weights(*weights(...), ...)``.
     """
-    device_only = method == "conservative"
     array, shape_in, shape_out, dev = _weights_device(
         coordinates_input, coordinates_output, axis_input, axis_output, None, method, bounds, perturb, seed,
-        want_host=not device_only)
+        want_host=False)
+    if isinstance(dev, Entries):
+        return _apply(dev, shape_in, shape_out, values_input, values_output, axis_input, axis_output, accumulate)
     if array is None:
         # 2D conservative: one device matrix per orthogonal element
         *_, shape_orth = _util.normalize_input_output_coordinates(

@@ -51,7 +51,9 @@ def weights(
 def _weights_device(coordinates_input, coordinates_output, axis_input, axis_output, weights_input, method,
                     bounds, perturb, seed, want_host: bool):
     """Build and return ``(array, shape_input, shape_output, device)`` where
-    ``device`` lists a :class:`DeviceWeights` per flat element (or None)."""
+    ``device`` lists a :class:`DeviceWeights` per flat element (or None).
+    Without ``want_host`` the array is None and the device part of 1D
+    weights is their :class:`Entries`."""
     unit_weights = getattr(weights_input, "unit", None)
     if unit_weights is not None:
         weights_input = getattr(weights_input, "value")
@@ -59,7 +61,7 @@ def _weights_device(coordinates_input, coordinates_output, axis_input, axis_outp
     if method == "multilinear":
         array, shape_in, shape_out, dev = _multilinear(
             coordinates_input, coordinates_output, axis_input, axis_output, weights_input, bounds, perturb,
-            seed)
+            seed, want_host)
     elif method == "conservative":
         array, shape_in, shape_out, dev = _conservative(
             coordinates_input, coordinates_output, axis_input, axis_output, weights_input, perturb, seed,
@@ -73,6 +75,16 @@ def _weights_device(coordinates_input, coordinates_output, axis_input, axis_outp
             ii, oo, vv = flat[k]
             flat[k] = (ii, oo, vv << unit_weights)
     return array, shape_in, shape_out, dev
+
+
+class Entries:
+    """Saved-layout entries of the flat elements of ``shape``, on the device:
+    (elements, stride) arrays, ``count`` of each row valid (None: all)."""
+
+    __slots__ = ("ind_in", "ind_out", "val", "count", "shape")
+
+    def __init__(self, ind_in, ind_out, val, count, shape):
+        self.ind_in, self.ind_out, self.val, self.count, self.shape = ind_in, ind_out, val, count, shape
 
 
 def _elements(nd: int, h_in, h_out, h_val, counts) -> np.ndarray:
@@ -126,7 +138,7 @@ def _conservative(ci, co, axis_input, axis_output, weights_input, perturb, seed,
         weights_input = np.broadcast_to(weights_input, shape_values_input)
 
     if len(axi) == 1:
-        array, dev = _conservative_1d(ci[0], co[0], axi, axo, weights_input, shape_orth)
+        array, dev = _conservative_1d(ci[0], co[0], axi, axo, weights_input, shape_orth, want_host)
         return array, shape_values_input, shape_values_output, dev
 
     array = np.empty(shape_orth, dtype=object)
@@ -158,7 +170,7 @@ def _conservative(ci, co, axis_input, axis_output, weights_input, perturb, seed,
     return (array if want_host else None), shape_values_input, shape_values_output, dev
 
 
-def _conservative_1d(x_in, x_out, axi, axo, weights_input, shape_orth):
+def _conservative_1d(x_in, x_out, axi, axo, weights_input, shape_orth, want_host):
     m = x_in.shape[axi[0]]
     n = x_out.shape[axo[0]]
     xi, si, nd = _rows(x_in, axi, m)
@@ -180,6 +192,8 @@ def _conservative_1d(x_in, x_out, axi, axo, weights_input, shape_orth):
     _lib.call("rg_conservative_1d", _device.ptr(d_xi), si, m, _device.ptr(d_xo), so, n, nd, _device.ptr(d_wi),
               sw, cap, _device.ptr(ind_in), _device.ptr(ind_out), _device.ptr(val), _device.ptr(count),
               _device.stream())
+    if not want_host:
+        return None, Entries(ind_in, ind_out, val, count, shape_orth)
     h_in, h_out, h_val, h_cnt = (_device.download(a) for a in (ind_in, ind_out, val, count))
     return _elements(nd, h_in, h_out, h_val, h_cnt.tolist()).reshape(shape_orth), [None] * nd
 
@@ -189,7 +203,7 @@ def _conservative_1d(x_in, x_out, axi, axo, weights_input, shape_orth):
 # ---------------------------------------------------------------------------
 
 
-def _multilinear(ci, co, axis_input, axis_output, weights_input, bounds, perturb, seed):
+def _multilinear(ci, co, axis_input, axis_output, weights_input, bounds, perturb, seed, want_host):
     # the cell search (find_indices, searchsorted) sees unperturbed coordinates
     ci_s, co_s, axi_s, axo_s, *_ = _util.normalize_input_output_coordinates(ci, co, axis_input, axis_output)
     if len(axi_s) != 1:
@@ -237,6 +251,8 @@ def _multilinear(ci, co, axis_input, axis_output, weights_input, bounds, perturb
     if bounds == "raise" and n_out.value:
         raise ValueError(
             f"{n_out.value} of the output points fall outside the input grid, and {bounds=}.")
+    if not want_host:
+        return None, shape_in, shape_out, Entries(ind_in, ind_out, val, None, shape_orth)
     h_in, h_out, h_val = (_device.download(a) for a in (ind_in, ind_out, val))
     return _elements(nd, h_in, h_out, h_val, [h_in.shape[1]] * nd).reshape(shape_orth), shape_in, shape_out, \
         [None] * nd

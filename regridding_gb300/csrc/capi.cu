@@ -42,13 +42,46 @@ int transpose_conservative_scale(const int64_t*, const int64_t*, const double*, 
 
 namespace {
 
-// entries of a COO list normalised to [0, n) (numpy-style negative indices)
-__global__ void normalise_coo(const int64_t* in, const int64_t* out, int64_t nnz, int64_t n_in,
-                              int64_t n_out, int32_t* in32, int32_t* out32, int64_t* pos,
-                              unsigned* bad) {
+// COO entries of one matrix (nd = 1) or of the nd blocks of a block diagonal
+// one: those of block d start at d * stride, and at place first[d] of all
+// entries (first null: d * stride, every block has `stride` of them).
+struct CooRows {
+    const int64_t *in, *out;
+    const double* val;
+    const int64_t* first;  // [nd + 1]
+    int64_t nd, stride;
+};
+
+// block and source of entry k
+__device__ __forceinline__ int64_t coo_source(const CooRows& C, int64_t k, int64_t* block) {
+    int64_t d = 0;
+    if (C.nd > 1 || C.first) {
+        if (C.first) {
+            int64_t lo = 0, hi = C.nd - 1;  // the last d with first[d] <= k
+            while (lo < hi) {
+                const int64_t mid = (lo + hi + 1) >> 1;
+                if (C.first[mid] <= k) lo = mid;
+                else hi = mid - 1;
+            }
+            d = lo;
+            k -= C.first[d];
+        } else {
+            d = k / C.stride;
+            k -= d * C.stride;
+        }
+    }
+    *block = d;
+    return d * C.stride + k;
+}
+
+// entries normalised to [0, n) (numpy-style negative indices), n cells a block
+__global__ void normalise_coo(CooRows C, int64_t nnz, int64_t n_in, int64_t n_out, int32_t* in32, int32_t* out32,
+                              int64_t* pos, unsigned* bad) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz;
          k += (int64_t)gridDim.x * blockDim.x) {
-        int64_t i = in[k], o = out[k];
+        int64_t d;
+        const int64_t src = coo_source(C, k, &d);
+        int64_t i = C.in[src], o = C.out[src];
         if (i < 0) i += n_in;
         if (o < 0) o += n_out;
         if (i < 0 || i >= n_in || o < 0 || o >= n_out) {
@@ -56,19 +89,20 @@ __global__ void normalise_coo(const int64_t* in, const int64_t* out, int64_t nnz
             i = 0;
             o = 0;
         }
-        in32[k] = (int32_t)i;
-        out32[k] = (int32_t)o;
+        in32[k] = (int32_t)(d * n_in + i);
+        out32[k] = (int32_t)(d * n_out + o);
         pos[k] = k;
     }
 }
 
-__global__ void gather_csr(const uint32_t* perm, const int32_t* in32, const double* val, int64_t nnz,
-                           int32_t* col, double* cval) {
+__global__ void gather_csr(const uint32_t* perm, const int32_t* in32, CooRows C, int64_t nnz, int32_t* col,
+                           double* cval) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz;
          k += (int64_t)gridDim.x * blockDim.x) {
         uint32_t e = perm[k];
+        int64_t d;
         col[k] = in32[e];
-        cval[k] = val[e];
+        cval[k] = C.val[coo_source(C, e, &d)];
     }
 }
 
@@ -178,6 +212,65 @@ void free_weights(rg_weights_s* W, cudaStream_t s) {
     dfree(W->ff_perm, s);
     dfree(W->dflags, s);
     delete W;
+}
+
+// Handle of nnz entries over C.nd blocks of n_out x n_in cells.
+int weights_from_entries(const CooRows& C, int64_t nnz, int64_t n_in, int64_t n_out, cudaStream_t s, rg_weights* out) {
+    *out = nullptr;
+    rg_weights_s* W = new (std::nothrow) rg_weights_s();
+    RG_CHECK(W, RG_ERR_ALLOC, "host allocation failed");
+    cudaGetDevice(&W->device);
+    const int64_t rows = C.nd * n_out;
+    W->n_in = C.nd * n_in;
+    W->n_out = rows;
+    W->nnz = nnz;
+    int32_t *in32 = nullptr, *out32 = nullptr;
+    int64_t* pos = nullptr;
+    uint32_t* perm = nullptr;
+    unsigned* bad = nullptr;
+    int st = RG_OK;
+    do {
+        if ((st = dalloc(&in32, (size_t)nnz, s))) break;
+        if ((st = dalloc(&out32, (size_t)nnz, s))) break;
+        if ((st = dalloc(&pos, (size_t)nnz, s))) break;
+        if ((st = dalloc(&perm, (size_t)nnz, s))) break;
+        if ((st = dalloc(&bad, 1, s))) break;
+        if ((st = dalloc(&W->row_ptr, (size_t)rows + 1, s))) break;
+        if ((st = dalloc(&W->col, (size_t)nnz, s))) break;
+        if ((st = dalloc(&W->val, (size_t)nnz, s))) break;
+        cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
+        if (nnz > 0)
+            normalise_coo<<<capped(nnz, 256), 256, 0, s>>>(C, nnz, n_in, n_out, in32, out32, pos, bad);
+        if (rows > 0) {
+            if ((st = bucket_sort(out32, pos, nnz, rows, W->row_ptr, perm, nullptr, s))) break;
+        } else {
+            cudaMemsetAsync(W->row_ptr, 0, sizeof(int64_t), s);
+        }
+        if (nnz > 0) gather_csr<<<capped(nnz, 256), 256, 0, s>>>(perm, in32, C, nnz, W->col, W->val);
+        unsigned hbad = 0;
+        small_to_host(&hbad, bad, sizeof(unsigned), s);
+        cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            set_error("rg_weights_from_coo: %s", cudaGetErrorString(e));
+            st = RG_ERR_CUDA;
+            break;
+        }
+        if (hbad) {
+            set_error("rg_weights_from_coo: an index is out of range for the given shapes");
+            st = RG_ERR_ARG;
+        }
+    } while (0);
+    dfree(in32, s);
+    dfree(out32, s);
+    dfree(pos, s);
+    dfree(perm, s);
+    dfree(bad, s);
+    if (st) {
+        free_weights(W, s);
+        return st;
+    }
+    *out = W;
+    return RG_OK;
 }
 
 }  // namespace
@@ -426,62 +519,35 @@ int rg_weights_from_coo(const int64_t* d_in, const int64_t* d_out, const double*
     RG_CHECK(nnz >= 0 && n_in >= 0 && n_out >= 0, RG_ERR_ARG, "rg_weights_from_coo: negative size");
     RG_CHECK(n_in < INT32_MAX && n_out < INT32_MAX, RG_ERR_UNSUPPORTED,
              "rg_weights_from_coo: more than 2^31 cells");
+    return weights_from_entries(CooRows{d_in, d_out, d_val, nullptr, 1, nnz}, nnz, n_in, n_out, (cudaStream_t)stream,
+                                out);
+}
+
+int rg_weights_block_diagonal(const int64_t* d_in, const int64_t* d_out, const double* d_val, const int64_t* d_count,
+                              int64_t nd, int64_t stride, int64_t n_in, int64_t n_out, rg_stream_t stream,
+                              rg_weights* out) {
+    rg::NvtxRange nvtx_range("rg_weights_block_diagonal");
+    RG_CHECK(out, RG_ERR_ARG, "rg_weights_block_diagonal: out is NULL");
+    RG_CHECK(nd >= 1 && stride >= 0 && n_in >= 0 && n_out >= 0, RG_ERR_ARG, "rg_weights_block_diagonal: bad size");
+    RG_CHECK(nd * n_in < INT32_MAX && nd * n_out < INT32_MAX && nd * stride < (int64_t)UINT32_MAX, RG_ERR_UNSUPPORTED,
+             "rg_weights_block_diagonal: more than 2^31 cells or 2^32 entries");
     *out = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
-    rg_weights_s* W = new (std::nothrow) rg_weights_s();
-    RG_CHECK(W, RG_ERR_ALLOC, "host allocation failed");
-    cudaGetDevice(&W->device);
-    W->n_in = n_in;
-    W->n_out = n_out;
-    W->nnz = nnz;
-    int32_t *in32 = nullptr, *out32 = nullptr;
-    int64_t* pos = nullptr;
-    uint32_t* perm = nullptr;
-    unsigned* bad = nullptr;
-    int st = RG_OK;
-    do {
-        if ((st = dalloc(&in32, (size_t)nnz, s))) break;
-        if ((st = dalloc(&out32, (size_t)nnz, s))) break;
-        if ((st = dalloc(&pos, (size_t)nnz, s))) break;
-        if ((st = dalloc(&perm, (size_t)nnz, s))) break;
-        if ((st = dalloc(&bad, 1, s))) break;
-        if ((st = dalloc(&W->row_ptr, (size_t)n_out + 1, s))) break;
-        if ((st = dalloc(&W->col, (size_t)nnz, s))) break;
-        if ((st = dalloc(&W->val, (size_t)nnz, s))) break;
-        cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
-        if (nnz > 0)
-            normalise_coo<<<capped(nnz, 256), 256, 0, s>>>(d_in, d_out, nnz, n_in, n_out, in32, out32, pos,
-                                                          bad);
-        if (n_out > 0) {
-            if ((st = bucket_sort(out32, pos, nnz, n_out, W->row_ptr, perm, nullptr, s))) break;
-        } else {
-            cudaMemsetAsync(W->row_ptr, 0, sizeof(int64_t), s);
-        }
-        if (nnz > 0) gather_csr<<<capped(nnz, 256), 256, 0, s>>>(perm, in32, d_val, nnz, W->col, W->val);
-        unsigned hbad = 0;
-        small_to_host(&hbad, bad, sizeof(unsigned), s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_error("rg_weights_from_coo: %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
-            break;
-        }
-        if (hbad) {
-            set_error("rg_weights_from_coo: an index is out of range for the given shapes");
-            st = RG_ERR_ARG;
-        }
-    } while (0);
-    dfree(in32, s);
-    dfree(out32, s);
-    dfree(pos, s);
-    dfree(perm, s);
-    dfree(bad, s);
-    if (st) {
-        free_weights(W, s);
-        return st;
+    if (d_count == nullptr)
+        return weights_from_entries(CooRows{d_in, d_out, d_val, nullptr, nd, stride}, nd * stride, n_in, n_out, s, out);
+    int64_t* first = nullptr;  // of every row's entries, and their total
+    int64_t nnz = 0;
+    int st = dalloc(&first, (size_t)nd + 1, s);
+    if (st == RG_OK) st = exclusive_scan_i64(d_count, first, nd, first + nd, s);
+    if (st == RG_OK) st = small_to_host(&nnz, first + nd, sizeof(int64_t), s);
+    if (st == RG_OK && cudaStreamSynchronize(s) != cudaSuccess) {
+        set_error("rg_weights_block_diagonal: %s", cudaGetErrorString(cudaGetLastError()));
+        st = RG_ERR_CUDA;
     }
-    *out = W;
-    return RG_OK;
+    if (st == RG_OK)
+        st = weights_from_entries(CooRows{d_in, d_out, d_val, first, nd, stride}, nnz, n_in, n_out, s, out);
+    dfree(first, s);
+    return st;
 }
 
 int rg_weights_info(rg_weights w, int64_t* nnz, int64_t* n_in, int64_t* n_out) {

@@ -1,5 +1,6 @@
 // 1D kernels: find_indices (brute and searchsorted), multilinear weights and
 // conservative 1D weights over batches of rows.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -134,51 +135,75 @@ __global__ void gather_multilinear(const uint32_t* __restrict__ perm, const int3
     }
 }
 
-// One thread per row: _weights_conservative_1d
-// (_weights_conservative_1d.py:59-318).  Grids are read through index maps
-// instead of reversed copies.  Raw entries go to [d*cap, d*cap + count).
-__global__ void conservative_1d_kernel(const double* __restrict__ xin, int64_t in_stride, int64_t m,
-                                       const double* __restrict__ xout, int64_t out_stride,
-                                       int64_t n, int64_t nd, const double* __restrict__ w_in,
-                                       int64_t w_stride, int64_t cap, int64_t* __restrict__ ind_in,
-                                       int64_t* __restrict__ ind_out, double* __restrict__ val,
-                                       int64_t* __restrict__ count, unsigned* flags) {
-    int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (d >= nd) return;
-    const double* ai = xin + d * in_stride;
-    const double* ao = xout + d * out_stride;
-    const bool rev_in = !(ai[0] < ai[m - 1]);
-    const bool rev_out = !(ao[0] < ao[n - 1]);
-    auto xs = [&](int64_t k) { return rev_in ? ai[m - 1 - k] : ai[k]; };
-    auto xt = [&](int64_t k) { return rev_out ? ao[n - 1 - k] : ao[k]; };
-    // cell length of the (possibly reversed) sweep grid
-    auto len_in = [&](int64_t k) { return dsub(xs(k + 1), xs(k)); };
-    const double st_left = xt(0), st_right = xt(n - 1);
-    int64_t base = d * cap, cnt = 0;
-    int64_t isw = 0, ist;
-    double p1 = xs(0);
-    bool outside;
+// One row of _weights_conservative_1d (_weights_conservative_1d.py:59-318).
+// Grids are read through index maps instead of reversed copies.
+struct Row1d {
+    const double *in, *out;
+    int64_t m, n;
+    bool rev_in, rev_out;
+    __device__ __forceinline__ double xs(int64_t k) const { return __ldg(in + (rev_in ? m - 1 - k : k)); }
+    __device__ __forceinline__ double xt(int64_t k) const { return __ldg(out + (rev_out ? n - 1 - k : k)); }
+    // weight of the piece p1..p2 of sweep cell isw, with the length of the
+    // (possibly reversed) sweep grid's cell at its saved index (negative
+    // indices wrap, as numpy indexing does)
+    __device__ __forceinline__ double weight(double p1, double p2, int64_t isw, const double* w_in) const {
+        const int64_t li = rev_in ? m - 2 - isw : isw;
+        double ratio = ddiv(dsub(p2, p1), dsub(xs(li + 1), xs(li)));
+        return w_in ? dmul(ratio, w_in[li]) : ratio;
+    }
+};
+
+// first k in [0, n) with at(k) >= v (or > v), at() ascending
+template <typename At>
+__device__ __forceinline__ int64_t first_not_below(const At& at, int64_t n, double v) {
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (at(mid) < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+template <typename At>
+__device__ __forceinline__ int64_t first_above(const At& at, int64_t n, double v) {
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (at(mid) <= v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// The sweep of one row by one thread, for grids that do not rise strictly: its
+// entries in sweep order, then in the saved order.  Every entry moves on in
+// the sweep grid or the static one and none moves back, so pairs are unique,
+// entries of one input are neighbours, and the saved order (by input, then
+// output) is the sweep's, reversed as a whole (reversed input) and within the
+// inputs (one of the grids reversed).
+__device__ int64_t sweep_1d(const Row1d& R, const double* w_in, int64_t cap, int64_t* ind_in, int64_t* ind_out,
+                            double* val, unsigned* flags) {
+    int64_t isw = 0, ist = MAXSIZE, cnt = 0;
+    double p1 = R.xs(0);
+    const double st_left = R.xt(0), st_right = R.xt(R.n - 1);
+    bool outside = true;
     if (st_left == p1) {
         outside = false;
         ist = 0;
     } else if (st_left < p1 && p1 < st_right) {
         outside = false;
-        // index_of_point on the reversed-or-not static grid
-        int64_t l = 0, r = n;
+        int64_t l = 0, r = R.n;
         while (r - l > 1) {
-            int64_t mid = (l + r) / 2;
-            if (xt(mid) > p1) r = mid;
+            const int64_t mid = (l + r) / 2;
+            if (R.xt(mid) > p1) r = mid;
             else l = mid;
         }
         ist = r - 1;
-    } else {
-        outside = true;
-        ist = MAXSIZE;
     }
-    while (isw < m - 1) {
-        double p2 = xs(isw + 1);
+    while (isw < R.m - 1) {
+        double p2 = R.xs(isw + 1);
         if (outside) {
-            double ps = xt(0);
+            const double ps = R.xt(0);
             if (p1 < ps && ps < p2) {
                 ist = 0;
                 p2 = ps;
@@ -190,10 +215,8 @@ __global__ void conservative_1d_kernel(const double* __restrict__ xin, int64_t i
             }
             if (ist < MAXSIZE) outside = false;
         } else {
-            int64_t iin = isw, iout = ist;
-            if (rev_in) iin = ~iin;
-            if (rev_out) iout = ~iout;
-            double ps = xt(ist + 1);
+            const int64_t at_sw = isw, at_st = ist;
+            const double ps = R.xt(ist + 1);
             if (p1 < ps && ps < p2) {
                 ist = ist + 1;
                 p2 = ps;
@@ -203,96 +226,151 @@ __global__ void conservative_1d_kernel(const double* __restrict__ xin, int64_t i
             } else {
                 isw = isw + 1;
             }
-            double length = dsub(p2, p1);
-            // negative indices wrap, as numpy indexing does
-            int64_t li = iin < 0 ? iin + (m - 1) : iin;
-            double ratio = ddiv(length, len_in(li));
-            if (w_in) ratio = dmul(ratio, w_in[d * w_stride + li]);
             if (cnt >= cap) {
                 atomicOr(flags, FLAG_CAPACITY);
                 break;
             }
-            ind_in[base + cnt] = iin;
-            ind_out[base + cnt] = iout;
-            val[base + cnt] = ratio;
+            ind_in[cnt] = R.rev_in ? ~at_sw : at_sw;
+            ind_out[cnt] = R.rev_out ? ~at_st : at_st;
+            val[cnt] = R.weight(p1, p2, at_sw, w_in);
             cnt++;
-            if (!(0 <= ist && ist < n - 1)) break;
+            if (!(0 <= ist && ist < R.n - 1)) break;
         }
         p1 = p2;
     }
-    count[d] = cnt;
-}
-
-// Per-row keys for ordering conservative 1D entries by (input, output):
-// negative (reversed-grid) indices are shifted by the row length, which keeps
-// their order because a row's indices all have the same sign.
-// Unused slots of a row (j >= count) are marked with PAD_INDEX and spread
-// over the row's own buckets with keys that sort after every real entry, so
-// no bucket grows long (the within-bucket ranking of long buckets is the
-// expensive part of the sort); the merge skips them.
-constexpr int64_t PAD_INDEX = INT64_MIN;
-
-__global__ void conservative_1d_keys(int64_t* __restrict__ ind_in,
-                                     const int64_t* __restrict__ ind_out,
-                                     const int64_t* __restrict__ count, int64_t nd, int64_t cap,
-                                     int64_t m, int64_t n, int32_t* __restrict__ bucket,
-                                     int64_t* __restrict__ skey) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nd * cap;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        int64_t d = k / cap, j = k % cap;
-        if (j < count[d]) {
-            int64_t i = ind_in[k];
-            int64_t o = ind_out[k];
-            if (i < 0) i += (m - 1);
-            if (o < 0) o += (n - 1);
-            bucket[k] = (int32_t)(d * (m - 1) + i);
-            skey[k] = (o << 32) | (int64_t)j;
-        } else {
-            ind_in[k] = PAD_INDEX;
-            bucket[k] = (int32_t)(d * (m - 1) + j % (m - 1));
-            skey[k] = ((int64_t)INT32_MAX << 32) | (int64_t)j;
+    auto reverse = [&](int64_t a, int64_t b) {
+        for (b--; a < b; a++, b--) {
+            const int64_t i = ind_in[a], o = ind_out[a];
+            const double v = val[a];
+            ind_in[a] = ind_in[b];
+            ind_out[a] = ind_out[b];
+            val[a] = val[b];
+            ind_in[b] = i;
+            ind_out[b] = o;
+            val[b] = v;
         }
-    }
+    };
+    if (R.rev_in) reverse(0, cnt);
+    if (R.rev_in != R.rev_out)
+        for (int64_t a = 0, b; a < cnt; a = b) {
+            for (b = a + 1; b < cnt && ind_in[b] == ind_in[a]; b++) {
+            }
+            reverse(a, b);
+        }
+    return cnt;
 }
 
-// Thread per row: gather the row's sorted entries and merge equal pairs
-// (add.reduceat association; pairs are unique in practice).
-__global__ void conservative_1d_merge(const uint32_t* __restrict__ perm, const int64_t* __restrict__ bptr,
-                                      const int64_t* __restrict__ in_raw,
-                                      const int64_t* __restrict__ out_raw,
-                                      const double* __restrict__ val_raw, int64_t nd, int64_t m,
-                                      int64_t cap, int64_t* __restrict__ ind_in,
-                                      int64_t* __restrict__ ind_out, double* __restrict__ val,
-                                      int64_t* __restrict__ count) {
-    int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (d >= nd) return;
-    int64_t s = bptr[d * (m - 1)], t = bptr[(d + 1) * (m - 1)];
-    int64_t w = 0;
-    int64_t g = s;
-    while (g < t) {
-        uint32_t e = perm[g];
-        int64_t ii = in_raw[e], oo = out_raw[e];
-        if (ii == PAD_INDEX) {  // unused slot (sorted last in its bucket)
-            g++;
+// One block per row.  Where both grids rise strictly in sweep order, the sweep
+// visits their vertices on the common range in order, a vertex of both once,
+// and emits one entry from each to the next: a merge.  Every vertex finds its
+// place by binary search: that of sweep vertex j is its rank among the sweep
+// vertices plus the static ones before it that are no sweep vertices (before,
+// in rank order), and so on for the static ones, so the entries are written
+// where they are saved, with no sort.  The former thread per row, sort by
+// buckets and thread per row for the merge spent 2.1 ms on 256 rows of 513 and
+// 385 vertices (chains of a few hundred dependent steps); this takes 52 us.
+constexpr int CONS_THREADS = 256;
+
+__global__ void __launch_bounds__(CONS_THREADS)
+    conservative_1d_rows(const double* __restrict__ xin, int64_t in_stride, int64_t m, const double* __restrict__ xout,
+                         int64_t out_stride, int64_t n, int64_t nd, const double* __restrict__ w_in, int64_t w_stride,
+                         int64_t cap, int64_t* __restrict__ ind_in, int64_t* __restrict__ ind_out,
+                         double* __restrict__ val, int64_t* __restrict__ count, int* __restrict__ rank_all,
+                         unsigned* flags) {
+    extern __shared__ int rank_shared[];
+    __shared__ int warp_sum[CONS_THREADS / 32];
+    __shared__ int running;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int64_t d = blockIdx.x; d < nd; d += gridDim.x) {
+        Row1d R{xin + d * in_stride, xout + d * out_stride, m, n, false, false};
+        R.rev_in = !(R.xs(0) < R.xs(m - 1));
+        R.rev_out = !(R.xt(0) < R.xt(n - 1));
+        const double* w_row = w_in ? w_in + d * w_stride : nullptr;
+        int64_t* o_in = ind_in + d * cap;
+        int64_t* o_out = ind_out + d * cap;
+        double* o_val = val + d * cap;
+        bool rises = true;
+        for (int64_t k = t; k + 1 < m; k += CONS_THREADS) rises = rises && R.xs(k) < R.xs(k + 1);
+        for (int64_t k = t; k + 1 < n; k += CONS_THREADS) rises = rises && R.xt(k) < R.xt(k + 1);
+        if (!__syncthreads_and(rises)) {
+            if (t == 0) count[d] = sweep_1d(R, w_row, cap, o_in, o_out, o_val, flags);
             continue;
         }
-        double acc = val_raw[e];
-        // group of equal pairs: first + (sequential from -0.0 over the rest,
-        // exact for the < 8 extra terms a 1D overlap can produce)
-        int64_t h = g + 1;
-        double rest = -0.0;
-        while (h < t && in_raw[perm[h]] == ii && out_raw[perm[h]] == oo) {
-            rest = dadd(rest, val_raw[perm[h]]);
-            h++;
+        const auto xs = [&](int64_t k) { return R.xs(k); };
+        const auto xt = [&](int64_t k) { return R.xt(k); };
+        // rank[k]: static vertices before k that are no sweep vertices
+        int* rank = rank_all ? rank_all + blockIdx.x * (n + 1) : rank_shared;
+        if (t == 0) running = 0;
+        for (int64_t k0 = 0; k0 <= n; k0 += CONS_THREADS) {
+            const int64_t k = k0 + t;
+            int own = 0;
+            if (k < n) {
+                const double v = R.xt(k);
+                const int64_t j = first_not_below(xs, m, v);
+                own = !(j < m && R.xs(j) == v);
+            }
+            int incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            if (lane == 31) warp_sum[warp] = incl;
+            __syncthreads();
+            int before = running;
+            for (int w = 0; w < warp; w++) before += warp_sum[w];
+            if (k <= n) rank[k] = before + incl - own;
+            __syncthreads();
+            if (t == CONS_THREADS - 1) running = before + incl;
         }
-        if (h - g > 1) acc = dadd(acc, rest);
-        ind_in[d * cap + w] = ii;
-        ind_out[d * cap + w] = oo;
-        val[d * cap + w] = acc;
-        w++;
-        g = h;
+        __syncthreads();
+        // the common range: its vertices are places 0 .. entries
+        const double a = fmax(R.xs(0), R.xt(0)), b = fmin(R.xs(m - 1), R.xt(n - 1));
+        const int64_t ja = first_not_below(xs, m, a), ka = first_not_below(xt, n, a);
+        const auto place_before = [&](int64_t j, int64_t k) { return j - ja + rank[k] - rank[ka]; };
+        const int64_t entries = a < b ? place_before(first_not_below(xs, m, b), first_not_below(xt, n, b)) : 0;
+        if (t == 0) {
+            count[d] = entries < cap ? entries : cap;
+            if (entries > cap) atomicOr(flags, FLAG_CAPACITY);
+        }
+        // sweep vertices j >= ja, then the other static vertices k >= ka
+        for (int64_t q = t; q < m + n && entries > 0; q += CONS_THREADS) {
+            int64_t j, k;  // cells that hold the piece from this vertex on
+            double p1;
+            int64_t place;
+            if (q < m) {
+                if (q < ja) continue;
+                j = q;
+                p1 = R.xs(j);
+                if (!(p1 < b)) continue;
+                k = first_above(xt, n, p1) - 1;
+                place = place_before(j, first_not_below(xt, n, p1));
+            } else {
+                k = q - m;
+                if (k < ka || rank[k + 1] == rank[k]) continue;
+                p1 = R.xt(k);
+                if (!(p1 < b)) continue;
+                j = first_above(xs, m, p1) - 1;
+                place = place_before(j + 1, k);
+            }
+            const double p2 = fmin(R.xs(j + 1), R.xt(k + 1));
+            // the saved place: inputs in order of their saved index, each
+            // input's entries in order of their output's
+            const double c1 = fmin(R.xs(j + 1), b);
+            const double c0 = fmax(R.xs(j), a);
+            const int64_t first = place_before(c0 == R.xs(j) ? j : ja, first_not_below(xt, n, c0));
+            const int64_t last = place_before(first_not_below(xs, m, c1), first_not_below(xt, n, c1));
+            int64_t at = place;
+            if (R.rev_in && R.rev_out) at = entries - 1 - place;
+            else if (R.rev_out) at = first + last - 1 - place;
+            else if (R.rev_in) at = entries - last + place - first;
+            if (at >= cap) continue;
+            o_in[at] = R.rev_in ? ~j : j;
+            o_out[at] = R.rev_out ? ~k : k;
+            o_val[at] = R.weight(p1, p2, j, w_row);
+        }
+        __syncthreads();
     }
-    count[d] = w;
 }
 
 __global__ void cell_length_kernel(const double* x, int64_t nd, int64_t n, double* len) {
@@ -417,35 +495,21 @@ int conservative_1d(const double* xin, int64_t in_stride, int64_t m, const doubl
     if (nd <= 0) return RG_OK;
     RG_CHECK(nd * (m - 1) < INT32_MAX && nd * cap < UINT32_MAX, RG_ERR_UNSUPPORTED,
              "conservative 1D: batch too large");
-    int64_t total = nd * cap;
-    int64_t *r_in = nullptr, *r_out = nullptr, *skey = nullptr, *bptr = nullptr;
-    double* r_val = nullptr;
-    int32_t* bucket = nullptr;
-    uint32_t* perm = nullptr;
     unsigned* flags = nullptr;
+    int* rank = nullptr;
     int st = RG_OK;
     do {
-        if ((st = dalloc(&r_in, (size_t)total, s))) break;
-        if ((st = dalloc(&r_out, (size_t)total, s))) break;
-        if ((st = dalloc(&r_val, (size_t)total, s))) break;
         if ((st = dalloc(&flags, 1, s))) break;
-        cudaMemsetAsync(flags, 0, sizeof(unsigned), s);
-        conservative_1d_kernel<<<grid_for(nd, 128), 128, 0, s>>>(xin, in_stride, m, xout, out_stride, n, nd,
-                                                                 w_in, w_stride, cap, r_in, r_out, r_val,
-                                                                 count, flags);
-        if ((st = dalloc(&bucket, (size_t)total, s))) break;
-        if ((st = dalloc(&skey, (size_t)total, s))) break;
-        unsigned g = grid_for(total, 256);
-        if (g > 65536) g = 65536;
-        conservative_1d_keys<<<g, 256, 0, s>>>(r_in, r_out, count, nd, cap, m, n, bucket, skey);
-        int64_t nb = nd * (m - 1);
-        if ((st = dalloc(&bptr, (size_t)nb + 1, s))) break;
-        if ((st = dalloc(&perm, (size_t)total, s))) break;
-        if ((st = bucket_sort(bucket, skey, total, nb, bptr, perm, nullptr, s))) break;
-        conservative_1d_merge<<<grid_for(nd, 128), 128, 0, s>>>(perm, bptr, r_in, r_out, r_val, nd, m, cap,
-                                                                ind_in, ind_out, val, count);
+        if ((st = zero_async(flags, sizeof(unsigned), s))) break;
+        // the ranks of a row's static vertices: shared memory up to 8191 of them
+        const unsigned blocks = (unsigned)std::min<int64_t>(nd, 152 * 8);
+        const size_t shared = n < 8192 ? (size_t)(n + 1) * sizeof(int) : 0;
+        if (shared == 0 && (st = dalloc(&rank, (size_t)blocks * (n + 1), s))) break;
+        conservative_1d_rows<<<blocks, CONS_THREADS, shared, s>>>(xin, in_stride, m, xout, out_stride, n, nd, w_in,
+                                                                  w_stride, cap, ind_in, ind_out, val, count, rank,
+                                                                  flags);
         unsigned fl = 0;
-        cudaMemcpyAsync(&fl, flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+        small_to_host(&fl, flags, sizeof(unsigned), s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             set_error("conservative 1D: %s", cudaGetErrorString(e));
@@ -457,13 +521,7 @@ int conservative_1d(const double* xin, int64_t in_stride, int64_t m, const doubl
             st = RG_ERR_ARG;
         }
     } while (0);
-    dfree(r_in, s);
-    dfree(r_out, s);
-    dfree(r_val, s);
-    dfree(skey, s);
-    dfree(bptr, s);
-    dfree(bucket, s);
-    dfree(perm, s);
+    dfree(rank, s);
     dfree(flags, s);
     return st;
 }
