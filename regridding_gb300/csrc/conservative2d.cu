@@ -278,23 +278,6 @@ __device__ bool cell_contains(const Grid& g, int64_t i, int64_t j, double px, do
     return w != 0;
 }
 
-// _index_of_point_local: _grids.py:282-349
-__device__ void locate_local(const Grid& g, double px, double py, int64_t i0, int64_t j0,
-                             int64_t* oi, int64_t* oj) {
-    int64_t ncx = g.nx - 1, ncy = g.ny - 1;
-    int64_t ia = i0 - 1 > 0 ? i0 - 1 : 0, ib = i0 + 2 < ncx ? i0 + 2 : ncx;
-    int64_t ja = j0 - 1 > 0 ? j0 - 1 : 0, jb = j0 + 2 < ncy ? j0 + 2 : ncy;
-    for (int64_t ii = ia; ii < ib; ii++)
-        for (int64_t jj = ja; jj < jb; jj++)
-            if (cell_contains(g, ii, jj, px, py)) {
-                *oi = ii;
-                *oj = jj;
-                return;
-            }
-    *oi = MAXSIZE;
-    *oj = MAXSIZE;
-}
-
 // _bilinear_interpolation: regridding/_interp_ndarray.py:226-269
 __device__ double bilinear(const double* a, int64_t sx, int64_t sy, double x, double y) {
     int64_t x00 = (int64_t)floor(x), y00 = (int64_t)floor(y);
@@ -312,39 +295,59 @@ __device__ double bilinear(const double* a, int64_t sx, int64_t sy, double x, do
 
 __device__ __forceinline__ bool floor_ok(double v) { return isfinite(v) && fabs(v) < 9.0e18; }
 
-// index_of_point_secant: _grids.py:352-463.  Returns false when the upstream
-// falls back to index_of_point_brute (singular Jacobian, no convergence, or an
-// iterate the upstream could not floor).
-__device__ bool locate_secant(const Grid& g, double px, double py, int64_t* oi, int64_t* oj) {
+// index_of_point_secant: _grids.py:352-463, by one warp (all lanes return the
+// same).  Returns false when the upstream falls back to index_of_point_brute
+// (singular Jacobian, no convergence, or an iterate the upstream could not
+// floor).  An iteration is one chain of dependent FP64 operations, and in one
+// lane its six interpolations and the nine cells of the local search were most
+// of it: lanes 0 to 5 take one interpolation each and lanes 0 to 8 one cell
+// (333 x 257 -> 250 x 193: seats 67 -> 48 us).
+__device__ bool locate_secant_warp(const Grid& g, double px, double py, int64_t* oi, int64_t* oj) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     const double h = 1e-3;
-    int64_t sx = g.nx, sy = g.ny;
+    const int64_t sx = g.nx, sy = g.ny, ncx = sx - 1, ncy = sy - 1;
+    // _index_of_point_local (_grids.py:282-349): the first containing cell of
+    // the 3 x 3 around (i0, j0), rows first
+    auto local = [&](int64_t i0, int64_t j0) {
+        const int64_t ii = i0 - 1 + lane / 3, jj = j0 - 1 + lane % 3;
+        const bool hit = lane < 9 && ii >= 0 && jj >= 0 && ii < ncx && jj < ncy && cell_contains(g, ii, jj, px, py);
+        const unsigned m = __ballot_sync(all, hit);
+        const int k = __ffs(m) - 1;
+        *oi = m ? i0 - 1 + k / 3 : MAXSIZE;
+        *oj = m ? j0 - 1 + k % 3 : MAXSIZE;
+    };
     double i = (double)sx / 2, j = (double)sy / 2;
     for (int it = 0; it < 100; it++) {
-        double xv = bilinear(g.x, sx, sy, i, j);
-        double yv = bilinear(g.y, sx, sy, i, j);
+        // lanes 0, 1: x and y at (i, j); 2, 3: at (i + h, j); 4, 5: at (i, j + h)
+        double v = 0.0;
+        if (lane < 6)
+            v = bilinear(lane & 1 ? g.y : g.x, sx, sy, lane >> 1 == 1 ? dadd(i, h) : i, lane >> 1 == 2 ? dadd(j, h) : j);
         if (!floor_ok(i) || !floor_ok(j)) return false;
-        int64_t i0 = (int64_t)floor(i), j0 = (int64_t)floor(j);
-        double ex = dsub(xv, px), ey = dsub(yv, py);
-        if (i0 >= 0 && j0 >= 0 && i0 < sx - 1 && j0 < sy - 1) {
+        const int64_t i0 = (int64_t)floor(i), j0 = (int64_t)floor(j);
+        const double xv = __shfl_sync(all, v, 0), yv = __shfl_sync(all, v, 1);
+        const double ex = dsub(xv, px), ey = dsub(yv, py);
+        if (i0 >= 0 && j0 >= 0 && i0 < ncx && j0 < ncy) {
             if (cell_contains(g, i0, j0, px, py)) {
-                locate_local(g, px, py, i0, j0, oi, oj);
+                local(i0, j0);
                 return true;
             }
         }
         if (fabs(ex) < 1e-10 && fabs(ey) < 1e-10) {
-            locate_local(g, px, py, i0, j0, oi, oj);
+            local(i0, j0);
             return true;
         }
-        double dx_di = ddiv(dsub(bilinear(g.x, sx, sy, dadd(i, h), j), xv), h);
-        double dx_dj = ddiv(dsub(bilinear(g.x, sx, sy, i, dadd(j, h)), xv), h);
-        double dy_di = ddiv(dsub(bilinear(g.y, sx, sy, dadd(i, h), j), yv), h);
-        double dy_dj = ddiv(dsub(bilinear(g.y, sx, sy, i, dadd(j, h)), yv), h);
-        double det = dsub(dmul(dx_di, dy_dj), dmul(dx_dj, dy_di));
+        // lanes 2, 3: dx/di, dy/di; 4, 5: dx/dj, dy/dj
+        const double slope = ddiv(dsub(v, lane & 1 ? yv : xv), h);
+        const double dx_di = __shfl_sync(all, slope, 2), dy_di = __shfl_sync(all, slope, 3);
+        const double dx_dj = __shfl_sync(all, slope, 4), dy_dj = __shfl_sync(all, slope, 5);
+        const double det = dsub(dmul(dx_di, dy_dj), dmul(dx_dj, dy_di));
         if (det == 0) return false;
-        double di = ddiv(dsub(dmul(dy_dj, ex), dmul(dx_dj, ey)), det);
-        double dj = ddiv(dadd(dmul(-dy_di, ex), dmul(dx_di, ey)), det);
-        i = dsub(i, di);
-        j = dsub(j, dj);
+        // lane 0: the step in i, lane 1: in j
+        const double a = lane & 1 ? dadd(dmul(-dy_di, ex), dmul(dx_di, ey)) : dsub(dmul(dy_dj, ex), dmul(dx_dj, ey));
+        const double step = ddiv(a, det);
+        i = dsub(i, __shfl_sync(all, step, 0));
+        j = dsub(j, __shfl_sync(all, step, 1));
     }
     return false;
 }
@@ -729,10 +732,7 @@ __global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
         for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
         if (w != 0) {
             int64_t i = MAXSIZE, j = MAXSIZE;
-            int ok = 0;
-            if (lane == 0) ok = locate_secant(S.g, x1, y1, &i, &j);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) locate_brute_warp(S.g, x1, y1, &i, &j);
+            if (!locate_secant_warp(S.g, x1, y1, &i, &j)) locate_brute_warp(S.g, x1, y1, &i, &j);
             if (i == MAXSIZE) {
                 // the upstream would index out of range here; report it and
                 // leave the line outside so the walk stays in bounds
@@ -1135,52 +1135,78 @@ __device__ __forceinline__ void chunk_walk_one(const Batch& B, const WalkState* 
     ends[g] = st;
 }
 
-// Chunks are handed out one at a time from a counter: a thread that finishes
-// a short chunk takes the next one instead of idling until the longest chunk
-// of its warp is done (walk lengths differ between chunks).
+// Every thread walks the chunk of its own number, then takes chunks from a
+// counter: a thread that finishes a short chunk takes the next one instead of
+// idling until the longest chunk of its warp is done (walk lengths differ
+// between chunks).  The lanes that come for a chunk together add to the
+// counter once.
 __global__ void __launch_bounds__(64)
     chunk_walk_kernel(Batch B, const WalkState* __restrict__ starts, WalkState* __restrict__ ends,
                       int64_t* __restrict__ counts, int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
                       double* __restrict__ s_val, unsigned long long* __restrict__ next_chunk) {
     const int64_t total = B.chunk_base[B.G];
-    for (;;) {
-        const int64_t g = (int64_t)atomicAdd(next_chunk, 1ull);
-        if (g >= total) return;
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x;
+    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    while (g < total) {
         chunk_walk_one(B, starts, ends, counts, s_in, s_out, s_val, g);
+        if (total <= threads) return;
+        const unsigned here = __activemask(), lane = threadIdx.x & 31u;
+        const unsigned leader = __ffs(here) - 1;
+        unsigned long long base = 0;
+        if (lane == leader) base = atomicAdd(next_chunk, (unsigned long long)__popc(here));
+        base = __shfl_sync(here, base, leader);
+        g = threads + (int64_t)base + __popc(here & ((1u << lane) - 1u));
     }
 }
 
-// One thread per line: walk chunks again, in order, wherever a chunk's start
-// differs from the previous chunk's end.
-__global__ void __launch_bounds__(64)
+// One warp per line: chunks are walked again, in order, wherever a chunk's
+// start differs from the previous chunk's end.  The lanes compare 32 chunks at
+// a time; a chunk walked again changes its own end, so the comparison goes on
+// from the chunk after it.  (A thread per line compared its chunks one dependent
+// load after another: 69 us for the 84 chunks a line of 333 x 257 -> 250 x 193,
+// now 4 us.)
+__global__ void __launch_bounds__(128)
     chunk_repair_kernel(Batch B, WalkState* __restrict__ starts, WalkState* __restrict__ ends,
                         int64_t* __restrict__ counts, int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
                         double* __restrict__ s_val, unsigned long long* __restrict__ n_repaired) {
-    int64_t line = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (line >= B.line_base[B.G]) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t line = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (line >= B.line_base[B.G]) return;  // whole warps
     const int pg = pair_of(B.line_base, B.G, line);
     const SweepParams& P = B.P[pg];
     const ChunkPlan& C = B.C[pg];
     unsigned* flags = B.flags + pg;
     int f = family_of(P, line);
-    const Family F = P.fam[f];
+    const Family& F = P.fam[f];
     const Static& S = P.st[F.st];
     int64_t li = line - F.line_base;
     const int64_t max_steps = 64 * (C.ch + 4 * (S.ncx + S.ncy) + 16);
     int64_t g0 = C.chunk_base[f] + li * C.nc[f];
-    for (int64_t c = 1; c < C.nc[f]; c++) {
-        WalkState prev = ends[g0 + c - 1];
-        WalkState cur = starts[g0 + c];
-        bool same = prev.outside == cur.outside && (prev.outside || (prev.stx == cur.stx && prev.sty == cur.sty));
-        if (same) continue;
-        atomicAdd(n_repaired, 1ull);
-        starts[g0 + c] = prev;
-        WalkState st = prev;
-        int64_t k = li * C.nc[f] + c;
-        int64_t base = C.slot_base[f] + k * C.cap[f];
-        counts[g0 + c] = walk_range<true>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in,
-                                          s_out, s_val, flags, max_steps);
-        ends[g0 + c] = st;
+    for (int64_t c0 = 1; c0 < C.nc[f];) {
+        bool same = true;
+        if (c0 + lane < C.nc[f]) {
+            const WalkState prev = ends[g0 + c0 + lane - 1], cur = starts[g0 + c0 + lane];
+            same = prev.outside == cur.outside && (prev.outside || (prev.stx == cur.stx && prev.sty == cur.sty));
+        }
+        const unsigned differ = __ballot_sync(0xffffffffu, !same);
+        if (!differ) {
+            c0 += 32;
+            continue;
+        }
+        const int64_t c = c0 + __ffs(differ) - 1;
+        if (lane == 0) {
+            atomicAdd(n_repaired, 1ull);
+            const WalkState prev = ends[g0 + c - 1];
+            starts[g0 + c] = prev;
+            WalkState st = prev;
+            int64_t k = li * C.nc[f] + c;
+            int64_t base = C.slot_base[f] + k * C.cap[f];
+            counts[g0 + c] = walk_range<true>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in,
+                                              s_out, s_val, flags, max_steps);
+            ends[g0 + c] = st;
+        }
+        __syncwarp();
+        c0 = c + 1;
     }
 }
 
@@ -1527,11 +1553,7 @@ __global__ void locate_points_kernel(Grid g, const double* px, const double* py,
     if (k >= n) return;
     double x = px[k], y = py[k];
     int64_t i = MAXSIZE, j = MAXSIZE;
-    int ok = 0;
-    if (method == 1) {
-        if (lane == 0) ok = locate_secant(g, x, y, &i, &j);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-    }
+    const bool ok = method == 1 && locate_secant_warp(g, x, y, &i, &j);
     if (!ok) locate_brute_warp(g, x, y, &i, &j);
     if (lane == 0) {
         oi[k] = i;
@@ -1712,7 +1734,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             const unsigned blocks = std::min<unsigned>(grid_for(chunks, 64), 152u * 8u);
             chunk_walk_kernel<<<blocks, 64, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep + 1);
         }
-        chunk_repair_kernel<<<grid_for(lines, 64), 64, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep);
+        chunk_repair_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep);
         zero_async(counts + chunks, sizeof(int64_t), s);
         if ((st = exclusive_scan_i64(counts, offsets, chunks + 1, total_dev, s))) break;
         int64_t nraw = 0;
