@@ -769,10 +769,13 @@ struct WalkState {
 // The body of the prange loop of _sweep_along_axis (:432-533) with
 // _step_outside_static (:547-698), _step_inside_static (:707-895) and
 // _calc_and_save_weights (:903-976) inlined, run on line li from vertex
-// st.sy until the walk reaches vertex j_end.  WRITE stores triples at
-// [wpos, wend); past wend it only counts (and flags the overflow).  Returns
-// the number of triples emitted.
-template <bool WRITE>
+// st.sy until the walk reaches vertex j_end.  EMIT_TRIPLES stores (input cell,
+// output cell, weight) for each of the line's sides at [wpos, wend),
+// EMIT_PIECES one (static cell, sweep segment, area) for both; past wend they
+// only count (and flag the overflow), as EMIT_COUNT does throughout.  Returns
+// the number of triples or pieces.
+constexpr int EMIT_COUNT = 0, EMIT_TRIPLES = 1, EMIT_PIECES = 2;
+template <int EMIT>
 __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Static& S, int64_t li, int64_t j_end,
                               WalkState& state, int64_t wpos, int64_t wend, int32_t* __restrict__ raw_in,
                               int32_t* __restrict__ raw_out, double* __restrict__ raw_val, unsigned* flags,
@@ -937,6 +940,17 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             // negation of area / a_in (times w_in): one division serves both
             double w_static = 0.0;
             bool have_static = false;
+            if constexpr (EMIT == EMIT_PIECES) {
+                if (wpos < wend) {
+                    raw_in[wpos] = (int32_t)(stx * S.ncy + sty);
+                    raw_out[wpos] = (int32_t)sy_idx;
+                    raw_val[wpos] = area;
+                } else {
+                    atomicOr(flags, FLAG_CAPACITY);
+                }
+                wpos++;
+                n_emit++;
+            } else
 #pragma unroll
             for (int side = 0; side < 2; side++) {
                 int64_t is = side == 0 ? li - 1 : li;
@@ -948,7 +962,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 if (F.sweep_input) { ii = a; ij = b; oi = stx; oj = sty; }
                 else { ii = stx; ij = sty; oi = a; oj = b; }
                 int64_t in_flat = ii * P.ncy_in + ij;
-                if (WRITE) {
+                if constexpr (EMIT == EMIT_TRIPLES) {
                     if (wpos < wend) {
                         double w;
                         if (!F.sweep_input && have_static) {
@@ -1009,7 +1023,7 @@ __global__ void __launch_bounds__(64)
     Seat seat = seats[line];
     WalkState state{seat.stx, seat.sty, 0, seat.outside, 0};
     const int64_t max_steps = 64 * (F.len + 4 * (S.ncx + S.ncy) + 16);
-    int64_t n = walk_range<WRITE>(P, F, S, line - F.line_base, F.len - 1, state,
+    int64_t n = walk_range<WRITE ? EMIT_TRIPLES : EMIT_COUNT>(P, F, S, line - F.line_base, F.len - 1, state,
                                   WRITE ? offsets[line] : 0, WRITE ? offsets[line + 1] : 0, raw_in, raw_out,
                                   raw_val, B.flags + pg, max_steps);
     if (!WRITE) counts[line] = n;
@@ -1024,15 +1038,19 @@ __global__ void __launch_bounds__(64)
 // chunked walk: every line is cut into chunks of CH sweep segments that are
 // walked in parallel.  A chunk starts from its vertex located in the static
 // grid; a per-line repair pass then re-walks, in order, every chunk whose
-// start disagrees with the end state of the chunk before it, so the triples
-// are exactly those of one sequential walk per line.
+// start disagrees with the end state of the chunk before it, so the pieces
+// are exactly those of one sequential walk per line.  A piece stands for the
+// triples of both cells that its line separates; their weights are divided
+// out where the triples are ordered, a piece per lane, and not in the walk,
+// whose FP64 instructions run with half their lanes (2048^2 -> 1536^2: walk
+// 4.71 -> 3.86 ms, the two ordering passes 1.38 -> 1.62 ms).
 // ---------------------------------------------------------------------------
 
 struct ChunkPlan {
     int64_t ch;              // sweep segments per chunk
     int64_t nc[4];           // chunks per line, per family
     int64_t chunk_base[5];   // first chunk id of each family (and the total)
-    int64_t cap[4];          // triple slots per chunk, per family
+    int64_t cap[4];          // piece slots per chunk, per family
     int64_t slot_base[4];    // first slot of each family
 };
 
@@ -1130,7 +1148,7 @@ __device__ __forceinline__ void chunk_walk_one(const Batch& B, const WalkState* 
     WalkState st = starts[g];
     int64_t base = C.slot_base[f] + k * C.cap[f];
     const int64_t max_steps = 64 * (C.ch + 4 * (S.ncx + S.ncy) + 16);
-    counts[g] = walk_range<true>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in, s_out,
+    counts[g] = walk_range<EMIT_PIECES>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in, s_out,
                                  s_val, flags, max_steps);
     ends[g] = st;
 }
@@ -1164,7 +1182,7 @@ __global__ void __launch_bounds__(64)
 // a time; a chunk walked again changes its own end, so the comparison goes on
 // from the chunk after it.  (A thread per line compared its chunks one dependent
 // load after another: 69 us for the 84 chunks a line of 333 x 257 -> 250 x 193,
-// now 4 us.)
+// now 6 us.)
 __global__ void __launch_bounds__(128)
     chunk_repair_kernel(Batch B, WalkState* __restrict__ starts, WalkState* __restrict__ ends,
                         int64_t* __restrict__ counts, int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
@@ -1201,7 +1219,7 @@ __global__ void __launch_bounds__(128)
             WalkState st = prev;
             int64_t k = li * C.nc[f] + c;
             int64_t base = C.slot_base[f] + k * C.cap[f];
-            counts[g0 + c] = walk_range<true>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in,
+            counts[g0 + c] = walk_range<EMIT_PIECES>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in,
                                               s_out, s_val, flags, max_steps);
             ends[g0 + c] = st;
         }
@@ -1210,24 +1228,48 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// One warp per chunk: move its triples from its slots to their place in the
-// emission order.
-
 // ---------------------------------------------------------------------------
 // merge (regridding/_weights/_weights_arrays.py:44-73)
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
-// Output-row ordering of the chunked walk's triples, read straight from the
-// chunks' slots (no compacted copy, no index indirection): chunk g's q-th
-// triple has raw position offsets[g] + q (the order of one sequential walk
-// per line), and it goes to the bucket of its output row with the key
-// (input cell << 32 | raw position), so that ordering each row by key gives
-// the same order as the bucket sort of the compacted triples: by input
-// cell, then by raw position.  One warp per chunk in the counting and
-// scattering passes (a chunk's consecutive triples often share a row, and
-// their lanes add to its counter once), one warp per row in the ranking.
+// Output-row ordering of the chunked walk's triples, made from the pieces in
+// the chunks' slots (no compacted copy, no index indirection): piece q of
+// chunk g has raw positions 2 (offsets[g] + q) and the next one for its two
+// triples (the order of one sequential walk per line), and each goes to the
+// bucket of its output row with the key (input cell << 32 | raw position), so
+// that ordering each row by key gives the same order as the bucket sort of the
+// compacted triples: by input cell, then by raw position.  In the counting and
+// scattering passes LANES lanes of a warp take a chunk, a piece per lane (a
+// chunk's consecutive triples often share a row, and their lanes add to its
+// counter once); 8 or 16 where chunks hold few pieces.  One warp per row in the
+// ranking.
 // ---------------------------------------------------------------------------
+
+// What a chunk's pieces share, and the cells of its piece's two triples
+// (_calc_and_save_weights, :903-976): side 0 lies below the line, side 1 above.
+struct PieceLine {
+    const SweepParams* P;
+    const Family* F;
+    int64_t li;
+    __device__ __forceinline__ bool has(int side) const { return side == 0 ? li >= 1 : li < F->lines - 1; }
+    __device__ __forceinline__ void cells(int side, int32_t stat, int32_t seg, int32_t* in, int32_t* out) const {
+        const int64_t is = side == 0 ? li - 1 : li;
+        const int64_t a = F->axis == 0 ? seg : is, b = F->axis == 0 ? is : seg;
+        const int32_t own = (int32_t)(a * (F->sweep_input ? P->ncy_in : P->ncy_out) + b);
+        *in = F->sweep_input ? own : stat;
+        *out = F->sweep_input ? stat : own;
+    }
+};
+
+// the chunk's line, and its first slot
+__device__ __forceinline__ PieceLine piece_line(const Batch& B, int pg, int64_t g, int64_t* base) {
+    const ChunkPlan& C = B.C[pg];
+    const int f = family_of_chunk(C, g);
+    const int64_t k = g - C.chunk_base[f];
+    *base = C.slot_base[f] + k * C.cap[f];
+    return PieceLine{&B.P[pg], &B.P[pg].fam[f], k / C.nc[f]};
+}
 
 __device__ __forceinline__ unsigned warp_row_add(unsigned* counters, int32_t b, bool active) {
     const unsigned lane = threadIdx.x & 31u;
@@ -1240,47 +1282,78 @@ __device__ __forceinline__ unsigned warp_row_add(unsigned* counters, int32_t b, 
     return base + __popc(peers & ((1u << lane) - 1u));
 }
 
-__global__ void slot_count_rows(Batch B, const int64_t* __restrict__ counts, const int32_t* __restrict__ s_out,
-                                unsigned* __restrict__ rows) {
-    const int lane = threadIdx.x & 31;
-    const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (g >= B.chunk_base[B.G]) return;  // warp-uniform
+template <int LANES>
+__global__ void slot_count_rows(Batch B, const int64_t* __restrict__ counts, const int32_t* __restrict__ s_cell,
+                                const int32_t* __restrict__ s_seg, unsigned* __restrict__ rows) {
+    const int lane = threadIdx.x & (LANES - 1);
+    const int64_t total = B.chunk_base[B.G];
+    int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
+    const bool valid = g < total;
+    if (!__any_sync(0xffffffffu, valid)) return;
+    if (!valid) g = total - 1;
     const int pg = pair_of(B.chunk_base, B.G, g);
-    const ChunkPlan& C = B.C[pg];
+    int64_t base;
+    const PieceLine L = piece_line(B, pg, g, &base);
     const int32_t ob = (int32_t)B.out_base[pg];
-    const int f = family_of_chunk(C, g);
-    const int64_t base = C.slot_base[f] + (g - C.chunk_base[f]) * C.cap[f];
-    const int64_t n = counts[g];
-    for (int64_t q0 = 0; q0 < n; q0 += 32) {
-        const int64_t q = q0 + lane;
+    const int64_t n = valid ? counts[g] : 0;
+    for (int64_t q = lane; __any_sync(0xffffffffu, q < n); q += LANES) {
         const bool active = q < n;
-        (void)warp_row_add(rows, active ? s_out[base + q] + ob : 0, active);
+        const int32_t cell = active ? s_cell[base + q] : 0, seg = active ? s_seg[base + q] : 0;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            int32_t in, out;
+            L.cells(side, cell, seg, &in, &out);
+            (void)warp_row_add(rows, active ? out + ob : 0, active && L.has(side));
+        }
     }
 }
 
+template <int LANES>
 __global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
-                                  const int32_t* __restrict__ s_in, const int32_t* __restrict__ s_out,
-                                  const double* __restrict__ s_val, const int64_t* __restrict__ row_start,
+                                  const int32_t* __restrict__ s_cell, const int32_t* __restrict__ s_seg,
+                                  const double* __restrict__ s_area, const int64_t* __restrict__ row_start,
                                   unsigned* __restrict__ cursor, int64_t* __restrict__ tkey,
                                   double* __restrict__ tval) {
-    const int lane = threadIdx.x & 31;
-    const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (g >= B.chunk_base[B.G]) return;  // warp-uniform
+    const int lane = threadIdx.x & (LANES - 1);
+    const int64_t total = B.chunk_base[B.G];
+    int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
+    const bool valid = g < total;
+    if (!__any_sync(0xffffffffu, valid)) return;
+    if (!valid) g = total - 1;
     const int pg = pair_of(B.chunk_base, B.G, g);
-    const ChunkPlan& C = B.C[pg];
+    int64_t base;
+    const PieceLine L = piece_line(B, pg, g, &base);
     const int32_t ob = (int32_t)B.out_base[pg];
-    const int f = family_of_chunk(C, g);
-    const int64_t base = C.slot_base[f] + (g - C.chunk_base[f]) * C.cap[f];
-    const int64_t n = counts[g], raw0 = offsets[g];
-    for (int64_t q0 = 0; q0 < n; q0 += 32) {
-        const int64_t q = q0 + lane;
+    const int64_t n = valid ? counts[g] : 0, raw0 = offsets[g];
+    const double* __restrict__ area_in = L.P->area_in;
+    const double* __restrict__ w_in = L.P->w_in;
+    for (int64_t q = lane; __any_sync(0xffffffffu, q < n); q += LANES) {
         const bool active = q < n;
-        const int32_t b = active ? s_out[base + q] + ob : 0;
-        const unsigned pos = warp_row_add(cursor, b, active);
-        if (active) {
-            const int64_t dst = row_start[b] + pos;
-            tkey[dst] = ((int64_t)s_in[base + q] << 32) | (int64_t)(uint32_t)(raw0 + q);
-            tval[dst] = s_val[base + q];
+        const int32_t cell = active ? s_cell[base + q] : 0, seg = active ? s_seg[base + q] : 0;
+        const double area = active ? s_area[base + q] : 0.0;
+        // a static input grid: both sides share the input cell, and
+        // -area / a_in (times w_in) is exactly the negation of area / a_in
+        // (times w_in): one division serves both
+        double shared = 0.0;
+        if (active && !L.F->sweep_input) {
+            shared = ddiv(area, __ldg(area_in + cell));
+            if (w_in) shared = dmul(shared, __ldg(w_in + cell));
+        }
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            const bool take = active && L.has(side);
+            int32_t in, out;
+            L.cells(side, cell, seg, &in, &out);
+            const unsigned pos = warp_row_add(cursor, take ? out + ob : 0, take);
+            if (!take) continue;
+            double w = side ? -shared : shared;
+            if (L.F->sweep_input) {
+                w = ddiv(side ? -area : area, __ldg(area_in + in));
+                if (w_in) w = dmul(w, __ldg(w_in + in));
+            }
+            const int64_t dst = row_start[out + ob] + pos;
+            tkey[dst] = ((int64_t)in << 32) | (int64_t)(uint32_t)(2 * (raw0 + q) + side);
+            tval[dst] = w;
         }
     }
 }
@@ -1672,7 +1745,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
     }
     *nraw_out = -1;
     if (ch <= 0) return RG_OK;
-    // fault injection for tests: RG_FAULT_CHUNK_SLOTS caps the triple slots
+    // fault injection for tests: RG_FAULT_CHUNK_SLOTS caps the piece slots
     // a chunk gets, so chunks overflow and the build takes its recovery path
     // (whole-line walks, which count exactly); the weights do not change
     int64_t slot_cap = INT64_MAX;
@@ -1697,7 +1770,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             if (!(cross < 1e6)) cross = 1e6;
             c.nc[f] = (F.len - 1 + ch - 1) / ch;
             c.chunk_base[f] = chunks;
-            c.cap[f] = std::min<int64_t>(2 * ch * (1 + (int64_t)cross) + 32, slot_cap);
+            c.cap[f] = std::min<int64_t>(ch * (1 + (int64_t)cross) + 16, slot_cap);
             c.slot_base[f] = slots;
             chunks += F.lines * c.nc[f];
             slots += F.lines * c.nc[f] * c.cap[f];
@@ -1737,10 +1810,11 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         chunk_repair_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep);
         zero_async(counts + chunks, sizeof(int64_t), s);
         if ((st = exclusive_scan_i64(counts, offsets, chunks + 1, total_dev, s))) break;
-        int64_t nraw = 0;
+        int64_t nraw = 0;  // pieces; up to two triples each
         small_to_host(&nraw, total_dev, sizeof(int64_t), s);
         small_to_host(fl.data(), B.flags, sizeof(unsigned) * fl.size(), s);
         cudaError_t e = cudaStreamSynchronize(s);
+        nraw *= 2;
         if (e != cudaSuccess) {
             set_error("conservative sweep (chunked walk): %s", cudaGetErrorString(e));
             st = RG_ERR_CUDA;
@@ -1753,9 +1827,8 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             zero_async(B.flags, sizeof(unsigned) * fl.size(), s);
             break;
         }
-        if (nraw >= (int64_t)UINT32_MAX) {
-            set_error("conservative sweep: %lld raw entries exceed 2^32", (long long)nraw);
-            st = RG_ERR_UNSUPPORTED;
+        if (nraw >= (int64_t)UINT32_MAX) {  // raw positions past 32 bits: the whole-line walk counts the triples
+            overflow = true;
             break;
         }
         {
@@ -1776,11 +1849,18 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 if ((st = dalloc(&tval, (size_t)std::max<int64_t>(nraw, 1), s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
                 zero_async(long_count, sizeof(unsigned), s);
-                slot_count_rows<<<grid_for(chunks * 32, 256), 256, 0, s>>>(B, counts, s_out, rowc);
+                // lanes per chunk for the pieces it holds on average
+                const int64_t mean = nraw / (2 * chunks);
+                const int lanes = mean > 20 ? 32 : mean > 10 ? 16 : 8;
+                const unsigned gc = grid_for(chunks * lanes, 256);
+                const auto count = lanes == 32 ? slot_count_rows<32> : lanes == 16 ? slot_count_rows<16> : slot_count_rows<8>;
+                const auto scatter = lanes == 32   ? slot_scatter_rows<32>
+                                     : lanes == 16 ? slot_scatter_rows<16>
+                                                   : slot_scatter_rows<8>;
+                count<<<gc, 256, 0, s>>>(B, counts, s_in, s_out, rowc);
                 if ((st = exclusive_scan_u32_to_i64(rowc, rows->row_start, nr + 1, nullptr, s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
-                slot_scatter_rows<<<grid_for(chunks * 32, 256), 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val,
-                                                                           rows->row_start, rowc, tkey, tval);
+                scatter<<<gc, 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val, rows->row_start, rowc, tkey, tval);
                 const unsigned gr = grid_for(nr * 32, 256) > 16384 ? 16384 : grid_for(nr * 32, 256);
                 rank_rows<<<gr, 256, 0, s>>>(rows->row_start, nr, tkey, tval, rows->in, rows->val, long_list,
                                              long_count);
