@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "inside.cuh"
 #include "seed.cuh"
 
 namespace rg {
@@ -140,16 +141,6 @@ __device__ __forceinline__ bool seg_hit(double x1, double y1, double x2, double 
 // certain; the walk computes the FP64 determinants of the edge it crosses
 // (its t is needed) and of the rare undecided candidates.
 // ---------------------------------------------------------------------------
-
-// v truncated to float32 from its bits: |v - f| < 2^-23 |v|.  Magnitudes
-// below 2^-126 give 0; magnitudes of 2^128 or more (and inf, NaN) clear ok.
-__device__ __forceinline__ float trunc_float(double v, bool& ok) {
-    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-    const unsigned ah = hi & 0x7fffffffu;
-    ok = ok && ah < 0x47f00000u;
-    const unsigned f = (hi & 0x80000000u) | ((ah - 0x38000000u) << 3) | (lo >> 29);
-    return ah < 0x38100000u ? 0.f : __uint_as_float(f);
-}
 
 // Where q = fl64(n / d) lies against [0, 1), given float32 values nf, df with
 // |nf - n| <= E and |df - d| <= E: 1 inside, 0 outside, -1 undecided.
@@ -262,13 +253,16 @@ struct Grid {
 };
 
 // point_is_inside_polygon on the 4 vertices of cell (i, j) in the order
-// (i,j), (i+1,j), (i+1,j+1), (i,j+1) (_grids.py:251-276)
+// (i,j), (i+1,j), (i+1,j+1), (i,j+1) (_grids.py:251-276), in float32 where
+// that is certain
 __device__ bool cell_contains(const Grid& g, int64_t i, int64_t j, double px, double py) {
     double vx[4], vy[4];
     vx[0] = g.X(i, j);         vy[0] = g.Y(i, j);
     vx[1] = g.X(i + 1, j);     vy[1] = g.Y(i + 1, j);
     vx[2] = g.X(i + 1, j + 1); vy[2] = g.Y(i + 1, j + 1);
     vx[3] = g.X(i, j + 1);     vy[3] = g.Y(i, j + 1);
+    const int dec = quad_contains_filter(vx, vy, px, py);
+    if (dec >= 0) return dec;
     double w = 0;
 #pragma unroll
     for (int v = 0; v < 4; v++) {
@@ -1071,7 +1065,10 @@ __device__ WalkState guess_state(const Static& S, double px, double py, int64_t 
     const Grid& g = S.g;
     const int64_t ncx = S.ncx, ncy = S.ncy;
     int64_t ci, cj;
-    seed_cell(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj);
+    const int single = locate_single(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj);
+    if (single == 1) return WalkState{ci, cj, sy, 0, 0};
+    if (single == 0) return w;
+    seed_cell<false>(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj);
     for (int step = 0; step < 64; step++) {
         if (cell_contains(g, ci, cj, px, py)) {
             w.stx = ci;

@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "inside.cuh"
 #include "seed.cuh"
 
 namespace rg {
@@ -58,14 +59,22 @@ __device__ __forceinline__ double wterm(double x, double y, double vx0, double v
     return 0.0;
 }
 
+struct Cell {
+    double vx[4], vy[4];
+    __device__ __forceinline__ Cell(const G2& g, int64_t i, int64_t j)
+        : vx{g.X(i, j), g.X(i + 1, j), g.X(i + 1, j + 1), g.X(i, j + 1)},
+          vy{g.Y(i, j), g.Y(i + 1, j), g.Y(i + 1, j + 1), g.Y(i, j + 1)} {}
+};
+
 __device__ bool contains(const G2& g, int64_t i, int64_t j, double px, double py) {
-    double vx[4] = {g.X(i, j), g.X(i + 1, j), g.X(i + 1, j + 1), g.X(i, j + 1)};
-    double vy[4] = {g.Y(i, j), g.Y(i + 1, j), g.Y(i + 1, j + 1), g.Y(i, j + 1)};
+    const Cell c(g, i, j);
+    const int dec = quad_contains_filter(c.vx, c.vy, px, py);
+    if (dec >= 0) return dec;
     double w = 0;
 #pragma unroll
     for (int v = 0; v < 4; v++) {
         int p = (v + 3) & 3;
-        w = w + wterm(px, py, vx[p], vy[p], vx[v], vy[v]);
+        w = w + wterm(px, py, c.vx[p], c.vy[p], c.vx[v], c.vy[v]);
     }
     return w != 0;
 }
@@ -94,9 +103,23 @@ __global__ void __launch_bounds__(128)
     if (k >= n) return;
     const int64_t ncx = g.nx - 1, ncy = g.ny - 1;
     const double p_x = px[k], p_y = py[k];
-    // starting guess: Newton on the bilinear index map (float32)
+    // nearly every point is settled in float32: inside a cell, or (a walk that
+    // left the grid) left to the winding number of the boundary; the others
+    // start again with float64 decisions
     int64_t ci, cj;
-    seed_cell(g.x, g.y, g.nx, g.ny, p_x, p_y, &ci, &cj);
+    const int single = locate_single(g.x, g.y, g.nx, g.ny, p_x, p_y, &ci, &cj);
+    if (single == 1) {
+        int64_t ri, rj;
+        lowest_local(g, p_x, p_y, ci, cj, &ri, &rj);
+        oi[k] = ri;
+        oj[k] = rj;
+        return;
+    }
+    if (single == 0) {
+        fails[atomicAdd(nfail, 1ull)] = k;
+        return;
+    }
+    seed_cell<false>(g.x, g.y, g.nx, g.ny, p_x, p_y, &ci, &cj);
     const int cap = 64 + 2 * (int)sqrt((double)(ncx + ncy));
     for (int step = 0; step < cap; step++) {
         if (contains(g, ci, cj, p_x, p_y)) {
