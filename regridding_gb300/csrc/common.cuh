@@ -158,8 +158,9 @@ struct FastDiv {
 // transfers (a 512^2 build took 6-9 ms instead of 1.3 ms next to a stream
 // copying 600 MB blocks); elsewhere cudaMemcpyAsync.  small_to_host is
 // stream-ordered: read the destination after synchronising the stream.
-// small_to_device returns once the source has been read (it synchronises the
-// stream when a kernel did the copy), so the source may be freed at once.
+// small_to_device returns once the source has been read (with the launch up to
+// 15 KB; above, it synchronises the stream when a kernel did the copy), so the
+// source may be freed at once.
 bool kernel_host_access();
 // cudaMemsetAsync(p, 0, n, s) as a kernel, for the small clears of the build
 int zero_async(void* p, size_t n, cudaStream_t s);

@@ -240,7 +240,7 @@ __device__ __forceinline__ int ybin(const YBins& b, double v) {
 
 // one block: y-range of the boundary vertices -> bin parameters
 __global__ void ybins_params(G2 g, int64_t nb, int nbins, YBins* out) {
-    __shared__ double smin[256], smax[256];
+    __shared__ double smin[1024], smax[1024];
     double lo = INFINITY, hi = -INFINITY;
     for (int64_t v = threadIdx.x; v < nb; v += blockDim.x) {
         double bx, by;
@@ -402,7 +402,7 @@ int locate_2d_walk(const double* x, const double* y, int64_t nx, int64_t ny, con
         cudaMemsetAsync(overflow, 0, sizeof(unsigned), s);
         G2 g{x, y, nx, ny};
         const unsigned eb = grid_for(nb, 128) > 1024 ? 1024 : grid_for(nb, 128);
-        ybins_params<<<1, 256, 0, s>>>(g, nb, nbins, bp);
+        ybins_params<<<1, 1024, 0, s>>>(g, nb, nbins, bp);
         ybins_fill<0><<<eb, 128, 0, s>>>(g, nb, bp, counts, nullptr, nullptr, cap, overflow);
         if ((st = exclusive_scan_u32_to_i64(counts, ptr, nbins + 1, total, s))) break;
         cudaMemsetAsync(counts, 0, sizeof(unsigned) * (nbins + 1), s);
