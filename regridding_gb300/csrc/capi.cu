@@ -338,10 +338,12 @@ __global__ void host_bytes_copy(unsigned char* __restrict__ dst, const unsigned 
 
 // Bytes that travel with the launch, as a kernel's argument: the source is
 // read when the launch is issued, so nothing waits for the device.
+template <int WORDS>
 struct ArgBytes {
-    unsigned long long w[496];  // 3968 bytes: the arguments of one launch stay under 4 KB
+    unsigned long long w[WORDS];
 };
-__global__ void store_bytes(unsigned char* __restrict__ dst, const __grid_constant__ ArgBytes src, unsigned n) {
+template <int WORDS>
+__global__ void store_bytes(unsigned char* __restrict__ dst, const __grid_constant__ ArgBytes<WORDS> src, unsigned n) {
     if ((((uintptr_t)dst | n) & 7) == 0) {
         for (unsigned k = threadIdx.x; k < n / 8; k += blockDim.x) ((unsigned long long*)dst)[k] = src.w[k];
     } else {
@@ -415,15 +417,24 @@ int small_to_host(void* h_dst, const void* d_src, size_t n, cudaStream_t s) {
 
 int small_to_device(void* d_dst, const void* h_src, size_t n, cudaStream_t s) {
     if (n == 0) return RG_OK;
-    // up to four launches that carry the bytes (2 us each, not waited for);
-    // above, a kernel that reads the host array costs a synchronisation (about
-    // 13 us, and eight of them in a build of one pair)
-    ArgBytes arg;
-    if (n <= 4 * sizeof(arg)) {
-        for (size_t k = 0; k < n; k += sizeof(arg)) {
-            const size_t m = n - k < sizeof(arg) ? n - k : sizeof(arg);
+    // up to 3968 bytes (arguments below 4 KB), and up to three launches of 32000
+    // (below the 32764 bytes a launch may carry), are not waited for; a kernel
+    // that reads the host array costs a synchronisation (13 us for a few bytes,
+    // of which a build of one pair had eight; 45 us for 34 KB)
+    constexpr size_t SMALL = 496 * 8, LARGE = 4000 * 8;
+    if (n <= SMALL) {
+        ArgBytes<496> arg;
+        memcpy(arg.w, h_src, n);
+        store_bytes<496><<<1, 256, 0, s>>>((unsigned char*)d_dst, arg, (unsigned)n);
+        RG_CUDA(cudaGetLastError());
+        return RG_OK;
+    }
+    if (n <= 3 * LARGE) {
+        ArgBytes<4000> arg;
+        for (size_t k = 0; k < n; k += LARGE) {
+            const size_t m = n - k < LARGE ? n - k : LARGE;
             memcpy(arg.w, (const char*)h_src + k, m);
-            store_bytes<<<1, 256, 0, s>>>((unsigned char*)d_dst + k, arg, (unsigned)m);
+            store_bytes<4000><<<1, 1024, 0, s>>>((unsigned char*)d_dst + k, arg, (unsigned)m);
         }
         RG_CUDA(cudaGetLastError());
         return RG_OK;

@@ -506,33 +506,46 @@ __global__ void cell_area_batch(const PrepGrid* __restrict__ P, int G, int64_t n
 // any order, so the partition does not matter).
 __global__ void __launch_bounds__(256) bbox_partial_batch(const PrepGrid* __restrict__ P, int nparts,
                                                           double* __restrict__ part) {
-    __shared__ double sh[4][256];
+    __shared__ long long sh[4][8];
     const int k = blockIdx.x / nparts, p = blockIdx.x % nparts;
     const Grid g = P[k].g;
     const int64_t n = g.nx * g.ny;
-    double a = INFINITY, b = INFINITY, c = -INFINITY, d = -INFINITY;
+    // extrema of the order keys (no FP64 instruction); NaN is left out, and
+    // no vertex gives the infinities
+    long long a = order_key(INFINITY), b = a, c = order_key(-INFINITY), d = c;
     for (int64_t v = (int64_t)p * blockDim.x + threadIdx.x; v < n; v += (int64_t)nparts * blockDim.x) {
         const double xv = g.x[v], yv = g.y[v];
-        a = fmin(a, xv);
-        b = fmin(b, yv);
-        c = fmax(c, xv);
-        d = fmax(d, yv);
-    }
-    sh[0][threadIdx.x] = a;
-    sh[1][threadIdx.x] = b;
-    sh[2][threadIdx.x] = c;
-    sh[3][threadIdx.x] = d;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            sh[0][threadIdx.x] = fmin(sh[0][threadIdx.x], sh[0][threadIdx.x + w]);
-            sh[1][threadIdx.x] = fmin(sh[1][threadIdx.x], sh[1][threadIdx.x + w]);
-            sh[2][threadIdx.x] = fmax(sh[2][threadIdx.x], sh[2][threadIdx.x + w]);
-            sh[3][threadIdx.x] = fmax(sh[3][threadIdx.x], sh[3][threadIdx.x + w]);
+        if (!any_nan(xv, xv, xv, xv)) {
+            a = min(a, order_key(xv));
+            c = max(c, order_key(xv));
         }
-        __syncthreads();
+        if (!any_nan(yv, yv, yv, yv)) {
+            b = min(b, order_key(yv));
+            d = max(d, order_key(yv));
+        }
     }
-    if (threadIdx.x < 4) part[((int64_t)k * nparts + p) * 4 + threadIdx.x] = sh[threadIdx.x][0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a = min(a, __shfl_xor_sync(0xffffffffu, a, o));
+        b = min(b, __shfl_xor_sync(0xffffffffu, b, o));
+        c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
+        d = max(d, __shfl_xor_sync(0xffffffffu, d, o));
+    }
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][warp] = a;
+        sh[1][warp] = b;
+        sh[2][warp] = c;
+        sh[3][warp] = d;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        long long r = sh[threadIdx.x][0];
+        for (int w = 1; w < 8; w++) r = threadIdx.x < 2 ? min(r, sh[threadIdx.x][w]) : max(r, sh[threadIdx.x][w]);
+        // the key's double: the keys' map is its own inverse
+        part[((int64_t)k * nparts + p) * 4 + threadIdx.x] =
+            __longlong_as_double(r ^ ((r >> 63) & 0x7fffffffffffffffll));
+    }
 }
 
 __global__ void bbox_combine_batch(const double* __restrict__ part, int nparts, int ngrids, double* __restrict__ out) {
@@ -682,11 +695,9 @@ __device__ __forceinline__ int pair_of(const int64_t* __restrict__ base, int G, 
     return lo;
 }
 
-// Starting state of every sweep line (:439-468): one warp per line.
-__global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
-    int lane = threadIdx.x & 31;
-    int64_t line = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (line >= B.line_base[B.G]) return;
+// Starting state of a sweep line (:439-468), by one warp.
+__device__ void seat_line(const Batch& B, int64_t line, Seat* seats) {
+    const int lane = threadIdx.x & 31;
     const int pg = pair_of(B.line_base, B.G, line);
     const SweepParams& P = B.P[pg];
     unsigned* flags = B.flags + pg;
@@ -739,6 +750,11 @@ __global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
         }
     }
     if (lane == 0) seats[line] = seat;
+}
+
+__global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
+    const int64_t line = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (line < B.line_base[B.G]) seat_line(B, line, seats);
 }
 
 // ---------------------------------------------------------------------------
@@ -1105,8 +1121,26 @@ __device__ WalkState guess_state(const Static& S, double px, double py, int64_t 
     return w;
 }
 
-__global__ void chunk_seat_kernel(Batch B, const Seat* __restrict__ seats, WalkState* __restrict__ starts) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Starts of all chunks: the first blocks seat the lines, a warp each, for the
+// lines' first chunks; the others guess, a thread for each further chunk.  Both
+// are chains of dependent steps on few threads, so they run side by side.
+__global__ void __launch_bounds__(128)
+    chunk_seat_kernel(Batch B, unsigned seat_blocks, Seat* __restrict__ seats, WalkState* __restrict__ starts) {
+    if (blockIdx.x < seat_blocks) {
+        const int64_t line = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+        if (line >= B.line_base[B.G]) return;
+        seat_line(B, line, seats);
+        if ((threadIdx.x & 31) == 0) {
+            const int pg = pair_of(B.line_base, B.G, line);
+            const SweepParams& P = B.P[pg];
+            const ChunkPlan& C = B.C[pg];
+            const int f = family_of(P, line);
+            const Seat s0 = seats[line];
+            starts[C.chunk_base[f] + (line - P.fam[f].line_base) * C.nc[f]] = WalkState{s0.stx, s0.sty, 0, s0.outside, 0};
+        }
+        return;
+    }
+    int64_t g = (blockIdx.x - seat_blocks) * (int64_t)blockDim.x + threadIdx.x;
     if (g >= B.chunk_base[B.G]) return;
     const int pg = pair_of(B.chunk_base, B.G, g);
     const SweepParams& P = B.P[pg];
@@ -1116,12 +1150,7 @@ __global__ void chunk_seat_kernel(Batch B, const Seat* __restrict__ seats, WalkS
     int64_t k = g - C.chunk_base[f];
     int64_t li = k / C.nc[f], c = k - li * C.nc[f];
     int64_t j0 = c * C.ch;
-    if (c == 0) {
-        Seat s0 = seats[F.line_base + li];
-        starts[g] = WalkState{s0.stx, s0.sty, 0, s0.outside, 0};
-    } else {
-        starts[g] = guess_state(P.st[F.st], F.SX(li, j0), F.SY(li, j0), j0);
-    }
+    if (c > 0) starts[g] = guess_state(P.st[F.st], F.SX(li, j0), F.SY(li, j0), j0);
 }
 
 __device__ __forceinline__ int64_t chunk_end(const ChunkPlan& C, const Family& F, int64_t c) {
@@ -1279,6 +1308,13 @@ __device__ __forceinline__ unsigned warp_row_add(unsigned* counters, int32_t b, 
     return base + __popc(peers & ((1u << lane) - 1u));
 }
 
+// A triple in its row's bucket: one 16-byte store (key and weight in arrays of
+// their own touched two sectors per triple: 2048^2 -> 1536^2 1.37 ms, now 1.07).
+struct __align__(16) Triple {
+    int64_t key;  // input cell << 32 | raw position
+    double w;
+};
+
 template <int LANES>
 __global__ void slot_count_rows(Batch B, const int64_t* __restrict__ counts, const int32_t* __restrict__ s_cell,
                                 const int32_t* __restrict__ s_seg, unsigned* __restrict__ rows) {
@@ -1309,8 +1345,7 @@ template <int LANES>
 __global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
                                   const int32_t* __restrict__ s_cell, const int32_t* __restrict__ s_seg,
                                   const double* __restrict__ s_area, const int64_t* __restrict__ row_start,
-                                  unsigned* __restrict__ cursor, int64_t* __restrict__ tkey,
-                                  double* __restrict__ tval) {
+                                  unsigned* __restrict__ cursor, Triple* __restrict__ triples) {
     const int lane = threadIdx.x & (LANES - 1);
     const int64_t total = B.chunk_base[B.G];
     int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
@@ -1348,9 +1383,8 @@ __global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, c
                 w = ddiv(side ? -area : area, __ldg(area_in + in));
                 if (w_in) w = dmul(w, __ldg(w_in + in));
             }
-            const int64_t dst = row_start[out + ob] + pos;
-            tkey[dst] = ((int64_t)in << 32) | (int64_t)(uint32_t)(2 * (raw0 + q) + side);
-            tval[dst] = w;
+            triples[row_start[out + ob] + pos] =
+                Triple{((int64_t)in << 32) | (int64_t)(uint32_t)(2 * (raw0 + q) + side), w};
         }
     }
 }
@@ -1360,8 +1394,8 @@ constexpr int ROW_SMALL = 64;  // rows ranked by one warp (two keys per lane)
 // One warp per output row of at most ROW_SMALL triples: each triple's rank
 // is the number of keys of its row below its own (keys are unique); the row
 // is written out in that order.  Longer rows are listed for rank_rows_long.
-__global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, const int64_t* __restrict__ tkey,
-                          const double* __restrict__ tval, int32_t* __restrict__ out_in,
+__global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
+                          int32_t* __restrict__ out_in,
                           double* __restrict__ out_val, int32_t* __restrict__ long_list,
                           unsigned* __restrict__ long_count) {
     const int lane = threadIdx.x & 31;
@@ -1372,8 +1406,9 @@ __global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, 
             if (lane == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)r;
             continue;
         }
-        const int64_t k0 = lane < n ? tkey[s + lane] : INT64_MAX;
-        const int64_t k1 = lane + 32 < n ? tkey[s + 32 + lane] : INT64_MAX;
+        const Triple none{INT64_MAX, 0.0};
+        const Triple t0 = lane < n ? triples[s + lane] : none, t1 = lane + 32 < n ? triples[s + 32 + lane] : none;
+        const int64_t k0 = t0.key, k1 = t1.key;
         int r0 = 0, r1 = 0;
         const int n0 = n < 32 ? (int)n : 32;
         for (int j = 0; j < n0; j++) {
@@ -1388,11 +1423,11 @@ __global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, 
         }
         if (lane < n) {
             out_in[s + r0] = (int32_t)(k0 >> 32);
-            out_val[s + r0] = tval[s + lane];
+            out_val[s + r0] = t0.w;
         }
         if (lane + 32 < n) {
             out_in[s + r1] = (int32_t)(k1 >> 32);
-            out_val[s + r1] = tval[s + 32 + lane];
+            out_val[s + r1] = t1.w;
         }
     }
 }
@@ -1402,8 +1437,8 @@ __global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, 
 constexpr int ROW_TILE = 2048;
 __global__ void __launch_bounds__(256)
     rank_rows_long(const int64_t* __restrict__ row_start, const int32_t* __restrict__ long_list,
-                   const unsigned* __restrict__ long_count, const int64_t* __restrict__ tkey,
-                   const double* __restrict__ tval, int32_t* __restrict__ out_in, double* __restrict__ out_val) {
+                   const unsigned* __restrict__ long_count, const Triple* __restrict__ triples,
+                   int32_t* __restrict__ out_in, double* __restrict__ out_val) {
     __shared__ int64_t tile[ROW_TILE];
     const unsigned nl = *long_count;
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
@@ -1415,13 +1450,13 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
-                mykey[k] = e < t ? tkey[e] : INT64_MAX;
+                mykey[k] = e < t ? triples[e].key : INT64_MAX;
                 rank[k] = 0;
             }
             for (int64_t q0 = 0; q0 < len; q0 += ROW_TILE) {
                 const int64_t m = len - q0 < ROW_TILE ? len - q0 : ROW_TILE;
                 __syncthreads();
-                for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = tkey[s + q0 + q];
+                for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
                 __syncthreads();
                 for (int64_t q = 0; q < m; q++) {
                     const int64_t kq = tile[q];
@@ -1434,7 +1469,7 @@ __global__ void __launch_bounds__(256)
                 const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
                 if (e < t) {
                     out_in[s + rank[k]] = (int32_t)(mykey[k] >> 32);
-                    out_val[s + rank[k]] = tval[e];
+                    out_val[s + rank[k]] = triples[e].w;
                 }
             }
         }
@@ -1644,7 +1679,7 @@ int locate_2d_exact(const double* x, const double* y, int64_t nx, int64_t ny, co
 std::atomic<int64_t> g_sweep_chunk{32};
 // the walk kernel keeps 8 blocks of 64 threads per SM: 152 x 512 threads
 constexpr int64_t kTargetChunks = 152 * 512;
-constexpr int64_t kMinChunk = 4;
+constexpr int64_t kMinChunk = 1;
 
 namespace {
 
@@ -1720,7 +1755,7 @@ struct SortedRows {
 // slots would not fit; fl receives every grid's error word.
 
 int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector<double>& bbox_h,
-                  const Seat* seats, int64_t lines, int64_t* total_dev, cudaStream_t s, int64_t* nraw_out,
+                  Seat* seats, int64_t lines, int64_t* total_dev, cudaStream_t s, int64_t* nraw_out,
                   std::vector<unsigned>& fl, ChunkPlan** plans_dev, int64_t** chunk_base_dev, SortedRows* rows) {
     const int G = B.G;
     // sweep segments per chunk: rg_set_sweep_chunk (default 32), the
@@ -1732,8 +1767,9 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         // Small batches: shorter chunks, so that the walk still has about
         // kTargetChunks threads (each chunk is one thread's sequential walk;
         // a 128^2 pair in chunks of 32 segments keeps 2,000 threads busy
-        // for 0.7 ms).  Every chunk length gives the same triples in the
-        // same order.
+        // for 0.7 ms), down to one segment (a start costs little beside the
+        // walk of a segment; 64^2 -> 48^2: walk 100 -> 34 us).  Every chunk length gives the same
+        // triples in the same order.
         int64_t segments = 0;
         for (int g = 0; g < G; g++)
             for (int f = 0; f < 4; f++) segments += P[g].fam[f].lines * (P[g].fam[f].len - 1);
@@ -1798,7 +1834,8 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         if ((st = dalloc(&s_out, (size_t)slots, s))) break;
         if ((st = dalloc(&s_val, (size_t)slots, s))) break;
         zero_async(n_rep, 2 * sizeof(unsigned long long), s);
-        chunk_seat_kernel<<<grid_for(chunks, 128), 128, 0, s>>>(B, seats, starts);
+        const unsigned seat_blocks = grid_for(lines * 32, 128);
+        chunk_seat_kernel<<<seat_blocks + grid_for(chunks, 128), 128, 0, s>>>(B, seat_blocks, seats, starts);
         {
             // resident blocks only: 8 blocks of 64 threads per SM
             const unsigned blocks = std::min<unsigned>(grid_for(chunks, 64), 152u * 8u);
@@ -1832,8 +1869,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             // order the triples by output row from the slots
             const int64_t nr = rows->n_rows;
             unsigned *rowc = nullptr, *long_count = nullptr;
-            int64_t* tkey = nullptr;
-            double* tval = nullptr;
+            Triple* triples = nullptr;
             int32_t* long_list = nullptr;
             do {
                 if ((st = dalloc(&rows->row_start, (size_t)nr + 1, s))) break;
@@ -1842,8 +1878,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 if ((st = dalloc(&rowc, (size_t)nr + 1, s))) break;
                 if ((st = dalloc(&long_count, 1, s))) break;
                 if ((st = dalloc(&long_list, (size_t)std::max<int64_t>(nr, 1), s))) break;
-                if ((st = dalloc(&tkey, (size_t)std::max<int64_t>(nraw, 1), s))) break;
-                if ((st = dalloc(&tval, (size_t)std::max<int64_t>(nraw, 1), s))) break;
+                if ((st = dalloc(&triples, (size_t)std::max<int64_t>(nraw, 1), s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
                 zero_async(long_count, sizeof(unsigned), s);
                 // lanes per chunk for the pieces it holds on average
@@ -1857,18 +1892,17 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 count<<<gc, 256, 0, s>>>(B, counts, s_in, s_out, rowc);
                 if ((st = exclusive_scan_u32_to_i64(rowc, rows->row_start, nr + 1, nullptr, s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
-                scatter<<<gc, 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val, rows->row_start, rowc, tkey, tval);
+                scatter<<<gc, 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val, rows->row_start, rowc, triples);
                 const unsigned gr = grid_for(nr * 32, 256) > 16384 ? 16384 : grid_for(nr * 32, 256);
-                rank_rows<<<gr, 256, 0, s>>>(rows->row_start, nr, tkey, tval, rows->in, rows->val, long_list,
+                rank_rows<<<gr, 256, 0, s>>>(rows->row_start, nr, triples, rows->in, rows->val, long_list,
                                              long_count);
-                rank_rows_long<<<1024, 256, 0, s>>>(rows->row_start, long_list, long_count, tkey, tval, rows->in,
+                rank_rows_long<<<1024, 256, 0, s>>>(rows->row_start, long_list, long_count, triples, rows->in,
                                                     rows->val);
             } while (0);
             dfree(rowc, s);
             dfree(long_count, s);
             dfree(long_list, s);
-            dfree(tkey, s);
-            dfree(tval, s);
+            dfree(triples, s);
             if (st) break;
         }
         e = cudaGetLastError();
@@ -1989,8 +2023,8 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             nedges_all += 2 * (r.g.nx - 1) + 2 * (r.g.ny - 1);
             max_verts = std::max(max_verts, r.g.nx * r.g.ny);
         }
-        // blocks per grid for the boxes: about 16 vertices a thread, 1..256
-        const int nparts = (int)std::min<int64_t>(256, std::max<int64_t>(1, (max_verts + 4095) / 4096));
+        // blocks per grid for the boxes: about 4 vertices a thread, 1..512
+        const int nparts = (int)std::min<int64_t>(512, std::max<int64_t>(1, (max_verts + 1023) / 1024));
         if ((st = upload(&SB.grids, PG, s))) break;
         if ((st = dalloc(&area_in, (size_t)in_base[G], s))) break;
         if ((st = dalloc(&bbox_d, (size_t)4 * NG, s))) break;
@@ -2113,7 +2147,6 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
 
         // seats and the sweep (sync 3)
         if ((st = dalloc(&seats, (size_t)lines, s))) break;
-        seat_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, seats);
         std::vector<unsigned> fl((size_t)G, 0u);
         int64_t nraw = 0;
         SortedRows rows;
@@ -2125,7 +2158,8 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         sorted_val = rows.val;
         if (st) break;
         if (nraw < 0) {
-            // a chunk overflowed its slots: walk whole lines instead
+            // a chunk overflowed its slots, or lines are not cut: walk whole lines
+            seat_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, seats);
             if ((st = sweep_lines(B, lines, seats, total_dev, s, &raw_in, &raw_out, &raw_val, &nraw, fl))) break;
         }
         for (int g = 0; g < G; g++) status[g] = walk_status(fl[g]);

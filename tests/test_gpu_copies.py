@@ -9,7 +9,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 3967, 3968, 3969, 7936, 7937, 15871, 15872, 15873, 100003])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 3967, 3968, 3969, 31999, 32000, 32001, 64000, 95999, 96000, 96001, 300003])
 @pytest.mark.parametrize("shift", [0, 1, 4, 8])
 def test_copy_from_host(n, shift):
     torch = pytest.importorskip("torch")
