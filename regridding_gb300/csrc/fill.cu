@@ -21,8 +21,8 @@
 // result equals the sequential sweep bit for bit.  The missing cells of each
 // (colour, phase) class are compacted once, in (slice, cell) order, into a
 // list of 64-bit entries (slice << 32 | cell); every iteration is then six
-// gather launches over the lists, and cells that are not missing cost
-// nothing.  Per updated cell: 6 FP64 operations, 4 neighbour reads, 1 write.
+// gathers over the lists (launches, or phases of one launch: fill_relax), and
+// cells that are not missing cost nothing.  Per updated cell: 6 FP64 operations, 4 neighbour reads, 1 write.
 //
 // Median.  A radix select on order-preserving integer keys of the valid,
 // non-NaN values (8-bit digits, most significant first: 8 histogram passes
@@ -30,6 +30,8 @@
 // lower median; the median is (lo + hi) / 2 in the array's dtype for an even
 // count (numpy's mean of the two middle elements), the middle element for an
 // odd count, and 0 for a slice without valid values.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace rg {
@@ -187,6 +189,138 @@ __global__ void fill_update(T* __restrict__ a, const uint64_t* __restrict__ list
     }
 }
 
+// ---------------------------------------------------------------------------
+// Few cells: all iterations in one launch.  A launch per class takes about 4.4
+// us however few cells it updates, and slices never read one another, so a
+// cluster of blocks relaxes its slice with a cluster barrier (hardware, all
+// blocks resident) between the classes.  The cluster's blocks read each
+// other's cells from L2; a thread keeps the first kRelaxKeep entries of the
+// two classes off the seams in registers, with their neighbours' places.
+// Bound by the barrier's and the gathers' latency (about 1 us a class), above a
+// few thousand cells per block by FP64 issue: 4 slices of 480 x 641, 8 %
+// missing, 100 iterations 0.88 -> 0.57 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRelaxThreads = 512;
+constexpr int kRelaxKeep = 2;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
+// a missing cell and its neighbours, within its slice
+struct GsCell {
+    uint32_t c, l, r, d, u;
+    __device__ __forceinline__ GsCell(uint32_t cell, uint32_t ny, const FastDiv& nx_div) : c(cell) {
+        const uint32_t nx = nx_div.d, j = nx_div.div(c), i = c - j * nx;
+        l = i ? c - 1 : c + nx - 1;
+        r = i + 1 == nx ? c + 1 - nx : c + 1;
+        d = j ? c - nx : c + (ny - 1) * nx;
+        u = j + 1 == ny ? i : c + nx;
+    }
+    GsCell() = default;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kRelaxThreads)
+    fill_relax(T* __restrict__ a, const uint64_t* __restrict__ list, const int64_t* __restrict__ offsets, int64_t nblocks,
+               int64_t tiles, uint32_t ny, FastDiv nx_div, GsConst k, int iterations) {
+    const unsigned C = cluster_size();
+    const int64_t t = blockIdx.x / C;
+    const unsigned first = cluster_rank() * kRelaxThreads + threadIdx.x, stride = C * kRelaxThreads;
+    T* s = a + t * (int64_t)ny * nx_div.d;
+    int64_t base[kClasses];
+    unsigned n[kClasses];
+#pragma unroll
+    for (int cls = 0; cls < kClasses; ++cls) {
+        base[cls] = offsets[cls * nblocks + t * tiles];
+        n[cls] = (unsigned)(offsets[cls * nblocks + (t + 1) * tiles] - base[cls]);
+    }
+    GsCell kept[2][kRelaxKeep];
+#pragma unroll
+    for (int colour = 0; colour < 2; ++colour)
+#pragma unroll
+        for (int h = 0; h < kRelaxKeep; ++h) {
+            const unsigned q = first + h * stride;
+            if (q < n[3 * colour]) kept[colour][h] = GsCell((uint32_t)__ldg(list + base[3 * colour] + q), ny, nx_div);
+        }
+    auto update = [&](const GsCell& g) {
+        __stcg(s + g.c, gs_value(__ldcg(s + g.l), __ldcg(s + g.r), __ldcg(s + g.d), __ldcg(s + g.u), k));
+    };
+    for (int it = 0; it < iterations; ++it) {
+#pragma unroll
+        for (int cls = 0; cls < kClasses; ++cls) {
+            if (n[cls] == 0) continue;  // of the slice: the same in all its blocks
+            unsigned q = first;
+            if (cls % 3 == 0) {
+                // both kept cells' loads are issued before either store
+                T v[kRelaxKeep];
+#pragma unroll
+                for (int h = 0; h < kRelaxKeep; ++h) {
+                    const GsCell& g = kept[cls / 3][h];
+                    if (first + h * stride < n[cls])
+                        v[h] = gs_value(__ldcg(s + g.l), __ldcg(s + g.r), __ldcg(s + g.d), __ldcg(s + g.u), k);
+                }
+#pragma unroll
+                for (int h = 0; h < kRelaxKeep; ++h)
+                    if (first + h * stride < n[cls]) __stcg(s + kept[cls / 3][h].c, v[h]);
+                q += kRelaxKeep * stride;
+            }
+            for (; q < n[cls]; q += stride) update(GsCell((uint32_t)__ldg(list + base[cls] + q), ny, nx_div));
+            cluster_barrier();
+        }
+    }
+}
+
+// The largest cluster, up to 16 blocks, of which nt run at a time (1 when none
+// does), for a kernel of kRelaxThreads threads.
+template <typename F>
+int cluster_for(F* kernel, int64_t nt, size_t smem) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaGetLastError();
+    for (int c = 16; c > 1; c /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim = {(unsigned)c, 1, 1};
+        cfg.gridDim = dim3((unsigned)(c * std::min<int64_t>(nt, 4096)));
+        cfg.blockDim = dim3(kRelaxThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (active >= nt) return c;
+    }
+    return 1;
+}
+
+template <typename F, typename... Args>
+cudaError_t launch_clusters(F* kernel, int64_t nt, int c, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {(unsigned)c, 1, 1};
+    cfg.gridDim = dim3((unsigned)(nt * c));
+    cfg.blockDim = dim3(kRelaxThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // a[where] = guess: one value per slice (kind 1) or one per cell (kind 2)
 template <typename T>
 __global__ void fill_seed(T* __restrict__ a, const uint8_t* __restrict__ where, int64_t nt, int64_t S,
@@ -312,33 +446,6 @@ __global__ void median_hist(const T* __restrict__ a, const uint8_t* __restrict__
     }
 }
 
-// the same over the copied candidate keys of each slice
-__global__ void median_hist_keys(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets,
-                                 int64_t nt, int shift, const MedianState* __restrict__ st,
-                                 unsigned* __restrict__ hist) {
-    __shared__ unsigned h[256];
-    const unsigned lane = threadIdx.x & 31u;
-    for (int64_t t = blockIdx.y; t < nt; t += gridDim.y) {
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) h[b] = 0;
-        __syncthreads();
-        const unsigned long long prefix = st[t].prefix, mask = st[t].mask;
-        const int64_t lo = offsets[t], hi = offsets[t + 1];
-        for (int64_t base = lo + blockIdx.x * (int64_t)blockDim.x; base < hi; base += (int64_t)gridDim.x * blockDim.x) {
-            const int64_t c = base + threadIdx.x;
-            unsigned bin = 0xffffffffu;
-            if (c < hi) {
-                const unsigned long long key = keys[c];
-                if ((key & mask) == prefix) bin = (unsigned)(key >> shift) & 255u;
-            }
-            hist_add(h, bin, lane);
-        }
-        __syncthreads();
-        for (int b = threadIdx.x; b < 256; b += blockDim.x)
-            if (h[b]) atomicAdd(&hist[t * 256 + b], h[b]);
-        __syncthreads();
-    }
-}
-
 // One warp per slice chooses the digit holding rank k (the first pass
 // counts the valid keys, which fixes k) and clears the histogram.
 __global__ void median_pick(MedianState* __restrict__ st, unsigned* __restrict__ hist, int64_t nt, int shift,
@@ -453,32 +560,103 @@ __global__ void median_compact(const T* __restrict__ a, const uint8_t* __restric
     }
 }
 
-// candidates <= the lower median, and the smallest candidate above it
-__global__ void median_upper_keys(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets,
-                                  int64_t nt, MedianState* __restrict__ st) {
-    __shared__ unsigned long long le, gt;
-    for (int64_t t = blockIdx.y; t < nt; t += gridDim.y) {
-        if (threadIdx.x == 0) {
-            le = 0;
-            gt = ~0ull;
+// The remaining digits from the copied candidate keys, one cluster per slice:
+// each block's histogram of a digit in shared memory, all blocks' summed
+// through it, the digit holding rank k chosen in every block alike; then the
+// candidates <= the lower median and the smallest one above it.  (A launch per
+// step took 14 us a digit on 4 slices of 480 x 641: 0.13 ms, now 0.04 ms.)
+__global__ void __launch_bounds__(kRelaxThreads)
+    median_digits(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets, int first_shift,
+                  MedianState* __restrict__ st) {
+    __shared__ unsigned h[256], all[256];
+    __shared__ unsigned long long prefix_s, le, gt;
+    __shared__ long long k_s;
+    const unsigned C = cluster_size(), rank = cluster_rank();
+    const int64_t t = blockIdx.x / C;
+    const int lane = threadIdx.x & 31;
+    const int64_t lo = offsets[t], hi = offsets[t + 1];
+    unsigned long long prefix = st[t].prefix, mask = st[t].mask;
+    long long k = st[t].k;
+    auto peer = [&](const void* p, unsigned r) {
+        unsigned at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(r));
+        return at;
+    };
+    if (threadIdx.x == 0) {
+        le = 0;
+        gt = ~0ull;
+    }
+    for (int shift = first_shift; shift >= 0 && hi > lo; shift -= 8) {
+        if (threadIdx.x < 256) h[threadIdx.x] = 0;
+        __syncthreads();
+        // whole warps: hist_add takes all lanes
+        for (int64_t base = lo + (int64_t)rank * kRelaxThreads; base < hi; base += (int64_t)C * kRelaxThreads) {
+            const int64_t c = base + threadIdx.x;
+            unsigned bin = 0xffffffffu;
+            if (c < hi) {
+                const unsigned long long key = __ldg(keys + c);
+                if ((key & mask) == prefix) bin = (unsigned)(key >> shift) & 255u;
+            }
+            hist_add(h, bin, lane);
+        }
+        cluster_barrier();
+        if (threadIdx.x < 256) {
+            unsigned sum = 0;
+            for (unsigned r = 0; r < C; ++r) {
+                unsigned v;
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer(&h[threadIdx.x], r)) : "memory");
+                sum += v;
+            }
+            all[threadIdx.x] = sum;
         }
         __syncthreads();
-        const unsigned long long lo = st[t].prefix;
-        unsigned long long my_le = 0, my_gt = ~0ull;
-        for (int64_t c = offsets[t] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < offsets[t + 1];
-             c += (int64_t)gridDim.x * blockDim.x) {
-            const unsigned long long key = keys[c];
-            if (key <= lo) ++my_le;
-            else if (key < my_gt) my_gt = key;
+        if (threadIdx.x < 32) {
+            unsigned c[8];
+            long long mine = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) mine += c[q] = all[lane * 8 + q];
+            long long incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const long long up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            const long long excl = incl - mine;
+            if (excl <= k && k < incl) {
+                long long acc = excl;
+                int q = 0;
+                for (; q < 7; ++q) {
+                    if (acc + (long long)c[q] > k) break;
+                    acc += c[q];
+                }
+                k_s = k - acc;
+                prefix_s = prefix | (unsigned long long)(lane * 8 + q) << shift;
+            }
         }
-        if (my_le) atomicAdd(&le, my_le);
-        if (my_gt != ~0ull) atomicMin(&gt, my_gt);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (le) atomicAdd(&st[t].count_le, le);
-            if (gt != ~0ull) atomicMin(&st[t].min_gt, gt);
-        }
-        __syncthreads();
+        cluster_barrier();  // (also: every block has read this one's histogram)
+        k = k_s;
+        prefix = prefix_s;
+        mask |= 255ull << shift;
+    }
+    __syncthreads();
+    unsigned long long my_le = 0, my_gt = ~0ull;
+    for (int64_t c = lo + (int64_t)rank * kRelaxThreads + threadIdx.x; c < hi; c += (int64_t)C * kRelaxThreads) {
+        const unsigned long long key = __ldg(keys + c);
+        if (key <= prefix) ++my_le;
+        else if (key < my_gt) my_gt = key;
+    }
+    if (my_le) atomicAdd(&le, my_le);
+    if (my_gt != ~0ull) atomicMin(&gt, my_gt);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (le) atomicAdd(&st[t].count_le, le);
+        if (gt != ~0ull) atomicMin(&st[t].min_gt, gt);
+    }
+    cluster_barrier();  // every block has read st[t]
+    if (rank == 0 && threadIdx.x == 0 && hi > lo) {
+        st[t].prefix = prefix;
+        st[t].mask = mask;
+        st[t].k = k;
     }
 }
 
@@ -540,7 +718,6 @@ int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out,
         const unsigned gw = grid_for(nt * 32, 256);  // a warp per slice
         median_init<<<g1, 256, 0, s>>>(st, nt);
         const dim3 grid = slice_grid(nt, S, 8192);
-        constexpr int kPasses = Keys<T>::kBits / 8;
         for (int pass = 0; pass < kDataPasses; ++pass) {
             const int shift = Keys<T>::kBits - 8 * (pass + 1);
             median_hist<T><<<grid, 256, 0, s>>>(a, where, nt, S, shift, st, hist);
@@ -554,14 +731,8 @@ int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out,
         RG_CUDA(cudaStreamSynchronize(s));
         if ((status = dalloc(&keys, total > 0 ? total : 1, s))) break;
         median_compact<T><<<grid, 256, 0, s>>>(a, where, nt, S, st, offsets, cursor, keys);
-        const int64_t per_slice = (total + nt - 1) / (nt > 0 ? nt : 1);
-        const dim3 kgrid = slice_grid(nt, per_slice, 4096);
-        for (int pass = kDataPasses; pass < kPasses; ++pass) {
-            const int shift = Keys<T>::kBits - 8 * (pass + 1);
-            median_hist_keys<<<kgrid, 256, 0, s>>>(keys, offsets, nt, shift, st, hist);
-            median_pick<<<gw, 256, 0, s>>>(st, hist, nt, shift, pass);
-        }
-        median_upper_keys<<<kgrid, 256, 0, s>>>(keys, offsets, nt, st);
+        RG_CUDA(launch_clusters(median_digits, nt, cluster_for(median_digits, nt, 0), s, keys, offsets,
+                                Keys<T>::kBits - 8 * (kDataPasses + 1), st));
         median_write<T><<<g1, 256, 0, s>>>(st, nt, out);
         RG_CUDA(cudaGetLastError());
     } while (0);
@@ -632,6 +803,26 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         // resident blocks, whose threads walk longer stretches of the list)
         const GsConst k = gs_constants(ny, nx);
         const FastDiv nx_div((uint32_t)nx);
+        // Few cells per slice: clusters.  A class of n cells takes about 4 us or
+        // n * 6 operations at 0.66 of the chip's FP64 rate (0.63 T/s) as a
+        // launch, and 1 us plus its slice's share at the cluster's rate as a
+        // phase.  Measured, launches and clusters, 100 iterations with the
+        // whole call: one 64 x 64 slice 1.24 and 0.81 ms, three of 101 x 607
+        // 1.93 and 1.14 ms, one of 700 x 700 1.61 and 1.52 ms, one of 768 x 768
+        // (float32) 1.39 and 1.47 ms: the line lies below the last two.
+        int64_t widest = 0;
+        for (int cls = 0; cls < kClasses; ++cls) widest = std::max(widest, starts[cls + 1] - starts[cls]);
+        const int c = nt <= 4096 ? cluster_for(fill_relax<T>, nt, 0) : 1;
+        const double op_us = 6.0 / (0.66 * 0.63e6);  // of one cell, the whole chip
+        const double launch_us = std::max(3.8, widest * op_us);
+        const double phase_us = 1.0 + (double)widest / nt * op_us * 152 / c * ((nt * c + 151) / 152);
+        if (phase_us < launch_us) {
+            for (int64_t done = 0; done < iterations; done += 1024)  // a launch stays below a few ms
+                RG_CUDA(launch_clusters(fill_relax<T>, nt, c, s, a, (const uint64_t*)list, (const int64_t*)offsets, nblocks,
+                                        tiles, (uint32_t)ny, nx_div, k,
+                                        (int)std::min<int64_t>(1024, iterations - done)));
+            break;
+        }
         for (int64_t it = 0; it < iterations; ++it) {
             for (int cls = 0; cls < kClasses; ++cls) {
                 const int64_t n = starts[cls + 1] - starts[cls];
