@@ -210,7 +210,8 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
 int tiled_lists_for(rg_weights_s* W, const float* vin, cudaStream_t s, int* g, bool* made);
 int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s);
 bool box_usable(const rg_weights_s* W, int64_t stack);
-int box_load(const rg_weights_s* W, const float* vin, int64_t stack);
+int box_load(const rg_weights_s* W, const void* vin, int64_t stack);
+int apply_wide_f64(const rg_weights_s* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s);
 int box_order_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_perm_for(rg_weights_s* W, cudaStream_t s, bool* made);
@@ -243,12 +244,27 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     // the exact float64 apply of a float32 stack stages input boxes too
     const bool exact_box = !transposed && acc == RG_ACC_EXACT && dtype_in == RG_F32 && dtype_out == RG_F64 &&
                            W->n_out > 0 && W->nnz > 0;
+    // and that of a float64 stack, from a handle's second such call on: the
+    // lists cost about as much as the second and third calls save, and gathers
+    // from global memory, which a first call takes, give the same bits
+    bool exact64 = !transposed && acc != RG_ACC_FAST && dtype_in == RG_F64 && dtype_out == RG_F64 && W->n_out > 0 &&
+                   W->nnz > 0 && stack >= 2;
+    if (exact64) {
+        std::lock_guard<std::mutex> lock(W->mu);
+        if (!W->box_perm) {
+            // (the lists are read back by the host: not while a graph is captured)
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            if (W->exact64_calls++ > 0) RG_CUDA(cudaStreamIsCapturing(s, &capture));
+            else exact64 = false;
+            exact64 = exact64 && capture == cudaStreamCaptureStatusNone;
+        }
+    }
     // the compensated apply: float32 stack, float64 output, float-float sums
     const bool ff_box = !transposed && acc == RG_ACC_COMPENSATED && dtype_in == RG_F32 && dtype_out == RG_F64 &&
                         W->n_out > 0 && W->nnz > 0;
     // (the patch lists keep a float32 copy of the weights in gather order)
     const bool need32 = ((acc == RG_ACC_FAST && dtype_out == RG_F32) || exact_box || ff_box) && W->nnz > 0;
-    int g = 0;
+    int g = 0, load64 = -1;
     bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false, ff_direct = false;
     {
         std::lock_guard<std::mutex> lock(W->mu);
@@ -265,7 +281,7 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
             made = true;
         }
         int load = -1;  // how the patch kernel fills its stages, -1: it does not take the call
-        if (((tiled && W->in_shape1 % 4 == 0) || exact_box || ff_box) && box_usable(W, stack)) {
+        if (((tiled && W->in_shape1 % 4 == 0) || exact_box || exact64 || ff_box) && box_usable(W, stack)) {
             RG_TRY(box_lists_for(W, s, &made));
             load = box_load(W, (const float*)vin, stack);
         }
@@ -283,6 +299,15 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
             }
             use_box = load != LOAD_SWIZZLED || W->box_cfg[stack_class(stack)] >= 0;
         }
+        // (boxes of more than 1536 cells, of coarse outputs with long rows, pay
+        // from 16 slices on: 1000 x 700 -> 500 x 350 with 4, 8 and 16 slices 48, 89
+        // and 171 us gathered, 55, 95 and 150 us staged; smaller boxes from two
+        // on: 1024^2 -> 768^2 with 4, 8 slices 84, 164 us gathered, 73, 133 staged;
+        // 2048^2 -> 1536^2 with 16 slices 1.20 and 0.94 ms, FP64 issue 0.65 ms)
+        exact64 = exact64 && load >= 0 &&
+                  (stack >= 16 || (W->box_residues ? 4 * W->box_residues : W->box_rows * W->box_cols) <= 1536);
+        load64 = load;
+        if (exact64) RG_TRY(box_perm_for(W, s, &made));
         if (exact_box && load >= 0) {
             use_box_exact = true;
             RG_TRY(box_perm_for(W, s, &made));
@@ -304,6 +329,10 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
             RG_TRY(rows_usable(W, (const float*)vin, stack, s, &made, &use_rows));
         if (tiled && !use_box && !use_rows) RG_TRY(tiled_lists_for(W, (const float*)vin, s, &g, &made));
         if (made) RG_CUDA(cudaStreamSynchronize(s));
+    }
+    if (exact64) {
+        const int st = apply_wide_f64(W, load64, (const double*)vin, (double*)vout, stack, s);
+        if (st != RG_ERR_UNSUPPORTED) return st;
     }
     if (use_rows) return apply_rows_launch(W, (const float*)vin, (float*)vout, stack, s);
     if (use_box_exact) {

@@ -781,24 +781,25 @@ EncodeTiledFn encode_tiled() {
 
 // Tensor map of the input stack: columns x rows x slices, boxes of box_rows
 // rows and `bs` slices of 32 columns with the 128-byte swizzle, or (wide)
-// box_pitch columns as they lie; or (LOAD_RESIDUES) groups of four rows x
+// `pitch` columns as they lie; or (LOAD_RESIDUES) groups of four rows x
 // their number.
-bool encode_stack(const rg_weights_s* W, const float* vin, int64_t stack, int bs, CUtensorMap* map) {
-    const bool wide = W->box_pitch > 0;
+bool encode_stack(const rg_weights_s* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map) {
+    const bool wide = pitch > 0;
+    const CUtensorMapDataType type = bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     if (W->box_residues) {
         const cuuint64_t dims[2] = {(cuuint64_t)W->in_shape1 * 4, (cuuint64_t)(stack * W->in_shape0 / 4)};
-        const cuuint64_t strides[1] = {(cuuint64_t)W->in_shape1 * 16};
-        const cuuint32_t box[2] = {(cuuint32_t)W->box_pitch, (cuuint32_t)((W->box_rows + 3) / 4)};
+        const cuuint64_t strides[1] = {(cuuint64_t)W->in_shape1 * 4 * bytes};
+        const cuuint32_t box[2] = {(cuuint32_t)pitch, (cuuint32_t)((W->box_rows + 3) / 4)};
         const cuuint32_t estr[2] = {1, 1};
-        return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)vin, dims, strides, box, estr,
+        return encode_tiled()(map, type, 2, (void*)vin, dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
     const cuuint64_t dims[3] = {(cuuint64_t)W->in_shape1, (cuuint64_t)W->in_shape0, (cuuint64_t)stack};
-    const cuuint64_t strides[2] = {(cuuint64_t)W->in_shape1 * 4, (cuuint64_t)W->n_in * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)(wide ? W->box_pitch : PBOX_C), (cuuint32_t)W->box_rows, (cuuint32_t)bs};
+    const cuuint64_t strides[2] = {(cuuint64_t)W->in_shape1 * bytes, (cuuint64_t)W->n_in * bytes};
+    const cuuint32_t box[3] = {(cuuint32_t)(wide ? pitch : PBOX_C), (cuuint32_t)W->box_rows, (cuuint32_t)bs};
     const cuuint32_t estr[3] = {1, 1, 1};
-    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)vin, dims, strides, box, estr,
+    return encode_tiled()(map, type, 3, (void*)vin, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -933,7 +934,7 @@ bool box_usable(const rg_weights_s* W, int64_t stack) {
 
 // How the patch kernel would fill its stages for this call, -1 when it does
 // not take it (the caller holds the handle's lock, box_lists_for has run).
-int box_load(const rg_weights_s* W, const float* vin, int64_t stack) {
+int box_load(const rg_weights_s* W, const void* vin, int64_t stack) {
     const bool aligned = W->in_shape1 % 4 == 0 && ((uintptr_t)vin & 15) == 0;
     if (W->box_state == 1) return aligned ? LOAD_SWIZZLED : -1;
     if (W->box_state != 2) return -1;
@@ -1224,7 +1225,7 @@ int launch_box_config_mode(const rg_weights_s* W, int cfg, const float* vin, voi
     // stage's other slices are never stored)
     const int bs = (int)std::min<int64_t>(c.sps, stack);
     CUtensorMap map;
-    if (!encode_stack(W, vin, stack, MODE == MODE_FAST ? bs : 1, &map)) return RG_ERR_UNSUPPORTED;
+    if (!encode_stack(W, vin, stack, MODE == MODE_FAST ? bs : 1, 0, 4, &map)) return RG_ERR_UNSUPPORTED;
     switch (cfg) {
         case 0: return launch_patch<4, 2, 0, MODE>(W, map, bs, vin, vout, stack, s);
         case 1: return launch_patch<4, 2, 4, MODE>(W, map, bs, vin, vout, stack, s);
@@ -1241,7 +1242,7 @@ int launch_ff_config(const rg_weights_s* W, int cfg, const float* vin, void* vou
     const FFConfig c = kFFConfigs[cfg];
     const int bs = (int)std::min<int64_t>(c.sps, stack);
     CUtensorMap map;
-    if (!encode_stack(W, vin, stack, 1, &map)) return RG_ERR_UNSUPPORTED;
+    if (!encode_stack(W, vin, stack, 1, 0, 4, &map)) return RG_ERR_UNSUPPORTED;
     switch (cfg) {
         case 0: return launch_patch<6, 2, 0, MODE_FF, 6>(W, map, bs, vin, vout, stack, s);
         case 1: return launch_patch<8, 2, 0, MODE_FF, 6>(W, map, bs, vin, vout, stack, s);
@@ -1390,7 +1391,7 @@ int apply_box_exact(const rg_weights_s* W, const float* vin, double* vout, int64
     if (W->box_state != 1) return RG_ERR_UNSUPPORTED;
     const int bs = (int)std::min<int64_t>(4, stack);
     CUtensorMap map;
-    if (!encode_stack(W, vin, stack, 1, &map)) return RG_ERR_UNSUPPORTED;
+    if (!encode_stack(W, vin, stack, 1, 0, 4, &map)) return RG_ERR_UNSUPPORTED;
     return launch_patch<4, 2, 0, MODE_EXACT>(W, map, bs, vin, vout, stack, s);
 }
 

@@ -14,24 +14,26 @@
 
 namespace rg {
 
-bool encode_stack(const rg_weights_s* W, const float* vin, int64_t stack, int bs, CUtensorMap* map);
+bool encode_stack(const rg_weights_s* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map);
 PatchGrid patch_grid(const rg_weights_s* W);
 BoxShape box_shape(const rg_weights_s* W);
 
 namespace {
 
-template <int PL, int SPS, int NST, int MODE, int LOAD>
-int launch_wide(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+// (box: the handle's, or for a handle of swizzled boxes a wide one of the same
+// extent)
+template <int PL, int SPS, int NST, int MODE, int LOAD, typename TIN>
+int launch_wide(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
     constexpr int CT = MODE == MODE_FF ? 6 : CACHED_T;
-    const auto kernel = apply_patch_tma<SPS, NST, 0, MODE, CT, LOAD, PL>;
-    const size_t smem = (size_t)NST * SPS * PL * sizeof(float);
+    const auto kernel = apply_patch_tma<SPS, NST, 0, MODE, CT, LOAD, PL, TIN>;
+    const size_t smem = (size_t)NST * SPS * PL * sizeof(TIN);
     static std::once_flag attr;
     std::call_once(attr, [&]() {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaGetLastError();
     });
     CUtensorMap map = {};
-    if (!encode_stack(W, vin, stack, 1, &map)) return RG_ERR_UNSUPPORTED;
+    if (!encode_stack(W, vin, stack, 1, box.pitch, (int)sizeof(TIN), &map)) return RG_ERR_UNSUPPORTED;
     const int64_t patches = W->box_patches;
     // split the stack over gridDim.y only when the patches alone give less
     // than ~4 waves of 4 blocks per SM on 152 SMs
@@ -43,7 +45,7 @@ int launch_wide(const rg_weights_s* W, const float* vin, void* vout, int64_t sta
     const dim3 grid((unsigned)patches, (unsigned)((stack + chunk - 1) / chunk));
     // bytes of one copy: a slice's box, or the rows of one residue
     const int rows = LOAD == LOAD_RESIDUES ? (W->box_rows + 3) / 4 : W->box_rows;
-    const unsigned box_bytes = (unsigned)(rows * W->box_pitch * 4);
+    const unsigned box_bytes = (unsigned)(rows * box.pitch * sizeof(TIN));
     constexpr bool OUT64 = MODE != MODE_FAST;
     constexpr bool FF = MODE == MODE_FF;
     kernel<<<grid, 32 * PATCH_WARPS, smem, s>>>(
@@ -51,36 +53,36 @@ int launch_wide(const rg_weights_s* W, const float* vin, void* vout, int64_t sta
         W->val32, W->val, OUT64 ? (double*)vout : nullptr, FastDiv((uint32_t)W->in_shape1), patch_grid(W), patches,
         W->box_origin, W->box_rows, SPS * PL, box_bytes, vin, W->n_in,
         OUT64 ? nullptr : (float*)vout, W->n_out, stack, chunk, W->dflags,
-        FF ? W->ff_perm : (OUT64 ? W->box_perm : nullptr), box_shape(W), W->box_extent);
+        FF ? W->ff_perm : (OUT64 ? W->box_perm : nullptr), box, W->box_extent);
     RG_CUDA(cudaGetLastError());
     return RG_OK;
 }
 
 // Slices per stage: a stage computes all its slices, also those past the end
 // of the stack, so one or two slices take stages of two; the largest boxes
-// too, to keep three blocks on an SM.
-template <int PL, int MODE, int LOAD>
-int launch_plane(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
-    if constexpr (PL <= 2304)
-        if (stack > 2) return launch_wide<PL, 4, 2, MODE, LOAD>(W, vin, vout, stack, s);
-    return launch_wide<PL, 2, 2, MODE, LOAD>(W, vin, vout, stack, s);
+// (from 9 KB a slice) too, to keep three blocks on an SM.
+template <int PL, int MODE, int LOAD, typename TIN>
+int launch_plane(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+    if constexpr (PL * sizeof(TIN) <= 2304 * 4)
+        if (stack > 2) return launch_wide<PL, 4, 2, MODE, LOAD>(W, box, vin, vout, stack, s);
+    return launch_wide<PL, 2, 2, MODE, LOAD>(W, box, vin, vout, stack, s);
 }
 
 // A slice's plane in a stage, the smallest of a few sizes that holds the box
 // (a constant, so that a gather's slices differ by constant offsets).
-template <int MODE, int LOAD>
-int launch_mode(const rg_weights_s* W, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
-    const int cells = W->box_residues ? 4 * W->box_residues : W->box_rows * W->box_pitch;
-    if (cells <= 1024) return launch_plane<1024, MODE, LOAD>(W, vin, vout, stack, s);
-    if (cells <= 1536) return launch_plane<1536, MODE, LOAD>(W, vin, vout, stack, s);
-    if (cells <= 2304) return launch_plane<2304, MODE, LOAD>(W, vin, vout, stack, s);
-    return launch_plane<3584, MODE, LOAD>(W, vin, vout, stack, s);
+template <int MODE, int LOAD, typename TIN>
+int launch_mode(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+    const int cells = box.residues ? 4 * box.residues : W->box_rows * box.pitch;
+    if (cells <= 1024) return launch_plane<1024, MODE, LOAD>(W, box, vin, vout, stack, s);
+    if (cells <= 1536) return launch_plane<1536, MODE, LOAD>(W, box, vin, vout, stack, s);
+    if (cells <= 2304) return launch_plane<2304, MODE, LOAD>(W, box, vin, vout, stack, s);
+    return launch_plane<3584, MODE, LOAD>(W, box, vin, vout, stack, s);
 }
 
-template <int MODE>
-int launch_load(const rg_weights_s* W, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
-    if (load == LOAD_WIDE) return launch_mode<MODE, LOAD_WIDE>(W, vin, vout, stack, s);
-    if constexpr (MODE != MODE_FAST) return launch_mode<MODE, LOAD_RESIDUES>(W, vin, vout, stack, s);
+template <int MODE, typename TIN>
+int launch_load(const rg_weights_s* W, int load, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+    if (load == LOAD_WIDE) return launch_mode<MODE, LOAD_WIDE>(W, box_shape(W), vin, vout, stack, s);
+    if constexpr (MODE != MODE_FAST) return launch_mode<MODE, LOAD_RESIDUES>(W, box_shape(W), vin, vout, stack, s);
     return RG_ERR_UNSUPPORTED;
 }
 
@@ -92,6 +94,14 @@ int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void
         case MODE_EXACT: return launch_load<MODE_EXACT>(W, load, vin, vout, stack, s);
         default: return launch_load<MODE_FF>(W, load, vin, vout, stack, s);
     }
+}
+
+// The exact apply of a float64 stack (box_load, box_perm_for first): as the
+// float32 one, in wide boxes also where that takes swizzled ones.
+int apply_wide_f64(const rg_weights_s* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s) {
+    if (load != LOAD_SWIZZLED) return launch_load<MODE_EXACT>(W, load, vin, vout, stack, s);
+    const BoxShape box{W->in_shape1 >= 36 ? 36 : 32, 0};
+    return launch_mode<MODE_EXACT, LOAD_WIDE>(W, box, vin, vout, stack, s);
 }
 
 }  // namespace rg

@@ -245,6 +245,7 @@ struct rg_weights_s {
     int2* box_origin = nullptr;
     int2* box_extent = nullptr;    // wide boxes: rows and columns of every patch's footprint
     uint16_t* box_slot = nullptr;  // per entry, in the order the TMA kernel gathers them
+    int exact64_calls = 0;         // exact applies of float64 stacks so far (until they have their order)
     uint8_t* box_perm = nullptr;   // exact apply: per patch, thread -> output (longest rows first)
     float* box_val = nullptr;      // float32 weights in that order
     // the compensated (float-float) apply: per entry its box slot, float32

@@ -78,7 +78,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
-__device__ __forceinline__ void tma_load_3d(float* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
         "[%5];\n" ::"r"(smem_u32(dst)),
@@ -233,7 +233,7 @@ __device__ __forceinline__ void ff_step2(uint64_t& h, uint64_t& l, uint64_t wh, 
     l = f2_add(l, f2_add(err, r));
 }
 
-__device__ __forceinline__ void tma_load_2d(float* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
             smem_u32(dst)),
@@ -241,14 +241,20 @@ __device__ __forceinline__ void tma_load_2d(float* dst, const CUtensorMap* map, 
         : "memory");
 }
 
-template <int SPS, int NST, int MINB, int MODE, int CT = CACHED_T, int LOAD = LOAD_SWIZZLED, int PL = PLANE>
+__device__ __forceinline__ double as_double(float v) { return widen(v); }
+__device__ __forceinline__ double as_double(double v) { return v; }
+
+// TIN: the stack's type (double in the exact mode's wide boxes only; "floats"
+// are cells then).
+template <int SPS, int NST, int MINB, int MODE, int CT = CACHED_T, int LOAD = LOAD_SWIZZLED, int PL = PLANE,
+          typename TIN = float>
 __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     apply_patch_tma(const __grid_constant__ CUtensorMap tmap, const int64_t* __restrict__ row_ptr,
                     const int32_t* __restrict__ col, const uint16_t* __restrict__ slot,
                     const float* __restrict__ bval, const float* __restrict__ blo, const float* __restrict__ val,
                     const double* __restrict__ dval, double* __restrict__ vout64, FastDiv nd,
                     PatchGrid P, int64_t n_patches, const int2* __restrict__ origin, int BR, int stage_floats,
-                    unsigned box_bytes, const float* __restrict__ vin, int64_t n_in, float* __restrict__ vout,
+                    unsigned box_bytes, const TIN* __restrict__ vin, int64_t n_in, float* __restrict__ vout,
                     int64_t n_out, int64_t stack, int64_t chunk, unsigned* __restrict__ flags,
                     const uint8_t* __restrict__ perm, BoxShape box, const int2* __restrict__ extent) {
     constexpr bool EXACT = MODE == MODE_EXACT;
@@ -276,7 +282,8 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     __shared__ uint16_t ex_slot[NX][32 * PATCH_WARPS];
     __shared__ float ex_hi[NXF][32 * PATCH_WARPS], ex_lo[NXL][32 * PATCH_WARPS];
     __shared__ double ex_d[NXD][32 * PATCH_WARPS];
-    extern __shared__ __align__(1024) float ring[];
+    extern __shared__ __align__(1024) unsigned char ring_bytes[];
+    TIN* ring = reinterpret_cast<TIN*>(ring_bytes);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int64_t p = blockIdx.x;
     // the thread's output: the warp tile layout, or for the exact and
@@ -310,15 +317,15 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     auto issue_residues = [&](int st, int64_t grp) {
         const int64_t z0 = d0 + grp * SPS;
         const int n = (int)(d1 - z0 < SPS ? d1 - z0 : SPS);
-        float* stage = ring + (int64_t)st * stage_floats;
+        TIN* stage = ring + (int64_t)st * stage_floats;
         if (z0 + n == stack && (stack - 1) * in_rows + org.x + ext.x > (stack * in_rows & ~(int64_t)3)) {
             for (int q = 0; q < n; q++)
                 for (int r = 0; r < ext.x; r++) {
                     const unsigned row = (unsigned)(org.x + r);
                     const int lead = (int)(row * nd.d & 3u);
-                    float* dst = stage + q * PL + (r & 3) * box.residues + (r >> 2) * box.pitch +
+                    TIN* dst = stage + q * PL + (r & 3) * box.residues + (r >> 2) * box.pitch +
                                  slice_shift(z0 + q);
-                    const float* src = vin + (z0 + q) * n_in + (int64_t)row * nd.d + org.y - lead;
+                    const TIN* src = vin + (z0 + q) * n_in + (int64_t)row * nd.d + org.y - lead;
                     const int cells = ext.y + lead;
                     for (int c = lane; c < cells; c += 32) dst[c] = __ldg(src + c);
                 }
@@ -375,12 +382,12 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
         if (o >= 0) {
             if constexpr (OUT64) {
                 for (int64_t d = d0; d < d1; d++) {
-                    const float* a = vin + d * n_in;
+                    const TIN* a = vin + d * n_in;
                     double acc = 0.0;
                     for (int64_t k = s; k < e; k++) acc = __dadd_rn(acc, __dmul_rn(dval[k], (double)__ldg(a + col[k])));
                     vout64[d * n_out + o] = acc;
                 }
-            } else {
+            } else if constexpr (sizeof(TIN) == 4) {
                 apply_direct(s, e, col, val, vin, n_in, out, n_out, d0, d1);
             }
         }
@@ -452,7 +459,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
             }
             return;
         }
-        const float* buf = ring + (int64_t)st * stage_floats;
+        const TIN* buf = ring + (int64_t)st * stage_floats;
         const int64_t ds = d0 + grp * SPS;
         int off[SPS];  // the slices' planes in the stage
 #pragma unroll
@@ -469,7 +476,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
 #pragma unroll
                         for (int q = 0; q < SPS; q++)
                             acc[q] = __dadd_rn(
-                                acc[q], __dmul_rn(wd[k], widen(cell_of(q, li[k]))));
+                                acc[q], __dmul_rn(wd[k], as_double(cell_of(q, li[k]))));
                     }
                 }
                 if constexpr (CT > 0) {
@@ -481,7 +488,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
 #pragma unroll
                             for (int q = 0; q < SPS; q++)
                                 acc[q] = __dadd_rn(acc[q],
-                                                   __dmul_rn(wk, widen(cell_of(q, sk))));
+                                                   __dmul_rn(wk, as_double(cell_of(q, sk))));
                         }
                     }
                 }
@@ -490,7 +497,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                     const int sk = box_slot_of<LOAD>(col[k], org, nd, box);
 #pragma unroll
                     for (int q = 0; q < SPS; q++)
-                        acc[q] = __dadd_rn(acc[q], __dmul_rn(wk, widen(cell_of(q, sk))));
+                        acc[q] = __dadd_rn(acc[q], __dmul_rn(wk, as_double(cell_of(q, sk))));
                 }
 #pragma unroll
                 for (int q = 0; q < SPS; q++)
@@ -579,7 +586,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                             // float64, stored order (the exact apply's sum)
                             r = 0.0;
                             for (int64_t k = s; k < e; k++)
-                                r = __dadd_rn(r, __dmul_rn(dval[k], widen(cell_of(q, box_slot_of<LOAD>(col[k], org, nd, box)))));
+                                r = __dadd_rn(r, __dmul_rn(dval[k], as_double(cell_of(q, box_slot_of<LOAD>(col[k], org, nd, box)))));
                         }
                         vout64[(ds + q) * n_out + o] = r;
                     }
