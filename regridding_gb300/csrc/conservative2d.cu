@@ -878,7 +878,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             // certain (almost always); only the edge found needs its crossing
             // parameter divided out.  Same edges, same order, same t.
             const double p2x = x2, p2y = y2;
-            const double dx12 = dsub(x1, p2x), dy12 = dsub(y1, p2y);
+            double dx12 = 0.0, dy12 = 0.0;  // of the segment, once an edge needs FP64
             int found = -1;
             double f_tdet = 0.0, f_det = 1.0;
             // float32 images of the segment for the crossing filter
@@ -906,6 +906,8 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                     if (ok) dec = crossing_filter(x1f, y1f, dx12f, dy12f, x3f, y3f, x4f, y4f, m);
                 }
                 if (dec == 0) continue;
+                dx12 = dsub(x1, p2x);
+                dy12 = dsub(y1, p2y);
                 const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
                 const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
                 const double tdet = dsub(dmul(x13, y34), dmul(y13, x34));
@@ -926,9 +928,10 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 break;
             }
             if (found >= 0) {
+                // x1 + t (p2 - x1), with p2 - x1 the negated difference at hand
                 const double t = ddiv(f_tdet, f_det);
-                x2 = dadd(x1, dmul(t, dsub(p2x, x1)));
-                y2 = dadd(y1, dmul(t, dsub(p2y, y1)));
+                x2 = dsub(x1, dmul(t, dx12));
+                y2 = dsub(y1, dmul(t, dy12));
             }
             int64_t nsy, nstx, nsty;
             if (found >= 0) {
@@ -1053,7 +1056,7 @@ __global__ void __launch_bounds__(64)
 // triples of both cells that its line separates; their weights are divided
 // out where the triples are ordered, a piece per lane, and not in the walk,
 // whose FP64 instructions run with half their lanes (2048^2 -> 1536^2: walk
-// 4.71 -> 3.86 ms, the two ordering passes 1.38 -> 1.62 ms).
+// 4.71 -> 3.86 ms, the two ordering passes 1.38 -> 1.62 ms then).
 // ---------------------------------------------------------------------------
 
 struct ChunkPlan {
