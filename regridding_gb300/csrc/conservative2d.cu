@@ -1273,7 +1273,8 @@ __global__ void __launch_bounds__(128)
 // chunk's consecutive triples often share a row, and their lanes add to its
 // counter once); 8 or 16 where chunks hold few pieces.  The counting pass keeps
 // every triple's place in its bucket, so the scattering one needs no atomics
-// (2048^2 -> 1536^2: counting 0.22 -> 0.26 ms, scattering 1.07 -> 0.93 ms).  One warp per row in the ranking.
+// (2048^2 -> 1536^2: counting 0.22 -> 0.26 ms, scattering 1.07 -> 0.93 ms).  order_rows
+// sorts and merges the buckets.
 // ---------------------------------------------------------------------------
 
 // What a chunk's pieces share, and the cells of its piece's two triples
@@ -1392,94 +1393,6 @@ __global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, c
     }
 }
 
-constexpr int ROW_SMALL = 64;  // rows ranked by one warp (two keys per lane)
-
-// One warp per output row of at most ROW_SMALL triples: each triple's rank
-// is the number of keys of its row below its own (keys are unique); the row
-// is written out in that order.  Longer rows are listed for rank_rows_long.
-__global__ void rank_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
-                          int32_t* __restrict__ out_in,
-                          double* __restrict__ out_val, int32_t* __restrict__ long_list,
-                          unsigned* __restrict__ long_count) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < nrows; r += nwarps) {
-        const int64_t s = row_start[r], n = row_start[r + 1] - s;  // warp-uniform
-        if (n > ROW_SMALL) {
-            if (lane == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)r;
-            continue;
-        }
-        const Triple none{INT64_MAX, 0.0};
-        const Triple t0 = lane < n ? triples[s + lane] : none, t1 = lane + 32 < n ? triples[s + 32 + lane] : none;
-        const int64_t k0 = t0.key, k1 = t1.key;
-        int r0 = 0, r1 = 0;
-        const int n0 = n < 32 ? (int)n : 32;
-        for (int j = 0; j < n0; j++) {
-            const int64_t kj = __shfl_sync(0xffffffffu, k0, j);
-            r0 += kj < k0;
-            r1 += kj < k1;
-        }
-        for (int j = 32; j < n; j++) {
-            const int64_t kj = __shfl_sync(0xffffffffu, k1, j - 32);
-            r0 += kj < k0;
-            r1 += kj < k1;
-        }
-        if (lane < n) {
-            out_in[s + r0] = (int32_t)(k0 >> 32);
-            out_val[s + r0] = t0.w;
-        }
-        if (lane + 32 < n) {
-            out_in[s + r1] = (int32_t)(k1 >> 32);
-            out_val[s + r1] = t1.w;
-        }
-    }
-}
-
-// One block per listed long row: keys staged in shared-memory tiles, every
-// thread ranks up to 8 triples per pass.
-constexpr int ROW_TILE = 2048;
-__global__ void __launch_bounds__(256)
-    rank_rows_long(const int64_t* __restrict__ row_start, const int32_t* __restrict__ long_list,
-                   const unsigned* __restrict__ long_count, const Triple* __restrict__ triples,
-                   int32_t* __restrict__ out_in, double* __restrict__ out_val) {
-    __shared__ int64_t tile[ROW_TILE];
-    const unsigned nl = *long_count;
-    for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
-        const int32_t r = long_list[li];
-        const int64_t s = row_start[r], t = row_start[r + 1], len = t - s;
-        for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
-            int64_t mykey[8];
-            int64_t rank[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
-                mykey[k] = e < t ? triples[e].key : INT64_MAX;
-                rank[k] = 0;
-            }
-            for (int64_t q0 = 0; q0 < len; q0 += ROW_TILE) {
-                const int64_t m = len - q0 < ROW_TILE ? len - q0 : ROW_TILE;
-                __syncthreads();
-                for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
-                __syncthreads();
-                for (int64_t q = 0; q < m; q++) {
-                    const int64_t kq = tile[q];
-#pragma unroll
-                    for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
-                if (e < t) {
-                    out_in[s + rank[k]] = (int32_t)(mykey[k] >> 32);
-                    out_val[s + rank[k]] = triples[e].w;
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
 __global__ void make_keys(const int32_t* raw_in, int64_t n, int64_t* skey) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * blockDim.x)
@@ -1550,6 +1463,213 @@ __device__ double pairwise_sum(const At& at, int64_t off, int64_t n) {
 }
 
 
+// Merges the entries [s, t) of a row, sorted by input cell, in place with the
+// add.reduceat association; at(k) and the stores are the caller's.  Returns
+// the end of the merged entries.
+template <typename In, typename At, typename Store>
+__device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& in, const At& at, const Store& store) {
+    int64_t w = s, g = s;
+    while (g < t) {
+        const int32_t c = in(g);
+        int64_t h = g + 1;
+        while (h < t && in(h) == c) h++;
+        // (a run of up to 128 is one block of the pairwise sum)
+        const double rest = h - g - 1 <= 128 ? pw_block(at, g + 1, h - g - 1) : pairwise_sum(at, g + 1, h - g - 1);
+        store(w, c, dadd(at(g), rest));
+        w++;
+        g = h;
+    }
+    return w;
+}
+
+// Buckets to merged rows, ORDER_ROWS rows per block.  A warp takes a row: each
+// triple's rank is the number of keys of its row below its own (keys are
+// unique), and the sorted row goes to shared memory; then a lane merges each
+// row there, and the block's merged entries are written without gaps from its
+// first bucket's start.  Blocks with a row of more than ROW_SMALL triples are
+// listed for order_rows_long.  (A launch each for ranking, merging and
+// compacting the rows through global memory took 0.78, 0.42 and 0.17 ms on
+// 2048^2 -> 1536^2: now ORDERMS and COPYMS ms.)
+constexpr int ORDER_ROWS = 32;
+constexpr int ORDER_THREADS = 128;
+constexpr int ROW_SMALL = 64;  // ranked by one warp (two keys per lane)
+
+// The rows' merged counts to the block's prefix (pre[ORDER_ROWS] their total)
+// and to row_nnz; by one warp.
+__device__ __forceinline__ void order_counts(int64_t r0, int64_t nrows, int mine, int* pre, int64_t* row_nnz) {
+    const int lane = threadIdx.x & 31;
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+    }
+    pre[lane + 1] = incl;
+    if (lane == 0) pre[0] = 0;
+    if (r0 + lane < nrows) row_nnz[r0 + lane] = mine;
+}
+
+__global__ void __launch_bounds__(ORDER_THREADS)
+    order_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
+               int32_t* __restrict__ tmp_col, double* __restrict__ tmp_val, int64_t* __restrict__ row_nnz,
+               int32_t* __restrict__ long_list, unsigned* __restrict__ long_count) {
+    __shared__ double val[ORDER_ROWS * ROW_SMALL];
+    __shared__ int32_t in[ORDER_ROWS * ROW_SMALL];
+    __shared__ int start[ORDER_ROWS + 1], pre[ORDER_ROWS + 1];
+    const int t = threadIdx.x, lane = t & 31;
+    const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, s0 = row_start[r0];
+    bool longer = false;
+    if (t <= ORDER_ROWS) {
+        const int64_t r = r0 + t < nrows ? r0 + t : nrows, s = row_start[r];
+        longer = t < ORDER_ROWS && r < nrows && row_start[r + 1] - s > ROW_SMALL;
+        start[t] = (int)(s - s0);
+    }
+    if (__syncthreads_or(longer)) {
+        if (t == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)blockIdx.x;
+        return;
+    }
+    for (int r = t >> 5; r < ORDER_ROWS; r += ORDER_THREADS / 32) {
+        const int s = start[r], n = start[r + 1] - s;  // warp-uniform
+        const Triple none{INT64_MAX, 0.0};
+        const Triple t0 = lane < n ? triples[s0 + s + lane] : none;
+        const Triple t1 = lane + 32 < n ? triples[s0 + s + 32 + lane] : none;
+        int a = 0, b = 0;
+        for (int j = 0; j < (n < 32 ? n : 32); j++) {
+            const int64_t kj = __shfl_sync(0xffffffffu, t0.key, j);
+            a += kj < t0.key;
+            b += kj < t1.key;
+        }
+        for (int j = 32; j < n; j++) {
+            const int64_t kj = __shfl_sync(0xffffffffu, t1.key, j - 32);
+            a += kj < t0.key;
+            b += kj < t1.key;
+        }
+        if (lane < n) {
+            in[s + a] = (int32_t)(t0.key >> 32);
+            val[s + a] = t0.w;
+        }
+        if (lane + 32 < n) {
+            in[s + b] = (int32_t)(t1.key >> 32);
+            val[s + b] = t1.w;
+        }
+    }
+    __syncthreads();
+    if (t < 32) {
+        const int s = start[t];
+        const int64_t end = merge_sorted(
+            s, start[t + 1], [&](int64_t k) { return in[k]; }, [&](int64_t k) { return val[k]; },
+            [&](int64_t k, int32_t c, double v) {
+                in[k] = c;
+                val[k] = v;
+            });
+        order_counts(r0, nrows, (int)(end - s), pre, row_nnz);
+    }
+    __syncthreads();
+    for (int e = t; e < pre[ORDER_ROWS]; e += ORDER_THREADS) {
+        int r = 0;
+#pragma unroll
+        for (int d = ORDER_ROWS / 2; d > 0; d >>= 1)
+            if (pre[r + d] <= e) r += d;
+        const int k = start[r] + e - pre[r];
+        tmp_col[s0 + e] = in[k];
+        tmp_val[s0 + e] = val[k];
+    }
+}
+
+// The listed blocks: every row ranked by the whole block, keys staged in shared-memory tiles, up to 8 triples per thread
+// and pass; then merged by a lane each, and moved together.
+constexpr int ROW_TILE = 2048;
+__global__ void __launch_bounds__(256)
+    order_rows_long(const int64_t* __restrict__ row_start, int64_t nrows, const int32_t* __restrict__ long_list,
+                    const unsigned* __restrict__ long_count, const Triple* __restrict__ triples,
+                    int32_t* tmp_col, double* tmp_val, int64_t* __restrict__ row_nnz) {
+    __shared__ int64_t tile[ROW_TILE];
+    __shared__ int pre[ORDER_ROWS + 1];
+    const unsigned nl = *long_count;
+    for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
+        const int64_t r0 = (int64_t)long_list[li] * ORDER_ROWS, s0 = row_start[r0];
+        for (int64_t r = r0; r < r0 + ORDER_ROWS && r < nrows; r++) {
+            const int64_t s = row_start[r], t = row_start[r + 1], len = t - s;
+            for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
+                int64_t mykey[8];
+                int64_t rank[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
+                    mykey[k] = e < t ? triples[e].key : INT64_MAX;
+                    rank[k] = 0;
+                }
+                for (int64_t q0 = 0; q0 < len; q0 += ROW_TILE) {
+                    const int64_t m = len - q0 < ROW_TILE ? len - q0 : ROW_TILE;
+                    __syncthreads();
+                    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
+                    __syncthreads();
+                    for (int64_t q = 0; q < m; q++) {
+                        const int64_t kq = tile[q];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
+                    if (e < t) {
+                        tmp_col[s + rank[k]] = (int32_t)(mykey[k] >> 32);
+                        tmp_val[s + rank[k]] = triples[e].w;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int64_t r = r0 + threadIdx.x;
+            int64_t n = 0;
+            if (r < nrows) {
+                const int64_t s = row_start[r];
+                n = merge_sorted(
+                        s, row_start[r + 1], [&](int64_t k) { return tmp_col[k]; },
+                        [&](int64_t k) { return tmp_val[k]; },
+                        [&](int64_t k, int32_t c, double v) {
+                            tmp_col[k] = c;
+                            tmp_val[k] = v;
+                        }) -
+                    s;
+            }
+            order_counts(r0, nrows, (int)n, pre, row_nnz);
+        }
+        __syncthreads();
+        // (entries move towards the front: a pass reads before any of it writes)
+        for (int r = 0; r < ORDER_ROWS && r0 + r < nrows; r++) {
+            const int64_t src = row_start[r0 + r] - pre[r];
+            for (int e0 = pre[r]; e0 < pre[r + 1]; e0 += blockDim.x) {
+                const int e = e0 + threadIdx.x;
+                const bool have = e < pre[r + 1];
+                const int32_t c = have ? tmp_col[src + e] : 0;
+                const double v = have ? tmp_val[src + e] : 0.0;
+                __syncthreads();
+                if (have) {
+                    tmp_col[s0 + e] = c;
+                    tmp_val[s0 + e] = v;
+                }
+                __syncthreads();
+            }
+        }
+    }
+}
+
+// The blocks' merged entries to their place in the CSR.
+__global__ void __launch_bounds__(ORDER_THREADS)
+    copy_blocks(const int64_t* __restrict__ row_start, const int64_t* __restrict__ row_ptr, int64_t nrows,
+                const int32_t* __restrict__ tmp_col, const double* __restrict__ tmp_val, int32_t* __restrict__ col,
+                double* __restrict__ val) {
+    const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, r1 = r0 + ORDER_ROWS < nrows ? r0 + ORDER_ROWS : nrows;
+    const int64_t s = row_start[r0], d = row_ptr[r0], n = row_ptr[r1] - d;
+    for (int64_t e = threadIdx.x; e < n; e += ORDER_THREADS) {
+        col[d + e] = tmp_col[s + e];
+        val[d + e] = tmp_val[s + e];
+    }
+}
+
 // One thread per output cell: merge equal input indices of the cell's sorted
 // raw entries with the add.reduceat association, first + pairwise(rest),
 // writing (col, value) compactly from the bucket start; count them.
@@ -1566,22 +1686,14 @@ __global__ void merge_rows(const int64_t* __restrict__ bptr, const int32_t* __re
                            double* __restrict__ tmp_val, int64_t* __restrict__ row_nnz) {
     SortedVal at{s_val};
     for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n_out;
-         o += (int64_t)gridDim.x * blockDim.x) {
-        int64_t s = bptr[o], t = bptr[o + 1];
-        int64_t w = s;
-        int64_t g = s;
-        while (g < t) {
-            int32_t c = s_in[g];
-            int64_t h = g + 1;
-            while (h < t && s_in[h] == c) h++;
-            double v = dadd(at(g), pairwise_sum(at, g + 1, h - g - 1));
-            tmp_col[w] = c;
-            tmp_val[w] = v;
-            w++;
-            g = h;
-        }
-        row_nnz[o] = w - s;
-    }
+         o += (int64_t)gridDim.x * blockDim.x)
+        row_nnz[o] = merge_sorted(
+                         bptr[o], bptr[o + 1], [&](int64_t k) { return s_in[k]; }, at,
+                         [&](int64_t k, int32_t c, double v) {
+                             tmp_col[k] = c;
+                             tmp_val[k] = v;
+                         }) -
+                     bptr[o];
 }
 
 __global__ void compact_rows(const int64_t* __restrict__ bptr, const int64_t* __restrict__ row_ptr,
@@ -1742,24 +1854,26 @@ int sweep_lines(const Batch& B, int64_t lines, const Seat* seats, int64_t* total
     return st;
 }
 
-// The triples ordered by output row straight from the chunks' slots
-// (slot_count_rows, slot_scatter_rows, rank_rows): row_start[n_rows + 1] and
-// the rows' input cells and values.
-struct SortedRows {
+// The triples merged by output row straight from the chunks' slots
+// (slot_count_rows, slot_scatter_rows, order_rows): row_start[n_rows + 1] of
+// the buckets, the rows' merged counts, and the merged entries of every
+// ORDER_ROWS rows from their first bucket's start on.
+struct MergedRows {
     int64_t n_rows = 0;
     int64_t* row_start = nullptr;
-    int32_t* in = nullptr;
+    int64_t* row_nnz = nullptr;
+    int32_t* col = nullptr;
     double* val = nullptr;
 };
 
 // Chunked walk over all lines of the batch (see chunk_walk_kernel), its
-// triples left in output-row order in *rows.  Sets *nraw_out to -1 (and
+// triples left merged by output row in *rows.  Sets *nraw_out to -1 (and
 // frees everything) when a chunk needed more slots than it was given or the
 // slots would not fit; fl receives every grid's error word.
 
 int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector<double>& bbox_h,
                   Seat* seats, int64_t lines, int64_t* total_dev, cudaStream_t s, int64_t* nraw_out,
-                  std::vector<unsigned>& fl, ChunkPlan** plans_dev, int64_t** chunk_base_dev, SortedRows* rows) {
+                  std::vector<unsigned>& fl, ChunkPlan** plans_dev, int64_t** chunk_base_dev, MergedRows* rows) {
     const int G = B.G;
     // sweep segments per chunk: rg_set_sweep_chunk (default 32), the
     // RG_SWEEP_CHUNK environment variable overriding it (0 walks whole lines)
@@ -1878,12 +1992,13 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             int32_t* long_list = nullptr;
             do {
                 if ((st = dalloc(&rows->row_start, (size_t)nr + 1, s))) break;
-                if ((st = dalloc(&rows->in, (size_t)std::max<int64_t>(nraw, 1), s))) break;
-                if ((st = dalloc(&rows->val, (size_t)std::max<int64_t>(nraw, 1), s))) break;
+                if ((st = dalloc(&rows->row_nnz, (size_t)nr + 1, s))) break;
+                if ((st = dalloc(&rows->col, (size_t)nraw, s))) break;
+                if ((st = dalloc(&rows->val, (size_t)nraw, s))) break;
                 if ((st = dalloc(&rowc, (size_t)nr + 1, s))) break;
                 if ((st = dalloc(&long_count, 1, s))) break;
-                if ((st = dalloc(&long_list, (size_t)std::max<int64_t>(nr, 1), s))) break;
-                if ((st = dalloc(&triples, (size_t)std::max<int64_t>(nraw, 1), s))) break;
+                if ((st = dalloc(&long_list, (size_t)(nr / ORDER_ROWS + 1), s))) break;
+                if ((st = dalloc(&triples, (size_t)nraw, s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
                 zero_async(long_count, sizeof(unsigned), s);
                 // lanes per chunk for the pieces it holds on average
@@ -1897,11 +2012,12 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 count<<<gc, 256, 0, s>>>(B, counts, s_in, s_out, rowc, s_pos);
                 if ((st = exclusive_scan_u32_to_i64(rowc, rows->row_start, nr + 1, nullptr, s))) break;
                 scatter<<<gc, 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val, s_pos, rows->row_start, triples);
-                const unsigned gr = grid_for(nr * 32, 256) > 16384 ? 16384 : grid_for(nr * 32, 256);
-                rank_rows<<<gr, 256, 0, s>>>(rows->row_start, nr, triples, rows->in, rows->val, long_list,
-                                             long_count);
-                rank_rows_long<<<1024, 256, 0, s>>>(rows->row_start, long_list, long_count, triples, rows->in,
-                                                    rows->val);
+                const unsigned blocks = grid_for(nr, ORDER_ROWS);
+                order_rows<<<blocks, ORDER_THREADS, 0, s>>>(rows->row_start, nr, triples, rows->col, rows->val,
+                                                            rows->row_nnz, long_list, long_count);
+                order_rows_long<<<std::min(blocks, 152u * 8u), 256, 0, s>>>(rows->row_start, nr, long_list, long_count,
+                                                                            triples, rows->col, rows->val,
+                                                                            rows->row_nnz);
             } while (0);
             dfree(rowc, s);
             dfree(long_count, s);
@@ -2154,14 +2270,16 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         if ((st = dalloc(&seats, (size_t)lines, s))) break;
         std::vector<unsigned> fl((size_t)G, 0u);
         int64_t nraw = 0;
-        SortedRows rows;
+        MergedRows rows;
         rows.n_rows = n_out_all;
         st = sweep_chunked(B, P, bbox_h, seats, lines, total_dev, s, &nraw, fl, &plans_dev, &chunk_base_dev,
                            &rows);
         bucket_ptr = rows.row_start;
-        sorted_in = rows.in;
-        sorted_val = rows.val;
+        row_nnz = rows.row_nnz;
+        tmp_col = rows.col;
+        tmp_val = rows.val;
         if (st) break;
+        const bool merged = bucket_ptr != nullptr;
         if (nraw < 0) {
             // a chunk overflowed its slots, or lines are not cut: walk whole lines
             seat_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, seats);
@@ -2194,12 +2312,14 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             raw_in = raw_out = nullptr;
             raw_val = nullptr;
         }
-        if ((st = dalloc(&tmp_col, (size_t)nraw, s))) break;
-        if ((st = dalloc(&tmp_val, (size_t)nraw, s))) break;
-        if ((st = dalloc(&row_nnz, (size_t)n_out_all + 1, s))) break;
+        if (!merged) {
+            if ((st = dalloc(&tmp_col, (size_t)nraw, s))) break;
+            if ((st = dalloc(&tmp_val, (size_t)nraw, s))) break;
+            if ((st = dalloc(&row_nnz, (size_t)n_out_all + 1, s))) break;
+            merge_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, sorted_in, sorted_val, n_out_all, tmp_col,
+                                                                tmp_val, row_nnz);
+        }
         zero_async(row_nnz + n_out_all, sizeof(int64_t), s);
-        merge_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, sorted_in, sorted_val, n_out_all, tmp_col,
-                                                            tmp_val, row_nnz);
         if ((st = dalloc(&row_ptr, (size_t)n_out_all + 1, s))) break;
         if ((st = exclusive_scan_i64(row_nnz, row_ptr, n_out_all + 1, total_dev, s))) break;
         if ((st = dalloc(&nnz_base_dev, (size_t)G + 1, s))) break;
@@ -2222,8 +2342,12 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         const int64_t nnz = nnz_base[G];
         if ((st = dalloc(&col, (size_t)nnz, s))) break;
         if ((st = dalloc(&val, (size_t)nnz, s))) break;
-        compact_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, row_ptr, tmp_col, tmp_val, n_out_all, col,
-                                                              val);
+        if (merged)
+            copy_blocks<<<grid_for(n_out_all, ORDER_ROWS), ORDER_THREADS, 0, s>>>(bucket_ptr, row_ptr, n_out_all, tmp_col,
+                                                                                  tmp_val, col, val);
+        else
+            compact_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, row_ptr, tmp_col, tmp_val, n_out_all, col,
+                                                                  val);
         e = cudaGetLastError();
         if (e != cudaSuccess) {
             set_error("conservative build: %s", cudaGetErrorString(e));

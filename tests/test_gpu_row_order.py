@@ -1,0 +1,41 @@
+"""Ordering of a build's triples by output row (order_rows, order_rows_long):
+rows of one warp (64 triples), of a block's tile (2048) and longer, mixed in
+one block of 32 rows and across blocks, against the oracle bit for bit."""
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def graded(parts, angle):
+    """A grid over [-1, 1]^2 whose lines lie at the given fractions, turned a little."""
+    t = -0.97 + 1.94 * np.asarray(parts)
+    y, x = np.meshgrid(t, t, indexing="ij")
+    return np.stack([x * np.cos(angle) - y * np.sin(angle), x * np.sin(angle) + y * np.cos(angle)])
+
+
+@pytest.mark.parametrize(
+    "n_in, parts",
+    [
+        (9, np.linspace(0, 1, 4)),  # one block, short rows
+        (12, np.linspace(0, 1, 34)),  # 33^2 rows: a last block of one row
+        (75, np.linspace(0, 1, 2)),  # one row, longer than two tiles
+        (60, np.r_[0, 0.7, 0.71, 0.72, 0.75, 0.8, 1]),  # long and short rows in a block
+        (40, np.r_[0, 0.5, np.linspace(0.52, 1, 40)]),  # blocks with and without long rows
+        (20, np.linspace(0, 1, 6)),  # rows around 64 triples
+    ],
+)
+def test_rows_of_every_length(n_in, parts):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import regridding_gb300 as rg
+
+    gi = graded(np.linspace(0, 1, n_in + 1) ** 1.1, 0.013) * 1.05
+    go = graded(parts, -0.021)
+    want = oracle.weights_conservative_2d(gi, go)
+    got = rg.build_conservative_2d(gi, go).export_numpy()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
