@@ -1463,8 +1463,15 @@ __device__ double pairwise_sum(const At& at, int64_t off, int64_t n) {
 }
 
 
+// The sum of the run [g, h), by the add.reduceat association (a run of up to
+// 129 is one block of the pairwise sum).
+template <typename At>
+__device__ __forceinline__ double run_sum(const At& at, int64_t g, int64_t h) {
+    return dadd(at(g), h - g - 1 <= 128 ? pw_block(at, g + 1, h - g - 1) : pairwise_sum(at, g + 1, h - g - 1));
+}
+
 // Merges the entries [s, t) of a row, sorted by input cell, in place with the
-// add.reduceat association; at(k) and the stores are the caller's.  Returns
+// run_sum; the reads and stores are the caller's.  Returns
 // the end of the merged entries.
 template <typename In, typename At, typename Store>
 __device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& in, const At& at, const Store& store) {
@@ -1473,26 +1480,29 @@ __device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& 
         const int32_t c = in(g);
         int64_t h = g + 1;
         while (h < t && in(h) == c) h++;
-        // (a run of up to 128 is one block of the pairwise sum)
-        const double rest = h - g - 1 <= 128 ? pw_block(at, g + 1, h - g - 1) : pairwise_sum(at, g + 1, h - g - 1);
-        store(w, c, dadd(at(g), rest));
+        store(w, c, run_sum(at, g, h));
         w++;
         g = h;
     }
     return w;
 }
 
-// Buckets to merged rows, ORDER_ROWS rows per block.  A warp takes a row: each
-// triple's rank is the number of keys of its row below its own (keys are
-// unique), and the sorted row goes to shared memory; then a lane merges each
-// row there, and the block's merged entries are written without gaps from its
-// first bucket's start.  Blocks with a row of more than ROW_SMALL triples are
-// listed for order_rows_long.  (A launch each for ranking, merging and
-// compacting the rows through global memory took 0.78, 0.42 and 0.17 ms on
-// 2048^2 -> 1536^2: now ORDERMS and COPYMS ms.)
+// Buckets to merged rows, ORDER_ROWS rows per block, a thread per triple, then
+// one per merged entry.  The keys go to shared memory; a triple's rank is the
+// number of keys of its row below its own (keys are unique); it is stored at
+// its rank, the first of a row marked.  Each run of one input cell is then
+// added up and written, without gaps from the block's first bucket's start.
+// Blocks with a row of more than ROW_SMALL or rows of more than BLOCK_TRIPLES
+// triples are listed for order_rows_long.  (2048^2 -> 1536^2, 22 triples per
+// row: 0.75 ms, and 0.07 ms for copy_blocks; bound by instructions, half of
+// them the ranking.  A warp per row in the ranking and a lane per row in the
+// merge took 0.98 ms; a launch each for ranking, merging and compacting
+// through global memory 0.78, 0.42 and 0.17 ms.)
 constexpr int ORDER_ROWS = 32;
-constexpr int ORDER_THREADS = 128;
-constexpr int ROW_SMALL = 64;  // ranked by one warp (two keys per lane)
+constexpr int ORDER_THREADS = 256;
+constexpr int ROW_SMALL = 256;       // a row's ranks cost its square
+constexpr int BLOCK_TRIPLES = 2048;  // 40 KB of shared memory
+constexpr int32_t ROW_HEAD = INT32_MIN;
 
 // The rows' merged counts to the block's prefix (pre[ORDER_ROWS] their total)
 // and to row_nnz; by one warp.
@@ -1513,66 +1523,76 @@ __global__ void __launch_bounds__(ORDER_THREADS)
     order_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
                int32_t* __restrict__ tmp_col, double* __restrict__ tmp_val, int64_t* __restrict__ row_nnz,
                int32_t* __restrict__ long_list, unsigned* __restrict__ long_count) {
-    __shared__ double val[ORDER_ROWS * ROW_SMALL];
-    __shared__ int32_t in[ORDER_ROWS * ROW_SMALL];
-    __shared__ int start[ORDER_ROWS + 1], pre[ORDER_ROWS + 1];
+    __shared__ int64_t key[BLOCK_TRIPLES];
+    __shared__ double val[BLOCK_TRIPLES];
+    __shared__ int32_t in[BLOCK_TRIPLES];
+    __shared__ int start[ORDER_ROWS + 1];
+    __shared__ unsigned heads[BLOCK_TRIPLES / 32 + 1];  // a bit per triple that begins a run
+    __shared__ int before[BLOCK_TRIPLES / 32 + 1];      // runs before each word of heads
     const int t = threadIdx.x, lane = t & 31;
     const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, s0 = row_start[r0];
     bool longer = false;
     if (t <= ORDER_ROWS) {
         const int64_t r = r0 + t < nrows ? r0 + t : nrows, s = row_start[r];
-        longer = t < ORDER_ROWS && r < nrows && row_start[r + 1] - s > ROW_SMALL;
+        longer = t == ORDER_ROWS ? s - s0 > BLOCK_TRIPLES : r < nrows && row_start[r + 1] - s > ROW_SMALL;
         start[t] = (int)(s - s0);
     }
     if (__syncthreads_or(longer)) {
         if (t == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)blockIdx.x;
         return;
     }
-    for (int r = t >> 5; r < ORDER_ROWS; r += ORDER_THREADS / 32) {
-        const int s = start[r], n = start[r + 1] - s;  // warp-uniform
-        const Triple none{INT64_MAX, 0.0};
-        const Triple t0 = lane < n ? triples[s0 + s + lane] : none;
-        const Triple t1 = lane + 32 < n ? triples[s0 + s + 32 + lane] : none;
-        int a = 0, b = 0;
-        for (int j = 0; j < (n < 32 ? n : 32); j++) {
-            const int64_t kj = __shfl_sync(0xffffffffu, t0.key, j);
-            a += kj < t0.key;
-            b += kj < t1.key;
-        }
-        for (int j = 32; j < n; j++) {
-            const int64_t kj = __shfl_sync(0xffffffffu, t1.key, j - 32);
-            a += kj < t0.key;
-            b += kj < t1.key;
-        }
-        if (lane < n) {
-            in[s + a] = (int32_t)(t0.key >> 32);
-            val[s + a] = t0.w;
-        }
-        if (lane + 32 < n) {
-            in[s + b] = (int32_t)(t1.key >> 32);
-            val[s + b] = t1.w;
-        }
-    }
+    const int n = start[ORDER_ROWS];
+    for (int e = t; e < n; e += ORDER_THREADS) key[e] = triples[s0 + e].key;
     __syncthreads();
-    if (t < 32) {
-        const int s = start[t];
-        const int64_t end = merge_sorted(
-            s, start[t + 1], [&](int64_t k) { return in[k]; }, [&](int64_t k) { return val[k]; },
-            [&](int64_t k, int32_t c, double v) {
-                in[k] = c;
-                val[k] = v;
-            });
-        order_counts(r0, nrows, (int)(end - s), pre, row_nnz);
-    }
-    __syncthreads();
-    for (int e = t; e < pre[ORDER_ROWS]; e += ORDER_THREADS) {
+    for (int e = t; e < n; e += ORDER_THREADS) {
         int r = 0;
 #pragma unroll
         for (int d = ORDER_ROWS / 2; d > 0; d >>= 1)
-            if (pre[r + d] <= e) r += d;
-        const int k = start[r] + e - pre[r];
-        tmp_col[s0 + e] = in[k];
-        tmp_val[s0 + e] = val[k];
+            if (start[r + d] <= e) r += d;
+        const int s = start[r], m = start[r + 1];
+        const int64_t mine = key[e];
+        int rank = 0;
+#pragma unroll 4
+        for (int j = s; j < m; j++) rank += key[j] < mine;
+        in[s + rank] = (int32_t)(mine >> 32) | (rank == 0 ? ROW_HEAD : 0);
+        val[s + rank] = triples[s0 + e].w;
+    }
+    __syncthreads();
+    const int words = n / 32 + 1;
+    for (int q = t >> 5; q < words; q += ORDER_THREADS / 32) {
+        const int e = q * 32 + lane;
+        const bool head = e < n && (in[e] < 0 || in[e] != (in[e - 1] & ~ROW_HEAD));
+        const unsigned word = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) heads[q] = word;
+    }
+    __syncthreads();
+    if (t < 32) {
+        int sum = 0;
+        for (int q0 = 0; q0 < words; q0 += 32) {
+            int incl = q0 + lane < words ? __popc(heads[q0 + lane]) : 0;
+            const int own = incl;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            if (q0 + lane < words) before[q0 + lane] = sum + incl - own;
+            sum += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    const auto runs_before = [&](int e) { return before[e >> 5] + __popc(heads[e >> 5] & ((1u << (e & 31)) - 1u)); };
+    if (t < ORDER_ROWS && r0 + t < nrows) row_nnz[r0 + t] = runs_before(start[t + 1]) - runs_before(start[t]);
+    uint16_t* run = reinterpret_cast<uint16_t*>(key);  // where each run begins
+    for (int e = t; e < n; e += ORDER_THREADS)
+        if (heads[e >> 5] >> (e & 31) & 1u) run[runs_before(e)] = (uint16_t)e;
+    const int runs = runs_before(n);
+    if (t == 0) run[runs] = (uint16_t)n;
+    __syncthreads();
+    for (int k = t; k < runs; k += ORDER_THREADS) {
+        const int g = run[k];
+        tmp_col[s0 + k] = in[g] & ~ROW_HEAD;
+        tmp_val[s0 + k] = run_sum([&](int64_t e) { return val[e]; }, g, run[k + 1]);
     }
 }
 
@@ -1658,13 +1678,14 @@ __global__ void __launch_bounds__(256)
 }
 
 // The blocks' merged entries to their place in the CSR.
-__global__ void __launch_bounds__(ORDER_THREADS)
+constexpr int COPY_THREADS = 128;
+__global__ void __launch_bounds__(COPY_THREADS)
     copy_blocks(const int64_t* __restrict__ row_start, const int64_t* __restrict__ row_ptr, int64_t nrows,
                 const int32_t* __restrict__ tmp_col, const double* __restrict__ tmp_val, int32_t* __restrict__ col,
                 double* __restrict__ val) {
     const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, r1 = r0 + ORDER_ROWS < nrows ? r0 + ORDER_ROWS : nrows;
     const int64_t s = row_start[r0], d = row_ptr[r0], n = row_ptr[r1] - d;
-    for (int64_t e = threadIdx.x; e < n; e += ORDER_THREADS) {
+    for (int64_t e = threadIdx.x; e < n; e += COPY_THREADS) {
         col[d + e] = tmp_col[s + e];
         val[d + e] = tmp_val[s + e];
     }
@@ -2343,7 +2364,7 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         if ((st = dalloc(&col, (size_t)nnz, s))) break;
         if ((st = dalloc(&val, (size_t)nnz, s))) break;
         if (merged)
-            copy_blocks<<<grid_for(n_out_all, ORDER_ROWS), ORDER_THREADS, 0, s>>>(bucket_ptr, row_ptr, n_out_all, tmp_col,
+            copy_blocks<<<grid_for(n_out_all, ORDER_ROWS), COPY_THREADS, 0, s>>>(bucket_ptr, row_ptr, n_out_all, tmp_col,
                                                                                   tmp_val, col, val);
         else
             compact_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, row_ptr, tmp_col, tmp_val, n_out_all, col,
