@@ -484,8 +484,9 @@ __device__ __forceinline__ int grid_of_edge(const PrepGrid* __restrict__ P, int 
     return lo;
 }
 
-// areas of the input cells of every pair, in area_in's order (pair by pair)
-__global__ void cell_area_batch(const PrepGrid* __restrict__ P, int G, int64_t ncells, double* __restrict__ out) {
+// Areas of the input cells of every pair, in area_in's order (pair by pair),
+// each with its reciprocal for area_ratio.
+__global__ void cell_area_batch(const PrepGrid* __restrict__ P, int G, int64_t ncells, double2* __restrict__ out) {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncells;
          c += (int64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = G - 1;
@@ -496,8 +497,30 @@ __global__ void cell_area_batch(const PrepGrid* __restrict__ P, int G, int64_t n
         }
         const Grid g = P[2 * lo].g;
         const int64_t local = c - P[2 * lo].cell_base, ncy = g.ny - 1;
-        out[c] = cell_area_at(g.x, g.y, g.ny, local / ncy, local % ncy);
+        const double a = cell_area_at(g.x, g.y, g.ny, local / ncy, local % ncy);
+        out[c] = make_double2(a, ddiv(1.0, a));
     }
+}
+
+// a / cell.x, correctly rounded, from the cell's rounded reciprocal cell.y:
+// two corrections by the exact remainder.  The product a * y is within 1.5
+// units of the quotient; the first correction leaves at most half a unit and
+// 2^-53 of one, and the second then rounds as the quotient does (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000", 1990: the
+// remainder is exact, and its product with y's error stays below the distance
+// of any quotient from a rounding boundary).  Operands outside 2^-400 .. 2^400,
+// where nothing here over- or underflows, zeros and NaN divide.  (Half the
+// FP64 operations of a division.  2048^2 -> 1536^2: with the loads of both sides
+// issued together the scattering pass takes 0.79 ms in place of 0.93, the
+// areas 0.20 in place of 0.16.)
+__device__ __forceinline__ bool ratio_range(double v) {
+    return ((unsigned)__double2hiint(v) >> 20 & 0x7ffu) - 623u <= 800u;
+}
+__device__ __forceinline__ double area_ratio(double a, double2 cell) {
+    if (!(ratio_range(a) && ratio_range(cell.x))) return ddiv(a, cell.x);
+    const double q0 = dmul(a, cell.y);
+    const double q1 = __fma_rn(__fma_rn(-cell.x, q0, a), cell.y, q0);
+    return __fma_rn(__fma_rn(-cell.x, q1, a), cell.y, q1);
 }
 
 // Bounding boxes (xmin, ymin, xmax, ymax) of every static grid: nparts
@@ -649,7 +672,7 @@ struct Family {
 struct SweepParams {
     Family fam[4];
     Static st[2];
-    const double* area_in;  // (ncx_in, ncy_in)
+    const double2* area_in;  // (ncx_in, ncy_in): area and its reciprocal
     const double* w_in;     // nullable
     int64_t ncy_in, ncy_out;
     int64_t total_lines;
@@ -981,8 +1004,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                         if (!F.sweep_input && have_static) {
                             w = -w_static;
                         } else {
-                            double ain = __ldg(P.area_in + in_flat);
-                            w = side == 0 ? ddiv(area, ain) : ddiv(-area, ain);
+                            w = area_ratio(side == 0 ? area : -area, __ldg(P.area_in + in_flat));
                             if (P.w_in) w = dmul(w, __ldg(P.w_in + in_flat));
                             if (!F.sweep_input && side == 0) {
                                 w_static = w;
@@ -1349,8 +1371,14 @@ __global__ void slot_count_rows(Batch B, const int64_t* __restrict__ counts, con
     }
 }
 
+// -v without the FP64 pipe
+__device__ __forceinline__ double negated(double v) {
+    return __hiloint2double(__double2hiint(v) ^ INT32_MIN, __double2loint(v));
+}
+
 template <int LANES>
-__global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
+__global__ void __launch_bounds__(256)
+    slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
                                   const int32_t* __restrict__ s_cell, const int32_t* __restrict__ s_seg,
                                   const double* __restrict__ s_area, const uint2* __restrict__ s_pos,
                                   const int64_t* __restrict__ row_start, Triple* __restrict__ triples) {
@@ -1362,34 +1390,41 @@ __global__ void slot_scatter_rows(Batch B, const int64_t* __restrict__ counts, c
     int64_t base;
     const PieceLine L = piece_line(B, pg, g, &base);
     const int32_t ob = (int32_t)B.out_base[pg];
-    const int64_t n = counts[g], raw0 = offsets[g];
-    const double* __restrict__ area_in = L.P->area_in;
+    const int n = (int)counts[g];
+    const unsigned order0 = 2 * (unsigned)offsets[g];
+    // the moving grid's cell beside segment seg is seg * step + own0 before the line, + own1 after it
+    const bool has0 = L.has(0), has1 = L.has(1), sweep_input = L.F->sweep_input;
+    const int32_t nc = (int32_t)(sweep_input ? L.P->ncy_in : L.P->ncy_out);
+    const int32_t step = L.F->axis == 0 ? nc : 1, other = L.F->axis == 0 ? 1 : nc;
+    const int32_t own1 = (int32_t)L.li * other, own0 = own1 - other;
+    const double2* __restrict__ area_in = L.P->area_in;
     const double* __restrict__ w_in = L.P->w_in;
-    for (int64_t q = lane; q < n; q += LANES) {
-        const int32_t cell = s_cell[base + q], seg = s_seg[base + q];
-        const double area = s_area[base + q];
-        const uint2 pos = s_pos[base + q];
+    row_start += ob;
+    s_cell += base;
+    s_seg += base;
+    s_area += base;
+    s_pos += base;
+    for (int q = lane; q < n; q += LANES) {
+        const int32_t cell = s_cell[q], seg = s_seg[q] * step;
+        const double area = s_area[q];
+        const uint2 pos = s_pos[q];
+        const int32_t c0 = seg + own0, c1 = seg + own1;
+        const int64_t to0 = has0 ? row_start[sweep_input ? cell : c0] + pos.x : 0;
+        const int64_t to1 = has1 ? row_start[sweep_input ? cell : c1] + pos.y : 0;
+        const int32_t in0 = sweep_input ? (has0 ? c0 : c1) : cell, in1 = sweep_input && has1 ? c1 : in0;
         // a static input grid: both sides share the input cell, and
         // -area / a_in (times w_in) is exactly the negation of area / a_in
         // (times w_in): one division serves both
-        double shared = 0.0;
-        if (!L.F->sweep_input) {
-            shared = ddiv(area, __ldg(area_in + cell));
-            if (w_in) shared = dmul(shared, __ldg(w_in + cell));
+        const double2 a0 = __ldg(area_in + in0);
+        double w0 = area_ratio(area, a0);
+        if (w_in) w0 = dmul(w0, __ldg(w_in + in0));
+        double w1 = negated(w0);
+        if (sweep_input) {
+            w1 = negated(area_ratio(area, __ldg(area_in + in1)));
+            if (w_in) w1 = dmul(w1, __ldg(w_in + in1));
         }
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            if (!L.has(side)) continue;
-            int32_t in, out;
-            L.cells(side, cell, seg, &in, &out);
-            double w = side ? -shared : shared;
-            if (L.F->sweep_input) {
-                w = ddiv(side ? -area : area, __ldg(area_in + in));
-                if (w_in) w = dmul(w, __ldg(w_in + in));
-            }
-            triples[row_start[out + ob] + (side ? pos.y : pos.x)] =
-                Triple{((int64_t)in << 32) | (int64_t)(uint32_t)(2 * (raw0 + q) + side), w};
-        }
+        if (has0) triples[to0] = Triple{(int64_t)in0 << 32 | (order0 + 2 * q), w0};
+        if (has1) triples[to1] = Triple{(int64_t)in1 << 32 | (order0 + 2 * q + 1), w1};
     }
 }
 
@@ -2123,7 +2158,7 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
     const int64_t lines = line_base[G], n_out_all = out_base[G];
 
     int st = RG_OK;
-    double* area_in = nullptr;
+    double2* area_in = nullptr;
     double* bbox_d = nullptr;
     StaticBatch SB;
     int64_t* totals = nullptr;

@@ -39,3 +39,21 @@ def test_rows_of_every_length(n_in, parts):
     want = oracle.weights_conservative_2d(gi, go)
     got = rg.build_conservative_2d(gi, go).export_numpy()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize(
+    "scale", [(1.0, 2.0**-385), (1.0, 2.0**-393), (1.0, 2.0**-420), (2.0**60, 2.0**345), (1e60, 1e61), (1e70, 1e70)]
+)
+def test_weights_at_any_scale(scale):
+    """area / cell area beside the limits 2^-400 and 2^400 of area_ratio's short form"""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import regridding_gb300 as rg
+
+    scale = np.reshape(scale, (2, 1, 1))
+    gi = graded(np.linspace(0, 1, 24) ** 1.1, 0.013) * 1.05 * scale
+    go = graded(np.linspace(0, 1, 18), -0.021) * scale
+    want = oracle.weights_conservative_2d(gi, go)
+    got = rg.build_conservative_2d(gi, go).export_numpy()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
