@@ -197,6 +197,25 @@ __device__ __forceinline__ int crossing_filter(float x1, float y1, float dx12, f
     return (in_t == 1 && in_u == 1) ? 1 : -1;
 }
 
+// seg_hit without the quotients where their bits decide (almost always), for
+// the edges of a cell that the filter leaves open.
+__device__ __noinline__ bool inside_hit(double x1, double y1, double x2, double y2, double x3, double y3, double x4,
+                                        double y4) {
+    if (!bboxes_intersect(x1, y1, x2, y2, x3, y3, x4, y4)) return false;
+    const double dx12 = dsub(x1, x2), dy12 = dsub(y1, y2);
+    const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
+    const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
+    const double tdet = dsub(dmul(x13, y34), dmul(y13, x34));
+    const double det = dsub(dmul(dx12, y34), dmul(dy12, x34));
+    const double udet = dsub(dmul(dx12, y13), dmul(dy12, x13));
+    const int in_t = quotient_in_unit(tdet, det);
+    const int in_u = quotient_in_unit(-udet, det);
+    if (in_t == 0 || in_u == 0) return false;
+    if (in_t > 0 && in_u > 0) return true;
+    const double t = ddiv(tdet, det), u = ddiv(-udet, det);
+    return (0 <= t && t < 1) && (0 <= u && u < 1);
+}
+
 // contribution of one boundary edge to the extended winding number of
 // point_is_inside_polygon (geometry.py:737-829)
 __device__ __forceinline__ double winding_term(double x, double y, double vx0, double vy0,
@@ -784,10 +803,9 @@ __global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
 // the walk
 // ---------------------------------------------------------------------------
 
-__constant__ int c_vtx_i[4] = {0, 1, 1, 0};   // indices_cell_vertex: _grids.py:153-158
-__constant__ int c_vtx_j[4] = {0, 0, 1, 1};
-__constant__ int c_nrm_i[4] = {-1, 0, 1, 0};  // cell_normals: _grids.py:143-148
-__constant__ int c_nrm_j[4] = {0, -1, 0, 1};
+// indices_cell_vertex: _grids.py:153-158
+__device__ __forceinline__ int vertex_i(int v) { return (v + 1) >> 1 & 1; }  // 0, 1, 1, 0
+__device__ __forceinline__ int vertex_j(int v) { return v >> 1; }            // 0, 0, 1, 1
 
 // State of a walk at a sweep vertex.  At every vertex the upstream's
 // entry-edge marker is back at sys.maxsize and the current point is the
@@ -808,11 +826,16 @@ struct WalkState {
 // only count (and flag the overflow), as EMIT_COUNT does throughout.  Returns
 // the number of triples or pieces.
 constexpr int EMIT_COUNT = 0, EMIT_TRIPLES = 1, EMIT_PIECES = 2;
+// -v without the FP64 pipe
+__device__ __forceinline__ double negated(double v) {
+    return __hiloint2double(__double2hiint(v) ^ INT32_MIN, __double2loint(v));
+}
+
 template <int EMIT>
 __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Static& S, int64_t li, int64_t j_end,
                               WalkState& state, int64_t wpos, int64_t wend, int32_t* __restrict__ raw_in,
                               int32_t* __restrict__ raw_out, double* __restrict__ raw_val, unsigned* flags,
-                              int64_t max_steps) {
+                              int64_t max_steps, unsigned lanes) {
     const Grid st = S.g;
     int64_t stx = state.stx, sty = state.sty;
     bool outside = state.outside;
@@ -822,13 +845,21 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
     int64_t steps = 0;
     double x1 = F.SX(li, sy_idx), y1 = F.SY(li, sy_idx);
 
-    while (sy_idx < j_end) {
-        if (++steps > max_steps) {
+    bool capped = false;
+    while (true) {
+        const bool live = sy_idx < j_end && !capped;
+        if (!__any_sync(lanes, live)) break;
+        bool inside = false;
+        double x2 = x1, y2 = y1;
+        if (live && ++steps > max_steps) {
             atomicOr(flags, FLAG_WALK_CAP);
-            break;
+            capped = true;
+        } else if (live) {
+            x2 = F.SX(li, sy_idx + 1);
+            y2 = F.SY(li, sy_idx + 1);
+            inside = !outside;
         }
-        double x2 = F.SX(li, sy_idx + 1), y2 = F.SY(li, sy_idx + 1);
-        if (outside) {
+        if (live && !capped && outside) {
             // _step_outside_static: smallest-t crossing of the static boundary,
             // candidates from the bins overlapping the segment's box
             const double p2x = x2, p2y = y2;
@@ -893,74 +924,71 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 edge_last = MAXSIZE;
                 sy_idx = sy_idx + 1;
             }
-        } else {
-            // _step_inside_static: first crossed edge of the current static
-            // cell other than the entry edge
-            // The hit test of each candidate edge is seg_hit's, with the two
-            // quotients placed against [0, 1) on their bits where that is
-            // certain (almost always); only the edge found needs its crossing
-            // parameter divided out.  Same edges, same order, same t.
-            const double p2x = x2, p2y = y2;
-            double dx12 = 0.0, dy12 = 0.0;  // of the segment, once an edge needs FP64
-            int found = -1;
-            double f_tdet = 0.0, f_det = 1.0;
+        }
+        __syncwarp(lanes);
+        // _step_inside_static: first crossed edge of the current static cell
+        // other than the entry edge.  The hit test of each candidate edge is
+        // seg_hit's, decided in float32 where that is certain (almost always);
+        // only the edge found needs its crossing parameter.  Same edges, same
+        // order, same t.
+        int found = -1;
+        if (inside) {
             // float32 images of the segment for the crossing filter
             bool seg_ok = true;
             const float x1f = trunc_float(x1, seg_ok), y1f = trunc_float(y1, seg_ok);
-            const float x2f = trunc_float(p2x, seg_ok), y2f = trunc_float(p2y, seg_ok);
+            const float x2f = trunc_float(x2, seg_ok), y2f = trunc_float(y2, seg_ok);
             const float dx12f = __fsub_rn(x1f, x2f), dy12f = __fsub_rn(y1f, y2f);
             const float mseg = fmaxf(fmaxf(fabsf(x1f), fabsf(y1f)), fmaxf(fabsf(x2f), fabsf(y2f)));
+            bool ok3 = seg_ok;
+            float x3f = trunc_float(st.X(stx, sty + 1), ok3), y3f = trunc_float(st.Y(stx, sty + 1), ok3);
 #pragma unroll 1
             for (int v = 0; v < 4; v++) {
-                if (v == edge_last) continue;
-                int vp = (v + 3) & 3;
-                double x3 = st.X(stx + c_vtx_i[vp], sty + c_vtx_j[vp]);
-                double y3 = st.Y(stx + c_vtx_i[vp], sty + c_vtx_j[vp]);
-                double x4 = st.X(stx + c_vtx_i[v], sty + c_vtx_j[v]);
-                double y4 = st.Y(stx + c_vtx_i[v], sty + c_vtx_j[v]);
-                if (!bboxes_intersect(x1, y1, p2x, p2y, x3, y3, x4, y4)) continue;
-                // 1: crossed, 0: not crossed (both certain), -1: the FP64 test decides
-                int dec = -1;
-                {
-                    bool ok = seg_ok;
-                    const float x3f = trunc_float(x3, ok), y3f = trunc_float(y3, ok);
-                    const float x4f = trunc_float(x4, ok), y4f = trunc_float(y4, ok);
+                const double x4 = st.X(stx + vertex_i(v), sty + vertex_j(v));
+                const double y4 = st.Y(stx + vertex_i(v), sty + vertex_j(v));
+                bool ok4 = seg_ok;
+                const float x4f = trunc_float(x4, ok4), y4f = trunc_float(y4, ok4);
+                if (found < 0 && v != edge_last) {
+                    // 1: crossed, 0: not crossed (both certain), -1: the FP64 test decides.
+                    // (A certain crossing is one of the boxes, too.)
+                    int dec = -1;
                     const float m = fmaxf(mseg, fmaxf(fmaxf(fabsf(x3f), fabsf(y3f)), fmaxf(fabsf(x4f), fabsf(y4f))));
-                    if (ok) dec = crossing_filter(x1f, y1f, dx12f, dy12f, x3f, y3f, x4f, y4f, m);
-                }
-                if (dec == 0) continue;
-                dx12 = dsub(x1, p2x);
-                dy12 = dsub(y1, p2y);
-                const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
-                const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
-                const double tdet = dsub(dmul(x13, y34), dmul(y13, x34));
-                const double det = dsub(dmul(dx12, y34), dmul(dy12, x34));
-                if (dec < 0) {
-                    const double udet = dsub(dmul(dx12, y13), dmul(dy12, x13));
-                    const int in_t = quotient_in_unit(tdet, det);
-                    const int in_u = quotient_in_unit(-udet, det);
-                    if (in_t == 0 || in_u == 0) continue;
-                    if (in_t < 0 || in_u < 0) {
-                        const double t = ddiv(tdet, det), u = ddiv(-udet, det);
-                        if (!((0 <= t && t < 1) && (0 <= u && u < 1))) continue;
+                    if (ok3 && ok4) dec = crossing_filter(x1f, y1f, dx12f, dy12f, x3f, y3f, x4f, y4f, m);
+                    if (dec < 0) {
+                        const int p = (v + 3) & 3;
+                        const double x3 = st.X(stx + vertex_i(p), sty + vertex_j(p));
+                        const double y3 = st.Y(stx + vertex_i(p), sty + vertex_j(p));
+                        dec = inside_hit(x1, y1, x2, y2, x3, y3, x4, y4);
                     }
+                    if (dec > 0) found = v;
                 }
-                found = v;
-                f_tdet = tdet;
-                f_det = det;
-                break;
+                x3f = x4f;
+                y3f = y4f;
+                ok3 = ok4;
             }
-            if (found >= 0) {
-                // x1 + t (p2 - x1), with p2 - x1 the negated difference at hand
-                const double t = ddiv(f_tdet, f_det);
-                x2 = dsub(x1, dmul(t, dx12));
-                y2 = dsub(y1, dmul(t, dy12));
-            }
+        }
+        __syncwarp(lanes);
+        if (found >= 0) {
+            const int p = (found + 3) & 3;
+            const double x3 = st.X(stx + vertex_i(p), sty + vertex_j(p));
+            const double y3 = st.Y(stx + vertex_i(p), sty + vertex_j(p));
+            const double x4 = st.X(stx + vertex_i(found), sty + vertex_j(found));
+            const double y4 = st.Y(stx + vertex_i(found), sty + vertex_j(found));
+            const double dx12 = dsub(x1, x2), dy12 = dsub(y1, y2);
+            const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
+            const double tdet = dsub(dmul(dsub(x1, x3), y34), dmul(dsub(y1, y3), x34));
+            const double det = dsub(dmul(dx12, y34), dmul(dy12, x34));
+            // x1 + t (x2 - x1), with x2 - x1 the negated difference at hand
+            const double t = ddiv(tdet, det);
+            x2 = dsub(x1, dmul(t, dx12));
+            y2 = dsub(y1, dmul(t, dy12));
+        }
+        __syncwarp(lanes);
+        if (inside) {
             int64_t nsy, nstx, nsty;
             if (found >= 0) {
                 nsy = sy_idx;
-                nstx = stx + c_nrm_i[found];
-                nsty = sty + c_nrm_j[found];
+                nstx = stx + (found & 1 ? 0 : found - 1);  // cell_normals: _grids.py:143-148
+                nsty = sty + (found & 1 ? found - 2 : 0);
                 edge_last = (found + 2) % 4;
             } else {
                 nsy = sy_idx + 1;
@@ -970,7 +998,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             }
             // _calc_and_save_weights: area_triangle, negated for axis 0
             double area = dmul(dsub(dmul(x1, y2), dmul(x2, y1)), 0.5);
-            if (F.axis == 0) area = -area;
+            if (F.axis == 0) area = negated(area);
             // when the static grid is the input grid both sides share the
             // input cell, and -area / a_in (times w_in) is exactly the
             // negation of area / a_in (times w_in): one division serves both
@@ -1032,7 +1060,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             stx = nstx;
             sty = nsty;
         }
-        x1 = x2;
+        x1 = x2;  // (unchanged where the walk has ended)
         y1 = y2;
     }
     state.stx = stx;
@@ -1050,6 +1078,7 @@ __global__ void __launch_bounds__(64)
                 const int64_t* __restrict__ offsets, int32_t* __restrict__ raw_in,
                 int32_t* __restrict__ raw_out, double* __restrict__ raw_val) {
     int64_t line = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const unsigned here = __ballot_sync(0xffffffffu, line < B.line_base[B.G]);
     if (line >= B.line_base[B.G]) return;
     const int pg = pair_of(B.line_base, B.G, line);
     const SweepParams& P = B.P[pg];
@@ -1060,7 +1089,7 @@ __global__ void __launch_bounds__(64)
     const int64_t max_steps = 64 * (F.len + 4 * (S.ncx + S.ncy) + 16);
     int64_t n = walk_range<WRITE ? EMIT_TRIPLES : EMIT_COUNT>(P, F, S, line - F.line_base, F.len - 1, state,
                                   WRITE ? offsets[line] : 0, WRITE ? offsets[line + 1] : 0, raw_in, raw_out,
-                                  raw_val, B.flags + pg, max_steps);
+                                  raw_val, B.flags + pg, max_steps, here);
     if (!WRITE) counts[line] = n;
     if (WRITE && B.out_base[pg] != 0) {
         // output rows of the batch: the pair's rows follow those of the pairs before it
@@ -1186,7 +1215,7 @@ __device__ __forceinline__ int64_t chunk_end(const ChunkPlan& C, const Family& F
 __device__ __forceinline__ void chunk_walk_one(const Batch& B, const WalkState* __restrict__ starts,
                                                WalkState* __restrict__ ends, int64_t* __restrict__ counts,
                                                int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
-                                               double* __restrict__ s_val, int64_t g) {
+                                               double* __restrict__ s_val, int64_t g, unsigned lanes) {
     const int pg = pair_of(B.chunk_base, B.G, g);
     const SweepParams& P = B.P[pg];
     const ChunkPlan& C = B.C[pg];
@@ -1200,7 +1229,7 @@ __device__ __forceinline__ void chunk_walk_one(const Batch& B, const WalkState* 
     int64_t base = C.slot_base[f] + k * C.cap[f];
     const int64_t max_steps = 64 * (C.ch + 4 * (S.ncx + S.ncy) + 16);
     counts[g] = walk_range<EMIT_PIECES>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in, s_out,
-                                 s_val, flags, max_steps);
+                                 s_val, flags, max_steps, lanes);
     ends[g] = st;
 }
 
@@ -1216,15 +1245,17 @@ __global__ void __launch_bounds__(64)
     const int64_t total = B.chunk_base[B.G];
     const int64_t threads = (int64_t)gridDim.x * blockDim.x;
     int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    while (g < total) {
-        chunk_walk_one(B, starts, ends, counts, s_in, s_out, s_val, g);
+    const unsigned lane = threadIdx.x & 31u;
+    while (true) {
+        const unsigned here = __ballot_sync(0xffffffffu, g < total);
+        if (here == 0) return;
+        if (g < total) chunk_walk_one(B, starts, ends, counts, s_in, s_out, s_val, g, here);
+        __syncwarp();
         if (total <= threads) return;
-        const unsigned here = __activemask(), lane = threadIdx.x & 31u;
-        const unsigned leader = __ffs(here) - 1;
         unsigned long long base = 0;
-        if (lane == leader) base = atomicAdd(next_chunk, (unsigned long long)__popc(here));
-        base = __shfl_sync(here, base, leader);
-        g = threads + (int64_t)base + __popc(here & ((1u << lane) - 1u));
+        if (lane == 0) base = atomicAdd(next_chunk, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        g = threads + (int64_t)base + lane;
     }
 }
 
@@ -1271,7 +1302,7 @@ __global__ void __launch_bounds__(128)
             int64_t k = li * C.nc[f] + c;
             int64_t base = C.slot_base[f] + k * C.cap[f];
             counts[g0 + c] = walk_range<EMIT_PIECES>(P, F, S, li, chunk_end(C, F, c), st, base, base + C.cap[f], s_in,
-                                              s_out, s_val, flags, max_steps);
+                                              s_out, s_val, flags, max_steps, 1u);
             ends[g0 + c] = st;
         }
         __syncwarp();
@@ -1369,11 +1400,6 @@ __global__ void slot_count_rows(Batch B, const int64_t* __restrict__ counts, con
         }
         if (active) s_pos[base + q] = make_uint2(pos[0], pos[1]);
     }
-}
-
-// -v without the FP64 pipe
-__device__ __forceinline__ double negated(double v) {
-    return __hiloint2double(__double2hiint(v) ^ INT32_MIN, __double2loint(v));
 }
 
 template <int LANES>
