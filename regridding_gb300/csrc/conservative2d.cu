@@ -197,22 +197,18 @@ __device__ __forceinline__ int crossing_filter(float x1, float y1, float dx12, f
     return (in_t == 1 && in_u == 1) ? 1 : -1;
 }
 
-// seg_hit without the quotients where their bits decide (almost always), for
-// the edges of a cell that the filter leaves open.
-__device__ __noinline__ bool inside_hit(double x1, double y1, double x2, double y2, double x3, double y3, double x4,
-                                        double y4) {
-    if (!bboxes_intersect(x1, y1, x2, y2, x3, y3, x4, y4)) return false;
-    const double dx12 = dsub(x1, x2), dy12 = dsub(y1, y2);
-    const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
-    const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
-    const double tdet = dsub(dmul(x13, y34), dmul(y13, x34));
-    const double det = dsub(dmul(dx12, y34), dmul(dy12, x34));
-    const double udet = dsub(dmul(dx12, y13), dmul(dy12, x13));
-    const int in_t = quotient_in_unit(tdet, det);
-    const int in_u = quotient_in_unit(-udet, det);
+// -v without the FP64 pipe
+__device__ __forceinline__ double negated(double v) {
+    return __hiloint2double(__double2hiint(v) ^ INT32_MIN, __double2loint(v));
+}
+
+// Whether the rounded quotients tdet / det and udet / det lie in [0, 1), from
+// their bits where these decide (almost always).
+__device__ __forceinline__ bool in_unit(double tdet, double udet, double det) {
+    const int in_t = quotient_in_unit(tdet, det), in_u = quotient_in_unit(udet, det);
     if (in_t == 0 || in_u == 0) return false;
     if (in_t > 0 && in_u > 0) return true;
-    const double t = ddiv(tdet, det), u = ddiv(-udet, det);
+    const double t = ddiv(tdet, det), u = ddiv(udet, det);
     return (0 <= t && t < 1) && (0 <= u && u < 1);
 }
 
@@ -826,11 +822,6 @@ struct WalkState {
 // only count (and flag the overflow), as EMIT_COUNT does throughout.  Returns
 // the number of triples or pieces.
 constexpr int EMIT_COUNT = 0, EMIT_TRIPLES = 1, EMIT_PIECES = 2;
-// -v without the FP64 pipe
-__device__ __forceinline__ double negated(double v) {
-    return __hiloint2double(__double2hiint(v) ^ INT32_MIN, __double2loint(v));
-}
-
 template <int EMIT>
 __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Static& S, int64_t li, int64_t j_end,
                               WalkState& state, int64_t wpos, int64_t wend, int32_t* __restrict__ raw_in,
@@ -846,12 +837,73 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
     double x1 = F.SX(li, sy_idx), y1 = F.SY(li, sy_idx);
 
     bool capped = false;
+    int first = 0;  // the edge that the search in a cell begins with
+
+    // the piece of the current segment from (x1, y1) to (xe, ye)
+    const auto emit = [&](double xe, double ye) {
+        // _calc_and_save_weights: area_triangle, negated for axis 0
+        double area = dmul(dsub(dmul(x1, ye), dmul(xe, y1)), 0.5);
+        if (F.axis == 0) area = negated(area);
+        // when the static grid is the input grid both sides share the
+        // input cell, and -area / a_in (times w_in) is exactly the
+        // negation of area / a_in (times w_in): one division serves both
+        double w_static = 0.0;
+        bool have_static = false;
+        if constexpr (EMIT == EMIT_PIECES) {
+            if (wpos < wend) {
+                raw_in[wpos] = (int32_t)(stx * S.ncy + sty);
+                raw_out[wpos] = (int32_t)sy_idx;
+                raw_val[wpos] = area;
+            } else {
+                atomicOr(flags, FLAG_CAPACITY);
+            }
+            wpos++;
+            n_emit++;
+        } else {
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                int64_t is = side == 0 ? li - 1 : li;
+                if (side == 0 && !(is >= 0)) continue;
+                if (side == 1 && !(is < F.lines - 1)) continue;
+                int64_t a = is, b = sy_idx;
+                if (F.axis == 0) { a = sy_idx; b = is; }
+                int64_t ii, ij, oi, oj;
+                if (F.sweep_input) { ii = a; ij = b; oi = stx; oj = sty; }
+                else { ii = stx; ij = sty; oi = a; oj = b; }
+                int64_t in_flat = ii * P.ncy_in + ij;
+                if constexpr (EMIT == EMIT_TRIPLES) {
+                    if (wpos < wend) {
+                        double w;
+                        if (!F.sweep_input && have_static) {
+                            w = -w_static;
+                        } else {
+                            w = area_ratio(side == 0 ? area : -area, __ldg(P.area_in + in_flat));
+                            if (P.w_in) w = dmul(w, __ldg(P.w_in + in_flat));
+                            if (!F.sweep_input && side == 0) {
+                                w_static = w;
+                                have_static = true;
+                            }
+                        }
+                        raw_in[wpos] = (int32_t)in_flat;
+                        raw_out[wpos] = (int32_t)(oi * P.ncy_out + oj);
+                        raw_val[wpos] = w;
+                    } else {
+                        // never write past the slots given to this walk
+                        atomicOr(flags, FLAG_CAPACITY);
+                    }
+                    wpos++;
+                }
+                n_emit++;
+            }
+        }
+    };
+
     while (true) {
         const bool live = sy_idx < j_end && !capped;
         if (!__any_sync(lanes, live)) break;
         bool inside = false;
         double x2 = x1, y2 = y1;
-        if (live && ++steps > max_steps) {
+        if (live && steps >= max_steps) {
             atomicOr(flags, FLAG_WALK_CAP);
             capped = true;
         } else if (live) {
@@ -924,49 +976,71 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 edge_last = MAXSIZE;
                 sy_idx = sy_idx + 1;
             }
+            steps++;
         }
         __syncwarp(lanes);
         // _step_inside_static: first crossed edge of the current static cell
         // other than the entry edge.  The hit test of each candidate edge is
-        // seg_hit's, decided in float32 where that is certain (almost always);
-        // only the edge found needs its crossing parameter.  Same edges, same
-        // order, same t.
+        // seg_hit's, decided in float32 where that is certain; an edge that is
+        // left open ends the search and is decided with its crossing below,
+        // where the FP64 operations of both are the same.  A lane whose
+        // segment ends in its cell writes that piece and searches with the
+        // next segment, so that most lanes come to the crossing with one to
+        // compute: an FP64 instruction costs the same for one lane as for 32.
+        // Same edges, same order, same t.
         int found = -1;
-        if (inside) {
-            // float32 images of the segment for the crossing filter
-            bool seg_ok = true;
-            const float x1f = trunc_float(x1, seg_ok), y1f = trunc_float(y1, seg_ok);
-            const float x2f = trunc_float(x2, seg_ok), y2f = trunc_float(y2, seg_ok);
-            const float dx12f = __fsub_rn(x1f, x2f), dy12f = __fsub_rn(y1f, y2f);
-            const float mseg = fmaxf(fmaxf(fabsf(x1f), fabsf(y1f)), fmaxf(fabsf(x2f), fabsf(y2f)));
-            bool ok3 = seg_ok;
-            float x3f = trunc_float(st.X(stx, sty + 1), ok3), y3f = trunc_float(st.Y(stx, sty + 1), ok3);
+        bool open = false;
+        bool look = inside;
 #pragma unroll 1
-            for (int v = 0; v < 4; v++) {
-                const double x4 = st.X(stx + vertex_i(v), sty + vertex_j(v));
-                const double y4 = st.Y(stx + vertex_i(v), sty + vertex_j(v));
-                bool ok4 = seg_ok;
-                const float x4f = trunc_float(x4, ok4), y4f = trunc_float(y4, ok4);
-                if (found < 0 && v != edge_last) {
-                    // 1: crossed, 0: not crossed (both certain), -1: the FP64 test decides.
-                    // (A certain crossing is one of the boxes, too.)
-                    int dec = -1;
-                    const float m = fmaxf(mseg, fmaxf(fmaxf(fabsf(x3f), fabsf(y3f)), fmaxf(fabsf(x4f), fabsf(y4f))));
-                    if (ok3 && ok4) dec = crossing_filter(x1f, y1f, dx12f, dy12f, x3f, y3f, x4f, y4f, m);
-                    if (dec < 0) {
-                        const int p = (v + 3) & 3;
-                        const double x3 = st.X(stx + vertex_i(p), sty + vertex_j(p));
-                        const double y3 = st.Y(stx + vertex_i(p), sty + vertex_j(p));
-                        dec = inside_hit(x1, y1, x2, y2, x3, y3, x4, y4);
+        for (int pass = 0; pass < 2; pass++) {
+            if (look) {
+                // float32 images of the segment for the crossing filter
+                bool seg_ok = true;
+                const float x1f = trunc_float(x1, seg_ok), y1f = trunc_float(y1, seg_ok);
+                const float x2f = trunc_float(x2, seg_ok), y2f = trunc_float(y2, seg_ok);
+                const float dx12f = __fsub_rn(x1f, x2f), dy12f = __fsub_rn(y1f, y2f);
+                const float mseg = fmaxf(fmaxf(fabsf(x1f), fabsf(y1f)), fmaxf(fabsf(x2f), fabsf(y2f)));
+                bool ok3 = seg_ok;
+                float x3f = trunc_float(st.X(stx, sty + 1), ok3), y3f = trunc_float(st.Y(stx, sty + 1), ok3);
+#pragma unroll 1
+                for (int v = 0; v < 4; v++) {
+                    const double x4 = st.X(stx + vertex_i(v), sty + vertex_j(v));
+                    const double y4 = st.Y(stx + vertex_i(v), sty + vertex_j(v));
+                    bool ok4 = seg_ok;
+                    const float x4f = trunc_float(x4, ok4), y4f = trunc_float(y4, ok4);
+                    if (found < 0 && v >= first && v != edge_last) {
+                        // 1: crossed, 0: not crossed (both certain), -1: open.
+                        // (A certain crossing is one of the boxes, too.)
+                        int dec = -1;
+                        const float m =
+                            fmaxf(mseg, fmaxf(fmaxf(fabsf(x3f), fabsf(y3f)), fmaxf(fabsf(x4f), fabsf(y4f))));
+                        if (ok3 && ok4) dec = crossing_filter(x1f, y1f, dx12f, dy12f, x3f, y3f, x4f, y4f, m);
+                        if (dec != 0) found = v;
+                        open = dec < 0;
                     }
-                    if (dec > 0) found = v;
+                    x3f = x4f;
+                    y3f = y4f;
+                    ok3 = ok4;
                 }
-                x3f = x4f;
-                y3f = y4f;
-                ok3 = ok4;
             }
+            __syncwarp(lanes);
+            if (pass == 1) break;
+            look = look && found < 0;
+            if (look) {
+                emit(x2, y2);
+                steps++;
+                edge_last = MAXSIZE;
+                first = 0;
+                x1 = x2;
+                y1 = y2;
+                look = inside = ++sy_idx < j_end;
+                if (inside) {
+                    x2 = F.SX(li, sy_idx + 1);
+                    y2 = F.SY(li, sy_idx + 1);
+                }
+            }
+            __syncwarp(lanes);
         }
-        __syncwarp(lanes);
         if (found >= 0) {
             const int p = (found + 3) & 3;
             const double x3 = st.X(stx + vertex_i(p), sty + vertex_j(p));
@@ -974,81 +1048,39 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             const double x4 = st.X(stx + vertex_i(found), sty + vertex_j(found));
             const double y4 = st.Y(stx + vertex_i(found), sty + vertex_j(found));
             const double dx12 = dsub(x1, x2), dy12 = dsub(y1, y2);
+            const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
             const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
-            const double tdet = dsub(dmul(dsub(x1, x3), y34), dmul(dsub(y1, y3), x34));
+            const double tdet = dsub(dmul(x13, y34), dmul(y13, x34));
             const double det = dsub(dmul(dx12, y34), dmul(dy12, x34));
-            // x1 + t (x2 - x1), with x2 - x1 the negated difference at hand
-            const double t = ddiv(tdet, det);
-            x2 = dsub(x1, dmul(t, dx12));
-            y2 = dsub(y1, dmul(t, dy12));
+            if (open) {
+                open = !bboxes_intersect(x1, y1, x2, y2, x3, y3, x4, y4) ||
+                       !in_unit(tdet, negated(dsub(dmul(dx12, y13), dmul(dy12, x13))), det);
+            }
+            if (!open) {
+                // x1 + t (x2 - x1), with x2 - x1 the negated difference at hand
+                const double t = ddiv(tdet, det);
+                x2 = dsub(x1, dmul(t, dx12));
+                y2 = dsub(y1, dmul(t, dy12));
+            }
         }
         __syncwarp(lanes);
+        if (open) {
+            // not crossed after all: on with the next edge
+            first = found + 1;
+            continue;
+        }
         if (inside) {
-            int64_t nsy, nstx, nsty;
+            emit(x2, y2);
+            steps++;
+            first = 0;
+            int64_t nstx = stx, nsty = sty;
             if (found >= 0) {
-                nsy = sy_idx;
-                nstx = stx + (found & 1 ? 0 : found - 1);  // cell_normals: _grids.py:143-148
-                nsty = sty + (found & 1 ? found - 2 : 0);
+                nstx += found & 1 ? 0 : found - 1;  // cell_normals: _grids.py:143-148
+                nsty += found & 1 ? found - 2 : 0;
                 edge_last = (found + 2) % 4;
             } else {
-                nsy = sy_idx + 1;
-                nstx = stx;
-                nsty = sty;
+                sy_idx++;
                 edge_last = MAXSIZE;
-            }
-            // _calc_and_save_weights: area_triangle, negated for axis 0
-            double area = dmul(dsub(dmul(x1, y2), dmul(x2, y1)), 0.5);
-            if (F.axis == 0) area = negated(area);
-            // when the static grid is the input grid both sides share the
-            // input cell, and -area / a_in (times w_in) is exactly the
-            // negation of area / a_in (times w_in): one division serves both
-            double w_static = 0.0;
-            bool have_static = false;
-            if constexpr (EMIT == EMIT_PIECES) {
-                if (wpos < wend) {
-                    raw_in[wpos] = (int32_t)(stx * S.ncy + sty);
-                    raw_out[wpos] = (int32_t)sy_idx;
-                    raw_val[wpos] = area;
-                } else {
-                    atomicOr(flags, FLAG_CAPACITY);
-                }
-                wpos++;
-                n_emit++;
-            } else
-#pragma unroll
-            for (int side = 0; side < 2; side++) {
-                int64_t is = side == 0 ? li - 1 : li;
-                if (side == 0 && !(is >= 0)) continue;
-                if (side == 1 && !(is < F.lines - 1)) continue;
-                int64_t a = is, b = sy_idx;
-                if (F.axis == 0) { a = sy_idx; b = is; }
-                int64_t ii, ij, oi, oj;
-                if (F.sweep_input) { ii = a; ij = b; oi = stx; oj = sty; }
-                else { ii = stx; ij = sty; oi = a; oj = b; }
-                int64_t in_flat = ii * P.ncy_in + ij;
-                if constexpr (EMIT == EMIT_TRIPLES) {
-                    if (wpos < wend) {
-                        double w;
-                        if (!F.sweep_input && have_static) {
-                            w = -w_static;
-                        } else {
-                            w = area_ratio(side == 0 ? area : -area, __ldg(P.area_in + in_flat));
-                            if (P.w_in) w = dmul(w, __ldg(P.w_in + in_flat));
-                            if (!F.sweep_input && side == 0) {
-                                w_static = w;
-                                have_static = true;
-                            }
-                        }
-                        raw_in[wpos] = (int32_t)in_flat;
-                        raw_out[wpos] = (int32_t)(oi * P.ncy_out + oj);
-                        raw_val[wpos] = w;
-                    } else {
-                        // never write past the slots given to this walk
-                        atomicOr(flags, FLAG_CAPACITY);
-                    }
-                    wpos++;
-                }
-                n_emit++;
             }
             if (!(nstx >= 0 && nsty >= 0 && nstx < S.ncx && nsty < S.ncy)) {
                 edge_last = stx * S.ncy + sty;
@@ -1056,7 +1088,6 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 nsty = MAXSIZE;
                 outside = true;
             }
-            sy_idx = nsy;
             stx = nstx;
             sty = nsty;
         }
