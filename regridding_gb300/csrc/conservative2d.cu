@@ -799,10 +799,6 @@ __global__ void __launch_bounds__(128) seat_kernel(Batch B, Seat* seats) {
 // the walk
 // ---------------------------------------------------------------------------
 
-// indices_cell_vertex: _grids.py:153-158
-__device__ __forceinline__ int vertex_i(int v) { return (v + 1) >> 1 & 1; }  // 0, 1, 1, 0
-__device__ __forceinline__ int vertex_j(int v) { return v >> 1; }            // 0, 0, 1, 1
-
 // State of a walk at a sweep vertex.  At every vertex the upstream's
 // entry-edge marker is back at sys.maxsize and the current point is the
 // vertex itself, so (outside, static cell) is the whole state.
@@ -812,6 +808,36 @@ struct WalkState {
     int outside;
     int pad;
 };
+
+// The bins of the static boundary that the box (x0, x1) x (y0, y1) of a
+// segment's float32 images may touch, one or two more than FP64 would give:
+// every candidate is tested against the segment itself, so more bins change
+// nothing.  False: certainly none (the box lies beside the boundary's).
+// *bx1 < 0: float32 cannot tell, FP64 has to.  An image is within 2^-23 of its
+// coordinate (at most m) or 2^-126; e is four times what two of them and the
+// roundings add up to.  (The box and bins in FP64 were a fifth of the walk's
+// FP64 operations on 2048^2 -> 1536^2.)
+__device__ __forceinline__ bool boundary_bins(const Static& S, bool ok, float x0, float x1, float y0, float y1, float m,
+                                              int* bx0, int* bx1, int* by0, int* by1) {
+    const float lx = trunc_float(S.blx, ok), ux = trunc_float(S.bux, ok);
+    const float ly = trunc_float(S.bly, ok), uy = trunc_float(S.buy, ok);
+    const Bins& B = S.bins;
+    const float ox = trunc_float(B.ox, ok), oy = trunc_float(B.oy, ok), inv = trunc_float(B.inv_h, ok);
+    m = fmaxf(m, fmaxf(fmaxf(fmaxf(fabsf(lx), fabsf(ux)), fmaxf(fabsf(ly), fabsf(uy))), fmaxf(fabsf(ox), fabsf(oy))));
+    *bx1 = -1;
+    ok = ok && m <= 1.0995116e12f;                                          // 2^40
+    const float e = __fadd_rn(__fmul_rn(9.53674316e-7f, m), 1.17549435e-36f);  // 2^-20 m + 100 * 2^-126
+    if (!ok) return true;
+    if (x1 + e < lx || x0 - e > ux || y1 + e < ly || y0 - e > uy) return false;
+    const float nx = (float)(B.nbx - 1), ny = (float)(B.nby - 1);
+    const float w = __fadd_rn(__fmul_rn(e, inv), __fmul_rn(9.53674316e-7f, fmaxf(nx, ny)));
+    if (!(w < 0.5f)) return true;
+    *bx0 = (int)fminf(fmaxf((x0 - ox) * inv - w, 0.f), nx);
+    *bx1 = (int)fminf(fmaxf((x1 - ox) * inv + w, 0.f), nx);
+    *by0 = (int)fminf(fmaxf((y0 - oy) * inv - w, 0.f), ny);
+    *by1 = (int)fminf(fmaxf((y1 - oy) * inv + w, 0.f), ny);
+    return true;
+}
 
 // The body of the prange loop of _sweep_along_axis (:432-533) with
 // _step_outside_static (:547-698), _step_inside_static (:707-895) and
@@ -827,16 +853,26 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                               WalkState& state, int64_t wpos, int64_t wend, int32_t* __restrict__ raw_in,
                               int32_t* __restrict__ raw_out, double* __restrict__ raw_val, unsigned* flags,
                               int64_t max_steps, unsigned lanes) {
-    const Grid st = S.g;
-    int64_t stx = state.stx, sty = state.sty;
+    // 32-bit indices: cells and vertices are counted below 2^31 and 2^32
+    const double* __restrict__ const vx = S.g.x;
+    const double* __restrict__ const vy = S.g.y;
+    const unsigned row = (unsigned)S.g.ny;  // vertices from one to the next along the first axis
+    const int ncx = (int)S.ncx, ncy = (int)S.ncy;
+    const auto vertex = [&](int x, int y, int v) {  // indices_cell_vertex: _grids.py:153-158
+        return (unsigned)x * row + (unsigned)y + ((v + 1) >> 1 & 1 ? row : 0u) + (unsigned)(v >> 1);
+    };
+    const int64_t along = F.transposed ? F.sweep.ny : 1;  // from one vertex of the line to the next
+    const double* __restrict__ const lx = F.sweep.x + (F.transposed ? li : li * F.sweep.ny);
+    const double* __restrict__ const ly = F.sweep.y + (F.transposed ? li : li * F.sweep.ny);
     bool outside = state.outside;
-    int64_t edge_last = MAXSIZE;
-    int64_t sy_idx = state.sy;
-    int64_t n_emit = 0;
-    int64_t steps = 0;
-    double x1 = F.SX(li, sy_idx), y1 = F.SY(li, sy_idx);
-
-    bool capped = false;
+    int stx = outside ? 0 : (int)state.stx, sty = outside ? 0 : (int)state.sty;
+    constexpr int NONE = -1;
+    int edge_last = NONE;
+    int sy_idx = (int)state.sy, end = (int)j_end;
+    int n_emit = 0;
+    int steps = 0;
+    const int step_limit = (int)(max_steps < INT32_MAX ? max_steps : INT32_MAX);
+    double x1 = __ldg(lx + sy_idx * along), y1 = __ldg(ly + sy_idx * along);
     int first = 0;  // the edge that the search in a cell begins with
 
     // the piece of the current segment from (x1, y1) to (xe, ye)
@@ -851,8 +887,8 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
         bool have_static = false;
         if constexpr (EMIT == EMIT_PIECES) {
             if (wpos < wend) {
-                raw_in[wpos] = (int32_t)(stx * S.ncy + sty);
-                raw_out[wpos] = (int32_t)sy_idx;
+                raw_in[wpos] = stx * ncy + sty;
+                raw_out[wpos] = sy_idx;
                 raw_val[wpos] = area;
             } else {
                 atomicOr(flags, FLAG_CAPACITY);
@@ -899,24 +935,24 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
     };
 
     while (true) {
-        const bool live = sy_idx < j_end && !capped;
+        const bool live = sy_idx < end;
         if (!__any_sync(lanes, live)) break;
         bool inside = false;
         double x2 = x1, y2 = y1;
-        if (live && steps >= max_steps) {
+        bool enter = false;
+        if (live && steps >= step_limit) {
             atomicOr(flags, FLAG_WALK_CAP);
-            capped = true;
+            end = sy_idx;
         } else if (live) {
-            x2 = F.SX(li, sy_idx + 1);
-            y2 = F.SY(li, sy_idx + 1);
+            x2 = __ldg(lx + (sy_idx + 1) * along);
+            y2 = __ldg(ly + (sy_idx + 1) * along);
             inside = !outside;
+            enter = outside;
         }
-        if (live && !capped && outside) {
+        if (enter) {
             // _step_outside_static: smallest-t crossing of the static boundary,
             // candidates from the bins overlapping the segment's box
             const double p2x = x2, p2y = y2;
-            double sminx = fmin(x1, p2x), smaxx = fmax(x1, p2x);
-            double sminy = fmin(y1, p2y), smaxy = fmax(y1, p2y);
             bool found = false;
             double t_min = INFINITY;
             // float32 images of the segment for the crossing filter
@@ -925,15 +961,17 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             const float x2f = trunc_float(p2x, seg_ok), y2f = trunc_float(p2y, seg_ok);
             const float dx12f = __fsub_rn(x1f, x2f), dy12f = __fsub_rn(y1f, y2f);
             const float mseg = fmaxf(fmaxf(fabsf(x1f), fabsf(y1f)), fmaxf(fabsf(x2f), fabsf(y2f)));
-            int64_t best_order = INT64_MAX;
-            int best_code = 0;
-            int64_t best_cell = 0;
-            if (!(smaxx < S.blx || sminx > S.bux || smaxy < S.bly || sminy > S.buy)) {
-                const Bins& B = S.bins;
-                int bx0 = bin_coord(sminx, B.ox, B.inv_h, B.nbx);
-                int bx1 = bin_coord(smaxx, B.ox, B.inv_h, B.nbx);
-                int by0 = bin_coord(sminy, B.oy, B.inv_h, B.nby);
-                int by1 = bin_coord(smaxy, B.oy, B.inv_h, B.nby);
+            int best_order = INT32_MAX, best_code = 0, best_cell = 0;
+            const Bins& B = S.bins;
+            int bx0, bx1, by0, by1;
+            if (boundary_bins(S, seg_ok, fminf(x1f, x2f), fmaxf(x1f, x2f), fminf(y1f, y2f), fmaxf(y1f, y2f), mseg, &bx0,
+                              &bx1, &by0, &by1)) {
+                if (bx1 < 0) {
+                    bx0 = bin_coord(fmin(x1, p2x), B.ox, B.inv_h, B.nbx);
+                    bx1 = bin_coord(fmax(x1, p2x), B.ox, B.inv_h, B.nbx);
+                    by0 = bin_coord(fmin(y1, p2y), B.oy, B.inv_h, B.nby);
+                    by1 = bin_coord(fmax(y1, p2y), B.oy, B.inv_h, B.nby);
+                }
                 for (int by = by0; by <= by1; by++) {
                     for (int bx = bx0; bx <= bx1; bx++) {
                         int64_t bin = (int64_t)by * B.nbx + bx;
@@ -953,12 +991,12 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                             }
                             double t;
                             if (!seg_hit(x1, y1, p2x, p2y, e.x3, e.y3, e.x4, e.y4, &t)) continue;
-                            if (e.cell == edge_last) continue;
+                            if ((int)e.cell == edge_last) continue;
                             if (t < t_min || (t == t_min && ek < best_order)) {
                                 t_min = t;
                                 best_order = ek;
                                 best_code = e.code;
-                                best_cell = e.cell;
+                                best_cell = (int)e.cell;
                                 found = true;
                             }
                         }
@@ -966,14 +1004,14 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 }
             }
             if (found) {
-                stx = best_cell / S.ncy;
-                sty = best_cell % S.ncy;
+                stx = best_cell / ncy;
+                sty = best_cell % ncy;
                 x2 = dadd(x1, dmul(t_min, dsub(p2x, x1)));
                 y2 = dadd(y1, dmul(t_min, dsub(p2y, y1)));
                 edge_last = best_code;
                 outside = false;
             } else {
-                edge_last = MAXSIZE;
+                edge_last = NONE;
                 sy_idx = sy_idx + 1;
             }
             steps++;
@@ -1001,13 +1039,13 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 const float dx12f = __fsub_rn(x1f, x2f), dy12f = __fsub_rn(y1f, y2f);
                 const float mseg = fmaxf(fmaxf(fabsf(x1f), fabsf(y1f)), fmaxf(fabsf(x2f), fabsf(y2f)));
                 bool ok3 = seg_ok;
-                float x3f = trunc_float(st.X(stx, sty + 1), ok3), y3f = trunc_float(st.Y(stx, sty + 1), ok3);
+                const unsigned k3 = vertex(stx, sty, 3);
+                float x3f = trunc_float(__ldg(vx + k3), ok3), y3f = trunc_float(__ldg(vy + k3), ok3);
 #pragma unroll 1
                 for (int v = 0; v < 4; v++) {
-                    const double x4 = st.X(stx + vertex_i(v), sty + vertex_j(v));
-                    const double y4 = st.Y(stx + vertex_i(v), sty + vertex_j(v));
+                    const unsigned k4 = vertex(stx, sty, v);
                     bool ok4 = seg_ok;
-                    const float x4f = trunc_float(x4, ok4), y4f = trunc_float(y4, ok4);
+                    const float x4f = trunc_float(__ldg(vx + k4), ok4), y4f = trunc_float(__ldg(vy + k4), ok4);
                     if (found < 0 && v >= first && v != edge_last) {
                         // 1: crossed, 0: not crossed (both certain), -1: open.
                         // (A certain crossing is one of the boxes, too.)
@@ -1029,24 +1067,21 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             if (look) {
                 emit(x2, y2);
                 steps++;
-                edge_last = MAXSIZE;
+                edge_last = NONE;
                 first = 0;
                 x1 = x2;
                 y1 = y2;
-                look = inside = ++sy_idx < j_end;
+                look = inside = ++sy_idx < end;
                 if (inside) {
-                    x2 = F.SX(li, sy_idx + 1);
-                    y2 = F.SY(li, sy_idx + 1);
+                    x2 = __ldg(lx + (sy_idx + 1) * along);
+                    y2 = __ldg(ly + (sy_idx + 1) * along);
                 }
             }
             __syncwarp(lanes);
         }
         if (found >= 0) {
-            const int p = (found + 3) & 3;
-            const double x3 = st.X(stx + vertex_i(p), sty + vertex_j(p));
-            const double y3 = st.Y(stx + vertex_i(p), sty + vertex_j(p));
-            const double x4 = st.X(stx + vertex_i(found), sty + vertex_j(found));
-            const double y4 = st.Y(stx + vertex_i(found), sty + vertex_j(found));
+            const unsigned k3 = vertex(stx, sty, (found + 3) & 3), k4 = vertex(stx, sty, found);
+            const double x3 = __ldg(vx + k3), y3 = __ldg(vy + k3), x4 = __ldg(vx + k4), y4 = __ldg(vy + k4);
             const double dx12 = dsub(x1, x2), dy12 = dsub(y1, y2);
             const double x13 = dsub(x1, x3), y13 = dsub(y1, y3);
             const double x34 = dsub(x3, x4), y34 = dsub(y3, y4);
@@ -1073,29 +1108,25 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             emit(x2, y2);
             steps++;
             first = 0;
-            int64_t nstx = stx, nsty = sty;
+            const int cell = stx * ncy + sty;
             if (found >= 0) {
-                nstx += found & 1 ? 0 : found - 1;  // cell_normals: _grids.py:143-148
-                nsty += found & 1 ? found - 2 : 0;
-                edge_last = (found + 2) % 4;
+                stx += found & 1 ? 0 : found - 1;  // cell_normals: _grids.py:143-148
+                sty += found & 1 ? found - 2 : 0;
+                edge_last = (found + 2) & 3;
             } else {
                 sy_idx++;
-                edge_last = MAXSIZE;
+                edge_last = NONE;
             }
-            if (!(nstx >= 0 && nsty >= 0 && nstx < S.ncx && nsty < S.ncy)) {
-                edge_last = stx * S.ncy + sty;
-                nstx = MAXSIZE;
-                nsty = MAXSIZE;
+            if (!(stx >= 0 && sty >= 0 && stx < ncx && sty < ncy)) {
+                edge_last = cell;
                 outside = true;
             }
-            stx = nstx;
-            sty = nsty;
         }
         x1 = x2;  // (unchanged where the walk has ended)
         y1 = y2;
     }
-    state.stx = stx;
-    state.sty = sty;
+    state.stx = outside ? MAXSIZE : stx;
+    state.sty = outside ? MAXSIZE : sty;
     state.sy = sy_idx;
     state.outside = outside;
     return n_emit;
