@@ -1610,7 +1610,7 @@ __device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& 
     return w;
 }
 
-// Buckets to merged rows, ORDER_ROWS rows per block, a thread per triple, then
+// Buckets to merged rows, `per` rows per block, a thread per triple, then
 // one per merged entry.  The keys go to shared memory; a triple's rank is the
 // number of keys of its row below its own (keys are unique); it is stored at
 // its rank, the first of a row marked.  Each run of one input cell is then
@@ -1621,15 +1621,22 @@ __device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& 
 // them the ranking.  A warp per row in the ranking and a lane per row in the
 // merge took 0.98 ms; a launch each for ranking, merging and compacting
 // through global memory 0.78, 0.42 and 0.17 ms.)
-constexpr int ORDER_ROWS = 32;
+// The host takes 32, 8 or 2 rows per block, for up to 40, 160 or more triples
+// per row, so that a block's rows mostly fit BLOCK_TRIPLES (2048^2 -> 300^2,
+// 230 triples per row: with 32 every block was listed and order_rows_long took
+// 10.2 ms; now 1.5.)
+constexpr int ORDER_ROWS = 32;  // at most
+__host__ __forceinline__ int order_rows_per_block(int64_t triples, int64_t rows) {
+    return triples <= 40 * rows ? 32 : triples <= 160 * rows ? 8 : 2;
+}
 constexpr int ORDER_THREADS = 256;
-constexpr int ROW_SMALL = 256;       // a row's ranks cost its square
+constexpr int ROW_SMALL = 1024;      // a row's ranks cost its square
 constexpr int BLOCK_TRIPLES = 2048;  // 40 KB of shared memory
 constexpr int32_t ROW_HEAD = INT32_MIN;
 
 // The rows' merged counts to the block's prefix (pre[ORDER_ROWS] their total)
 // and to row_nnz; by one warp.
-__device__ __forceinline__ void order_counts(int64_t r0, int64_t nrows, int mine, int* pre, int64_t* row_nnz) {
+__device__ __forceinline__ void order_counts(int64_t r0, int64_t r1, int mine, int* pre, int64_t* row_nnz) {
     const int lane = threadIdx.x & 31;
     int incl = mine;
 #pragma unroll
@@ -1639,9 +1646,10 @@ __device__ __forceinline__ void order_counts(int64_t r0, int64_t nrows, int mine
     }
     pre[lane + 1] = incl;
     if (lane == 0) pre[0] = 0;
-    if (r0 + lane < nrows) row_nnz[r0 + lane] = mine;
+    if (r0 + lane < r1) row_nnz[r0 + lane] = mine;
 }
 
+template <int PER>
 __global__ void __launch_bounds__(ORDER_THREADS)
     order_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
                int32_t* __restrict__ tmp_col, double* __restrict__ tmp_val, int64_t* __restrict__ row_nnz,
@@ -1649,28 +1657,28 @@ __global__ void __launch_bounds__(ORDER_THREADS)
     __shared__ int64_t key[BLOCK_TRIPLES];
     __shared__ double val[BLOCK_TRIPLES];
     __shared__ int32_t in[BLOCK_TRIPLES];
-    __shared__ int start[ORDER_ROWS + 1];
+    __shared__ int start[PER + 1];
     __shared__ unsigned heads[BLOCK_TRIPLES / 32 + 1];  // a bit per triple that begins a run
     __shared__ int before[BLOCK_TRIPLES / 32 + 1];      // runs before each word of heads
     const int t = threadIdx.x, lane = t & 31;
-    const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, s0 = row_start[r0];
+    const int64_t r0 = (int64_t)blockIdx.x * PER, s0 = row_start[r0];
     bool longer = false;
-    if (t <= ORDER_ROWS) {
+    if (t <= PER) {
         const int64_t r = r0 + t < nrows ? r0 + t : nrows, s = row_start[r];
-        longer = t == ORDER_ROWS ? s - s0 > BLOCK_TRIPLES : r < nrows && row_start[r + 1] - s > ROW_SMALL;
+        longer = t == PER ? s - s0 > BLOCK_TRIPLES : r < nrows && row_start[r + 1] - s > ROW_SMALL;
         start[t] = (int)(s - s0);
     }
     if (__syncthreads_or(longer)) {
         if (t == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)blockIdx.x;
         return;
     }
-    const int n = start[ORDER_ROWS];
+    const int n = start[PER];
     for (int e = t; e < n; e += ORDER_THREADS) key[e] = triples[s0 + e].key;
     __syncthreads();
     for (int e = t; e < n; e += ORDER_THREADS) {
         int r = 0;
 #pragma unroll
-        for (int d = ORDER_ROWS / 2; d > 0; d >>= 1)
+        for (int d = PER / 2; d > 0; d >>= 1)
             if (start[r + d] <= e) r += d;
         const int s = start[r], m = start[r + 1];
         const int64_t mine = key[e];
@@ -1705,7 +1713,7 @@ __global__ void __launch_bounds__(ORDER_THREADS)
     }
     __syncthreads();
     const auto runs_before = [&](int e) { return before[e >> 5] + __popc(heads[e >> 5] & ((1u << (e & 31)) - 1u)); };
-    if (t < ORDER_ROWS && r0 + t < nrows) row_nnz[r0 + t] = runs_before(start[t + 1]) - runs_before(start[t]);
+    if (t < PER && r0 + t < nrows) row_nnz[r0 + t] = runs_before(start[t + 1]) - runs_before(start[t]);
     uint16_t* run = reinterpret_cast<uint16_t*>(key);  // where each run begins
     for (int e = t; e < n; e += ORDER_THREADS)
         if (heads[e >> 5] >> (e & 31) & 1u) run[runs_before(e)] = (uint16_t)e;
@@ -1723,15 +1731,16 @@ __global__ void __launch_bounds__(ORDER_THREADS)
 // and pass; then merged by a lane each, and moved together.
 constexpr int ROW_TILE = 2048;
 __global__ void __launch_bounds__(256)
-    order_rows_long(const int64_t* __restrict__ row_start, int64_t nrows, const int32_t* __restrict__ long_list,
+    order_rows_long(const int64_t* __restrict__ row_start, int64_t nrows, int per, const int32_t* __restrict__ long_list,
                     const unsigned* __restrict__ long_count, const Triple* __restrict__ triples,
                     int32_t* tmp_col, double* tmp_val, int64_t* __restrict__ row_nnz) {
     __shared__ int64_t tile[ROW_TILE];
     __shared__ int pre[ORDER_ROWS + 1];
     const unsigned nl = *long_count;
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
-        const int64_t r0 = (int64_t)long_list[li] * ORDER_ROWS, s0 = row_start[r0];
-        for (int64_t r = r0; r < r0 + ORDER_ROWS && r < nrows; r++) {
+        const int64_t r0 = (int64_t)long_list[li] * per, s0 = row_start[r0];
+        const int64_t r1 = r0 + per < nrows ? r0 + per : nrows;
+        for (int64_t r = r0; r < r1; r++) {
             const int64_t s = row_start[r], t = row_start[r + 1], len = t - s;
             for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
                 int64_t mykey[8];
@@ -1747,10 +1756,18 @@ __global__ void __launch_bounds__(256)
                     __syncthreads();
                     for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
                     __syncthreads();
-                    for (int64_t q = 0; q < m; q++) {
-                        const int64_t kq = tile[q];
+                    // (eight keys for each read of the tile, or the one of a short row)
+                    if (t - e0 > blockDim.x) {
+                        for (int64_t q = 0; q < m; q++) {
+                            const int64_t kq = tile[q];
 #pragma unroll
-                        for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
+                            for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
+                        }
+                    } else {
+                        int below = 0;
+#pragma unroll 4
+                        for (int q = 0; q < (int)m; q++) below += tile[q] < mykey[0];
+                        rank[0] += below;
                     }
                 }
 #pragma unroll
@@ -1767,7 +1784,7 @@ __global__ void __launch_bounds__(256)
         if (threadIdx.x < 32) {
             const int64_t r = r0 + threadIdx.x;
             int64_t n = 0;
-            if (r < nrows) {
+            if (r < r1) {
                 const int64_t s = row_start[r];
                 n = merge_sorted(
                         s, row_start[r + 1], [&](int64_t k) { return tmp_col[k]; },
@@ -1778,11 +1795,11 @@ __global__ void __launch_bounds__(256)
                         }) -
                     s;
             }
-            order_counts(r0, nrows, (int)n, pre, row_nnz);
+            order_counts(r0, r1, (int)n, pre, row_nnz);
         }
         __syncthreads();
         // (entries move towards the front: a pass reads before any of it writes)
-        for (int r = 0; r < ORDER_ROWS && r0 + r < nrows; r++) {
+        for (int r = 0; r0 + r < r1; r++) {
             const int64_t src = row_start[r0 + r] - pre[r];
             for (int e0 = pre[r]; e0 < pre[r + 1]; e0 += blockDim.x) {
                 const int e = e0 + threadIdx.x;
@@ -1803,10 +1820,10 @@ __global__ void __launch_bounds__(256)
 // The blocks' merged entries to their place in the CSR.
 constexpr int COPY_THREADS = 128;
 __global__ void __launch_bounds__(COPY_THREADS)
-    copy_blocks(const int64_t* __restrict__ row_start, const int64_t* __restrict__ row_ptr, int64_t nrows,
+    copy_blocks(const int64_t* __restrict__ row_start, const int64_t* __restrict__ row_ptr, int64_t nrows, int per,
                 const int32_t* __restrict__ tmp_col, const double* __restrict__ tmp_val, int32_t* __restrict__ col,
                 double* __restrict__ val) {
-    const int64_t r0 = (int64_t)blockIdx.x * ORDER_ROWS, r1 = r0 + ORDER_ROWS < nrows ? r0 + ORDER_ROWS : nrows;
+    const int64_t r0 = (int64_t)blockIdx.x * per, r1 = r0 + per < nrows ? r0 + per : nrows;
     const int64_t s = row_start[r0], d = row_ptr[r0], n = row_ptr[r1] - d;
     for (int64_t e = threadIdx.x; e < n; e += COPY_THREADS) {
         col[d + e] = tmp_col[s + e];
@@ -2001,9 +2018,10 @@ int sweep_lines(const Batch& B, int64_t lines, const Seat* seats, int64_t* total
 // The triples merged by output row straight from the chunks' slots
 // (slot_count_rows, slot_scatter_rows, order_rows): row_start[n_rows + 1] of
 // the buckets, the rows' merged counts, and the merged entries of every
-// ORDER_ROWS rows from their first bucket's start on.
+// `per` rows from their first bucket's start on.
 struct MergedRows {
     int64_t n_rows = 0;
+    int per = 0;
     int64_t* row_start = nullptr;
     int64_t* row_nnz = nullptr;
     int32_t* col = nullptr;
@@ -2141,7 +2159,8 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 if ((st = dalloc(&rows->val, (size_t)nraw, s))) break;
                 if ((st = dalloc(&rowc, (size_t)nr + 1, s))) break;
                 if ((st = dalloc(&long_count, 1, s))) break;
-                if ((st = dalloc(&long_list, (size_t)(nr / ORDER_ROWS + 1), s))) break;
+                rows->per = order_rows_per_block(nraw, nr);
+                if ((st = dalloc(&long_list, (size_t)(nr / rows->per + 1), s))) break;
                 if ((st = dalloc(&triples, (size_t)nraw, s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
                 zero_async(long_count, sizeof(unsigned), s);
@@ -2156,11 +2175,12 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 count<<<gc, 256, 0, s>>>(B, counts, s_in, s_out, rowc, s_pos);
                 if ((st = exclusive_scan_u32_to_i64(rowc, rows->row_start, nr + 1, nullptr, s))) break;
                 scatter<<<gc, 256, 0, s>>>(B, counts, offsets, s_in, s_out, s_val, s_pos, rows->row_start, triples);
-                const unsigned blocks = grid_for(nr, ORDER_ROWS);
-                order_rows<<<blocks, ORDER_THREADS, 0, s>>>(rows->row_start, nr, triples, rows->col, rows->val,
-                                                            rows->row_nnz, long_list, long_count);
-                order_rows_long<<<std::min(blocks, 152u * 8u), 256, 0, s>>>(rows->row_start, nr, long_list, long_count,
-                                                                            triples, rows->col, rows->val,
+                const unsigned blocks = grid_for(nr, rows->per);
+                const auto order = rows->per == 32 ? order_rows<32> : rows->per == 8 ? order_rows<8> : order_rows<2>;
+                order<<<blocks, ORDER_THREADS, 0, s>>>(rows->row_start, nr, triples, rows->col, rows->val,
+                                                       rows->row_nnz, long_list, long_count);
+                order_rows_long<<<std::min(blocks, 152u * 8u), 256, 0, s>>>(rows->row_start, nr, rows->per, long_list,
+                                                                            long_count, triples, rows->col, rows->val,
                                                                             rows->row_nnz);
             } while (0);
             dfree(rowc, s);
@@ -2487,8 +2507,8 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         if ((st = dalloc(&col, (size_t)nnz, s))) break;
         if ((st = dalloc(&val, (size_t)nnz, s))) break;
         if (merged)
-            copy_blocks<<<grid_for(n_out_all, ORDER_ROWS), COPY_THREADS, 0, s>>>(bucket_ptr, row_ptr, n_out_all, tmp_col,
-                                                                                  tmp_val, col, val);
+            copy_blocks<<<grid_for(n_out_all, rows.per), COPY_THREADS, 0, s>>>(bucket_ptr, row_ptr, n_out_all, rows.per,
+                                                                               tmp_col, tmp_val, col, val);
         else
             compact_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, row_ptr, tmp_col, tmp_val, n_out_all, col,
                                                                   val);
