@@ -501,20 +501,20 @@ __device__ __forceinline__ int grid_of_edge(const PrepGrid* __restrict__ P, int 
 
 // Areas of the input cells of every pair, in area_in's order (pair by pair),
 // each with its reciprocal for area_ratio.
-__global__ void cell_area_batch(const PrepGrid* __restrict__ P, int G, int64_t ncells, double2* __restrict__ out) {
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncells;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        int lo = 0, hi = G - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (P[2 * mid].cell_base <= c) lo = mid;
-            else hi = mid - 1;
-        }
-        const Grid g = P[2 * lo].g;
-        const int64_t local = c - P[2 * lo].cell_base, ncy = g.ny - 1;
-        const double a = cell_area_at(g.x, g.y, g.ny, local / ncy, local % ncy);
-        out[c] = make_double2(a, ddiv(1.0, a));
+__device__ __forceinline__ void cell_areas(unsigned block, const PrepGrid* __restrict__ P, int G, int64_t ncells,
+                                           double2* __restrict__ out) {
+    const int64_t c = block * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= ncells) return;
+    int lo = 0, hi = G - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (P[2 * mid].cell_base <= c) lo = mid;
+        else hi = mid - 1;
     }
+    const Grid g = P[2 * lo].g;
+    const int64_t local = c - P[2 * lo].cell_base, ncy = g.ny - 1;
+    const double a = cell_area_at(g.x, g.y, g.ny, local / ncy, local % ncy);
+    out[c] = make_double2(a, ddiv(1.0, a));
 }
 
 // a / cell.x, correctly rounded, from the cell's rounded reciprocal cell.y:
@@ -542,10 +542,10 @@ __device__ __forceinline__ double area_ratio(double a, double2 cell) {
 // blocks of 256 threads per grid fold strided vertices into partial
 // extrema, then one warp per grid combines them (min and max are exact in
 // any order, so the partition does not matter).
-__global__ void __launch_bounds__(256) bbox_partial_batch(const PrepGrid* __restrict__ P, int nparts,
-                                                          double* __restrict__ part) {
+__device__ __forceinline__ void box_parts(unsigned block, const PrepGrid* __restrict__ P, int nparts,
+                                          double* __restrict__ part) {
     __shared__ long long sh[4][8];
-    const int k = blockIdx.x / nparts, p = blockIdx.x % nparts;
+    const int k = block / nparts, p = block % nparts;
     const Grid g = P[k].g;
     const int64_t n = g.nx * g.ny;
     // extrema of the order keys (no FP64 instruction); NaN is left out, and
@@ -612,12 +612,22 @@ __global__ void bbox_combine_batch(const double* __restrict__ part, int nparts, 
     }
 }
 
-__global__ void boundary_edges_batch(const PrepGrid* __restrict__ P, int ngrids, int64_t nedges,
-                                     Edge* __restrict__ edges) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nedges;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int k = grid_of_edge(P, ngrids, e);
+// What the builds of a batch prepare from the vertices alone, by one launch of
+// 256 threads a block: the first box_blocks blocks the parts of the bounding
+// boxes, edge_blocks the boundary edges, the rest the input cells' areas.
+__global__ void __launch_bounds__(256)
+    prepare_batch(const PrepGrid* __restrict__ P, int G, unsigned box_blocks, int nparts, double* __restrict__ part,
+                  unsigned edge_blocks, int64_t nedges, Edge* __restrict__ edges, int64_t ncells,
+                  double2* __restrict__ areas) {
+    if (blockIdx.x < box_blocks) {
+        box_parts(blockIdx.x, P, nparts, part);
+    } else if (blockIdx.x < box_blocks + edge_blocks) {
+        const int64_t e = (blockIdx.x - box_blocks) * (int64_t)blockDim.x + threadIdx.x;
+        if (e >= nedges) return;
+        const int k = grid_of_edge(P, 2 * G, e);
         edges[e] = boundary_edge(P[k].g, e - P[k].edge_base);
+    } else {
+        cell_areas(blockIdx.x - box_blocks - edge_blocks, P, G, ncells, areas);
     }
 }
 
@@ -1241,7 +1251,8 @@ __device__ WalkState guess_state(const Static& S, double px, double py, int64_t 
 // lines' first chunks; the others guess, a thread for each further chunk.  Both
 // are chains of dependent steps on few threads, so they run side by side.
 __global__ void __launch_bounds__(128)
-    chunk_seat_kernel(Batch B, unsigned seat_blocks, Seat* __restrict__ seats, WalkState* __restrict__ starts) {
+    chunk_seat_kernel(Batch B, unsigned seat_blocks, Seat* __restrict__ seats, WalkState* __restrict__ starts,
+                      int64_t* __restrict__ counts) {
     if (blockIdx.x < seat_blocks) {
         const int64_t line = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
         if (line >= B.line_base[B.G]) return;
@@ -1257,7 +1268,10 @@ __global__ void __launch_bounds__(128)
         return;
     }
     int64_t g = (blockIdx.x - seat_blocks) * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= B.chunk_base[B.G]) return;
+    if (g >= B.chunk_base[B.G]) {
+        if (g == B.chunk_base[B.G]) counts[g] = 0;  // the scan's last element
+        return;
+    }
     const int pg = pair_of(B.chunk_base, B.G, g);
     const SweepParams& P = B.P[pg];
     const ChunkPlan& C = B.C[pg];
@@ -1663,6 +1677,7 @@ __global__ void __launch_bounds__(ORDER_THREADS)
     const int t = threadIdx.x, lane = t & 31;
     const int64_t r0 = (int64_t)blockIdx.x * PER, s0 = row_start[r0];
     bool longer = false;
+    if (t == 0 && blockIdx.x == 0) row_nnz[nrows] = 0;  // the scan's last element
     if (t <= PER) {
         const int64_t r = r0 + t < nrows ? r0 + t : nrows, s = row_start[r];
         longer = t == PER ? s - s0 > BLOCK_TRIPLES : r < nrows && row_start[r + 1] - s > ROW_SMALL;
@@ -1978,8 +1993,46 @@ int upload(T** d, const std::vector<T>& h, cudaStream_t s) {
     return RG_OK;
 }
 
+// Small arrays that go to the device together: one allocation, one copy.
+struct Pack {
+    std::vector<unsigned char> bytes;
+    unsigned char* dev = nullptr;
+    size_t add(const void* src, size_t n) {  // null: zeros
+        const size_t at = (bytes.size() + 15) & ~(size_t)15;
+        bytes.resize(at + n, 0);
+        if (src) memcpy(bytes.data() + at, src, n);
+        return at;
+    }
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        return add(v.data(), sizeof(T) * v.size());
+    }
+    int to_device(cudaStream_t s) {
+        RG_TRY(dalloc(&dev, bytes.size(), s));
+        return small_to_device(dev, bytes.data(), bytes.size(), s);
+    }
+    template <typename T>
+    T* at(size_t offset) const {
+        return reinterpret_cast<T*>(dev + offset);
+    }
+};
+
+// A count on the device and the grids' error words, which follow it, by one copy.
+int count_and_flags(const int64_t* total_dev, int64_t* total, std::vector<unsigned>& fl, cudaStream_t s) {
+    std::vector<unsigned char> buf(sizeof(int64_t) + sizeof(unsigned) * fl.size());
+    RG_TRY(small_to_host(buf.data(), total_dev, buf.size(), s));
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        set_error("conservative sweep: %s", cudaGetErrorString(e));
+        return RG_ERR_CUDA;
+    }
+    memcpy(total, buf.data(), sizeof(int64_t));
+    memcpy(fl.data(), buf.data() + sizeof(int64_t), sizeof(unsigned) * fl.size());
+    return RG_OK;
+}
+
 // One thread per line over all lines of the batch, count then write
-// (synchronises once).  fl receives every grid's error word.
+// (synchronises once; total_dev with the error words behind it).  fl receives every grid's error word.
 int sweep_lines(const Batch& B, int64_t lines, const Seat* seats, int64_t* total_dev, cudaStream_t s,
                 int32_t** raw_in, int32_t** raw_out, double** raw_val, int64_t* nraw_out, std::vector<unsigned>& fl) {
     int64_t *counts = nullptr, *offsets = nullptr;
@@ -1991,14 +2044,7 @@ int sweep_lines(const Batch& B, int64_t lines, const Seat* seats, int64_t* total
         zero_async(counts + lines, sizeof(int64_t), s);
         if ((st = exclusive_scan_i64(counts, offsets, lines + 1, total_dev, s))) break;
         int64_t nraw = 0;
-        small_to_host(&nraw, total_dev, sizeof(int64_t), s);
-        small_to_host(fl.data(), B.flags, sizeof(unsigned) * fl.size(), s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_error("conservative sweep (count walk): %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
-            break;
-        }
+        if ((st = count_and_flags(total_dev, &nraw, fl, s))) break;
         if (nraw >= (int64_t)UINT32_MAX) {
             set_error("conservative sweep: %lld raw entries exceed 2^32", (long long)nraw);
             st = RG_ERR_UNSUPPORTED;
@@ -2035,7 +2081,7 @@ struct MergedRows {
 
 int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector<double>& bbox_h,
                   Seat* seats, int64_t lines, int64_t* total_dev, cudaStream_t s, int64_t* nraw_out,
-                  std::vector<unsigned>& fl, ChunkPlan** plans_dev, int64_t** chunk_base_dev, MergedRows* rows) {
+                  std::vector<unsigned>& fl, unsigned char** plans_dev, MergedRows* rows) {
     const int G = B.G;
     // sweep segments per chunk: rg_set_sweep_chunk (default 32), the
     // RG_SWEEP_CHUNK environment variable overriding it (0 walks whole lines)
@@ -2101,40 +2147,36 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
     int st = RG_OK;
     bool overflow = false;
     do {
-        if ((st = upload(plans_dev, C, s))) break;
-        if ((st = upload(chunk_base_dev, chunk_base, s))) break;
-        B.C = *plans_dev;
-        B.chunk_base = *chunk_base_dev;
+        // the plans, and two counts: chunks repaired, next chunk of the walk
+        Pack pack;
+        const size_t plans_at = pack.add(C), base_at = pack.add(chunk_base);
+        const size_t rep_at = pack.add(nullptr, 2 * sizeof(unsigned long long));
+        st = pack.to_device(s);
+        *plans_dev = pack.dev;
+        if (st) break;
+        B.C = pack.at<ChunkPlan>(plans_at);
+        B.chunk_base = pack.at<int64_t>(base_at);
+        n_rep = pack.at<unsigned long long>(rep_at);
         if ((st = dalloc(&starts, (size_t)chunks, s))) break;
         if ((st = dalloc(&ends, (size_t)chunks, s))) break;
         if ((st = dalloc(&counts, (size_t)chunks + 1, s))) break;
         if ((st = dalloc(&offsets, (size_t)chunks + 1, s))) break;
-        if ((st = dalloc(&n_rep, 2, s))) break;  // chunks repaired, next chunk of the walk
         if ((st = dalloc(&s_in, (size_t)slots, s))) break;
         if ((st = dalloc(&s_out, (size_t)slots, s))) break;
         if ((st = dalloc(&s_val, (size_t)slots, s))) break;
         if ((st = dalloc(&s_pos, (size_t)slots, s))) break;
-        zero_async(n_rep, 2 * sizeof(unsigned long long), s);
         const unsigned seat_blocks = grid_for(lines * 32, 128);
-        chunk_seat_kernel<<<seat_blocks + grid_for(chunks, 128), 128, 0, s>>>(B, seat_blocks, seats, starts);
+        chunk_seat_kernel<<<seat_blocks + grid_for(chunks + 1, 128), 128, 0, s>>>(B, seat_blocks, seats, starts, counts);
         {
             // resident blocks only: 8 blocks of 64 threads per SM
             const unsigned blocks = std::min<unsigned>(grid_for(chunks, 64), 152u * 8u);
             chunk_walk_kernel<<<blocks, 64, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep + 1);
         }
         chunk_repair_kernel<<<grid_for(lines * 32, 128), 128, 0, s>>>(B, starts, ends, counts, s_in, s_out, s_val, n_rep);
-        zero_async(counts + chunks, sizeof(int64_t), s);
         if ((st = exclusive_scan_i64(counts, offsets, chunks + 1, total_dev, s))) break;
         int64_t nraw = 0;  // pieces; up to two triples each
-        small_to_host(&nraw, total_dev, sizeof(int64_t), s);
-        small_to_host(fl.data(), B.flags, sizeof(unsigned) * fl.size(), s);
-        cudaError_t e = cudaStreamSynchronize(s);
+        if ((st = count_and_flags(total_dev, &nraw, fl, s))) break;
         nraw *= 2;
-        if (e != cudaSuccess) {
-            set_error("conservative sweep (chunked walk): %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
-            break;
-        }
         bool cap = false;
         for (unsigned f : fl) cap = cap || (f & FLAG_CAPACITY);
         if (cap) {
@@ -2149,7 +2191,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         {
             // order the triples by output row from the slots
             const int64_t nr = rows->n_rows;
-            unsigned *rowc = nullptr, *long_count = nullptr;
+            unsigned *rowc = nullptr, *long_count = nullptr;  // (one allocation)
             Triple* triples = nullptr;
             int32_t* long_list = nullptr;
             do {
@@ -2157,13 +2199,12 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 if ((st = dalloc(&rows->row_nnz, (size_t)nr + 1, s))) break;
                 if ((st = dalloc(&rows->col, (size_t)nraw, s))) break;
                 if ((st = dalloc(&rows->val, (size_t)nraw, s))) break;
-                if ((st = dalloc(&rowc, (size_t)nr + 1, s))) break;
-                if ((st = dalloc(&long_count, 1, s))) break;
+                if ((st = dalloc(&rowc, (size_t)nr + 2, s))) break;
+                long_count = rowc + nr + 1;
                 rows->per = order_rows_per_block(nraw, nr);
                 if ((st = dalloc(&long_list, (size_t)(nr / rows->per + 1), s))) break;
                 if ((st = dalloc(&triples, (size_t)nraw, s))) break;
-                zero_async(rowc, sizeof(unsigned) * (nr + 1), s);
-                zero_async(long_count, sizeof(unsigned), s);
+                zero_async(rowc, sizeof(unsigned) * (nr + 2), s);
                 // lanes per chunk for the pieces it holds on average
                 const int64_t mean = nraw / (2 * chunks);
                 const int lanes = mean > 20 ? 32 : mean > 10 ? 16 : 8;
@@ -2184,12 +2225,11 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                                                                             rows->row_nnz);
             } while (0);
             dfree(rowc, s);
-            dfree(long_count, s);
             dfree(long_list, s);
             dfree(triples, s);
             if (st) break;
         }
-        e = cudaGetLastError();
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             set_error("conservative sweep (compaction): %s", cudaGetErrorString(e));
             st = RG_ERR_CUDA;
@@ -2201,7 +2241,6 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
     dfree(ends, s);
     dfree(counts, s);
     dfree(offsets, s);
-    dfree(n_rep, s);
     dfree(s_in, s);
     dfree(s_out, s);
     dfree(s_val, s);
@@ -2211,10 +2250,12 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
 }
 
 // Per-grid sizes of the merged CSR: nnz_base[g] = row_ptr[out_base[g]].
-__global__ void nnz_bases(const int64_t* __restrict__ row_ptr, const int64_t* __restrict__ out_base, int G,
-                          int64_t* __restrict__ nnz_base) {
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= G; g += gridDim.x * blockDim.x)
+__global__ void nnz_bases(const int64_t* __restrict__ row_ptr, const int64_t* __restrict__ out_base,
+                          const unsigned* __restrict__ flags, int G, int64_t* __restrict__ nnz_base) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= G; g += gridDim.x * blockDim.x) {
         nnz_base[g] = row_ptr[out_base[g]];
+        if (g < G) nnz_base[G + 1 + g] = flags[g];  // the grids' error words behind them
+    }
 }
 
 // Copy every grid's rows and entries of the merged CSR to its own arrays.
@@ -2270,9 +2311,9 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
     double* bbox_d = nullptr;
     StaticBatch SB;
     int64_t* totals = nullptr;
-    SweepParams* P_dev = nullptr;
-    int64_t *line_base_dev = nullptr, *out_base_dev = nullptr, *chunk_base_dev = nullptr;
-    ChunkPlan* plans_dev = nullptr;
+    unsigned char* head_dev = nullptr;  // the sweep parameters, bases, total and error words
+    const int64_t* out_base_dev = nullptr;
+    unsigned char* plans_dev = nullptr;
     Seat* seats = nullptr;
     int64_t* total_dev = nullptr;
     unsigned* flags = nullptr;
@@ -2315,10 +2356,10 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         if ((st = dalloc(&bbox_d, (size_t)4 * NG, s))) break;
         if ((st = dalloc(&SB.bbox_part, (size_t)4 * NG * nparts, s))) break;
         if ((st = dalloc(&SB.edges, (size_t)nedges_all, s))) break;
-        cell_area_batch<<<grid_for(in_base[G], 256), 256, 0, s>>>(SB.grids, G, in_base[G], area_in);
-        bbox_partial_batch<<<(unsigned)(NG * nparts), 256, 0, s>>>(SB.grids, nparts, SB.bbox_part);
+        const unsigned box_blocks = (unsigned)(NG * nparts), edge_blocks = grid_for(nedges_all, 256);
+        prepare_batch<<<box_blocks + edge_blocks + grid_for(in_base[G], 256), 256, 0, s>>>(
+            SB.grids, G, box_blocks, nparts, SB.bbox_part, edge_blocks, nedges_all, SB.edges, in_base[G], area_in);
         bbox_combine_batch<<<grid_for((int64_t)NG * 32, 128), 128, 0, s>>>(SB.bbox_part, nparts, NG, bbox_d);
-        boundary_edges_batch<<<grid_for(nedges_all, 128), 128, 0, s>>>(SB.grids, NG, nedges_all, SB.edges);
         std::vector<double> bbox_h((size_t)4 * NG);
         small_to_host(bbox_h.data(), bbox_d, sizeof(double) * 4 * NG, s);
         cudaError_t e = cudaStreamSynchronize(s);
@@ -2415,16 +2456,19 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             P[g].ncy_in = q.nyi - 1;
             P[g].ncy_out = q.nyo - 1;
         }
-        if ((st = upload(&P_dev, P, s))) break;
-        if ((st = upload(&line_base_dev, line_base, s))) break;
-        if ((st = upload(&out_base_dev, out_base, s))) break;
-        if ((st = dalloc(&flags, (size_t)G, s))) break;
-        if ((st = dalloc(&total_dev, 1, s))) break;
-        zero_async(flags, sizeof(unsigned) * G, s);
+        Pack pack;
+        const size_t P_at = pack.add(P), line_at = pack.add(line_base), out_at = pack.add(out_base);
+        const size_t total_at = pack.add(nullptr, sizeof(int64_t) + sizeof(unsigned) * G);
+        st = pack.to_device(s);
+        head_dev = pack.dev;
+        if (st) break;
+        out_base_dev = pack.at<int64_t>(out_at);
+        total_dev = pack.at<int64_t>(total_at);
+        flags = pack.at<unsigned>(total_at + sizeof(int64_t));
         Batch B;
-        B.P = P_dev;
+        B.P = pack.at<SweepParams>(P_at);
         B.C = nullptr;
-        B.line_base = line_base_dev;
+        B.line_base = pack.at<int64_t>(line_at);
         B.chunk_base = nullptr;
         B.out_base = out_base_dev;
         B.flags = flags;
@@ -2436,8 +2480,7 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         int64_t nraw = 0;
         MergedRows rows;
         rows.n_rows = n_out_all;
-        st = sweep_chunked(B, P, bbox_h, seats, lines, total_dev, s, &nraw, fl, &plans_dev, &chunk_base_dev,
-                           &rows);
+        st = sweep_chunked(B, P, bbox_h, seats, lines, total_dev, s, &nraw, fl, &plans_dev, &rows);
         bucket_ptr = rows.row_start;
         row_nnz = rows.row_nnz;
         tmp_col = rows.col;
@@ -2482,16 +2525,14 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             if ((st = dalloc(&row_nnz, (size_t)n_out_all + 1, s))) break;
             merge_rows<<<grid_for(n_out_all, 128), 128, 0, s>>>(bucket_ptr, sorted_in, sorted_val, n_out_all, tmp_col,
                                                                 tmp_val, row_nnz);
+            zero_async(row_nnz + n_out_all, sizeof(int64_t), s);
         }
-        zero_async(row_nnz + n_out_all, sizeof(int64_t), s);
         if ((st = dalloc(&row_ptr, (size_t)n_out_all + 1, s))) break;
         if ((st = exclusive_scan_i64(row_nnz, row_ptr, n_out_all + 1, total_dev, s))) break;
-        if ((st = dalloc(&nnz_base_dev, (size_t)G + 1, s))) break;
-        nnz_bases<<<grid_for(G + 1, 128), 128, 0, s>>>(row_ptr, out_base_dev, G, nnz_base_dev);
-        std::vector<int64_t> nnz_base((size_t)G + 1, 0);
-        small_to_host(nnz_base.data(), nnz_base_dev, sizeof(int64_t) * (G + 1), s);
-        std::vector<unsigned> fl2((size_t)G, 0u);
-        small_to_host(fl2.data(), flags, sizeof(unsigned) * G, s);
+        if ((st = dalloc(&nnz_base_dev, 2 * (size_t)G + 1, s))) break;
+        nnz_bases<<<grid_for(G + 1, 128), 128, 0, s>>>(row_ptr, out_base_dev, flags, G, nnz_base_dev);
+        std::vector<int64_t> nnz_base(2 * (size_t)G + 1, 0);  // the bases, then the error words
+        small_to_host(nnz_base.data(), nnz_base_dev, sizeof(int64_t) * nnz_base.size(), s);
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             set_error("conservative build (merge): %s", cudaGetErrorString(e));
@@ -2499,7 +2540,7 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             break;
         }
         for (int g = 0; g < G; g++)
-            if (status[g] == RG_OK && (fl2[g] & FLAG_CAPACITY)) {
+            if (status[g] == RG_OK && (nnz_base[G + 1 + g] & FLAG_CAPACITY)) {
                 set_error("conservative sweep: the write walk disagreed with the count walk");
                 status[g] = RG_ERR_WALK;
             }
@@ -2610,14 +2651,9 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
     dfree(bbox_d, s);
     SB.free(s);
     dfree(totals, s);
-    dfree(P_dev, s);
-    dfree(line_base_dev, s);
-    dfree(out_base_dev, s);
-    dfree(chunk_base_dev, s);
+    dfree(head_dev, s);
     dfree(plans_dev, s);
     dfree(seats, s);
-    dfree(total_dev, s);
-    dfree(flags, s);
     dfree(raw_in, s);
     dfree(raw_out, s);
     dfree(raw_val, s);
