@@ -1309,11 +1309,11 @@ __device__ __forceinline__ void chunk_walk_one(const Batch& B, const WalkState* 
     ends[g] = st;
 }
 
-// Every thread walks the chunk of its own number, then takes chunks from a
-// counter: a thread that finishes a short chunk takes the next one instead of
-// idling until the longest chunk of its warp is done (walk lengths differ
-// between chunks).  The lanes that come for a chunk together add to the
-// counter once.
+// Every warp walks the 32 chunks of its own number, then takes 32 more from a
+// counter.  Its lanes step together (walk_range): lanes that finish early wait,
+// which costs less than the divergence did when every lane took its next chunk
+// by itself (2048^2 -> 1536^2: 2.1 ms, 3.7 ms before; FP64 issue takes 55 % of
+// it, the latency of the steps the rest).
 __global__ void __launch_bounds__(64)
     chunk_walk_kernel(Batch B, const WalkState* __restrict__ starts, WalkState* __restrict__ ends,
                       int64_t* __restrict__ counts, int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
@@ -1968,8 +1968,11 @@ int locate_2d_exact(const double* x, const double* y, int64_t nx, int64_t ny, co
 }
 
 std::atomic<int64_t> g_sweep_chunk{32};
-// the walk kernel keeps 8 blocks of 64 threads per SM: 152 x 512 threads
-constexpr int64_t kTargetChunks = 152 * 512;
+// two chunks for each thread of the walk (8 blocks of 64 per SM): lengths
+// differ, and a second round evens them out (one chunk per thread against two:
+// 1024^2 -> 200^2 1.73 and 1.32 ms with the apply, 700^2 -> 500^2 0.93 and 0.89;
+// 333x257 and 16 pairs of 32 to 256 the same; 2048^2 is above either)
+constexpr int64_t kTargetChunks = 152 * 1024;
 constexpr int64_t kMinChunk = 1;
 
 namespace {
@@ -2090,9 +2093,8 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         ch = atoll(env);
     } else if (ch > kMinChunk) {
         // Small batches: shorter chunks, so that the walk still has about
-        // kTargetChunks threads (each chunk is one thread's sequential walk;
-        // a 128^2 pair in chunks of 32 segments keeps 2,000 threads busy
-        // for 0.7 ms), down to one segment (a start costs little beside the
+        // kTargetChunks chunks (each is one thread's sequential walk; a 128^2
+        // pair in chunks of 32 segments keeps 2,000 threads busy for 0.7 ms), down to one segment (a start costs little beside the
         // walk of a segment; 64^2 -> 48^2: walk 100 -> 34 us).  Every chunk length gives the same
         // triples in the same order.
         int64_t segments = 0;
