@@ -1207,7 +1207,8 @@ __device__ WalkState guess_state(const Static& S, double px, double py, int64_t 
     const Grid& g = S.g;
     const int64_t ncx = S.ncx, ncy = S.ncy;
     int64_t ci, cj;
-    const int single = locate_single(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj);
+    const int single = locate_single(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj,
+                                     [&](int64_t i, int64_t j) { return cell_contains(g, i, j, px, py); });
     if (single == 1) return WalkState{ci, cj, sy, 0, 0};
     if (single == 0) return w;
     seed_cell<false>(g.x, g.y, g.nx, g.ny, px, py, &ci, &cj);
@@ -2207,9 +2208,12 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 if ((st = dalloc(&long_list, (size_t)(nr / rows->per + 1), s))) break;
                 if ((st = dalloc(&triples, (size_t)nraw, s))) break;
                 zero_async(rowc, sizeof(unsigned) * (nr + 2), s);
-                // lanes per chunk for the pieces it holds on average
+                // lanes per chunk for the pieces it holds on average (the lines at
+                // 20 and 10 against 48 and 24, builds with their applies: 512^2 ->
+                // 384^2 688 and 677 us, 700^2 -> 500^2 911 and 893, 1024^2 -> 768^2
+                // 1.50 and 1.47 ms, 2048^2 -> 1536^2 the same)
                 const int64_t mean = nraw / (2 * chunks);
-                const int lanes = mean > 20 ? 32 : mean > 10 ? 16 : 8;
+                const int lanes = mean > 48 ? 32 : mean > 24 ? 16 : 8;
                 const unsigned gc = grid_for(chunks * lanes, 256);
                 const auto count = lanes == 32 ? slot_count_rows<32> : lanes == 16 ? slot_count_rows<16> : slot_count_rows<8>;
                 const auto scatter = lanes == 32   ? slot_scatter_rows<32>

@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(128)
     // left the grid) left to the winding number of the boundary; the others
     // start again with float64 decisions
     int64_t ci, cj;
-    const int single = locate_single(g.x, g.y, g.nx, g.ny, p_x, p_y, &ci, &cj);
+    const int single = locate_single(g.x, g.y, g.nx, g.ny, p_x, p_y, &ci, &cj,
+                                     [&](int64_t i, int64_t j) { return contains(g, i, j, p_x, p_y); });
     if (single == 1) {
         int64_t ri, rj;
         lowest_local(g, p_x, p_y, ci, cj, &ri, &rj);
