@@ -183,7 +183,8 @@ int rg_weights_free(rg_weights w, rg_stream_t stream);
  * lists and entry orders) and its first in each stack size class (1, 2-3,
  * 4-7, ..., 64 and more slices: the autotuner times its configurations on
  * that call, unless an earlier handle of the same kind was tuned) synchronise
- * `stream`; later applies are asynchronous. */
+ * `stream`, as do the first exact apply of a float32 stack and the second of
+ * a float64 one (from then on staged as well); later applies are asynchronous. */
 int rg_apply(rg_weights w, const void* d_vin, int dtype_in, void* d_vout, int dtype_out,
              int64_t stack, int acc, rg_stream_t stream);
 

@@ -21,7 +21,7 @@ __device__ __forceinline__ float trunc_float(double v, bool& ok) {
 // -1 undecided.  GB300 issues FP64 at 1/64 of its FP32 rate, and the test's
 // eight differences, four products and two crossings were most of a locate.
 // (593 K points in a 1024^2 grid: the walk kernel 596 us in FP64, 205 us with
-// this test, 73 us with the walk itself decided in float32 too.)
+// this test, 66 us with the walk itself decided in float32 too.)
 //
 // With m the largest magnitude of the coordinates and S the largest of the
 // eight float32 differences to the point, every difference is within D =
