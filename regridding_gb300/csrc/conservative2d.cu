@@ -881,11 +881,21 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
     const unsigned row = (unsigned)S.g.ny;  // vertices from one to the next along the first axis
     const int ncx = (int)S.ncx, ncy = (int)S.ncy;
     const auto vertex = [&](int x, int y, int v) {  // indices_cell_vertex: _grids.py:153-158
+#ifdef RG_DEBUG
+        if (!debug_in_grid(x + ((v + 1) >> 1 & 1), y + (v >> 1), S.g.nx, S.g.ny)) return 0u;
+#endif
         return (unsigned)x * row + (unsigned)y + ((v + 1) >> 1 & 1 ? row : 0u) + (unsigned)(v >> 1);
     };
     const int64_t along = F.transposed ? F.sweep.ny : 1;  // from one vertex of the line to the next
     const double* __restrict__ const lx = F.sweep.x + (F.transposed ? li : li * F.sweep.ny);
     const double* __restrict__ const ly = F.sweep.y + (F.transposed ? li : li * F.sweep.ny);
+    const auto line_vertex = [&](const double* __restrict__ line, int k) {
+#ifdef RG_DEBUG
+        if (!debug_in_grid(F.transposed ? k : li, F.transposed ? li : k, F.sweep.nx, F.sweep.ny))
+            return __longlong_as_double(0x7ff8000000000000ll);
+#endif
+        return __ldg(line + k * along);
+    };
     bool outside = state.outside;
     int stx = outside ? 0 : (int)state.stx, sty = outside ? 0 : (int)state.sty;
     constexpr int NONE = -1;
@@ -894,7 +904,7 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
     int n_emit = 0;
     int steps = 0;
     const int step_limit = (int)(max_steps < INT32_MAX ? max_steps : INT32_MAX);
-    double x1 = __ldg(lx + sy_idx * along), y1 = __ldg(ly + sy_idx * along);
+    double x1 = line_vertex(lx, sy_idx), y1 = line_vertex(ly, sy_idx);
     int first = 0;  // the edge that the search in a cell begins with
 
     // the piece of the current segment from (x1, y1) to (xe, ye)
@@ -966,8 +976,8 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
             atomicOr(flags, FLAG_WALK_CAP);
             end = sy_idx;
         } else if (live) {
-            x2 = __ldg(lx + (sy_idx + 1) * along);
-            y2 = __ldg(ly + (sy_idx + 1) * along);
+            x2 = line_vertex(lx, sy_idx + 1);
+            y2 = line_vertex(ly, sy_idx + 1);
             inside = !outside;
             enter = outside;
         }
@@ -1095,8 +1105,8 @@ __device__ int64_t walk_range(const SweepParams& P, const Family& F, const Stati
                 y1 = y2;
                 look = inside = ++sy_idx < end;
                 if (inside) {
-                    x2 = __ldg(lx + (sy_idx + 1) * along);
-                    y2 = __ldg(ly + (sy_idx + 1) * along);
+                    x2 = line_vertex(lx, sy_idx + 1);
+                    y2 = line_vertex(ly, sy_idx + 1);
                 }
             }
             __syncwarp(lanes);
