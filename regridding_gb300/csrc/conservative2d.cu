@@ -1630,9 +1630,9 @@ __device__ __forceinline__ double run_sum(const At& at, int64_t g, int64_t h) {
     return dadd(at(g), h - g - 1 <= 128 ? pw_block(at, g + 1, h - g - 1) : pairwise_sum(at, g + 1, h - g - 1));
 }
 
-// Merges the entries [s, t) of a row, sorted by input cell, in place with the
-// run_sum; the reads and stores are the caller's.  Returns
-// the end of the merged entries.
+// Merges the entries [s, t) of a row, sorted by input cell, by run_sum; the
+// reads and stores (in place) are the caller's.  Returns the end of the merged
+// entries.
 template <typename In, typename At, typename Store>
 __device__ __forceinline__ int64_t merge_sorted(int64_t s, int64_t t, const In& in, const At& at, const Store& store) {
     int64_t w = s, g = s;
