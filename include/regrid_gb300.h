@@ -52,7 +52,10 @@ typedef struct CUstream_st* rg_stream_t; /* == cudaStream_t */
  * unevaluated pair of floats (error-free products by FMA, Knuth's two-sum) on
  * the FP32 pipe, the pair added in double at the end.  Result within
  * (1.1e-14 + (n + 2)^2 * 3.6e-15) * sum_k |w_k x_k| of the exact sum for rows
- * of n entries (checked to 1e-12 relative against the upstream float64 apply).
+ * of n entries, 1e-12 of sums of one sign for n <= 14.  Longer rows are summed in
+ * float64, bit for bit as RG_ACC_EXACT, except where the input footprints of
+ * 16 x 16 output cells fit boxes of 32 x 32 input cells, whose rows are short
+ * (about 9 entries; one of 60 is off by some 5e-14).
  * A float32 partial sum that overflows, or a non-finite input or weight,
  * sends that output and slice to the exact float64 sum instead.
  * Every other dtype combination computes as RG_ACC_EXACT. */
@@ -177,8 +180,9 @@ int rg_weights_free(rg_weights w, rg_stream_t stream);
  * float64 result bit for bit (dtype_out must be RG_F64, or RG_F32 for the
  * upstream in-place float32 output, which rounds after every update);
  * RG_ACC_FAST accumulates in dtype_out with FMA; RG_ACC_COMPENSATED gives a
- * float64 result within 1e-12 of the upstream's for float32 input, about 5x
- * faster than RG_ACC_EXACT on GB300 (see its definition above).
+ * float64 result within 1e-12 of the upstream's (sums of one sign, see its
+ * definition above) for float32 input, about 5x
+ * faster than RG_ACC_EXACT on GB300.
  * The first fast or compensated apply of a handle (which builds its tile
  * lists and entry orders) and its first in each stack size class (1, 2-3,
  * 4-7, ..., 64 and more slices: the autotuner times its configurations on

@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(32 * WARPS)
 // The input footprint of every patch, one block of 256 threads each, a thread
 // per output cell: its first row and column (a multiple of 4, where a tensor
 // copy can start) and its extent, (-1, -1) and 0 without entries.  stats: the
-// most rows and columns, and the patches larger than 32 x 32.
+// most rows and columns, the patches larger than 32 x 32, and the output rows
+// of more than FF_ROW_MAX entries.
 __global__ void __launch_bounds__(32 * PATCH_WARPS)
     patch_footprints(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col, PatchGrid P, FastDiv nd,
                      int2* __restrict__ origin, int2* __restrict__ extent, unsigned* __restrict__ stats) {
@@ -300,6 +301,8 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS)
         cmin = min(cmin, cc);
         cmax = max(cmax, cc);
     }
+    const unsigned longer = __ballot_sync(0xffffffffu, e - s > FF_ROW_MAX);
+    if (lane == 0 && longer) atomicAdd(&stats[3], (unsigned)__popc(longer));
     rmin = __reduce_min_sync(0xffffffffu, rmin);
     cmin = __reduce_min_sync(0xffffffffu, cmin);
     rmax = __reduce_max_sync(0xffffffffu, rmax);
@@ -1086,7 +1089,7 @@ int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
     }
     W->box_cb = 4;
     RG_CHECK(most < 0x7fffffff, RG_ERR_UNSUPPORTED, "apply: too many output patches");
-    unsigned* stats = nullptr;  // [candidate][rows, columns, larger than 32 x 32, -]
+    unsigned* stats = nullptr;  // [candidate][rows, columns, larger than 32 x 32, long rows]
     int st = RG_OK;
     int state = -1;
     auto footprints = [&](int k) {
@@ -1137,6 +1140,7 @@ int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made) {
             footprints(best);
         }
         const WideBox b = wide_box(h[best], W->in_shape1);
+        W->box_long = h[0][3];
         W->box_patches = patch_count(patch_grid(W));
         // the box has to lie in a tensor's extent
         if (b.rows == 0 || b.rows > 256 || b.pitch > 256 || b.cells() > WIDE_MAX) break;

@@ -240,6 +240,7 @@ struct rg_weights_s {
     int box_state = 0;  // 0 not built, 1 ready, 2 ready with wide boxes, -1 not applicable
     int box_rows = 0, box_cols = 0, box_pitch = 0, box_residues = 0, box_cb = 4;
     int64_t box_patches = 0;
+    int64_t box_long = 0;  // wide boxes: output rows too long for float-float sums (FF_ROW_MAX)
     // configuration chosen by the autotuner per stack class (-1 not tuned, -2 none fits)
     int box_cfg[rg::kStackClasses] = {-1, -1, -1, -1, -1, -1, -1};
     int2* box_origin = nullptr;

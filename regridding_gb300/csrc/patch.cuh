@@ -176,6 +176,16 @@ __device__ __forceinline__ double widen_normal(unsigned u) {
 //              in double once per output.  Entries in the gather order.
 constexpr int MODE_FAST = 0, MODE_EXACT = 1, MODE_FF = 2;
 
+// Longest row that MODE_FF sums as float pairs in a wide box: their error,
+// (1.5 2^-47 + (n + 2)^2 2^-48) sum |w x|, is then below 1e-12 of the sum (and
+// is approached where roundings have one sign: n equal terms, n = 250, are off by
+// 1e-12).  Longer rows are summed in float64, in stored order.  (Boxes of 32
+// swizzled columns hold patches whose rows have about 9 entries; their kernel
+// tests nothing.)
+constexpr int FF_ROW_MAX = 14;
+// One in this many rows may be long; with more, the exact kernel takes the call.
+constexpr int FF_LONG_SHARE = 16;
+
 // Packed pairs of float32 (two slices of one output): the sm_100-family
 // f32x2 instructions apply one IEEE operation, rounded to nearest, to both
 // halves, at the issue cost of one scalar instruction.
@@ -398,7 +408,10 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     // past its own row have zero weights and slot 0: such a step leaves the
     // pair (h, l) unchanged for a finite input word; a non-finite one makes
     // the sum NaN, which sends that output and slice to the exact loop.
-    const int kwarp = MODE == MODE_FF ? __reduce_max_sync(0xffffffffu, nk) : nk;
+    // a long row's lane takes no float-float step: its entries here are none
+    const bool long_row = MODE == MODE_FF && LOAD != LOAD_SWIZZLED && nk > FF_ROW_MAX;
+    const int nf = long_row ? 0 : nk;
+    const int kwarp = MODE == MODE_FF ? __reduce_max_sync(0xffffffffu, nf) : nk;
     // PLANES: every slice of a stage has its own 4 KB plane, 1024-byte
     // aligned, so all slices see the same swizzle phase and a gather's
     // slices differ by constant offsets.  Otherwise the rows of slice q start
@@ -420,8 +433,8 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
             wd[k] = k < nk ? dval[s + k] : 0.0;
             w[k] = 0.f;
         } else if constexpr (MODE == MODE_FF) {
-            li[k] = k < nk ? (int)slot[s + k] : 0;
-            const float a = k < nk ? bval[s + k] : 0.f, b = k < nk ? blo[s + k] : 0.f;
+            li[k] = k < nf ? (int)slot[s + k] : 0;
+            const float a = k < nf ? bval[s + k] : 0.f, b = k < nf ? blo[s + k] : 0.f;
             fh[k] = f2_pack(a, a);
             fhn[k] = f2_pack(-a, -a);
             fl[k] = f2_pack(b, b);
@@ -434,7 +447,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     if constexpr (CT > 0) {
 #pragma unroll
         for (int j = 0; j < NX; j++) {
-            const bool has = CT + j < nk;
+            const bool has = CT + j < nf;
             if constexpr (EXACT) {
                 ex_slot[j][t] = has ? (uint16_t)box_slot_of<LOAD>(col[s + CT + j], org, nd, box) : (uint16_t)0;
                 ex_d[j][t] = has ? dval[s + CT + j] : 0.0;
@@ -534,7 +547,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                         }
                     }
                 }
-                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < e; k++) {
+                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < s + nf; k++) {
                     const float wk = bval[k], wlk = blo[k];
                     const uint64_t kh = f2_pack(wk, wk), khn = f2_pack(-wk, -wk), kl = f2_pack(wlk, wlk);
                     const int a = slot[k];
@@ -557,7 +570,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                 // branch, and stored without further tests (per-slice tests
                 // and branches were a measured share of the instruction
                 // stream).  Anything else takes the per-slice path.
-                bool usual = ds + SPS <= d1;
+                bool usual = ds + SPS <= d1 && !long_row;
 #pragma unroll
                 for (int q = 0; q < SPS; q++)
                     usual = usual & normal_bits(__float_as_uint(h[q])) & normal_bits(__float_as_uint(l[q]));
@@ -577,13 +590,13 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                             r = __dadd_rn(widen_normal(uh), widen_normal(ul));
                         } else if (nk == 0) {
                             r = 0.0;
-                        } else if (finite_bits(h[q]) && finite_bits(l[q])) {
+                        } else if (!long_row && finite_bits(h[q]) && finite_bits(l[q])) {
                             r = __dadd_rn(widen(h[q]), widen(l[q]));
                         } else {
-                            // a float32 partial sum overflowed, or an input or
-                            // a weight is not finite (or a padded step read a
-                            // non-finite word): this output and slice in
-                            // float64, stored order (the exact apply's sum)
+                            // a long row, or a float32 partial sum overflowed,
+                            // or an input or a weight is not finite (or a padded
+                            // step read a non-finite word): this output and slice
+                            // in float64, stored order (the exact apply's sum)
                             r = 0.0;
                             for (int64_t k = s; k < e; k++)
                                 r = __dadd_rn(r, __dmul_rn(dval[k], as_double(cell_of(q, box_slot_of<LOAD>(col[k], org, nd, box)))));
