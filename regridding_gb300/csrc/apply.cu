@@ -165,28 +165,29 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
 }  // namespace
 
 int tiled_lists_for(rg_weights_s* W, const float* vin, cudaStream_t s, int* g, bool* made);
-int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s);
-bool box_usable(const rg_weights_s* W, int64_t stack);
-int box_load(const rg_weights_s* W, const void* vin, int64_t stack);
-int apply_wide_f64(const rg_weights_s* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s);
+int apply_tiled(const rg_weights_state* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s);
+bool box_usable(const rg_weights_state* W, int64_t stack);
+int box_load(const rg_weights_state* W, const void* vin, int64_t stack);
+int apply_wide_f64(const rg_weights_state* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s);
 int box_order_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_perm_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int ff_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
-int apply_box(const rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
-int apply_box_exact(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s);
-int apply_box_ff(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s);
+int apply_box(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
+int apply_box_exact(const rg_weights_state* W, const float* vin, double* vout, int64_t stack, cudaStream_t s);
+int apply_box_ff(const rg_weights_state* W, const float* vin, double* vout, int64_t stack, cudaStream_t s);
 int tune_box_fast(rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
 int tune_box_ff(rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s);
 int rows_usable(rg_weights_s* W, const float* vin, int64_t stack, cudaStream_t s, bool* made, bool* ok);
-int apply_rows_launch(const rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
+int apply_rows_launch(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
 int ensure_transposed(rg_weights_s* W, cudaStream_t s);
 
 // Every apply goes through here.  The per-handle state an apply needs beyond
 // the CSR (the transposed CSR, the float32 copy of the weights, the warp-tile
 // lists) is made on first use under the handle's mutex and finished (the
 // stream synchronised) before the lock is released, so calls from other
-// threads and streams only ever see complete state.
+// threads and streams only ever see complete state.  The launches read a copy
+// of it taken under the lock.
 int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_in, void* vout,
                   int dtype_out, int64_t stack, int acc, cudaStream_t s) {
     RG_CHECK(dtype_in == RG_F32 || dtype_in == RG_F64, RG_ERR_ARG, "apply: bad input dtype");
@@ -223,6 +224,7 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     const bool need32 = ((acc == RG_ACC_FAST && dtype_out == RG_F32) || exact_box || ff_box) && W->nnz > 0;
     int g = 0, load64 = -1;
     bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false;
+    rg_weights_state now;
     {
         std::lock_guard<std::mutex> lock(W->mu);
         bool made = false;
@@ -287,22 +289,23 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
             RG_TRY(rows_usable(W, (const float*)vin, stack, s, &made, &use_rows));
         if (tiled && !use_box && !use_rows) RG_TRY(tiled_lists_for(W, (const float*)vin, s, &g, &made));
         if (made) RG_CUDA(cudaStreamSynchronize(s));
+        now = *W;
     }
     if (exact64) {
-        const int st = apply_wide_f64(W, load64, (const double*)vin, (double*)vout, stack, s);
+        const int st = apply_wide_f64(&now, load64, (const double*)vin, (double*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
     }
-    if (use_rows) return apply_rows_launch(W, (const float*)vin, (float*)vout, stack, s);
+    if (use_rows) return apply_rows_launch(&now, (const float*)vin, (float*)vout, stack, s);
     if (use_box_exact) {
-        const int st = apply_box_exact(W, (const float*)vin, (double*)vout, stack, s);
+        const int st = apply_box_exact(&now, (const float*)vin, (double*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
     }
     if (use_box_ff) {
-        const int st = apply_box_ff(W, (const float*)vin, (double*)vout, stack, s);
+        const int st = apply_box_ff(&now, (const float*)vin, (double*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
     }
     if (use_box) {
-        const int st = apply_box(W, (const float*)vin, (float*)vout, stack, s);
+        const int st = apply_box(&now, (const float*)vin, (float*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
         // the tuned configuration does not take this call (fewer slices than
         // a stage): the warp-staged kernel does, with its own lists
@@ -310,12 +313,13 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
         bool made = false;
         RG_TRY(tiled_lists_for(W, (const float*)vin, s, &g, &made));
         if (made) RG_CUDA(cudaStreamSynchronize(s));
+        now = *W;
     }
-    if (tiled) return apply_tiled(W, g, (const float*)vin, (float*)vout, stack, s);
+    if (tiled) return apply_tiled(&now, g, (const float*)vin, (float*)vout, stack, s);
     if (!transposed)
-        return apply_csr(W->row_ptr, W->col, W->val, W->val32, W->nnz, W->n_out, W->n_in, W->out_shape0,
-                         W->out_shape1, vin, dtype_in, vout, dtype_out, stack, acc, s);
-    return apply_csr(W->t_row_ptr, W->t_col, W->t_val, W->t_val32, W->nnz, W->n_in, W->n_out, 0, 0, vin,
+        return apply_csr(now.row_ptr, now.col, now.val, now.val32, now.nnz, now.n_out, now.n_in, now.out_shape0,
+                         now.out_shape1, vin, dtype_in, vout, dtype_out, stack, acc, s);
+    return apply_csr(now.t_row_ptr, now.t_col, now.t_val, now.t_val32, now.nnz, now.n_in, now.n_out, 0, 0, vin,
                      dtype_in, vout, dtype_out, stack, acc, s);
 }
 

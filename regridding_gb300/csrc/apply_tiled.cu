@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(32 * WARPS)
     }
 }
 
-TileShape tile_shape(const rg_weights_s* W) {
+TileShape tile_shape(const rg_weights_state* W) {
     TileShape T;
     if (W->out_shape0 > 0 && W->out_shape1 > 0 && W->out_shape0 * W->out_shape1 == W->n_out) {
         T.n0 = W->out_shape0;
@@ -786,7 +786,7 @@ EncodeTiledFn encode_tiled() {
 // rows and `bs` slices of 32 columns with the 128-byte swizzle, or (wide)
 // `pitch` columns as they lie; or (LOAD_RESIDUES) groups of four rows x
 // their number.
-bool encode_stack(const rg_weights_s* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map) {
+bool encode_stack(const rg_weights_state* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map) {
     const bool wide = pitch > 0;
     const CUtensorMapDataType type = bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     if (W->box_residues) {
@@ -897,7 +897,7 @@ int tiled_lists_for(rg_weights_s* W, const float* vin, cudaStream_t s, int* g, b
     return RG_OK;
 }
 
-int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
+int apply_tiled(const rg_weights_state* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
     const bool vec = g == 1;
     const TileShape T = tile_shape(W);
     const int64_t wtiles = W->t_tiles;
@@ -928,7 +928,7 @@ int apply_tiled(const rg_weights_s* W, int g, const float* vin, float* vout, int
 
 // Whether the patch kernel may take calls with this handle: output and input
 // grid shapes known.
-bool box_usable(const rg_weights_s* W, int64_t stack) {
+bool box_usable(const rg_weights_state* W, int64_t stack) {
     return W->box_state >= 0 && W->out_shape0 > 0 && W->out_shape1 > 0 &&
            W->out_shape0 * W->out_shape1 == W->n_out && W->in_shape0 > 0 && W->in_shape1 > 0 &&
            W->in_shape0 * W->in_shape1 == W->n_in && stack >= 1 && W->n_in < INT32_MAX && stack < INT32_MAX &&
@@ -937,7 +937,7 @@ bool box_usable(const rg_weights_s* W, int64_t stack) {
 
 // How the patch kernel would fill its stages for this call, -1 when it does
 // not take it (the caller holds the handle's lock, box_lists_for has run).
-int box_load(const rg_weights_s* W, const void* vin, int64_t stack) {
+int box_load(const rg_weights_state* W, const void* vin, int64_t stack) {
     const bool aligned = W->in_shape1 % 4 == 0 && ((uintptr_t)vin & 15) == 0;
     if (W->box_state == 1) return aligned ? LOAD_SWIZZLED : -1;
     if (W->box_state != 2) return -1;
@@ -947,9 +947,9 @@ int box_load(const rg_weights_s* W, const void* vin, int64_t stack) {
     return stack * W->in_shape0 / 4 >= (W->box_rows + 3) / 4 ? LOAD_RESIDUES : -1;
 }
 
-BoxShape box_shape(const rg_weights_s* W) { return BoxShape{W->box_pitch, W->box_residues}; }
+BoxShape box_shape(const rg_weights_state* W) { return BoxShape{W->box_pitch, W->box_residues}; }
 
-PatchGrid patch_grid(const rg_weights_s* W) {
+PatchGrid patch_grid(const rg_weights_state* W) {
     PatchGrid P;
     P.n0 = W->out_shape0;
     P.n1 = W->out_shape1;
@@ -1184,7 +1184,7 @@ constexpr FFConfig kFFConfigs[] = {{6, 2, 0, 6}, {8, 2, 0, 6}, {4, 2, 0, 6}, {4,
 constexpr int kNumFFConfigs = (int)(sizeof(kFFConfigs) / sizeof(kFFConfigs[0]));
 
 template <int SPS, int NST, int MINB, int MODE = MODE_FAST, int CT = CACHED_T>
-int launch_patch(const rg_weights_s* W, const CUtensorMap& map, int box_slices, const float* vin, void* vout,
+int launch_patch(const rg_weights_state* W, const CUtensorMap& map, int box_slices, const float* vin, void* vout,
                  int64_t stack, cudaStream_t s) {
     const int BR = W->box_rows;
     // stages (and with planes, every slice) start on 1024-byte boundaries
@@ -1222,7 +1222,7 @@ int launch_patch(const rg_weights_s* W, const CUtensorMap& map, int box_slices, 
 }
 
 template <int MODE>
-int launch_box_config_mode(const rg_weights_s* W, int cfg, const float* vin, void* vout, int64_t stack,
+int launch_box_config_mode(const rg_weights_state* W, int cfg, const float* vin, void* vout, int64_t stack,
                            cudaStream_t s) {
     const BoxConfig c = kBoxConfigs[cfg];
     // a stack shorter than a stage: the box carries only its slices (the
@@ -1242,7 +1242,7 @@ int launch_box_config_mode(const rg_weights_s* W, int cfg, const float* vin, voi
     return RG_ERR_UNSUPPORTED;
 }
 
-int launch_ff_config(const rg_weights_s* W, int cfg, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+int launch_ff_config(const rg_weights_state* W, int cfg, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
     const FFConfig c = kFFConfigs[cfg];
     const int bs = (int)std::min<int64_t>(c.sps, stack);
     CUtensorMap map;
@@ -1260,7 +1260,7 @@ int launch_ff_config(const rg_weights_s* W, int cfg, const float* vin, void* vou
 }
 
 // MODE_FAST (float32 vout, kBoxConfigs) or MODE_FF (float64 vout, kFFConfigs).
-int launch_box_config(const rg_weights_s* W, int mode, int cfg, const float* vin, void* vout, int64_t stack,
+int launch_box_config(const rg_weights_state* W, int mode, int cfg, const float* vin, void* vout, int64_t stack,
                       cudaStream_t s) {
     if (mode == MODE_FF) return launch_ff_config(W, cfg, vin, vout, stack, s);
     return launch_box_config_mode<MODE_FAST>(W, cfg, vin, vout, stack, s);
@@ -1360,12 +1360,12 @@ int tune_box(rg_weights_s* W, int mode, const float* vin, void* vout, int64_t st
     return RG_OK;
 }
 
-int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s);
+int apply_wide(const rg_weights_state* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s);
 
 // Launch the TMA apply; returns RG_ERR_UNSUPPORTED (nothing launched) when
 // the tuned configuration does not take this call, so the caller can take
 // another kernel.
-int apply_box(const rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
+int apply_box(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
     if (W->box_state == 2) return apply_wide(W, MODE_FAST, box_load(W, vin, stack), vin, vout, stack, s);
     const int cfg = W->box_cfg[stack_class(stack)];
     if (cfg < 0) return RG_ERR_UNSUPPORTED;
@@ -1373,7 +1373,7 @@ int apply_box(const rg_weights_s* W, const float* vin, float* vout, int64_t stac
 }
 
 // The compensated (float-float) TMA apply with its tuned configuration.
-int apply_box_ff(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
+int apply_box_ff(const rg_weights_state* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
     const int cfg = W->box_cfg_ff[stack_class(stack)];
     if (W->box_state == 2) return apply_wide(W, MODE_FF, box_load(W, vin, stack), vin, vout, stack, s);
     if (W->box_state != 1 || cfg < 0 || !W->ff_slot || !W->ff_perm) return RG_ERR_UNSUPPORTED;
@@ -1390,7 +1390,7 @@ int tune_box_ff(rg_weights_s* W, const float* vin, double* vout, int64_t stack, 
 
 // The exact (float64) TMA apply: 4 slices per stage, 2 stages (FP64 issue,
 // not the staging, bounds it).
-int apply_box_exact(const rg_weights_s* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
+int apply_box_exact(const rg_weights_state* W, const float* vin, double* vout, int64_t stack, cudaStream_t s) {
     if (W->box_state == 2) return apply_wide(W, MODE_EXACT, box_load(W, vin, stack), vin, vout, stack, s);
     if (W->box_state != 1) return RG_ERR_UNSUPPORTED;
     const int bs = (int)std::min<int64_t>(4, stack);
@@ -1433,7 +1433,7 @@ int rows_usable(rg_weights_s* W, const float* vin, int64_t stack, cudaStream_t s
     return RG_OK;
 }
 
-int apply_rows_launch(const rg_weights_s* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
+int apply_rows_launch(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
     const int stage_floats = (int)((W->n_in + 31) & ~31ll);  // stages start on 128-byte boundaries
     const size_t smem = (size_t)ROWS_NST * stage_floats * sizeof(float);
     static std::once_flag attr;

@@ -14,16 +14,16 @@
 
 namespace rg {
 
-bool encode_stack(const rg_weights_s* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map);
-PatchGrid patch_grid(const rg_weights_s* W);
-BoxShape box_shape(const rg_weights_s* W);
+bool encode_stack(const rg_weights_state* W, const void* vin, int64_t stack, int bs, int pitch, int bytes, CUtensorMap* map);
+PatchGrid patch_grid(const rg_weights_state* W);
+BoxShape box_shape(const rg_weights_state* W);
 
 namespace {
 
 // (box: the handle's, or for a handle of swizzled boxes a wide one of the same
 // extent)
 template <int PL, int SPS, int NST, int MODE, int LOAD, typename TIN>
-int launch_wide(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+int launch_wide(const rg_weights_state* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
     constexpr int CT = MODE == MODE_FF ? 6 : CACHED_T;
     const auto kernel = apply_patch_tma<SPS, NST, 0, MODE, CT, LOAD, PL, TIN>;
     const size_t smem = (size_t)NST * SPS * PL * sizeof(TIN);
@@ -62,7 +62,7 @@ int launch_wide(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout,
 // of the stack, so one or two slices take stages of two; the largest boxes
 // (from 9 KB a slice) too, to keep three blocks on an SM.
 template <int PL, int MODE, int LOAD, typename TIN>
-int launch_plane(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+int launch_plane(const rg_weights_state* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
     if constexpr (PL * sizeof(TIN) <= 2304 * 4)
         if (stack > 2) return launch_wide<PL, 4, 2, MODE, LOAD>(W, box, vin, vout, stack, s);
     return launch_wide<PL, 2, 2, MODE, LOAD>(W, box, vin, vout, stack, s);
@@ -71,7 +71,7 @@ int launch_plane(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout
 // A slice's plane in a stage, the smallest of a few sizes that holds the box
 // (a constant, so that a gather's slices differ by constant offsets).
 template <int MODE, int LOAD, typename TIN>
-int launch_mode(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+int launch_mode(const rg_weights_state* W, BoxShape box, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
     const int cells = box.residues ? 4 * box.residues : W->box_rows * box.pitch;
     if (cells <= 1024) return launch_plane<1024, MODE, LOAD>(W, box, vin, vout, stack, s);
     if (cells <= 1536) return launch_plane<1536, MODE, LOAD>(W, box, vin, vout, stack, s);
@@ -80,7 +80,7 @@ int launch_mode(const rg_weights_s* W, BoxShape box, const TIN* vin, void* vout,
 }
 
 template <int MODE, typename TIN>
-int launch_load(const rg_weights_s* W, int load, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
+int launch_load(const rg_weights_state* W, int load, const TIN* vin, void* vout, int64_t stack, cudaStream_t s) {
     if (load == LOAD_WIDE) return launch_mode<MODE, LOAD_WIDE>(W, box_shape(W), vin, vout, stack, s);
     if constexpr (MODE != MODE_FAST) return launch_mode<MODE, LOAD_RESIDUES>(W, box_shape(W), vin, vout, stack, s);
     return RG_ERR_UNSUPPORTED;
@@ -88,7 +88,7 @@ int launch_load(const rg_weights_s* W, int load, const TIN* vin, void* vout, int
 
 }  // namespace
 
-int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
+int apply_wide(const rg_weights_state* W, int mode, int load, const float* vin, void* vout, int64_t stack, cudaStream_t s) {
     switch (mode) {
         case MODE_FAST: return launch_load<MODE_FAST>(W, load, vin, vout, stack, s);
         case MODE_EXACT: return launch_load<MODE_EXACT>(W, load, vin, vout, stack, s);
@@ -98,7 +98,7 @@ int apply_wide(const rg_weights_s* W, int mode, int load, const float* vin, void
 
 // The exact apply of a float64 stack (box_load, box_perm_for first): as the
 // float32 one, in wide boxes also where that takes swizzled ones.
-int apply_wide_f64(const rg_weights_s* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s) {
+int apply_wide_f64(const rg_weights_state* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s) {
     if (load != LOAD_SWIZZLED) return launch_load<MODE_EXACT>(W, load, vin, vout, stack, s);
     const BoxShape box{W->in_shape1 >= 36 ? 36 : 32, 0};
     return launch_mode<MODE_EXACT, LOAD_WIDE>(W, box, vin, vout, stack, s);

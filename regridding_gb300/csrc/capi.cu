@@ -174,17 +174,25 @@ int column_order(rg_weights_s* W, int32_t** row_of, uint32_t** perm, int64_t** c
     return st;
 }
 
-// Frees what box_lists_for and the entry orders made (no work in flight).
-void drop_patch_lists(rg_weights_s* W) {
+// Puts aside what box_lists_for and the entry orders made, for a new shape:
+// the lists stay as they are until the handle is freed.
+int retire_patch_lists(rg_weights_s* W) {
+    try {
+        W->retired.reserve(W->retired.size() + 9);
+    } catch (const std::bad_alloc&) {
+        set_error("host allocation failed");
+        return RG_ERR_ALLOC;
+    }
     for (void* p : {(void*)W->box_origin, (void*)W->box_extent, (void*)W->box_slot, (void*)W->box_val,
                     (void*)W->box_perm, (void*)W->ff_perm, (void*)W->ff_slot, (void*)W->ff_hi, (void*)W->ff_lo})
-        dfree(p, nullptr);
+        if (p) W->retired.push_back(p);
     W->box_origin = W->box_extent = nullptr;
     W->box_slot = W->ff_slot = nullptr;
     W->box_val = W->ff_hi = W->ff_lo = nullptr;
     W->box_perm = W->ff_perm = nullptr;
     W->box_state = 0;
     W->box_cb = 4;
+    return RG_OK;
 }
 
 void free_weights(rg_weights_s* W, cudaStream_t s) {
@@ -201,6 +209,7 @@ void free_weights(rg_weights_s* W, cudaStream_t s) {
         dfree(W->t_gidx[g], s);
         dfree(W->t_slot[g], s);
     }
+    for (void* p : W->retired) dfree(p, s);
     dfree(W->box_origin, s);
     dfree(W->box_extent, s);
     dfree(W->box_slot, s);
@@ -603,10 +612,7 @@ int rg_weights_set_output_shape(rg_weights w, int64_t n0, int64_t n1) {
     if (w->out_shape0 == n0 && w->out_shape1 == n1) return RG_OK;
     RG_CHECK(!w->tiled_ready[0] && !w->tiled_ready[1] && !w->box_val, RG_ERR_ARG,
              "rg_weights_set_output_shape: the output tiling is fixed once a fast float32 apply has run");
-    if (w->box_state != 0) {  // patch lists of the former shape, perhaps in use on some stream
-        RG_CUDA(cudaDeviceSynchronize());
-        drop_patch_lists(w);
-    }
+    if (w->box_state != 0) RG_TRY(retire_patch_lists(w));
     w->out_shape0 = n0;
     w->out_shape1 = n1;
     return RG_OK;
@@ -637,12 +643,9 @@ int rg_weights_set_input_shape(rg_weights w, int64_t n0, int64_t n1) {
              (long long)n1, (long long)w->n_in);
     std::lock_guard<std::mutex> lock(w->mu);
     if (w->in_shape0 == n0 && w->in_shape1 == n1) return RG_OK;
-    if (w->box_state != 0 && w->in_shape1 % 4 != 0 && !w->box_val) {
-        // exact or compensated applies made patch lists for rows that are
-        // not whole 16-byte chunks; they may still be in use on some stream
-        RG_CUDA(cudaDeviceSynchronize());
-        drop_patch_lists(w);
-    }
+    // (exact or compensated applies made patch lists for rows that are not
+    // whole 16-byte chunks)
+    if (w->box_state != 0 && w->in_shape1 % 4 != 0 && !w->box_val) RG_TRY(retire_patch_lists(w));
     RG_CHECK(w->box_state == 0, RG_ERR_ARG,
              "rg_weights_set_input_shape: the input tiling is fixed once a fast float32 apply has run");
     w->in_shape0 = n0;

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -208,7 +209,10 @@ inline int stack_class(int64_t stack) {
 // Opaque weight matrix of one orthogonal element, resident on the device.
 // Rows are output cells, columns input cells; entries of each row are sorted
 // by column, which is also the order the upstream apply accumulates them.
-struct rg_weights_s {
+// What an apply's launches read; a call copies it under the handle's lock and
+// launches from the copy, so that a shape set meanwhile (which makes other
+// lists) does not reach it.
+struct rg_weights_state {
     int64_t n_in = 0, n_out = 0, nnz = 0;
     int64_t* row_ptr = nullptr;  // [n_out + 1]
     int32_t* col = nullptr;      // [nnz]
@@ -260,7 +264,13 @@ struct rg_weights_s {
     unsigned* dflags = nullptr;  // device error word of the asynchronous (TMA) apply
     int rows_maxlen = -1;        // longest row (for the row kernel; -1 not known yet)
     int device = 0;
-    std::mutex mu;  // guards the lazily made state above (made on first use by an apply)
+};
+
+struct rg_weights_s : rg_weights_state {
+    std::mutex mu;  // guards the lazily made state (made on first use by an apply)
+    // patch lists of former shapes, which calls in flight or captured graphs
+    // may still read: freed with the handle
+    std::vector<void*> retired;
 };
 
 namespace rg {
