@@ -142,7 +142,8 @@ int rg_weights_info(rg_weights w, int64_t* nnz, int64_t* n_in, int64_t* n_out);
 
 /* Record the 2D shape of the output cells (rows of the matrix) so the apply
  * can tile them in two dimensions.  Optional; the shape cannot change once a
- * fast float32 apply has run with the handle (RG_ERR_ARG).
+ * fast float32 apply has run with the handle (RG_ERR_ARG).  Lists that other
+ * applies made for a former shape are kept until the handle is freed.
  *
  * Handles may be shared between threads and streams: the state an apply
  * makes on first use (float32 weights, tile lists, transposed CSR) is made
@@ -157,9 +158,10 @@ int rg_weights_export_coo(rg_weights w, int64_t* d_in, int64_t* d_out, double* d
                           rg_stream_t stream);
 
 /* Record the 2D shape of the input cells (columns of the matrix), which
- * lets the fast float32 apply stage input boxes with tensor-map copies.
- * Optional (weights built by rg_build_conservative_2d have it); fixed once a
- * fast float32 apply has run (RG_ERR_ARG). */
+ * lets the applies stage input boxes with tensor-map copies.  Optional
+ * (weights built by rg_build_conservative_2d have it); fixed (RG_ERR_ARG) once
+ * an apply of a 16-byte aligned float32 stack has met both shapes, with input
+ * rows of a multiple of 4 cells. */
 int rg_weights_set_input_shape(rg_weights w, int64_t n0, int64_t n1);
 
 /* Synchronise `stream` and report a failure that an earlier asynchronous

@@ -166,6 +166,7 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
 
 int tiled_lists_for(rg_weights_s* W, const float* vin, cudaStream_t s, int* g, bool* made);
 int apply_tiled(const rg_weights_state* W, int g, const float* vin, float* vout, int64_t stack, cudaStream_t s);
+bool shapes_usable(const rg_weights_state* W, int64_t stack);
 bool box_usable(const rg_weights_state* W, int64_t stack);
 int box_load(const rg_weights_state* W, const void* vin, int64_t stack);
 int apply_wide_f64(const rg_weights_state* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s);
@@ -239,6 +240,8 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
                 transposed ? W->t_val : W->val, *v32, W->nnz);
             made = true;
         }
+        if ((tiled || exact_box || ff_box) && W->in_shape1 % 4 == 0 && ((uintptr_t)vin & 15) == 0 && shapes_usable(W, stack))
+            W->in_fixed = true;
         int load = -1;  // how the patch kernel fills its stages, -1: it does not take the call
         if (((tiled && W->in_shape1 % 4 == 0) || exact_box || exact64 || ff_box) && box_usable(W, stack)) {
             RG_TRY(box_lists_for(W, s, &made));

@@ -928,12 +928,13 @@ int apply_tiled(const rg_weights_state* W, int g, const float* vin, float* vout,
 
 // Whether the patch kernel may take calls with this handle: output and input
 // grid shapes known.
-bool box_usable(const rg_weights_state* W, int64_t stack) {
-    return W->box_state >= 0 && W->out_shape0 > 0 && W->out_shape1 > 0 &&
+bool shapes_usable(const rg_weights_state* W, int64_t stack) {
+    return W->out_shape0 > 0 && W->out_shape1 > 0 &&
            W->out_shape0 * W->out_shape1 == W->n_out && W->in_shape0 > 0 && W->in_shape1 > 0 &&
            W->in_shape0 * W->in_shape1 == W->n_in && stack >= 1 && W->n_in < INT32_MAX && stack < INT32_MAX &&
            encode_tiled() != nullptr;
 }
+bool box_usable(const rg_weights_state* W, int64_t stack) { return W->box_state >= 0 && shapes_usable(W, stack); }
 
 // How the patch kernel would fill its stages for this call, -1 when it does
 // not take it (the caller holds the handle's lock, box_lists_for has run).

@@ -643,11 +643,10 @@ int rg_weights_set_input_shape(rg_weights w, int64_t n0, int64_t n1) {
              (long long)n1, (long long)w->n_in);
     std::lock_guard<std::mutex> lock(w->mu);
     if (w->in_shape0 == n0 && w->in_shape1 == n1) return RG_OK;
-    // (exact or compensated applies made patch lists for rows that are not
-    // whole 16-byte chunks)
-    if (w->box_state != 0 && w->in_shape1 % 4 != 0 && !w->box_val) RG_TRY(retire_patch_lists(w));
-    RG_CHECK(w->box_state == 0, RG_ERR_ARG,
-             "rg_weights_set_input_shape: the input tiling is fixed once a fast float32 apply has run");
+    RG_CHECK(!w->in_fixed, RG_ERR_ARG,
+             "rg_weights_set_input_shape: the input tiling is fixed once a float32 apply has staged it");
+    // (lists of float64 stacks, of rows that are no whole 16-byte chunks, or made by calls off a boundary)
+    if (w->box_state != 0) RG_TRY(retire_patch_lists(w));
     w->in_shape0 = n0;
     w->in_shape1 = n1;
     return RG_OK;

@@ -227,6 +227,7 @@ struct rg_weights_state {
     // shape for the tensor-map (TMA) staging of the input slices
     int64_t out_shape0 = 0, out_shape1 = 0;
     int64_t in_shape0 = 0, in_shape1 = 0;
+    bool in_fixed = false;  // a float32 apply has staged 16-byte aligned rows of that shape
     // warp-tile lists of the float32 fast apply, built on first use; index 0
     // lists single cells, index 1 lists 32-byte sectors of 8 cells
     bool tiled_ready[2] = {false, false};

@@ -88,3 +88,31 @@ def test_applies_beside_new_shapes():
         t.join()
     assert not bad
     dw.free()
+
+
+@pytest.mark.parametrize("calls", ["two float64", "unaligned float32"])
+def test_input_shape_stays_open(calls):
+    """Calls that stage no aligned float32 rows leave the input shape free."""
+    torch, dw, v, want = handle((40, 48), (30, 33))
+    if calls == "two float64":
+        for _ in range(2):
+            dw.apply(v.double())
+    else:
+        off = torch.empty(v.numel() + 1, device="cuda")[1:].reshape(v.shape)
+        off.copy_(v)
+        dw.apply(off)
+    assert set_shape(dw, "input", (48, 40)) == 0
+    for x in (v.double(), v.double(), v):
+        np.testing.assert_array_equal(dw.apply(x).cpu().numpy(), want)
+    dw.free()
+
+
+@pytest.mark.parametrize("mode", ["exact", "compensated", "fast"])
+def test_input_shape_is_fixed_by_staged_rows(mode):
+    from regridding_gb300 import _lib
+
+    torch, dw, v, want = handle((40, 48), (30, 33))
+    dw.apply(v, accumulate=mode)
+    assert set_shape(dw, "input", (48, 40)) == _lib.RG_ERR_ARG
+    assert set_shape(dw, "input", (40, 48)) == 0
+    dw.free()
