@@ -183,6 +183,19 @@ int rows_usable(rg_weights_s* W, const float* vin, int64_t stack, cudaStream_t s
 int apply_rows_launch(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s);
 int ensure_transposed(rg_weights_s* W, cudaStream_t s);
 
+// Whether compensated calls sum float pairs (else they compute as exact).
+bool float_pairs(const rg_weights_state* W) {
+    return W->box_state == 1 || W->box_long * FF_LONG_SHARE <= W->n_out;
+}
+
+// Whether an exact (or compensated) call over a float32 stack finds all that
+// box_lists_for and its like would make.
+bool lists_ready(const rg_weights_state* W, bool ff, int64_t stack) {
+    if (W->box_state <= 0) return W->box_state < 0;
+    if (!ff || !float_pairs(W)) return W->box_perm != nullptr;
+    return W->ff_slot && (W->box_state == 2 || W->box_cfg_ff[stack_class(stack)] != -1);
+}
+
 // Every apply goes through here.  The per-handle state an apply needs beyond
 // the CSR (the transposed CSR, the float32 copy of the weights, the warp-tile
 // lists) is made on first use under the handle's mutex and finished (the
@@ -242,8 +255,16 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
         }
         if ((tiled || exact_box || ff_box) && W->in_shape1 % 4 == 0 && ((uintptr_t)vin & 15) == 0 && shapes_usable(W, stack))
             W->in_fixed = true;
+        // the lists of a call are read back by the host: while a graph is captured
+        // float32 stacks with float64 sums gather where they are not there yet
+        bool boxes = box_usable(W, stack);
+        if ((exact_box || ff_box) && boxes && !lists_ready(W, ff_box, stack)) {
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            RG_CUDA(cudaStreamIsCapturing(s, &capture));
+            boxes = capture == cudaStreamCaptureStatusNone;
+        }
         int load = -1;  // how the patch kernel fills its stages, -1: it does not take the call
-        if (((tiled && W->in_shape1 % 4 == 0) || exact_box || exact64 || ff_box) && box_usable(W, stack)) {
+        if (((tiled && W->in_shape1 % 4 == 0) || exact_box || exact64 || ff_box) && boxes) {
             RG_TRY(box_lists_for(W, s, &made));
             load = box_load(W, (const float*)vin, stack);
         }
@@ -273,7 +294,7 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
         // compensated calls whose rows are too long for float-float sums, whose
         // footprints are too large for any box, without shapes or off a 16-byte
         // boundary of the swizzled box compute as exact
-        const bool ff_rows = W->box_state == 1 || W->box_long * FF_LONG_SHARE <= W->n_out;
+        const bool ff_rows = float_pairs(W);
         if ((exact_box || (ff_box && !ff_rows)) && load >= 0) {
             use_box_exact = true;
             RG_TRY(box_perm_for(W, s, &made));

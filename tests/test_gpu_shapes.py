@@ -116,3 +116,20 @@ def test_input_shape_is_fixed_by_staged_rows(mode):
     assert set_shape(dw, "input", (48, 40)) == _lib.RG_ERR_ARG
     assert set_shape(dw, "input", (40, 48)) == 0
     dw.free()
+
+
+@pytest.mark.parametrize("shape_in", [(41, 43), (40, 48)])
+@pytest.mark.parametrize("mode", ["exact", "compensated"])
+def test_first_call_under_capture(shape_in, mode):
+    """A captured call makes no lists (the host would read them back): where a
+    fast apply has made the float32 weights, its gathers are captured."""
+    torch, dw, v, want = handle(shape_in, (30, 33))
+    out = torch.empty(want.shape, dtype=torch.float64, device="cuda")
+    dw.apply(v, accumulate="fast")
+    graph = captured(torch, lambda: dw.apply(v, out=out, accumulate=mode))
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
+        assert near(dw.apply(v, accumulate=mode), want)
+    dw.free()
