@@ -319,7 +319,10 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
         const int st = apply_wide_f64(&now, load64, (const double*)vin, (double*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
     }
-    if (use_rows) return apply_rows_launch(&now, (const float*)vin, (float*)vout, stack, s);
+    if (use_rows) {
+        const int st = apply_rows_launch(&now, (const float*)vin, (float*)vout, stack, s);
+        if (st != RG_ERR_UNSUPPORTED) return st;
+    }
     if (use_box_exact) {
         const int st = apply_box_exact(&now, (const float*)vin, (double*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
@@ -331,8 +334,11 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     if (use_box) {
         const int st = apply_box(&now, (const float*)vin, (float*)vout, stack, s);
         if (st != RG_ERR_UNSUPPORTED) return st;
+    }
+    if (use_rows || use_box) {
         // the tuned configuration does not take this call (fewer slices than
-        // a stage): the warp-staged kernel does, with its own lists
+        // a stage), or the device not the kernel's shared memory: the
+        // warp-staged kernel does, with its own lists
         std::lock_guard<std::mutex> lock(W->mu);
         bool made = false;
         RG_TRY(tiled_lists_for(W, (const float*)vin, s, &g, &made));

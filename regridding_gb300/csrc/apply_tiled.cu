@@ -1194,12 +1194,8 @@ int launch_patch(const rg_weights_state* W, const CUtensorMap& map, int box_slic
     const unsigned box_bytes = (unsigned)((PLANES ? 1 : box_slices) * BR * PBOX_C * 4);
     const size_t smem = (size_t)NST * stage_floats * sizeof(float);
     if (smem > 200 * 1024) return RG_ERR_UNSUPPORTED;
-    static std::once_flag attr;
-    std::call_once(attr, []() {
-        cudaFuncSetAttribute(apply_patch_tma<SPS, NST, MINB, MODE, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
-        cudaGetLastError();
-    });
+    static SharedLimit limit;
+    if (!allow_shared((const void*)apply_patch_tma<SPS, NST, MINB, MODE, CT>, 200 * 1024, limit)) return RG_ERR_UNSUPPORTED;
     const int64_t patches = W->box_patches;
     // split the stack over gridDim.y only when the patches alone give less
     // than ~4 waves of 4 blocks per SM on 152 SMs
@@ -1437,11 +1433,8 @@ int rows_usable(rg_weights_s* W, const float* vin, int64_t stack, cudaStream_t s
 int apply_rows_launch(const rg_weights_state* W, const float* vin, float* vout, int64_t stack, cudaStream_t s) {
     const int stage_floats = (int)((W->n_in + 31) & ~31ll);  // stages start on 128-byte boundaries
     const size_t smem = (size_t)ROWS_NST * stage_floats * sizeof(float);
-    static std::once_flag attr;
-    std::call_once(attr, []() {
-        cudaFuncSetAttribute(apply_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaGetLastError();
-    });
+    static SharedLimit limit;
+    if (!allow_shared((const void*)apply_rows, 200 * 1024, limit)) return RG_ERR_UNSUPPORTED;
     const int64_t blocks = std::min<int64_t>(stack, 152 * 2);
     apply_rows<<<(unsigned)blocks, ROWS_THREADS, smem, s>>>(W->row_ptr, W->col, W->val32, vin, W->n_in, vout,
                                                             W->n_out, stack, stage_floats, W->dflags);

@@ -27,11 +27,8 @@ int launch_wide(const rg_weights_state* W, BoxShape box, const TIN* vin, void* v
     constexpr int CT = MODE == MODE_FF ? 6 : CACHED_T;
     const auto kernel = apply_patch_tma<SPS, NST, 0, MODE, CT, LOAD, PL, TIN>;
     const size_t smem = (size_t)NST * SPS * PL * sizeof(TIN);
-    static std::once_flag attr;
-    std::call_once(attr, [&]() {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaGetLastError();
-    });
+    static SharedLimit limit;
+    if (!allow_shared((const void*)kernel, 200 * 1024, limit)) return RG_ERR_UNSUPPORTED;
     CUtensorMap map = {};
     if (!encode_stack(W, vin, stack, 1, box.pitch, (int)sizeof(TIN), &map)) return RG_ERR_UNSUPPORTED;
     const int64_t patches = W->box_patches;

@@ -284,6 +284,18 @@ int weights_from_entries(const CooRows& C, int64_t nnz, int64_t n_in, int64_t n_
 
 }  // namespace
 
+bool allow_shared(const void* kernel, size_t bytes, SharedLimit& known) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const bool keep = dev >= 0 && dev < 64;
+    const signed char before = keep ? known[dev].load(std::memory_order_acquire) : 0;
+    if (before) return before > 0;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    if (keep) known[dev].store(ok ? 1 : -1, std::memory_order_release);
+    return ok;
+}
+
 void init_pool_once() {
     static std::once_flag flags[64];
     int dev = 0;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdio>
 #include <mutex>
 #include <string>
@@ -165,6 +166,12 @@ struct FastDiv {
 bool kernel_host_access();
 // cudaMemsetAsync(p, 0, n, s) as a kernel, for the small clears of the build
 int zero_async(void* p, size_t n, cudaStream_t s);
+
+// Lets a kernel take `bytes` of dynamic shared memory on the current device
+// (the limit belongs to a device; known: a kernel's own, what has been set on
+// each).  False where the device does not allow it.
+typedef std::atomic<signed char> SharedLimit[64];
+bool allow_shared(const void* kernel, size_t bytes, SharedLimit& known);
 int small_to_host(void* h_dst, const void* d_src, size_t n, cudaStream_t s);
 int small_to_device(void* d_dst, const void* h_src, size_t n, cudaStream_t s);
 

@@ -146,3 +146,19 @@ def test_debug_library_builds_with_every_symbol():
     for name in declared_symbols():
         assert hasattr(dbg, name), name
     assert dbg.rg_version() == _lib.load().rg_version()
+
+
+def test_shared_memory_limits_are_set_per_device():
+    """cudaFuncSetAttribute acts on the current device only: kernels that take
+    more than 48 KB ask allow_shared at every launch, and nothing sets the
+    limit once for the process."""
+    import pathlib
+    import re
+
+    csrc = pathlib.Path(__file__).resolve().parent.parent / "regridding_gb300" / "csrc"
+    sites = [(f.name, m.start()) for f in csrc.iterdir() if f.suffix in (".cu", ".cuh")
+             for m in re.finditer("cudaFuncAttributeMaxDynamicSharedMemorySize", f.read_text())]
+    assert [name for name, _ in sites] == ["capi.cu"]
+    for name in ("apply_wide.cu", "apply_tiled.cu"):
+        text = (csrc / name).read_text()
+        assert text.count("SharedLimit limit;") == text.count("allow_shared(") >= 1
