@@ -169,6 +169,7 @@ int apply_tiled(const rg_weights_state* W, int g, const float* vin, float* vout,
 bool shapes_usable(const rg_weights_state* W, int64_t stack);
 bool box_usable(const rg_weights_state* W, int64_t stack);
 int box_load(const rg_weights_state* W, const void* vin, int64_t stack);
+bool exact_staged(const rg_weights_state* W, int load, int bytes, int64_t stack);
 int apply_wide_f64(const rg_weights_state* W, int load, const double* vin, double* vout, int64_t stack, cudaStream_t s);
 int box_order_for(rg_weights_s* W, cudaStream_t s, bool* made);
 int box_lists_for(rg_weights_s* W, cudaStream_t s, bool* made);
@@ -282,20 +283,14 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
             }
             use_box = load != LOAD_SWIZZLED || W->box_cfg[stack_class(stack)] >= 0;
         }
-        // (boxes of more than 1536 cells, of coarse outputs with long rows, pay
-        // from 16 slices on: 1000 x 700 -> 500 x 350 with 4, 8 and 16 slices 48, 89
-        // and 171 us gathered, 55, 95 and 150 us staged; smaller boxes from two
-        // on: 1024^2 -> 768^2 with 4, 8 slices 84, 164 us gathered, 73, 133 staged;
-        // 2048^2 -> 1536^2 with 16 slices 1.20 and 0.94 ms, FP64 issue 0.65 ms)
-        exact64 = exact64 && load >= 0 &&
-                  (stack >= 16 || (W->box_residues ? 4 * W->box_residues : W->box_rows * W->box_cols) <= 1536);
+        exact64 = exact64 && load >= 0 && exact_staged(W, load, 8, stack);
         load64 = load;
         if (exact64) RG_TRY(box_perm_for(W, s, &made));
         // compensated calls whose rows are too long for float-float sums, whose
         // footprints are too large for any box, without shapes or off a 16-byte
         // boundary of the swizzled box compute as exact
         const bool ff_rows = float_pairs(W);
-        if ((exact_box || (ff_box && !ff_rows)) && load >= 0) {
+        if ((exact_box || (ff_box && !ff_rows)) && load >= 0 && exact_staged(W, load, 4, stack)) {
             use_box_exact = true;
             RG_TRY(box_perm_for(W, s, &made));
         }
