@@ -1392,6 +1392,11 @@ __global__ void __launch_bounds__(128)
             c0 += 32;
             continue;
         }
+        // A walk of the pair has met its step cap: its weights are an error, and
+        // a line that cycles would do so in each of its chunks again.
+        unsigned fl = 0;
+        if (lane == 0) fl = *(const volatile unsigned*)flags;
+        if (__shfl_sync(0xffffffffu, fl, 0) & FLAG_WALK_CAP) return;
         const int64_t c = c0 + __ffs(differ) - 1;
         if (lane == 0) {
             atomicAdd(n_repaired, 1ull);

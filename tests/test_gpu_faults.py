@@ -55,6 +55,29 @@ def test_undersized_chunk_slots_take_the_recovery_path(rg, monkeypatch):
             assert_same(g, e)
 
 
+def test_cycling_walks_end_soon(rg, monkeypatch):
+    """A pair whose walk cycles around a shared vertex is reported about as
+    soon as its whole lines are walked: the line's further chunks are not
+    walked to their step caps, too (five times as long)."""
+    import time
+
+    import torch
+
+    from regridding_gb300 import workloads
+
+    gi, go = ([torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in g]
+              for g in (workloads.distorted_grid(65, 0.3, 0.02), workloads.rect_grid(49, -1.05, 1.05)))
+    seconds = []
+    for chunk in ("0", None):
+        monkeypatch.setenv("RG_SWEEP_CHUNK", chunk) if chunk else monkeypatch.delenv("RG_SWEEP_CHUNK")
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        with pytest.raises(rg.RegridError, match="step cap"):
+            rg.build_conservative_2d(gi, go)
+        seconds.append(time.perf_counter() - t0)
+    assert seconds[1] < 3 * seconds[0], seconds
+
+
 def test_debug_library_builds_and_matches():
     code = f"""
 import sys
