@@ -446,6 +446,33 @@ __global__ void median_hist(const T* __restrict__ a, const uint8_t* __restrict__
     }
 }
 
+// the same over the copied candidate keys of each slice
+__global__ void median_hist_keys(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets,
+                                 int64_t nt, int shift, const MedianState* __restrict__ st,
+                                 unsigned* __restrict__ hist) {
+    __shared__ unsigned h[256];
+    const unsigned lane = threadIdx.x & 31u;
+    for (int64_t t = blockIdx.y; t < nt; t += gridDim.y) {
+        for (int b = threadIdx.x; b < 256; b += blockDim.x) h[b] = 0;
+        __syncthreads();
+        const unsigned long long prefix = st[t].prefix, mask = st[t].mask;
+        const int64_t lo = offsets[t], hi = offsets[t + 1];
+        for (int64_t base = lo + blockIdx.x * (int64_t)blockDim.x; base < hi; base += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t c = base + threadIdx.x;
+            unsigned bin = 0xffffffffu;
+            if (c < hi) {
+                const unsigned long long key = keys[c];
+                if ((key & mask) == prefix) bin = (unsigned)(key >> shift) & 255u;
+            }
+            hist_add(h, bin, lane);
+        }
+        __syncthreads();
+        for (int b = threadIdx.x; b < 256; b += blockDim.x)
+            if (h[b]) atomicAdd(&hist[t * 256 + b], h[b]);
+        __syncthreads();
+    }
+}
+
 // One warp per slice chooses the digit holding rank k (the first pass
 // counts the valid keys, which fixes k) and clears the histogram.
 __global__ void median_pick(MedianState* __restrict__ st, unsigned* __restrict__ hist, int64_t nt, int shift,
@@ -565,6 +592,7 @@ __global__ void median_compact(const T* __restrict__ a, const uint8_t* __restric
 // through it, the digit holding rank k chosen in every block alike; then the
 // candidates <= the lower median and the smallest one above it.  (A launch per
 // step took 14 us a digit on 4 slices of 480 x 641: 0.13 ms, now 0.04 ms.)
+// For few candidates (median_clusters); where many fill the chip, median_hist_keys.
 __global__ void __launch_bounds__(kRelaxThreads)
     median_digits(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets, int first_shift,
                   MedianState* __restrict__ st) {
@@ -660,6 +688,35 @@ __global__ void __launch_bounds__(kRelaxThreads)
     }
 }
 
+// candidates <= the lower median, and the smallest candidate above it
+__global__ void median_upper_keys(const unsigned long long* __restrict__ keys, const int64_t* __restrict__ offsets,
+                                  int64_t nt, MedianState* __restrict__ st) {
+    __shared__ unsigned long long le, gt;
+    for (int64_t t = blockIdx.y; t < nt; t += gridDim.y) {
+        if (threadIdx.x == 0) {
+            le = 0;
+            gt = ~0ull;
+        }
+        __syncthreads();
+        const unsigned long long lo = st[t].prefix;
+        unsigned long long my_le = 0, my_gt = ~0ull;
+        for (int64_t c = offsets[t] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < offsets[t + 1];
+             c += (int64_t)gridDim.x * blockDim.x) {
+            const unsigned long long key = keys[c];
+            if (key <= lo) ++my_le;
+            else if (key < my_gt) my_gt = key;
+        }
+        if (my_le) atomicAdd(&le, my_le);
+        if (my_gt != ~0ull) atomicMin(&gt, my_gt);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (le) atomicAdd(&st[t].count_le, le);
+            if (gt != ~0ull) atomicMin(&st[t].min_gt, gt);
+        }
+        __syncthreads();
+    }
+}
+
 template <typename T>
 __global__ void median_write(const MedianState* __restrict__ st, int64_t nt, T* __restrict__ out) {
     using KT = Keys<T>;
@@ -697,6 +754,18 @@ dim3 slice_grid(int64_t nt, int64_t S, int64_t per_block) {
     return dim3((unsigned)gx, (unsigned)(ty < 1 ? 1 : ty));
 }
 
+// Whether clusters of c blocks a slice find the remaining digits of nt slices
+// with `total` candidates: a pass takes them 0.26 us for every kRelaxThreads * c
+// candidates of a slice, and launches about 9 us and the candidates at 2 TB/s.
+// (float64, launches and clusters, on the whole median: one slice of 512^2 with
+// 241 K candidates 181 and 174 us, one of 1024^2 with 0.77 M 189 and 255, one of
+// 2048^2 with 3.9 M 0.29 and 1.06 ms, 64 of 1024^2 with 0.96 M each 3.07 and 2.90
+// ms.  More slices than run at a time, one block each: 5000 of 4096, float32, 400
+// and 428 us.)
+bool median_clusters(int64_t total, int64_t nt, int c) {
+    return c > 1 && 0.26 * (double)total / ((double)nt * c * kRelaxThreads) <= 9.0 + (double)total * 8 / 2e6;
+}
+
 template <typename T>
 int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out, cudaStream_t s) {
     MedianState* st = nullptr;
@@ -731,8 +800,19 @@ int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out,
         RG_CUDA(cudaStreamSynchronize(s));
         if ((status = dalloc(&keys, total > 0 ? total : 1, s))) break;
         median_compact<T><<<grid, 256, 0, s>>>(a, where, nt, S, st, offsets, cursor, keys);
-        RG_CUDA(launch_clusters(median_digits, nt, cluster_for(median_digits, nt, 0), s, keys, offsets,
-                                Keys<T>::kBits - 8 * (kDataPasses + 1), st));
+        constexpr int kPasses = Keys<T>::kBits / 8;
+        const int c = cluster_for(median_digits, nt, 0);
+        if (median_clusters(total, nt, c)) {
+            RG_CUDA(launch_clusters(median_digits, nt, c, s, keys, offsets, Keys<T>::kBits - 8 * (kDataPasses + 1), st));
+        } else {
+            const dim3 kgrid = slice_grid(nt, (total + nt - 1) / nt, 4096);
+            for (int pass = kDataPasses; pass < kPasses; ++pass) {
+                const int shift = Keys<T>::kBits - 8 * (pass + 1);
+                median_hist_keys<<<kgrid, 256, 0, s>>>(keys, offsets, nt, shift, st, hist);
+                median_pick<<<gw, 256, 0, s>>>(st, hist, nt, shift, pass);
+            }
+            median_upper_keys<<<kgrid, 256, 0, s>>>(keys, offsets, nt, st);
+        }
         median_write<T><<<g1, 256, 0, s>>>(st, nt, out);
         RG_CUDA(cudaGetLastError());
     } while (0);

@@ -139,6 +139,50 @@ def test_gpu_median(torch):
         np.testing.assert_array_equal(out.cpu().numpy(), exp.astype(dtype))
 
 
+def _median(a, where, torch):
+    from regridding_gb300 import _device, _lib
+
+    out = torch.empty(a.shape[0], dtype=a.dtype, device="cuda")
+    _lib.call("rg_fill_median", _device.ptr(a), _lib.RG_F64 if a.dtype == torch.float64 else _lib.RG_F32,
+              _device.ptr(where), a.shape[0], a.shape[1], _device.ptr(out), _device.stream())
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("nt,cells", [(1, 250_001), (1, 600_000), (1, 1 << 22), (3, 700_001), (40, 60_000), (700, 999)])
+def test_gpu_median_of_close_values(torch, dtype, nt, cells):
+    """Slices whose values share their leading digits, on both sides of the
+    candidate counts that clusters take, against numpy's median."""
+    rng = np.random.default_rng(33)
+    a = (1000 + 1e-3 * rng.normal(0, 1, (nt, cells))).astype(dtype)
+    where = rng.uniform(0, 1, a.shape) < 0.05
+    got = _median(torch.from_numpy(a).cuda(), torch.from_numpy(where.astype(np.uint8)).cuda(), torch)
+    want = oracle.fill_median_guess(a, where, (1,))[:, 0].astype(dtype)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+def test_gpu_median_of_one_large_slice(torch):
+    """The median of 2^24 close values takes one slice about as long as 64
+    (the latter fill the chip; one slice on 16 blocks took seven times that)."""
+    import time
+
+    a = 1000 + 1e-3 * torch.randn(1 << 24, dtype=torch.float64, device="cuda")
+    where = torch.zeros(1 << 24, dtype=torch.uint8, device="cuda")
+    seconds = {}
+    for nt in (64, 1):
+        times = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            _median(a.reshape(nt, -1), where, torch)
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t0)
+        seconds[nt] = min(times)
+    assert seconds[1] < 3 * seconds[64], seconds
+
+
 @pytest.mark.gpu
 def test_gpu_axis_of_length_one(torch):
     import regridding_gb300 as rg
