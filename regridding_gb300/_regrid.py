@@ -223,17 +223,23 @@ def _short_elements(flat: np.ndarray, groups: dict, first: dict):
     return Entries(*(_device.upload(h) for h in host), _device.upload(count), (len(arrays),)), element
 
 
+# Input and output of a block diagonal matrix's slices on the device, at most
+# (an element's own slices are never cut).
+BLOCK_BYTES = 1 << 30
+
+
 def _apply_blocks(entries, n_in: int, n_out: int, element: np.ndarray, v_in: np.ndarray, in_dtype, out: np.ndarray,
                   accumulate: str) -> None:
     """Slice ``d`` of ``v_in`` through element ``element[d]`` of the device
     ``entries`` into ``out[d]``: block diagonal matrices over as many
-    elements as 2^31 cells hold, each with one apply.  (The elements one by
-    one, 256 spectra of 512 -> 384 cells: 118 ms.)"""
+    elements as 2^31 cells and BLOCK_BYTES hold, each with one apply.  (The
+    elements one by one, 256 spectra of 512 -> 384 cells: 118 ms.)"""
     t = _device.torch()
     if element.size == 0:
         return
     nd, stride = entries.ind_in.shape
-    most = max(1, min((2**31 - 2) // max(n_in, n_out, 1), (2**32 - 2) // max(stride, 1)))
+    nbytes = element.size // nd * (n_in * np.dtype(in_dtype).itemsize + n_out * out.dtype.itemsize)
+    most = max(1, min((2**31 - 2) // max(n_in, n_out, 1), (2**32 - 2) // max(stride, 1), BLOCK_BYTES // max(nbytes, 1)))
     # slices of an element side by side: (slices, elements)
     order = np.argsort(element, kind="stable").reshape(nd, -1)
     for d in range(0, nd, most):
@@ -241,14 +247,16 @@ def _apply_blocks(entries, n_in: int, n_out: int, element: np.ndarray, v_in: np.
         count = None if entries.count is None else entries.count[d:d + most]
         dw = _device.DeviceWeights.block_diagonal(entries.ind_in[d:d + most], entries.ind_out[d:d + most],
                                                   entries.val[d:d + most], count, n_in, n_out)
-        whole = rows.size == element.size and np.array_equal(rows.reshape(-1), np.arange(element.size))
-        src = _device.upload(v_in if whole else v_in[rows.reshape(-1)], in_dtype)
+        at = rows.reshape(-1)
+        if np.array_equal(at, np.arange(at[0], at[0] + at.size)):
+            at = slice(at[0], at[0] + at.size)
+        src = _device.upload(v_in[at], in_dtype)
         dst = t.empty((rows.shape[0], rows.shape[1] * n_out), dtype=_device.torch_dtype(out.dtype), device="cuda")
         dw.apply(src.reshape(rows.shape[0], -1), out=dst, accumulate=accumulate)
-        if whole:
-            t.from_numpy(out).copy_(dst.reshape(-1, n_out))
+        if isinstance(at, slice):
+            t.from_numpy(out[at]).copy_(dst.reshape(-1, n_out))
         else:
-            out[rows.reshape(-1)] = _device.download(dst).reshape(-1, n_out)
+            out[at] = _device.download(dst).reshape(-1, n_out)
         dw.free()
 
 
