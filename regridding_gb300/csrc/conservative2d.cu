@@ -2166,7 +2166,9 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
         c.chunk_base[4] = chunks;
     }
     chunk_base[G] = chunks;
-    if (slots * 16 > (int64_t)24 << 30 || slots >= (int64_t)1 << 40) return RG_OK;  // too big: walk lines
+    // too big: walk lines (a slot: a piece and its two triples' places)
+    constexpr int64_t SLOT_BYTES = 2 * sizeof(int32_t) + sizeof(double) + sizeof(uint2);
+    if (slots > ((int64_t)24 << 30) / SLOT_BYTES) return RG_OK;
 
     WalkState *starts = nullptr, *ends = nullptr;
     int64_t *counts = nullptr, *offsets = nullptr;
