@@ -38,6 +38,32 @@
 #include <vector>
 
 #include "common.cuh"
+
+#ifdef RG_DEBUG
+// Debug builds (-DRG_DEBUG, regridding_gb300._build.build(debug=True)): the
+// grid reads whose place is computed (seats, guesses, walk) are
+// bounds-checked.  A read outside the array sets FLAG_BOUNDS here and yields
+// NaN (no trap: the build runs to its end and the host turns the flag into
+// RG_ERR_WALK).
+namespace rg {
+namespace {
+__device__ unsigned g_debug_flags;
+__device__ __forceinline__ bool debug_in_grid(int64_t i, int64_t j, int64_t nx, int64_t ny) {
+    if (i >= 0 && j >= 0 && i < nx && j < ny) return true;
+    atomicOr(&g_debug_flags, FLAG_BOUNDS);
+    return false;
+}
+}  // namespace
+}  // namespace rg
+#define RG_GRID_READ(a, i, j) \
+    (debug_in_grid(i, j, nx, ny) ? __ldg((a) + (i) * ny + (j)) : __longlong_as_double(0x7ff8000000000000ll))
+#define RG_FLAT_READ(a, k, n) \
+    (debug_in_grid(0, k, 1, n) ? __ldg((a) + (k)) : __longlong_as_double(0x7ff8000000000000ll))
+#else
+#define RG_GRID_READ(a, i, j) __ldg((a) + (i) * ny + (j))
+#define RG_FLAT_READ(a, k, n) __ldg((a) + (k))
+#endif
+
 #include "inside.cuh"
 #include "seed.cuh"
 
@@ -245,23 +271,6 @@ __device__ __forceinline__ double winding_term(double x, double y, double vx0, d
     return 0.0;
 }
 
-#ifdef RG_DEBUG
-// Debug builds (-DRG_DEBUG, regridding_gb300._build.build(debug=True)): every
-// grid read of the build is bounds-checked.  A read outside the array sets
-// FLAG_BOUNDS here and yields NaN (no trap: the build runs to its end and
-// the host turns the flag into RG_ERR_WALK).
-__device__ unsigned g_debug_flags;
-__device__ __forceinline__ bool debug_in_grid(int64_t i, int64_t j, int64_t nx, int64_t ny) {
-    if (i >= 0 && j >= 0 && i < nx && j < ny) return true;
-    atomicOr(&g_debug_flags, FLAG_BOUNDS);
-    return false;
-}
-#define RG_GRID_READ(a, i, j) \
-    (debug_in_grid(i, j, nx, ny) ? __ldg((a) + (i) * ny + (j)) : __longlong_as_double(0x7ff8000000000000ll))
-#else
-#define RG_GRID_READ(a, i, j) __ldg((a) + (i) * ny + (j))
-#endif
-
 struct Grid {
     const double* x;
     const double* y;
@@ -297,8 +306,9 @@ __device__ double bilinear(const double* a, int64_t sx, int64_t sy, double x, do
     else if (x00 > sx - 2) x00 = sx - 2;
     if (y00 < 0) y00 = 0;
     else if (y00 > sy - 2) y00 = sy - 2;
-    double a00 = __ldg(a + x00 * sy + y00), a01 = __ldg(a + x00 * sy + y00 + 1);
-    double a10 = __ldg(a + (x00 + 1) * sy + y00), a11 = __ldg(a + (x00 + 1) * sy + y00 + 1);
+    const int64_t k = x00 * sy + y00, n = sx * sy;
+    double a00 = RG_FLAT_READ(a, k, n), a01 = RG_FLAT_READ(a, k + 1, n);
+    double a10 = RG_FLAT_READ(a, k + sy, n), a11 = RG_FLAT_READ(a, k + sy + 1, n);
     double dx = dsub(x, (double)x00), dy = dsub(y, (double)y00);
     double w00 = dmul(dsub(1.0, dx), dsub(1.0, dy)), w01 = dmul(dsub(1.0, dx), dy);
     double w10 = dmul(dx, dsub(1.0, dy)), w11 = dmul(dx, dy);
@@ -2665,7 +2675,10 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
             st = RG_ERR_CUDA;
             break;
         }
+    } while (0);
+
 #ifdef RG_DEBUG
+    if (st == RG_OK) {  // (a build that fails otherwise leaves the word to the next)
         unsigned dbg = 0;
         const unsigned zero = 0;
         cudaMemcpyFromSymbolAsync(&dbg, g_debug_flags, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, s);
@@ -2673,14 +2686,12 @@ int build_batch(const PairSpec* pairs, int G, cudaStream_t s, rg_weights_s** W, 
         if (cudaStreamSynchronize(s) != cudaSuccess) {
             set_error("conservative build (debug flags): %s", cudaGetErrorString(cudaGetLastError()));
             st = RG_ERR_CUDA;
-            break;
-        }
-        if (dbg & FLAG_BOUNDS) {
+        } else if (dbg & FLAG_BOUNDS) {
             set_error("conservative build: debug bounds check: a grid read fell outside its array");
             for (int g = 0; g < G; g++) status[g] = RG_ERR_WALK;
         }
+    }
 #endif
-    } while (0);
 
     dfree(area_in, s);
     dfree(bbox_d, s);
@@ -2726,3 +2737,12 @@ extern "C" int rg_set_sweep_chunk(int64_t segments) {
     return RG_OK;
 }
 
+#ifdef RG_DEBUG
+// Debug builds, for tests of the reporting: sets the bounds word as a read
+// outside an array does.
+extern "C" int rg_debug_out_of_bounds() {
+    const unsigned word = rg::FLAG_BOUNDS;
+    RG_CUDA(cudaMemcpyToSymbol(rg::g_debug_flags, &word, sizeof(word)));
+    return RG_OK;
+}
+#endif

@@ -5,6 +5,11 @@
 
 #include "inside.cuh"
 
+// Element k of an array of n (a debug build's checked read, where one is defined).
+#ifndef RG_FLAT_READ
+#define RG_FLAT_READ(a, k, n) __ldg((a) + (k))
+#endif
+
 namespace rg {
 
 // Approximate cell (ci, cj) of point (px, py) in the grid of nx x ny
@@ -22,8 +27,8 @@ __device__ __forceinline__ bool seed_cell(const double* __restrict__ X, const do
     float fi = 0.5f * (float)ncx, fj = 0.5f * (float)ncy;
     bool ok = true;
     const float fx = SINGLE ? trunc_float(px, ok) : 0.f, fy = SINGLE ? trunc_float(py, ok) : 0.f;
-    auto dx_of = [&](int64_t v) { return SINGLE ? trunc_float(__ldg(X + v), ok) - fx : (float)(__ldg(X + v) - px); };
-    auto dy_of = [&](int64_t v) { return SINGLE ? trunc_float(__ldg(Y + v), ok) - fy : (float)(__ldg(Y + v) - py); };
+    auto dx_of = [&](int64_t v) { return SINGLE ? trunc_float(RG_FLAT_READ(X, v, nx * ny), ok) - fx : (float)(RG_FLAT_READ(X, v, nx * ny) - px); };
+    auto dy_of = [&](int64_t v) { return SINGLE ? trunc_float(RG_FLAT_READ(Y, v, nx * ny), ok) - fy : (float)(RG_FLAT_READ(Y, v, nx * ny) - py); };
     for (int it = 0; it < 16; it++) {
         int64_t i0 = (int64_t)floorf(fi), j0 = (int64_t)floorf(fj);
         i0 = i0 < 0 ? 0 : (i0 > ncx - 1 ? ncx - 1 : i0);
@@ -71,8 +76,9 @@ __device__ __forceinline__ int locate_single(const double* __restrict__ X, const
     if (!seed_cell<true>(X, Y, nx, ny, px, py, &i, &j)) return -1;
     for (int step = 0; step < 16; step++) {
         const int64_t v00 = i * ny + j, v10 = v00 + ny;
-        const double vx[4] = {__ldg(X + v00), __ldg(X + v10), __ldg(X + v10 + 1), __ldg(X + v00 + 1)};
-        const double vy[4] = {__ldg(Y + v00), __ldg(Y + v10), __ldg(Y + v10 + 1), __ldg(Y + v00 + 1)};
+        const auto at = [&](const double* a, int64_t v) { return RG_FLAT_READ(a, v, nx * ny); };
+        const double vx[4] = {at(X, v00), at(X, v10), at(X, v10 + 1), at(X, v00 + 1)};
+        const double vy[4] = {at(Y, v00), at(Y, v10), at(Y, v10 + 1), at(Y, v00 + 1)};
         const QuadFilter q(vx, vy, px, py);
         int in = q.contains();
         if (in < 0) in = contains(i, j) ? 1 : 0;

@@ -99,3 +99,30 @@ print('debug ok', _lib.load()._name)
     res = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=900)
     assert res.returncode == 0, res.stdout + res.stderr
     assert "debug ok" in res.stdout
+
+
+def test_debug_library_reports_a_single_pairs_bounds():
+    """A bounds word set while one pair is built (here by the host, as a read
+    outside an array would) fails that build, and not the next one."""
+    code = f"""
+import sys
+sys.path.insert(0, {ROOT!r})
+import regridding_gb300 as rg
+from regridding_gb300 import _lib, workloads
+gi = workloads.distorted_grid(33, 0.3, 0.02)
+go = workloads.perturb(workloads.rect_grid(25, -1.05, 1.05))
+rg.build_conservative_2d(gi, go)
+assert _lib.load().rg_debug_out_of_bounds() == _lib.RG_OK
+try:
+    rg.build_conservative_2d(gi, go)
+except rg.RegridError as e:
+    assert 'bounds check' in str(e), e
+else:
+    raise SystemExit('not reported')
+rg.build_conservative_2d(gi, go)
+print('reported')
+"""
+    env = dict(os.environ, RG_DEBUG="1")
+    res = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=900)
+    assert res.returncode == 0, res.stdout + res.stderr
+    assert "reported" in res.stdout
