@@ -129,10 +129,28 @@ __global__ void __launch_bounds__(kClassifyThreads) fill_lists(const uint8_t* __
     }
 }
 
-// the start of every class in the scanned offsets, and the total
-__global__ void fill_class_starts(const int64_t* __restrict__ offsets, int64_t nblocks, int64_t* __restrict__ out) {
-    const int k = threadIdx.x;
-    if (k <= kClasses) out[k] = offsets[k * nblocks];
+// The start of every class in the scanned offsets, and the total; behind them
+// the most entries of one slice in every class, for up to kRelaxSlices slices.
+// A warp per class.
+constexpr int kRelaxSlices = 152;
+__global__ void __launch_bounds__(32 * kClasses)
+    fill_class_starts(const int64_t* __restrict__ offsets, int64_t nblocks, int64_t nt, int64_t tiles,
+                      int64_t* __restrict__ out) {
+    const int k = threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (threadIdx.x <= kClasses) out[threadIdx.x] = offsets[threadIdx.x * nblocks];
+    int64_t most = 0;
+    if (nt <= kRelaxSlices)
+        for (int64_t t = lane; t < nt; t += 32) {
+            const int64_t* at = offsets + k * nblocks + t * tiles;
+            const int64_t n = at[tiles] - at[0];
+            most = n > most ? n : most;
+        }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const int64_t other = __shfl_xor_sync(0xffffffffu, most, d);
+        most = other > most ? other : most;
+    }
+    if (lane == 0) out[kClasses + 1 + k] = most;
 }
 
 struct GsConst {
@@ -863,13 +881,13 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         const int64_t ncounts = kClasses * nblocks + 1;
         if ((status = dalloc(&counts, ncounts, s))) break;
         if ((status = dalloc(&offsets, ncounts, s))) break;
-        if ((status = dalloc(&starts_dev, kClasses + 1, s))) break;
+        if ((status = dalloc(&starts_dev, 2 * kClasses + 1, s))) break;
         RG_CUDA(cudaMemsetAsync(counts, 0, ncounts * sizeof(unsigned), s));
         const dim3 cgrid((unsigned)tiles, (unsigned)(nt < 65535 ? nt : 65535));
         fill_count<<<cgrid, kClassifyThreads, 0, s>>>(where, nt, (uint32_t)ny, (uint32_t)nx, tiles, counts);
         if ((status = exclusive_scan_u32_to_i64(counts, offsets, ncounts, nullptr, s))) break;
-        fill_class_starts<<<1, 32, 0, s>>>(offsets, nblocks, starts_dev);
-        int64_t starts[kClasses + 1];
+        fill_class_starts<<<1, 32 * kClasses, 0, s>>>(offsets, nblocks, nt, tiles, starts_dev);
+        int64_t starts[2 * kClasses + 1];
         RG_CUDA(cudaMemcpyAsync(starts, starts_dev, sizeof(starts), cudaMemcpyDeviceToHost, s));
         RG_CUDA(cudaStreamSynchronize(s));
         const int64_t total = starts[kClasses];
@@ -883,21 +901,27 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         // resident blocks, whose threads walk longer stretches of the list)
         const GsConst k = gs_constants(ny, nx);
         const FastDiv nx_div((uint32_t)nx);
-        // Few cells per slice: clusters.  A class of n cells takes about 4 us or
-        // n * 6 operations at 0.66 of the chip's FP64 rate (0.63 T/s) as a
-        // launch, and 1 us plus its slice's share at the cluster's rate as a
-        // phase.  Measured, launches and clusters, 100 iterations with the
-        // whole call: one 64 x 64 slice 1.24 and 0.81 ms, three of 101 x 607
-        // 1.93 and 1.14 ms, one of 700 x 700 1.61 and 1.52 ms, one of 768 x 768
-        // (float32) 1.39 and 1.47 ms: the line lies below the last two.
-        int64_t widest = 0;
-        for (int cls = 0; cls < kClasses; ++cls) widest = std::max(widest, starts[cls + 1] - starts[cls]);
-        const int c = nt <= 4096 ? cluster_for(fill_relax<T>, nt, 0) : 1;
+        // Few cells per slice: clusters, of one block per SM at most (16 slices of
+        // 256^2, float32, two blocks per SM: 4.6 us a phase, one: 2.4).  A class
+        // takes at least 3.9 us as a launch, and as a phase 2.3 us (float32 2.7)
+        // and 1.5 us (1.8) per 1000 cells of a block.  Launches and clusters, us,
+        // 100 iterations: one 64 x 64 slice 880 and 510, one of 700 x 700 with 1 %
+        // missing 878 and 635, with 8 % 879 and 962 (float32: 1086), 4 of 480 x 641
+        // with 8 % 1741 and 974; more slices than SMs, of 1 %: 1000 of 100 x 101 2170
+        // and 4000, 5000 of 32 x 32 955 and 14800.
+        int c = nt <= kRelaxSlices ? cluster_for(fill_relax<T>, nt, 0) : 0;
+        while (c > 1 && nt * c > kRelaxSlices) c /= 2;
         const double op_us = 6.0 / (0.66 * 0.63e6);  // of one cell, the whole chip
-        const double launch_us = std::max(3.8, widest * op_us);
-        const double phase_us = 1.0 + (double)widest / nt * op_us * 152 / c * ((nt * c + 151) / 152);
-        if (phase_us < launch_us) {
-            for (int64_t done = 0; done < iterations; done += 1024)  // a launch stays below a few ms
+        double launches_us = 0, phases_us = 0;
+        for (int cls = 0; cls < kClasses && c > 0; ++cls) {
+            const int64_t n = starts[cls + 1] - starts[cls];
+            if (n == 0) continue;
+            const double block = (double)starts[kClasses + 1 + cls] / c / 1000;
+            launches_us += std::max(3.9, n * op_us);
+            phases_us += sizeof(T) == 8 ? 2.3 + 1.5 * block : 2.7 + 1.8 * block;
+        }
+        if (phases_us < launches_us) {
+            for (int64_t done = 0; done < iterations; done += 1024)  // (at most some 25 ms a launch)
                 RG_CUDA(launch_clusters(fill_relax<T>, nt, c, s, a, (const uint64_t*)list, (const int64_t*)offsets, nblocks,
                                         tiles, (uint32_t)ny, nx_div, k,
                                         (int)std::min<int64_t>(1024, iterations - done)));
