@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kClassifyThreads) fill_lists(const uint8_t* __
 // the most entries of one slice in every class, for up to kRelaxSlices slices.
 // A warp per class.
 constexpr int kRelaxSlices = 152;
+constexpr size_t kRelaxShared = 120 * 1024;  // of an SM's 228 KB
 __global__ void __launch_bounds__(32 * kClasses)
     fill_class_starts(const int64_t* __restrict__ offsets, int64_t nblocks, int64_t nt, int64_t tiles,
                       int64_t* __restrict__ out) {
@@ -326,13 +327,14 @@ int cluster_for(F* kernel, int64_t nt, size_t smem) {
 }
 
 template <typename F, typename... Args>
-cudaError_t launch_clusters(F* kernel, int64_t nt, int c, cudaStream_t s, Args... args) {
+cudaError_t launch_clusters(F* kernel, int64_t nt, int c, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim = {(unsigned)c, 1, 1};
     cfg.gridDim = dim3((unsigned)(nt * c));
     cfg.blockDim = dim3(kRelaxThreads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -821,7 +823,7 @@ int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out,
         constexpr int kPasses = Keys<T>::kBits / 8;
         const int c = cluster_for(median_digits, nt, 0);
         if (median_clusters(total, nt, c)) {
-            RG_CUDA(launch_clusters(median_digits, nt, c, s, keys, offsets, Keys<T>::kBits - 8 * (kDataPasses + 1), st));
+            RG_CUDA(launch_clusters(median_digits, nt, c, 0, s, keys, offsets, Keys<T>::kBits - 8 * (kDataPasses + 1), st));
         } else {
             const dim3 kgrid = slice_grid(nt, (total + nt - 1) / nt, 4096);
             for (int pass = kDataPasses; pass < kPasses; ++pass) {
@@ -901,15 +903,18 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         // resident blocks, whose threads walk longer stretches of the list)
         const GsConst k = gs_constants(ny, nx);
         const FastDiv nx_div((uint32_t)nx);
-        // Few cells per slice: clusters, of one block per SM at most (16 slices of
-        // 256^2, float32, two blocks per SM: 4.6 us a phase, one: 2.4).  A class
+        // Few cells per slice: clusters, of one block per SM (which the shared
+        // memory they ask for sees to: 16 slices of 256^2, float32, 1 %, with two
+        // blocks on an SM 4.6 us a phase, with one 2.6).  A class
         // takes at least 3.9 us as a launch, and as a phase 2.3 us (float32 2.7)
         // and 1.5 us (1.8) per 1000 cells of a block.  Launches and clusters, us,
         // 100 iterations: one 64 x 64 slice 880 and 510, one of 700 x 700 with 1 %
         // missing 878 and 635, with 8 % 879 and 962 (float32: 1086), 4 of 480 x 641
         // with 8 % 1741 and 974; more slices than SMs, of 1 %: 1000 of 100 x 101 2170
         // and 4000, 5000 of 32 x 32 955 and 14800.
-        int c = nt <= kRelaxSlices ? cluster_for(fill_relax<T>, nt, 0) : 0;
+        static SharedLimit limit;
+        int c = nt <= kRelaxSlices && allow_shared((const void*)fill_relax<T>, kRelaxShared, limit)
+                    ? cluster_for(fill_relax<T>, nt, kRelaxShared) : 0;
         while (c > 1 && nt * c > kRelaxSlices) c /= 2;
         const double op_us = 6.0 / (0.66 * 0.63e6);  // of one cell, the whole chip
         double launches_us = 0, phases_us = 0;
@@ -922,7 +927,7 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         }
         if (phases_us < launches_us) {
             for (int64_t done = 0; done < iterations; done += 1024)  // (at most some 25 ms a launch)
-                RG_CUDA(launch_clusters(fill_relax<T>, nt, c, s, a, (const uint64_t*)list, (const int64_t*)offsets, nblocks,
+                RG_CUDA(launch_clusters(fill_relax<T>, nt, c, kRelaxShared, s, a, (const uint64_t*)list, (const int64_t*)offsets, nblocks,
                                         tiles, (uint32_t)ny, nx_div, k,
                                         (int)std::min<int64_t>(1024, iterations - done)));
             break;
