@@ -52,8 +52,8 @@ typedef struct CUstream_st* rg_stream_t; /* == cudaStream_t */
  * unevaluated pair of floats (error-free products by FMA, Knuth's two-sum) on
  * the FP32 pipe, the pair added in double at the end.  Result within
  * (1.1e-14 + (n + 2)^2 * 3.6e-15) * sum_k |w_k x_k| of the exact sum for rows
- * of n entries, 1e-12 of sums of one sign for n <= 14.  Longer rows are summed in
- * float64, bit for bit as RG_ACC_EXACT, except where the input footprints of
+ * of n entries (half of that where all w_k x_k have one sign: 1e-12 for n <= 20).
+ * Rows of more than 20 entries are summed in float64, bit for bit as RG_ACC_EXACT, except where the input footprints of
  * 16 x 16 output cells fit boxes of 32 x 32 input cells, whose rows are short
  * (about 9 entries; one of 60 is off by some 5e-14).
  * A float32 partial sum that overflows, or a non-finite input or weight,

@@ -39,6 +39,11 @@ __device__ __forceinline__ int64_t tile_row(const Tile& T, int64_t tile, int tid
 // MODE 1: exact double update rounded to float32 after every entry (numpy's
 //         in-place float32 output)
 // MODE 2: fast, accumulate in the output type with FMA
+// MODE 3: compensated (float32 input, float64 output): rows of up to FF_ROW_MAX
+//         entries by the float-float sums of the patch kernel, two slices at a
+//         time, for footprints too large for its boxes (777 x 611 -> 311 x 244
+//         rotated by 0.45, 8 slices: 91 us as MODE 0, 44 so); longer ones as
+//         MODE 0
 template <typename Tin, typename Tout, int MODE, typename Tw>
 __global__ void __launch_bounds__(APPLY_BLOCK)
     apply_kernel(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
@@ -57,9 +62,49 @@ __global__ void __launch_bounds__(APPLY_BLOCK)
         c[k] = k < nk ? col[s + k] : 0;
         w[k] = k < nk ? val[s + k] : (Tw)0;
     }
+    if constexpr (MODE == 3) {
+        if (nk <= FF_ROW_MAX) {
+            float hi[CACHED], lo[CACHED];
+#pragma unroll
+            for (int k = 0; k < CACHED; k++) {
+                hi[k] = (float)w[k];
+                lo[k] = __double2float_rn(__dsub_rn(w[k], (double)hi[k]));
+            }
+            for (int64_t d = d0; d < d1; d += 2) {
+                const Tin* a = vin + d * n_in;
+                const Tin* b = d + 1 < d1 ? a + n_in : a;
+                uint64_t h2 = 0ull, l2 = 0ull;
+                auto step = [&](int32_t cell, float wh, float wl) {
+                    ff_step2(h2, l2, f2_pack(wh, wh), f2_pack(-wh, -wh), f2_pack(wl, wl),
+                             f2_pack(ldg_cast(a + cell), ldg_cast(b + cell)));
+                };
+#pragma unroll
+                for (int k = 0; k < CACHED; k++)
+                    if (k < nk) step(c[k], hi[k], lo[k]);
+                for (int64_t k = s + CACHED; k < e; k++) {
+                    const float wh = (float)val[k];
+                    step(col[k], wh, __double2float_rn(__dsub_rn(val[k], (double)wh)));
+                }
+                const float2 h = f2_unpack(h2), l = f2_unpack(l2);
+                auto store = [&](int64_t dd, const Tin* x, float hv, float lv) {
+                    double r = 0.0;
+                    if (finite_bits(hv) && finite_bits(lv)) {
+                        r = __dadd_rn(widen(hv), widen(lv));
+                    } else {  // as the patch kernel: this output and slice in float64, stored order
+                        for (int64_t k = s; k < e; k++)
+                            r = __dadd_rn(r, __dmul_rn((double)val[k], (double)ldg_cast(x + col[k])));
+                    }
+                    vout[dd * n_out + o] = (Tout)r;
+                };
+                store(d, a, h.x, l.x);
+                if (d + 1 < d1) store(d + 1, b, h.y, l.y);
+            }
+            return;
+        }
+    }
     for (int64_t d = d0; d < d1; d++) {
         const Tin* a = vin + d * n_in;
-        if (MODE == 0) {
+        if (MODE == 0 || MODE == 3) {
             double acc = 0.0;
 #pragma unroll
             for (int k = 0; k < CACHED; k++)
@@ -133,7 +178,10 @@ int apply_csr(const int64_t* row_ptr, const int32_t* col, const double* val, con
     RG_CHECK(acc == RG_ACC_EXACT || acc == RG_ACC_FAST || acc == RG_ACC_COMPENSATED, RG_ERR_ARG,
              "apply: bad accumulation mode");
     if (stack <= 0 || n_rows <= 0) return RG_OK;
-    if (acc != RG_ACC_FAST) {  // exact, or compensated where the staged kernel does not take the call
+    if (acc == RG_ACC_COMPENSATED && dtype_in == RG_F32 && dtype_out == RG_F64)
+        return launch<float, double, 3, double>(row_ptr, col, val, n_rows, shape0, shape1, vin, n_cols, vout, stack,
+                                                s);
+    if (acc != RG_ACC_FAST) {
         if (dtype_out == RG_F64) {
             if (dtype_in == RG_F32)
                 return launch<float, double, 0, double>(row_ptr, col, val, n_rows, shape0, shape1, vin, n_cols,
@@ -238,7 +286,7 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     // (the patch lists keep a float32 copy of the weights in gather order)
     const bool need32 = ((acc == RG_ACC_FAST && dtype_out == RG_F32) || exact_box || ff_box) && W->nnz > 0;
     int g = 0, load64 = -1;
-    bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false;
+    bool use_box = false, use_rows = false, use_box_exact = false, use_box_ff = false, ff_direct = false;
     rg_weights_state now;
     {
         std::lock_guard<std::mutex> lock(W->mu);
@@ -286,9 +334,10 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
         exact64 = exact64 && load >= 0 && exact_staged(W, load, 8, stack);
         load64 = load;
         if (exact64) RG_TRY(box_perm_for(W, s, &made));
-        // compensated calls whose rows are too long for float-float sums, whose
-        // footprints are too large for any box, without shapes or off a 16-byte
-        // boundary of the swizzled box compute as exact
+        // compensated calls with too many rows too long for float-float sums, those
+        // without shapes and those off a 16-byte boundary of the swizzled box
+        // compute as exact; footprints too large for any box gather
+        ff_direct = ff_box && W->box_state == -1;
         const bool ff_rows = float_pairs(W);
         if ((exact_box || (ff_box && !ff_rows)) && load >= 0 && exact_staged(W, load, 4, stack)) {
             use_box_exact = true;
@@ -343,9 +392,12 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     if (tiled) return apply_tiled(&now, g, (const float*)vin, (float*)vout, stack, s);
     if (!transposed)
         return apply_csr(now.row_ptr, now.col, now.val, now.val32, now.nnz, now.n_out, now.n_in, now.out_shape0,
-                         now.out_shape1, vin, dtype_in, vout, dtype_out, stack, acc, s);
+                         now.out_shape1, vin, dtype_in, vout, dtype_out, stack,
+                         acc == RG_ACC_COMPENSATED && !ff_direct ? RG_ACC_EXACT : acc, s);
+    // (a compensated call is defined for the matrix itself; its transpose computes as exact)
     return apply_csr(now.t_row_ptr, now.t_col, now.t_val, now.t_val32, now.nnz, now.n_in, now.n_out, 0, 0, vin,
-                     dtype_in, vout, dtype_out, stack, acc, s);
+                     dtype_in, vout, dtype_out, stack,
+                     acc == RG_ACC_COMPENSATED ? RG_ACC_EXACT : acc, s);
 }
 
 }  // namespace rg

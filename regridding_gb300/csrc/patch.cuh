@@ -176,15 +176,21 @@ __device__ __forceinline__ double widen_normal(unsigned u) {
 //              in double once per output.  Entries in the gather order.
 constexpr int MODE_FAST = 0, MODE_EXACT = 1, MODE_FF = 2;
 
-// Longest row that MODE_FF sums as float pairs in a wide box: their error,
-// (1.5 2^-47 + (n + 2)^2 2^-48) sum |w x|, is then below 1e-12 of the sum (and
-// is approached where roundings have one sign: n equal terms, n = 250, are off by
-// 1e-12).  Longer rows are summed in float64, in stored order.  (Boxes of 32
-// swizzled columns hold patches whose rows have about 9 entries; their kernel
-// tests nothing.)
-constexpr int FF_ROW_MAX = 14;
+// Longest row that MODE_FF sums as float pairs in a wide box.  With u = 2^-24
+// and sums S of one sign, every product is off by at most 3 u^2 of its term, the
+// rounding of err + r by u^2 (S + 2 of the term), and that of the k-th l by
+// u |l| <= u^2 (k + 2) S: in all u^2 (n^2 / 2 + 3.5 n + 5) S, and 2^-53 S for the
+// last addition, below 1e-12 S for n <= 20.  (Where roundings have one sign the
+// bound is approached: 250 equal terms are off by 1e-12, 4,000 by 2.7e-10.)
+// Longer rows are summed in float64, in stored order.  (Boxes of 32 swizzled
+// columns hold patches whose rows have about 9 entries; their kernel tests
+// nothing.)
+constexpr int FF_ROW_MAX = 20;
 // One in this many rows may be long; with more, the exact kernel takes the call.
-constexpr int FF_LONG_SHARE = 16;
+// (2048^2 -> 819^2 rotated by 0.45, one row in 30 long, 1, 2, 4, 8, 16 slices:
+// 97, 124, 189, 321, 587 us with the long rows here, 76 (gathered), 111, 178, 309,
+// 568 exact; without long rows 52, 56, 72, 103, 168.)
+constexpr int FF_LONG_SHARE = 64;
 
 // Packed pairs of float32 (two slices of one output): the sm_100-family
 // f32x2 instructions apply one IEEE operation, rounded to nearest, to both
