@@ -1686,9 +1686,8 @@ constexpr int ROW_SMALL = 1024;      // a row's ranks cost its square
 constexpr int BLOCK_TRIPLES = 2048;  // 40 KB of shared memory
 constexpr int32_t ROW_HEAD = INT32_MIN;
 
-// The rows' merged counts to the block's prefix (pre[ORDER_ROWS] their total)
-// and to row_nnz; by one warp.
-__device__ __forceinline__ void order_counts(int64_t r0, int64_t r1, int mine, int* pre, int64_t* row_nnz) {
+// Rows' merged counts to their prefix (pre[ORDER_ROWS] the total); by one warp.
+__device__ __forceinline__ void order_counts(int mine, int* pre) {
     const int lane = threadIdx.x & 31;
     int incl = mine;
 #pragma unroll
@@ -1698,14 +1697,13 @@ __device__ __forceinline__ void order_counts(int64_t r0, int64_t r1, int mine, i
     }
     pre[lane + 1] = incl;
     if (lane == 0) pre[0] = 0;
-    if (r0 + lane < r1) row_nnz[r0 + lane] = mine;
 }
 
 template <int PER>
 __global__ void __launch_bounds__(ORDER_THREADS)
     order_rows(const int64_t* __restrict__ row_start, int64_t nrows, const Triple* __restrict__ triples,
                int32_t* __restrict__ tmp_col, double* __restrict__ tmp_val, int64_t* __restrict__ row_nnz,
-               int32_t* __restrict__ long_list, unsigned* __restrict__ long_count) {
+               int2* __restrict__ long_list, unsigned* __restrict__ long_count) {
     __shared__ int64_t key[BLOCK_TRIPLES];
     __shared__ double val[BLOCK_TRIPLES];
     __shared__ int32_t in[BLOCK_TRIPLES];
@@ -1722,7 +1720,7 @@ __global__ void __launch_bounds__(ORDER_THREADS)
         start[t] = (int)(s - s0);
     }
     if (__syncthreads_or(longer)) {
-        if (t == 0) long_list[atomicAdd(long_count, 1u)] = (int32_t)blockIdx.x;
+        if (t == 0) long_list[atomicAdd(long_count, 1u)] = make_int2((int)blockIdx.x, 0);
         return;
     }
     const int n = start[PER];
@@ -1780,85 +1778,172 @@ __global__ void __launch_bounds__(ORDER_THREADS)
     }
 }
 
-// The listed blocks: every row ranked by the whole block, keys staged in shared-memory tiles, up to 8 triples per thread
-// and pass; then merged by a lane each, and moved together.
+// A row of up to ROW_SHORT triples ranked and merged by a warp, through its
+// triples' place; returns its merged entries.
+constexpr int ROW_SHORT = 256;
+__device__ int order_short_row(int64_t s, int len, Triple* triples, int32_t* tmp_col, double* tmp_val) {
+    const int lane = threadIdx.x & 31;
+    constexpr int OWN = ROW_SHORT / 32;
+    int64_t key[OWN];
+    int rank[OWN];
+#pragma unroll
+    for (int k = 0; k < OWN; k++) {
+        key[k] = lane + 32 * k < len ? triples[s + lane + 32 * k].key : INT64_MAX;
+        rank[k] = 0;
+    }
+    for (int j = 0; j < len; j++) {
+        const int64_t other = triples[s + j].key;
+#pragma unroll
+        for (int k = 0; k < OWN; k++) rank[k] += other < key[k];
+    }
+#pragma unroll
+    for (int k = 0; k < OWN; k++)
+        if (lane + 32 * k < len) {
+            tmp_col[s + rank[k]] = (int32_t)(key[k] >> 32);
+            tmp_val[s + rank[k]] = triples[s + lane + 32 * k].w;
+        }
+    __syncwarp();
+    int runs = 0;
+    for (int e0 = 0; e0 < len; e0 += 32) {
+        const int e = e0 + lane;
+        const int32_t c = e < len ? tmp_col[s + e] : 0;
+        const bool head = e < len && (e == 0 || tmp_col[s + e - 1] != c);
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        if (head) {
+            int h = e + 1;
+            while (h < len && tmp_col[s + h] == c) h++;
+            triples[s + runs + __popc(heads & ((1u << lane) - 1u))] =
+                Triple{c, run_sum([&](int64_t k) { return tmp_val[k]; }, s + e, s + h)};
+        }
+        runs += __popc(heads);
+    }
+    __syncwarp();
+    for (int k = lane; k < runs; k += 32) {
+        tmp_col[s + k] = (int32_t)triples[s + k].key;
+        tmp_val[s + k] = triples[s + k].w;
+    }
+    return runs;
+}
+
+// The listed blocks (.x; .y counts their finished turns), a row per block and
+// turn, its short rows together in one, a warp each: ranked with the keys staged in shared-memory tiles, up to 8 triples per
+// thread and pass, and merged by a thread per run; the block that finishes a
+// listed block's last row moves its rows together.  (63 pairs of 64^2 and one of
+// 512^2 -> 8^2 in a batch, whose 64 rows of 36,000 triples lie in two blocks of
+// 32: 14 ms; with a block for all rows of a listed one 270.  512^2 -> 8^2
+// alone 11 and 21 ms.)
 constexpr int ROW_TILE = 2048;
-__global__ void __launch_bounds__(256)
-    order_rows_long(const int64_t* __restrict__ row_start, int64_t nrows, int per, const int32_t* __restrict__ long_list,
-                    const unsigned* __restrict__ long_count, const Triple* __restrict__ triples,
-                    int32_t* tmp_col, double* tmp_val, int64_t* __restrict__ row_nnz) {
+__global__ void __launch_bounds__(ORDER_THREADS)
+    order_rows_long(const int64_t* __restrict__ row_start, int64_t nrows, int per, int2* __restrict__ long_list,
+                    const unsigned* __restrict__ long_count, Triple* triples, int32_t* tmp_col, double* tmp_val,
+                    int64_t* row_nnz) {
     __shared__ int64_t tile[ROW_TILE];
-    __shared__ int pre[ORDER_ROWS + 1];
-    const unsigned nl = *long_count;
-    for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
-        const int64_t r0 = (int64_t)long_list[li] * per, s0 = row_start[r0];
+    __shared__ int pre[ORDER_ROWS + 1], warp_heads[ORDER_THREADS / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // (rows first: turns of few rows, at the end, leave no SM with more of the long ones)
+    const int64_t rows = (int64_t)*long_count * per, items = rows + *long_count;
+    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const bool together = item >= rows;
+        int2* listed = long_list + (together ? item - rows : item / per);
+        const int64_t r0 = (int64_t)listed->x * per, s0 = row_start[r0];
         const int64_t r1 = r0 + per < nrows ? r0 + per : nrows;
-        for (int64_t r = r0; r < r1; r++) {
-            const int64_t s = row_start[r], t = row_start[r + 1], len = t - s;
-            for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
-                int64_t mykey[8];
-                int64_t rank[8];
+        const int64_t r = together ? r0 : r0 + item % per;
+        // the listed block's turns: its long rows, and the short ones together
+        const unsigned longer = __ballot_sync(0xffffffffu, r0 + lane < r1 && row_start[r0 + lane + 1] - row_start[r0 + lane] > ROW_SHORT);
+        if (!together && (r >= r1 || !(longer >> (r - r0) & 1u))) continue;
+        if (together)
+            for (int q = warp; r0 + q < r1; q += ORDER_THREADS / 32)
+                if (!(longer >> q & 1u))
+                    row_nnz[r0 + q] = order_short_row(row_start[r0 + q], (int)(row_start[r0 + q + 1] - row_start[r0 + q]),
+                                                      triples, tmp_col, tmp_val);
+        const int64_t s = together ? 0 : row_start[r], t = together ? 0 : row_start[r + 1], len = t - s;
+        for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
+            int64_t mykey[8];
+            int64_t rank[8];
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
-                    mykey[k] = e < t ? triples[e].key : INT64_MAX;
-                    rank[k] = 0;
-                }
-                for (int64_t q0 = 0; q0 < len; q0 += ROW_TILE) {
-                    const int64_t m = len - q0 < ROW_TILE ? len - q0 : ROW_TILE;
-                    __syncthreads();
-                    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
-                    __syncthreads();
-                    // (eight keys for each read of the tile, or the one of a short row)
-                    if (t - e0 > blockDim.x) {
-                        for (int64_t q = 0; q < m; q++) {
-                            const int64_t kq = tile[q];
+            for (int k = 0; k < 8; k++) {
+                const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
+                mykey[k] = e < t ? triples[e].key : INT64_MAX;
+                rank[k] = 0;
+            }
+            for (int64_t q0 = 0; q0 < len; q0 += ROW_TILE) {
+                const int64_t m = len - q0 < ROW_TILE ? len - q0 : ROW_TILE;
+                __syncthreads();
+                for (int64_t q = threadIdx.x; q < m; q += blockDim.x) tile[q] = triples[s + q0 + q].key;
+                __syncthreads();
+                // (eight keys for each read of the tile, or the one of a short row)
+                if (t - e0 > blockDim.x) {
+                    for (int64_t q = 0; q < m; q++) {
+                        const int64_t kq = tile[q];
 #pragma unroll
-                            for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
-                        }
-                    } else {
-                        int below = 0;
+                        for (int k = 0; k < 8; k++) rank[k] += kq < mykey[k];
+                    }
+                } else {
+                    int below = 0;
 #pragma unroll 4
-                        for (int q = 0; q < (int)m; q++) below += tile[q] < mykey[0];
-                        rank[0] += below;
-                    }
+                    for (int q = 0; q < (int)m; q++) below += tile[q] < mykey[0];
+                    rank[0] += below;
                 }
+            }
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
-                    if (e < t) {
-                        tmp_col[s + rank[k]] = (int32_t)(mykey[k] >> 32);
-                        tmp_val[s + rank[k]] = triples[e].w;
-                    }
+            for (int k = 0; k < 8; k++) {
+                const int64_t e = e0 + threadIdx.x + (int64_t)k * blockDim.x;
+                if (e < t) {
+                    tmp_col[s + rank[k]] = (int32_t)(mykey[k] >> 32);
+                    tmp_val[s + rank[k]] = triples[e].w;
                 }
             }
         }
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            const int64_t r = r0 + threadIdx.x;
-            int64_t n = 0;
-            if (r < r1) {
-                const int64_t s = row_start[r];
-                n = merge_sorted(
-                        s, row_start[r + 1], [&](int64_t k) { return tmp_col[k]; },
-                        [&](int64_t k) { return tmp_val[k]; },
-                        [&](int64_t k, int32_t c, double v) {
-                            tmp_col[k] = c;
-                            tmp_val[k] = v;
-                        }) -
-                    s;
+        // a thread adds up each run; the merged row goes through its triples' place
+        int runs = 0;
+        for (int64_t e0 = s; e0 < t; e0 += blockDim.x) {
+            __syncthreads();
+            const int64_t e = e0 + threadIdx.x;
+            const int32_t c = e < t ? tmp_col[e] : 0;
+            const bool head = e < t && (e == s || tmp_col[e - 1] != c);
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            if ((threadIdx.x & 31) == 0) warp_heads[threadIdx.x >> 5] = __popc(heads);
+            __syncthreads();
+            int at = runs + __popc(heads & ((1u << (threadIdx.x & 31)) - 1u));
+            for (int w = 0; w < ORDER_THREADS / 32; w++) {
+                at += w < (threadIdx.x >> 5) ? warp_heads[w] : 0;
+                runs += warp_heads[w];
             }
-            order_counts(r0, r1, (int)n, pre, row_nnz);
+            if (head) {
+                int64_t h = e + 1;
+                while (h < t && tmp_col[h] == c) h++;
+                triples[s + at] = Triple{c, run_sum([&](int64_t k) { return tmp_val[k]; }, e, h)};
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < runs; k += blockDim.x) {
+            tmp_col[s + k] = (int32_t)triples[s + k].key;
+            tmp_val[s + k] = triples[s + k].w;
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (!together) row_nnz[r] = runs;
+            __threadfence();
+            last = atomicAdd(&listed->y, 1) == __popc(longer);
+            __threadfence();
+        }
+        __syncthreads();
+        if (!last) continue;
+        if (threadIdx.x < 32) {
+            const int64_t row = r0 + threadIdx.x;
+            order_counts(row < r1 ? (int)__ldcg(row_nnz + row) : 0, pre);
         }
         __syncthreads();
         // (entries move towards the front: a pass reads before any of it writes)
-        for (int r = 0; r0 + r < r1; r++) {
-            const int64_t src = row_start[r0 + r] - pre[r];
-            for (int e0 = pre[r]; e0 < pre[r + 1]; e0 += blockDim.x) {
+        for (int q = 0; r0 + q < r1; q++) {
+            const int64_t src = row_start[r0 + q] - pre[q];
+            for (int e0 = pre[q]; e0 < pre[q + 1]; e0 += blockDim.x) {
                 const int e = e0 + threadIdx.x;
-                const bool have = e < pre[r + 1];
-                const int32_t c = have ? tmp_col[src + e] : 0;
-                const double v = have ? tmp_val[src + e] : 0.0;
+                const bool have = e < pre[q + 1];
+                const int32_t c = have ? __ldcg(tmp_col + src + e) : 0;
+                const double v = have ? __ldcg(tmp_val + src + e) : 0.0;
                 __syncthreads();
                 if (have) {
                     tmp_col[s0 + e] = c;
@@ -1867,6 +1952,7 @@ __global__ void __launch_bounds__(256)
                 __syncthreads();
             }
         }
+        __syncthreads();
     }
 }
 
@@ -2235,7 +2321,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
             const int64_t nr = rows->n_rows;
             unsigned *rowc = nullptr, *long_count = nullptr;  // (one allocation)
             Triple* triples = nullptr;
-            int32_t* long_list = nullptr;
+            int2* long_list = nullptr;
             do {
                 if ((st = dalloc(&rows->row_start, (size_t)nr + 1, s))) break;
                 if ((st = dalloc(&rows->row_nnz, (size_t)nr + 1, s))) break;
@@ -2265,7 +2351,7 @@ int sweep_chunked(Batch& B, const std::vector<SweepParams>& P, const std::vector
                 const auto order = rows->per == 32 ? order_rows<32> : rows->per == 8 ? order_rows<8> : order_rows<2>;
                 order<<<blocks, ORDER_THREADS, 0, s>>>(rows->row_start, nr, triples, rows->col, rows->val,
                                                        rows->row_nnz, long_list, long_count);
-                order_rows_long<<<std::min(blocks, 152u * 8u), 256, 0, s>>>(rows->row_start, nr, rows->per, long_list,
+                order_rows_long<<<std::min(grid_for(2 * nr, 1), 152u * 8u), ORDER_THREADS, 0, s>>>(rows->row_start, nr, rows->per, long_list,
                                                                             long_count, triples, rows->col, rows->val,
                                                                             rows->row_nnz);
             } while (0);

@@ -57,3 +57,40 @@ def test_weights_at_any_scale(scale):
     want = oracle.weights_conservative_2d(gi, go)
     got = rg.build_conservative_2d(gi, go).export_numpy()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_long_rows_side_by_side():
+    """A coarse pair whose 64 rows have some 36,000 triples each takes about as
+    long beside 63 fine pairs, where they lie in two blocks of 32 rows, as
+    alone, where each pair of rows has a block (in series they took ten times
+    as long)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import time
+
+    from regridding_gb300 import batching, workloads
+
+    def device(grid):
+        return tuple(torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in grid)
+
+    gi = np.stack(np.meshgrid(np.linspace(0, 1, 513), np.linspace(0, 1, 513), indexing="ij"))
+    go = np.stack(np.meshgrid(np.linspace(0.013, 0.977, 9), np.linspace(0.013, 0.977, 9), indexing="ij"))
+    coarse = device(gi + 1e-4 * np.sin(40 * gi[::-1])), device(go + 1e-7 * np.sin(9 * go[::-1]))
+    rng = np.random.default_rng(2)
+    fine = [tuple(device(g) for g in workloads.grid_pair(rng, 64)) for _ in range(63)]
+    seconds = []
+    for pairs in ([coarse], fine + [coarse]):
+        times = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            built = batching.build_batch(pairs)
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t0)
+            last = built[-1].export_numpy()
+            for dw in built:
+                dw.free()
+        seconds.append((min(times), last))
+    assert all(np.array_equal(a, b) for a, b in zip(seconds[0][1], seconds[1][1]))
+    assert seconds[1][0] < 3 * seconds[0][0], [t for t, _ in seconds]
