@@ -55,6 +55,33 @@ def test_undersized_chunk_slots_take_the_recovery_path(rg, monkeypatch):
             assert_same(g, e)
 
 
+def test_graded_grids_keep_to_their_chunks(rg):
+    """Lines that lie ten times as far apart at the rim as in the middle fit
+    the chunks' slots: a build takes about twice that of even lines (by whole
+    lines, after an overflow, twelve times)."""
+    import time
+
+    import torch
+
+    from regridding_gb300 import workloads
+
+    x, y = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in workloads.distorted_grid(513, 0.1, 0.02))
+    even = workloads.perturb(workloads.rect_grid(385, -0.95, 0.95))
+    seconds = []
+    for power in (1, 2):
+        go = [torch.from_numpy(np.sign(a) * np.abs(a) ** power).cuda() for a in even]
+        times = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            dw = rg.build_conservative_2d((x, y), go)
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t0)
+            dw.free()
+        seconds.append(min(times))
+    assert seconds[1] < 5 * seconds[0], seconds
+
+
 def test_cycling_walks_end_soon(rg, monkeypatch):
     """A pair whose walk cycles around a shared vertex is reported about as
     soon as its whole lines are walked: the line's further chunks are not
