@@ -141,6 +141,8 @@ struct Row1d {
     const double *in, *out;
     int64_t m, n;
     bool rev_in, rev_out;
+    __device__ __forceinline__ Row1d(const double* a, const double* b, int64_t m, int64_t n)
+        : in(a), out(b), m(m), n(n), rev_in(!(a[0] < a[m - 1])), rev_out(!(b[0] < b[n - 1])) {}
     __device__ __forceinline__ double xs(int64_t k) const { return __ldg(in + (rev_in ? m - 1 - k : k)); }
     __device__ __forceinline__ double xt(int64_t k) const { return __ldg(out + (rev_out ? n - 1 - k : k)); }
     // weight of the piece p1..p2 of sweep cell isw, with the length of the
@@ -175,88 +177,100 @@ __device__ __forceinline__ int64_t first_above(const At& at, int64_t n, double v
     return lo;
 }
 
-// The sweep of one row by one thread, for grids that do not rise strictly: its
-// entries in sweep order, then in the saved order.  Every entry moves on in
-// the sweep grid or the static one and none moves back, so pairs are unique,
-// entries of one input are neighbours, and the saved order (by input, then
-// output) is the sweep's, reversed as a whole (reversed input) and within the
-// inputs (one of the grids reversed).
+// The sweep of one row, entry by entry.
+struct Sweep1d {
+    int64_t isw = 0, ist = MAXSIZE;
+    double p1;
+    bool outside = true, ended = false;
+
+    __device__ __forceinline__ Sweep1d(const Row1d& R) : p1(R.xs(0)) {
+        const double left = R.xt(0), right = R.xt(R.n - 1);
+        if (left == p1) {
+            outside = false;
+            ist = 0;
+        } else if (left < p1 && p1 < right) {
+            outside = false;
+            int64_t l = 0, r = R.n;
+            while (r - l > 1) {
+                const int64_t mid = (l + r) / 2;
+                if (R.xt(mid) > p1) r = mid;
+                else l = mid;
+            }
+            ist = r - 1;
+        }
+    }
+    __device__ __forceinline__ bool live(const Row1d& R) const { return !ended && isw < R.m - 1; }
+    // One step; true when it made an entry, of cells sw and st from `from` to `to`.
+    __device__ __forceinline__ bool step(const Row1d& R, int64_t* sw, int64_t* st, double* from, double* to) {
+        double p2 = R.xs(isw + 1);
+        *sw = isw;
+        *st = ist;
+        *from = p1;
+        const bool entry = !outside;
+        const double ps = R.xt(outside ? 0 : ist + 1);
+        if (p1 < ps && ps < p2) {
+            ist = outside ? 0 : ist + 1;
+            p2 = ps;
+        } else {
+            if (ps == p2) ist = outside ? 0 : ist + 1;
+            isw = isw + 1;
+        }
+        if (entry) ended = !(0 <= ist && ist < R.n - 1);
+        else outside = !(ist < MAXSIZE);
+        *to = p1 = p2;
+        return entry;
+    }
+};
+
+// The entries of one row by one thread, in the saved order.  Every entry moves
+// on in the sweep grid or the static one and none moves back, so pairs are
+// unique, entries of one input are neighbours, and the saved order (by input,
+// then output) is the sweep's, reversed as a whole (reversed input: a sweep
+// ahead counts the entries) and within the inputs (one of the grids reversed:
+// each input's entries are turned round once they are written).
 __device__ int64_t sweep_1d(const Row1d& R, const double* w_in, int64_t cap, int64_t* ind_in, int64_t* ind_out,
                             double* val, unsigned* flags) {
-    int64_t isw = 0, ist = MAXSIZE, cnt = 0;
-    double p1 = R.xs(0);
-    const double st_left = R.xt(0), st_right = R.xt(R.n - 1);
-    bool outside = true;
-    if (st_left == p1) {
-        outside = false;
-        ist = 0;
-    } else if (st_left < p1 && p1 < st_right) {
-        outside = false;
-        int64_t l = 0, r = R.n;
-        while (r - l > 1) {
-            const int64_t mid = (l + r) / 2;
-            if (R.xt(mid) > p1) r = mid;
-            else l = mid;
+    int64_t sw, st, total = 0, cnt = 0;
+    double from, to;
+    if (R.rev_in)
+        for (Sweep1d ahead(R); ahead.live(R);) total += ahead.step(R, &sw, &st, &from, &to);
+    const auto place = [&](int64_t k) { return R.rev_in ? total - 1 - k : k; };
+    const bool turn = R.rev_in != R.rev_out;
+    int64_t own = -1, first = 0;  // the current input and its first entry
+    const auto turn_round = [&]() {
+        int64_t a = place(first), b = place(cnt - 1);
+        if (a > b) {
+            const int64_t t = a;
+            a = b;
+            b = t;
         }
-        ist = r - 1;
-    }
-    while (isw < R.m - 1) {
-        double p2 = R.xs(isw + 1);
-        if (outside) {
-            const double ps = R.xt(0);
-            if (p1 < ps && ps < p2) {
-                ist = 0;
-                p2 = ps;
-            } else if (ps == p2) {
-                isw = isw + 1;
-                ist = 0;
-            } else {
-                isw = isw + 1;
-            }
-            if (ist < MAXSIZE) outside = false;
-        } else {
-            const int64_t at_sw = isw, at_st = ist;
-            const double ps = R.xt(ist + 1);
-            if (p1 < ps && ps < p2) {
-                ist = ist + 1;
-                p2 = ps;
-            } else if (ps == p2) {
-                ist = ist + 1;
-                isw = isw + 1;
-            } else {
-                isw = isw + 1;
-            }
-            if (cnt >= cap) {
-                atomicOr(flags, FLAG_CAPACITY);
-                break;
-            }
-            ind_in[cnt] = R.rev_in ? ~at_sw : at_sw;
-            ind_out[cnt] = R.rev_out ? ~at_st : at_st;
-            val[cnt] = R.weight(p1, p2, at_sw, w_in);
-            cnt++;
-            if (!(0 <= ist && ist < R.n - 1)) break;
-        }
-        p1 = p2;
-    }
-    auto reverse = [&](int64_t a, int64_t b) {
-        for (b--; a < b; a++, b--) {
-            const int64_t i = ind_in[a], o = ind_out[a];
+        for (; a < b; a++, b--) {
+            const int64_t o = ind_out[a];
             const double v = val[a];
-            ind_in[a] = ind_in[b];
             ind_out[a] = ind_out[b];
             val[a] = val[b];
-            ind_in[b] = i;
             ind_out[b] = o;
             val[b] = v;
         }
     };
-    if (R.rev_in) reverse(0, cnt);
-    if (R.rev_in != R.rev_out)
-        for (int64_t a = 0, b; a < cnt; a = b) {
-            for (b = a + 1; b < cnt && ind_in[b] == ind_in[a]; b++) {
-            }
-            reverse(a, b);
+    for (Sweep1d sweep(R); sweep.live(R);) {
+        if (!sweep.step(R, &sw, &st, &from, &to)) continue;
+        if (turn && sw != own) {
+            if (cnt - first > 1) turn_round();
+            own = sw;
+            first = cnt;
         }
+        const int64_t at = place(cnt);
+        if (at >= cap) {
+            atomicOr(flags, FLAG_CAPACITY);
+            return 0;
+        }
+        ind_in[at] = R.rev_in ? ~sw : sw;
+        ind_out[at] = R.rev_out ? ~st : st;
+        val[at] = R.weight(from, to, sw, w_in);
+        cnt++;
+    }
+    if (turn && cnt - first > 1) turn_round();
     return cnt;
 }
 
@@ -269,6 +283,10 @@ __device__ int64_t sweep_1d(const Row1d& R, const double* w_in, int64_t cap, int
 // where they are saved, with no sort.  The former thread per row, sort by
 // buckets and thread per row for the merge spent 2.1 ms on 256 rows of 513 and
 // 385 vertices (chains of a few hundred dependent steps); this takes 52 us.
+// The first `few` rows that do not rise strictly are swept by the block's
+// first thread, beside the other blocks; further ones are listed for
+// conservative_1d_sweeps.  (10,000 such rows of 513 and 385 vertices one thread
+// a block: 16 ms, now 1.7.)
 constexpr int CONS_THREADS = 256;
 
 __global__ void __launch_bounds__(CONS_THREADS)
@@ -276,15 +294,13 @@ __global__ void __launch_bounds__(CONS_THREADS)
                          int64_t out_stride, int64_t n, int64_t nd, const double* __restrict__ w_in, int64_t w_stride,
                          int64_t cap, int64_t* __restrict__ ind_in, int64_t* __restrict__ ind_out,
                          double* __restrict__ val, int64_t* __restrict__ count, int* __restrict__ rank_all,
-                         unsigned* flags) {
+                         unsigned* flags, int32_t* __restrict__ list, unsigned* __restrict__ n_list, unsigned few) {
     extern __shared__ int rank_shared[];
     __shared__ int warp_sum[CONS_THREADS / 32];
     __shared__ int running;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int64_t d = blockIdx.x; d < nd; d += gridDim.x) {
-        Row1d R{xin + d * in_stride, xout + d * out_stride, m, n, false, false};
-        R.rev_in = !(R.xs(0) < R.xs(m - 1));
-        R.rev_out = !(R.xt(0) < R.xt(n - 1));
+        const Row1d R(xin + d * in_stride, xout + d * out_stride, m, n);
         const double* w_row = w_in ? w_in + d * w_stride : nullptr;
         int64_t* o_in = ind_in + d * cap;
         int64_t* o_out = ind_out + d * cap;
@@ -293,7 +309,11 @@ __global__ void __launch_bounds__(CONS_THREADS)
         for (int64_t k = t; k + 1 < m; k += CONS_THREADS) rises = rises && R.xs(k) < R.xs(k + 1);
         for (int64_t k = t; k + 1 < n; k += CONS_THREADS) rises = rises && R.xt(k) < R.xt(k + 1);
         if (!__syncthreads_and(rises)) {
-            if (t == 0) count[d] = sweep_1d(R, w_row, cap, o_in, o_out, o_val, flags);
+            if (t == 0) {
+                const unsigned at = atomicAdd(n_list, 1u);
+                if (at < few) count[d] = sweep_1d(R, w_row, cap, o_in, o_out, o_val, flags);
+                else list[at - few] = (int32_t)d;
+            }
             continue;
         }
         const auto xs = [&](int64_t k) { return R.xs(k); };
@@ -370,6 +390,22 @@ __global__ void __launch_bounds__(CONS_THREADS)
             o_val[at] = R.weight(p1, p2, j, w_row);
         }
         __syncthreads();
+    }
+}
+
+// A thread per row: the listed ones (list null: all nd).
+__global__ void __launch_bounds__(128)
+    conservative_1d_sweeps(const double* __restrict__ xin, int64_t in_stride, int64_t m, const double* __restrict__ xout,
+                           int64_t out_stride, int64_t n, int64_t nd, const double* __restrict__ w_in, int64_t w_stride,
+                           int64_t cap, int64_t* __restrict__ ind_in, int64_t* __restrict__ ind_out,
+                           double* __restrict__ val, int64_t* __restrict__ count, unsigned* flags,
+                           const int32_t* __restrict__ list, int64_t n_list) {
+    const int64_t total = list ? n_list : nd;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t d = list ? list[q] : q;
+        const Row1d R(xin + d * in_stride, xout + d * out_stride, m, n);
+        count[d] = sweep_1d(R, w_in ? w_in + d * w_stride : nullptr, cap, ind_in + d * cap, ind_out + d * cap,
+                            val + d * cap, flags);
     }
 }
 
@@ -487,6 +523,16 @@ int multilinear_1d(const double* xin, int64_t in_stride, int64_t m, const double
     return st;
 }
 
+// Whether a thread takes each row (else a block).  A block takes about 20 ns
+// and 0.17 ns a vertex of a row, the chip over; a thread 3.3 us a vertex at most,
+// for as many rows as run at a time.  Blocks and threads, us: rows of 64 and 48
+// vertices, 3,000: 134 and 150, 6,000: 250 and 150, 100,000: 3650 and 550 (one of
+// the grids reversed: 610); of 17 and 9, 4,000: 130 and 57; of 513 and 385, 10,000:
+// 1610 and 1120, 20,000: 3180 and 1580 (reversed 2770).
+static bool rows_by_threads(int64_t nd, int64_t m, int64_t n) {
+    return nd * (20 + 0.17 * (m + n)) > 3300.0 * (m + n);
+}
+
 int conservative_1d(const double* xin, int64_t in_stride, int64_t m, const double* xout,
                     int64_t out_stride, int64_t n, int64_t nd, const double* w_in, int64_t w_stride,
                     int64_t cap, int64_t* ind_in, int64_t* ind_out, double* val, int64_t* count,
@@ -495,28 +541,46 @@ int conservative_1d(const double* xin, int64_t in_stride, int64_t m, const doubl
     if (nd <= 0) return RG_OK;
     RG_CHECK(nd * (m - 1) < INT32_MAX && nd * cap < UINT32_MAX, RG_ERR_UNSUPPORTED,
              "conservative 1D: batch too large");
-    unsigned* flags = nullptr;
+    const bool threads = rows_by_threads(nd, m, n);
+    // uneven rows swept in place: all, where every block has one row at most
+    const unsigned blocks = (unsigned)std::min<int64_t>(nd, 152 * 8), few = nd <= blocks ? blocks : 32;
+    unsigned* flags = nullptr;  // conditions met, the uneven rows' count, and the list of those past `few`
     int* rank = nullptr;
+    int32_t* list = nullptr;
     int st = RG_OK;
     do {
-        if ((st = dalloc(&flags, 1, s))) break;
-        if ((st = zero_async(flags, sizeof(unsigned), s))) break;
-        // the ranks of a row's static vertices: shared memory up to 8191 of them
-        const unsigned blocks = (unsigned)std::min<int64_t>(nd, 152 * 8);
-        const size_t shared = n < 8192 ? (size_t)(n + 1) * sizeof(int) : 0;
-        if (shared == 0 && (st = dalloc(&rank, (size_t)blocks * (n + 1), s))) break;
-        conservative_1d_rows<<<blocks, CONS_THREADS, shared, s>>>(xin, in_stride, m, xout, out_stride, n, nd, w_in,
-                                                                  w_stride, cap, ind_in, ind_out, val, count, rank,
-                                                                  flags);
-        unsigned fl = 0;
-        small_to_host(&fl, flags, sizeof(unsigned), s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
+        if ((st = dalloc(&flags, 2 + (threads ? 0 : (size_t)(nd - std::min<int64_t>(nd, few))), s))) break;
+        if ((st = zero_async(flags, 2 * sizeof(unsigned), s))) break;
+        const auto sweeps = [&](int64_t rows) {
+            conservative_1d_sweeps<<<std::min(grid_for(rows, 128), 152u * 16u), 128, 0, s>>>(
+                xin, in_stride, m, xout, out_stride, n, nd, w_in, w_stride, cap, ind_in, ind_out, val, count, flags, list, rows);
+        };
+        unsigned fl[2] = {0, 0};
+        const auto read = [&]() {
+            small_to_host(fl, flags, sizeof(fl), s);
+            const cudaError_t e = cudaStreamSynchronize(s);
+            if (e == cudaSuccess) return (int)RG_OK;
             set_error("conservative 1D: %s", cudaGetErrorString(e));
-            st = RG_ERR_CUDA;
-            break;
+            return (int)RG_ERR_CUDA;
+        };
+        if (threads) {
+            sweeps(nd);
+            if ((st = read())) break;
+        } else {
+            list = (int32_t*)(flags + 2);
+            // the ranks of a row's static vertices: shared memory up to 8191 of them
+            const size_t shared = n < 8192 ? (size_t)(n + 1) * sizeof(int) : 0;
+            if (shared == 0 && (st = dalloc(&rank, (size_t)blocks * (n + 1), s))) break;
+            conservative_1d_rows<<<blocks, CONS_THREADS, shared, s>>>(xin, in_stride, m, xout, out_stride, n, nd, w_in,
+                                                                      w_stride, cap, ind_in, ind_out, val, count, rank,
+                                                                      flags, list, flags + 1, few);
+            if ((st = read())) break;
+            if (fl[1] > few) {
+                sweeps(fl[1] - few);
+                if ((st = read())) break;
+            }
         }
-        if (fl & FLAG_CAPACITY) {
+        if (fl[0] & FLAG_CAPACITY) {
             set_error("conservative 1D: per-row capacity %lld exceeded", (long long)cap);
             st = RG_ERR_ARG;
         }

@@ -92,3 +92,56 @@ def test_rows_equal_elements(method, lead, axis, dtype):
         w32 = np.zeros(want.shape, dtype="float32")
         rg.regrid_from_weights(*one, vd, values_output=w32, axis_input=-1, axis_output=-1)
         np.testing.assert_array_equal(into[..., d, :] if axis == -1 else into[..., d], w32)
+
+
+@pytest.mark.parametrize("flip", ["", "x", "y", "xy"])
+def test_many_rows_equal_few(flip):
+    """30,000 short rows at a time, every third with a repeated or falling
+    step, and a hundred of them alone: the same bits."""
+    import regridding_gb300 as rg
+
+    rng = np.random.default_rng(11)
+    x = np.sort(rng.uniform(0, 1, (30_000, 34)), axis=1)
+    y = np.sort(rng.uniform(-0.1, 1.1, (30_000, 27)), axis=1)
+    x[::3, 7] = x[::3, 6]
+    y[1::9, 5] = y[1::9, 4]
+    x[2::27, 9] = x[2::27, 5]
+    x = x[:, ::-1] if "x" in flip else x
+    y = y[:, ::-1] if "y" in flip else y
+    many, *_ = rg.weights((x,), (y,), axis_input=-1, axis_output=-1, method="conservative")
+    for k in (0, 1, 2, 15_000, 29_900):
+        few, *_ = rg.weights((x[k:k + 100],), (y[k:k + 100],), axis_input=-1, axis_output=-1, method="conservative")
+        for a, b in zip(few, many[k:k + 100]):
+            for p, q in zip(a, b):
+                np.testing.assert_array_equal(p, q)
+
+
+def test_uneven_rows_take_no_longer():
+    """10,000 rows with a repeated vertex take about as long as without (a
+    block for each row's one sweeping thread made them ten times slower)."""
+    import time
+
+    import torch
+
+    from regridding_gb300 import _device, _lib
+
+    nd, m, n = 10_000, 513, 385
+    cap = m + n + 2
+    y = torch.linspace(-0.05, 1.05, n, dtype=torch.float64, device="cuda").repeat(nd, 1)
+    x = torch.sort(torch.rand(nd, m, dtype=torch.float64, device="cuda"), dim=1).values
+    ii, oo = (torch.empty(nd, cap, dtype=torch.int64, device="cuda") for _ in range(2))
+    vv, count = torch.empty(nd, cap, dtype=torch.float64, device="cuda"), torch.empty(nd, dtype=torch.int64, device="cuda")
+    seconds = []
+    for uneven in (False, True):
+        if uneven:
+            x[:, m // 2] = x[:, m // 2 - 1]
+        times = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            _lib.call("rg_conservative_1d", _device.ptr(x), m, m, _device.ptr(y), n, n, nd, None, 0, cap,
+                      _device.ptr(ii), _device.ptr(oo), _device.ptr(vv), _device.ptr(count), _device.stream())
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t0)
+        seconds.append(min(times))
+    assert seconds[1] < 3 * seconds[0], seconds
