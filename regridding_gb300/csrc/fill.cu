@@ -300,13 +300,13 @@ __global__ void __launch_bounds__(kRelaxThreads)
     }
 }
 
-// The largest cluster, up to 16 blocks, of which nt run at a time (1 when none
+// The largest cluster, up to `most` blocks, of which nt run at a time (1 when none
 // does), for a kernel of kRelaxThreads threads.
 template <typename F>
-int cluster_for(F* kernel, int64_t nt, size_t smem) {
+int cluster_for(F* kernel, int64_t nt, size_t smem, int most) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaGetLastError();
-    for (int c = 16; c > 1; c /= 2) {
+    for (int c = most; c > 1; c /= 2) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -821,7 +821,7 @@ int median_impl(const T* a, const uint8_t* where, int64_t nt, int64_t S, T* out,
         if ((status = dalloc(&keys, total > 0 ? total : 1, s))) break;
         median_compact<T><<<grid, 256, 0, s>>>(a, where, nt, S, st, offsets, cursor, keys);
         constexpr int kPasses = Keys<T>::kBits / 8;
-        const int c = cluster_for(median_digits, nt, 0);
+        const int c = cluster_for(median_digits, nt, 0, 16);
         if (median_clusters(total, nt, c)) {
             RG_CUDA(launch_clusters(median_digits, nt, c, 0, s, keys, offsets, Keys<T>::kBits - 8 * (kDataPasses + 1), st));
         } else {
@@ -912,20 +912,24 @@ int gauss_seidel_impl(T* a, const uint8_t* where, int64_t nt, int64_t ny, int64_
         // missing 878 and 635, with 8 % 879 and 962 (float32: 1086), 4 of 480 x 641
         // with 8 % 1741 and 974; more slices than SMs, of 1 %: 1000 of 100 x 101 2170
         // and 4000, 5000 of 32 x 32 955 and 14800.
-        static SharedLimit limit;
-        int c = nt <= kRelaxSlices && allow_shared((const void*)fill_relax<T>, kRelaxShared, limit)
-                    ? cluster_for(fill_relax<T>, nt, kRelaxShared) : 0;
-        while (c > 1 && nt * c > kRelaxSlices) c /= 2;
         const double op_us = 6.0 / (0.66 * 0.63e6);  // of one cell, the whole chip
-        double launches_us = 0, phases_us = 0;
-        for (int cls = 0; cls < kClasses && c > 0; ++cls) {
-            const int64_t n = starts[cls + 1] - starts[cls];
-            if (n == 0) continue;
-            const double block = (double)starts[kClasses + 1 + cls] / c / 1000;
-            launches_us += std::max(3.9, n * op_us);
-            phases_us += sizeof(T) == 8 ? 2.3 + 1.5 * block : 2.7 + 1.8 * block;
-        }
-        if (phases_us < launches_us) {
+        const auto faster = [&](int c) {
+            double launches_us = 0, phases_us = 0;
+            for (int cls = 0; cls < kClasses; ++cls) {
+                const int64_t n = starts[cls + 1] - starts[cls];
+                if (n == 0) continue;
+                const double block = (double)starts[kClasses + 1 + cls] / c / 1000;
+                launches_us += std::max(3.9, n * op_us);
+                phases_us += sizeof(T) == 8 ? 2.3 + 1.5 * block : 2.7 + 1.8 * block;
+            }
+            return phases_us < launches_us;
+        };
+        // (the driver is asked only where the largest cluster would do)
+        int c = 16;
+        while (c > 1 && nt * c > kRelaxSlices) c /= 2;
+        static SharedLimit limit;
+        if (nt <= kRelaxSlices && faster(c) && allow_shared((const void*)fill_relax<T>, kRelaxShared, limit) &&
+            faster(c = cluster_for(fill_relax<T>, nt, kRelaxShared, c))) {
             for (int64_t done = 0; done < iterations; done += 1024)  // (at most some 25 ms a launch)
                 RG_CUDA(launch_clusters(fill_relax<T>, nt, c, kRelaxShared, s, a, (const uint64_t*)list, (const int64_t*)offsets, nblocks,
                                         tiles, (uint32_t)ny, nx_div, k,
