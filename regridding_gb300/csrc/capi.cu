@@ -438,10 +438,12 @@ int small_to_host(void* h_dst, const void* d_src, size_t n, cudaStream_t s) {
 
 int small_to_device(void* d_dst, const void* h_src, size_t n, cudaStream_t s) {
     if (n == 0) return RG_OK;
-    // up to 3968 bytes (arguments below 4 KB), and up to three launches of 32000
-    // (below the 32764 bytes a launch may carry), are not waited for; a kernel
-    // that reads the host array costs a synchronisation (13 us for a few bytes,
-    // of which a build of one pair had eight; 45 us for 34 KB)
+    // up to 3968 bytes (arguments below 4 KB), and up to 32000 (below the 32764 a
+    // launch may carry), are not waited for; a kernel that reads the host array
+    // costs a synchronisation (13 us for a few bytes, of which a build of one
+    // pair had eight).  An upload that is waited for, by argument and by such a
+    // kernel: 4 KB 45 and 51 us, 16 KB 47 and 45, 32 KB 50 and 45; two and three
+    // launches, 48 KB 57 and 43, 80 KB 68 and 43.
     constexpr size_t SMALL = 496 * 8, LARGE = 4000 * 8;
     if (n <= SMALL) {
         ArgBytes<496> arg;
@@ -450,13 +452,10 @@ int small_to_device(void* d_dst, const void* h_src, size_t n, cudaStream_t s) {
         RG_CUDA(cudaGetLastError());
         return RG_OK;
     }
-    if (n <= 3 * LARGE) {
+    if (n <= LARGE) {
         ArgBytes<4000> arg;
-        for (size_t k = 0; k < n; k += LARGE) {
-            const size_t m = n - k < LARGE ? n - k : LARGE;
-            memcpy(arg.w, (const char*)h_src + k, m);
-            store_bytes<4000><<<1, 1024, 0, s>>>((unsigned char*)d_dst + k, arg, (unsigned)m);
-        }
+        memcpy(arg.w, h_src, n);
+        store_bytes<4000><<<1, 1024, 0, s>>>((unsigned char*)d_dst, arg, (unsigned)n);
         RG_CUDA(cudaGetLastError());
         return RG_OK;
     }

@@ -161,7 +161,7 @@ struct FastDiv {
 // copying 600 MB blocks); elsewhere cudaMemcpyAsync.  small_to_host is
 // stream-ordered: read the destination after synchronising the stream.
 // small_to_device returns once the source has been read (with the launch up to
-// 94 KB; above, it synchronises the stream when a kernel did the copy), so the
+// 31 KB; above, it synchronises the stream when a kernel did the copy), so the
 // source may be freed at once.
 bool kernel_host_access();
 // cudaMemsetAsync(p, 0, n, s) as a kernel, for the small clears of the build
