@@ -190,7 +190,9 @@ int rg_weights_free(rg_weights w, rg_stream_t stream);
  * 4-7, ..., 64 and more slices: the autotuner times its configurations on
  * that call, unless an earlier handle of the same kind was tuned) synchronise
  * `stream`, as do the first exact apply of a float32 stack and the second of
- * a float64 one (from then on staged as well); later applies are asynchronous. */
+ * a float64 one (from then on staged as well); later applies are asynchronous.
+ * While `stream` is captured, exact and compensated applies whose lists are
+ * missing gather from global memory. */
 int rg_apply(rg_weights w, const void* d_vin, int dtype_in, void* d_vout, int dtype_out,
              int64_t stack, int acc, rg_stream_t stream);
 

@@ -1373,7 +1373,7 @@ __global__ void __launch_bounds__(64)
 // a time; a chunk walked again changes its own end, so the comparison goes on
 // from the chunk after it.  (A thread per line compared its chunks one dependent
 // load after another: 69 us for the 84 chunks a line of 333 x 257 -> 250 x 193,
-// now 6 us.)
+// now 4 us.)
 __global__ void __launch_bounds__(128)
     chunk_repair_kernel(Batch B, WalkState* __restrict__ starts, WalkState* __restrict__ ends,
                         int64_t* __restrict__ counts, int32_t* __restrict__ s_in, int32_t* __restrict__ s_out,
@@ -1826,9 +1826,10 @@ __device__ int order_short_row(int64_t s, int len, Triple* triples, int32_t* tmp
 }
 
 // The listed blocks (.x; .y counts their finished turns), a row per block and
-// turn, its short rows together in one, a warp each: ranked with the keys staged in shared-memory tiles, up to 8 triples per
-// thread and pass, and merged by a thread per run; the block that finishes a
-// listed block's last row moves its rows together.  (63 pairs of 64^2 and one of
+// turn, its short rows together in one, a warp each: ranked with the keys staged
+// in shared-memory tiles, up to 8 triples per thread and pass, and merged by a
+// thread per run; the block that finishes a listed block's last turn moves its
+// rows together.  (63 pairs of 64^2 and one of
 // 512^2 -> 8^2 in a batch, whose 64 rows of 36,000 triples lie in two blocks of
 // 32: 14 ms; with a block for all rows of a listed one 270.  512^2 -> 8^2
 // alone 11 and 21 ms.)
@@ -1850,13 +1851,14 @@ __global__ void __launch_bounds__(ORDER_THREADS)
         const int64_t r1 = r0 + per < nrows ? r0 + per : nrows;
         const int64_t r = together ? r0 : r0 + item % per;
         // the listed block's turns: its long rows, and the short ones together
-        const unsigned longer = __ballot_sync(0xffffffffu, r0 + lane < r1 && row_start[r0 + lane + 1] - row_start[r0 + lane] > ROW_SHORT);
+        const bool mine = r0 + lane < r1 && row_start[r0 + lane + 1] - row_start[r0 + lane] > ROW_SHORT;
+        const unsigned longer = __ballot_sync(0xffffffffu, mine);
         if (!together && (r >= r1 || !(longer >> (r - r0) & 1u))) continue;
         if (together)
             for (int q = warp; r0 + q < r1; q += ORDER_THREADS / 32)
                 if (!(longer >> q & 1u))
-                    row_nnz[r0 + q] = order_short_row(row_start[r0 + q], (int)(row_start[r0 + q + 1] - row_start[r0 + q]),
-                                                      triples, tmp_col, tmp_val);
+                    row_nnz[r0 + q] = order_short_row(
+                        row_start[r0 + q], (int)(row_start[r0 + q + 1] - row_start[r0 + q]), triples, tmp_col, tmp_val);
         const int64_t s = together ? 0 : row_start[r], t = together ? 0 : row_start[r + 1], len = t - s;
         for (int64_t e0 = s; e0 < t; e0 += (int64_t)blockDim.x * 8) {
             int64_t mykey[8];

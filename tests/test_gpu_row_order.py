@@ -72,7 +72,7 @@ def test_long_rows_side_by_side():
     from regridding_gb300 import batching, workloads
 
     def device(grid):
-        return tuple(torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in grid)
+        return tuple(torch.tensor(np.asarray(a), device="cuda") for a in grid)
 
     gi = np.stack(np.meshgrid(np.linspace(0, 1, 513), np.linspace(0, 1, 513), indexing="ij"))
     go = np.stack(np.meshgrid(np.linspace(0.013, 0.977, 9), np.linspace(0.013, 0.977, 9), indexing="ij"))
