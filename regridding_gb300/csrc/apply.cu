@@ -270,16 +270,6 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     // from global memory, which a first call takes, give the same bits
     bool exact64 = !transposed && acc != RG_ACC_FAST && dtype_in == RG_F64 && dtype_out == RG_F64 && W->n_out > 0 &&
                    W->nnz > 0 && stack >= 2;
-    if (exact64) {
-        std::lock_guard<std::mutex> lock(W->mu);
-        if (!W->box_perm) {
-            // (the lists are read back by the host: not while a graph is captured)
-            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-            if (W->exact64_calls++ > 0) RG_CUDA(cudaStreamIsCapturing(s, &capture));
-            else exact64 = false;
-            exact64 = exact64 && capture == cudaStreamCaptureStatusNone;
-        }
-    }
     // the compensated apply: float32 stack, float64 output, float-float sums
     const bool ff_box = !transposed && acc == RG_ACC_COMPENSATED && dtype_in == RG_F32 && dtype_out == RG_F64 &&
                         W->n_out > 0 && W->nnz > 0;
@@ -291,6 +281,13 @@ int apply_weights(rg_weights_s* W, bool transposed, const void* vin, int dtype_i
     {
         std::lock_guard<std::mutex> lock(W->mu);
         bool made = false;
+        if (exact64 && !W->box_perm) {
+            // (the lists are read back by the host: not while a graph is captured)
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            if (W->exact64_calls++ > 0) RG_CUDA(cudaStreamIsCapturing(s, &capture));
+            else exact64 = false;
+            exact64 = exact64 && capture == cudaStreamCaptureStatusNone;
+        }
         if (transposed && W->t_row_ptr == nullptr) {
             RG_TRY(ensure_transposed(W, s));
             made = true;
