@@ -53,9 +53,10 @@ typedef struct CUstream_st* rg_stream_t; /* == cudaStream_t */
  * the FP32 pipe, the pair added in double at the end.  Result within
  * (1.1e-14 + (n + 2)^2 * 3.6e-15) * sum_k |w_k x_k| of the exact sum for rows
  * of n entries (half of that where all w_k x_k have one sign: 1e-12 for n <= 20).
- * Rows of more than 20 entries are summed in float64, bit for bit as RG_ACC_EXACT, except where the input footprints of
- * 16 x 16 output cells fit boxes of 32 x 32 input cells, whose rows are short
- * (about 9 entries; one of 60 is off by some 5e-14).
+ * Rows of more than 20 entries are summed in float64, bit for bit as
+ * RG_ACC_EXACT, except where the input footprints of 16 x 16 output cells fit
+ * boxes of 32 x 32 input cells, whose rows are short (about 9 entries; one of
+ * 60 is off by some 5e-14).
  * A float32 partial sum that overflows, or a non-finite input or weight,
  * sends that output and slice to the exact float64 sum instead.
  * Every other dtype combination computes as RG_ACC_EXACT. */
@@ -183,8 +184,8 @@ int rg_weights_free(rg_weights w, rg_stream_t stream);
  * upstream in-place float32 output, which rounds after every update);
  * RG_ACC_FAST accumulates in dtype_out with FMA; RG_ACC_COMPENSATED gives a
  * float64 result within 1e-12 of the upstream's (sums of one sign, see its
- * definition above) for float32 input, about 5x
- * faster than RG_ACC_EXACT on GB300.
+ * definition above) for float32 input, about 5x faster than RG_ACC_EXACT on
+ * GB300.
  * The first fast or compensated apply of a handle (which builds its tile
  * lists and entry orders) and its first in each stack size class (1, 2-3,
  * 4-7, ..., 64 and more slices: the autotuner times its configurations on

@@ -228,9 +228,9 @@ class DeviceWeights:
         ``accumulate="exact"`` reproduces the upstream float64 result bit for
         bit (float64 output, or an upstream-style in-place float32 ``out``);
         ``"fast"`` accumulates in the output dtype with FMA; ``"compensated"``
-        gives a float64 output within 1e-12 relative of the exact sum
-        (float32 input: float-float arithmetic on the FP32 pipe; other dtypes
-        compute as ``"exact"``).
+        gives a float64 output within 1e-12 relative of the exact sum where
+        its terms have one sign (float32 input: float-float arithmetic on the
+        FP32 pipe, long rows in float64; other dtypes compute as ``"exact"``).
         """
         t = torch()
         if accumulate not in _lib.RG_ACC:

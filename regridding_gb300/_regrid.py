@@ -57,9 +57,10 @@ def regrid_from_weights(
     with FMA (float32 output for float32 input unless ``values_output`` says
     otherwise): the HBM-bandwidth path, within about 1e-6 relative of the
     float64 result.  ``accumulate="compensated"`` returns the upstream's
-    float64 output within 1e-12 relative of it, computed for float32 input
-    in float-float arithmetic on the FP32 pipe, about 5x faster than
-    ``"exact"`` on GB300 (other inputs compute as ``"exact"``).
+    float64 output within 1e-12 relative of it where a sum's terms have one
+    sign, computed for float32 input in float-float arithmetic on the FP32
+    pipe (long rows in float64), about 5x faster than ``"exact"`` on GB300
+    (other inputs compute as ``"exact"``).
     """
     return _apply(weights, shape_input, shape_output, values_input, values_output, axis_input, axis_output, accumulate)
 

@@ -228,8 +228,8 @@ struct Sweep1d {
 // then output) is the sweep's, reversed as a whole (reversed input: a sweep
 // ahead counts the entries) and within the inputs (one of the grids reversed:
 // each input's entries are turned round once they are written).
-__device__ __noinline__ int64_t sweep_1d(const Row1d& R, const double* w_in, int64_t cap, int64_t* ind_in, int64_t* ind_out,
-                            double* val, unsigned* flags) {
+__device__ __noinline__ int64_t sweep_1d(const Row1d& R, const double* w_in, int64_t cap, int64_t* ind_in,
+                                         int64_t* ind_out, double* val, unsigned* flags) {
     int64_t sw, st, total = 0, cnt = 0;
     double from, to;
     if (R.rev_in)
