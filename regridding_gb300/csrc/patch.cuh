@@ -417,6 +417,9 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
     // a long row's lane takes no float-float step: its entries here are none
     const bool long_row = MODE == MODE_FF && LOAD != LOAD_SWIZZLED && nk > FF_ROW_MAX;
     const int nf = long_row ? 0 : nk;
+    // (written so: with s + nf the swizzled kernel of six slices takes 80 registers
+    // for 64, 577 us for 573, and with a choice of s and e the wide ones 617 for 600)
+    const int64_t ef = LOAD == LOAD_SWIZZLED ? e : s + nf;
     const int kwarp = MODE == MODE_FF ? __reduce_max_sync(0xffffffffu, nf) : nk;
     // PLANES: every slice of a stage has its own 4 KB plane, 1024-byte
     // aligned, so all slices see the same swizzle phase and a gather's
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(32 * PATCH_WARPS, MINB)
                         }
                     }
                 }
-                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < s + nf; k++) {
+                for (int64_t k = s + (CT > 0 ? CT + NX : 0); k < ef; k++) {
                     const float wk = bval[k], wlk = blo[k];
                     const uint64_t kh = f2_pack(wk, wk), khn = f2_pack(-wk, -wk), kl = f2_pack(wlk, wlk);
                     const int a = slot[k];
